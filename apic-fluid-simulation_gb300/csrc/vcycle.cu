@@ -139,12 +139,41 @@ __global__ void __launch_bounds__(kSegBlock) k_prolong_red(Level c, Level f, int
     ph_prolong(c, f, nseg, gwarp(), gnwarps(), 0, last, extra, w0);
 }
 
+// CG on a coarsest level that is too large for the shared-memory tail (a
+// grid whose sides stop halving early: 1000 x 600 ends at 125 x 75).  The
+// arrays that every iteration reads move into shared memory, the most used
+// first, as many as fit (`nsm` of them: directions, couplings, diagonal,
+// residual); the rest stay in L2.  Mask and coefficients do not change
+// during a solve: their copies start while the previous kernel drains.
+constexpr size_t kCoarseSmemBudget = 220 * 1024;
+inline __host__ __device__ size_t coarse_smem_bytes(uint32_t words, uint32_t padded, int nsm) {
+    return 4ull * (words + size_t(nsm) * padded);
+}
 __global__ void __launch_bounds__(kTailThreads) k_coarse_solve(Level L, float* __restrict__ cs, float* __restrict__ cap,
                                                                float* __restrict__ cr, const Ctl* __restrict__ ctl,
-                                                               int exact) {
+                                                               int exact, int nsm) {
+    extern __shared__ uint32_t sm[];
+    CgArrays A{L.fluid, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, cs, cap, cr, nsm > 3};
+    float* f = reinterpret_cast<float*>(sm + L.words);
+    auto copy = [&](float* dst, const float* src) {
+        for (uint32_t i = threadIdx.x; i < L.padded; i += kTailThreads) cp_async4(dst + i, src + i);
+        return dst;
+    };
+    if (nsm > 0) {
+        for (uint32_t i = threadIdx.x; i < L.words; i += kTailThreads) cp_async4(sm + i, L.fluid + i);
+        A.bits = sm;
+        A.cs = f;
+        if (nsm > 1) A.px = copy(f + L.padded, L.px);
+        if (nsm > 2) A.py = copy(f + 2 * L.padded, L.py);
+        if (nsm > 3) A.diag = copy(f + 3 * L.padded, L.diag);
+        if (nsm > 4) A.cr = f + 4 * L.padded;
+        if (nsm > 5) A.cap = f + 5 * L.padded;
+    }
     pdl_wait();
+    cp_async_wait_all();
     if (ctl->pcg_done) return;
-    cta_coarse_cg(L.fluid, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, cs, cap, cr, exact != 0);
+    __syncthreads();
+    cta_coarse_cg(A, exact != 0);
 }
 
 __global__ void __launch_bounds__(kTailThreads) k_vcycle_tail(TailParams tp, const Ctl* ctl) {
@@ -309,6 +338,8 @@ void plan_vcycle(Scene& s) {
     if (s.tail_first < s.nlevels) {
         s.tail_smem = bytes;
         cudaFuncSetAttribute(k_vcycle_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTailSmemBudget));
+    } else {
+        cudaFuncSetAttribute(k_coarse_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoarseSmemBudget));
     }
     plan_vcycle_dsm(s);
 }
@@ -365,8 +396,10 @@ bool enqueue_vcycle(Scene& s, bool base_red_done, int rz_mode, bool residual_exi
         }
         if (l == last) {
             restrict_plain(l);
-            launch(pdl, k_coarse_solve, 1, kTailThreads, 0, st, L[l], s.cg_s, s.cg_ap, s.cg_r, s.ctl,
-                   coarse_cg_exact(s) ? 1 : 0);
+            int nsm = 6;
+            while (nsm > 0 && coarse_smem_bytes(L[l].words, L[l].padded, nsm) > kCoarseSmemBudget) --nsm;
+            launch(pdl, k_coarse_solve, 1, kTailThreads, nsm ? coarse_smem_bytes(L[l].words, L[l].padded, nsm) : 0, st,
+                   L[l], s.cg_s, s.cg_ap, s.cg_r, s.ctl, coarse_cg_exact(s) ? 1 : 0, nsm);
             break;
         }
         restrict_red(l);

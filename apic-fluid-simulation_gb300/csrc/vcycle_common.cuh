@@ -144,200 +144,388 @@ __device__ __forceinline__ float prolonged(float e, float ec, uint32_t reps) {
     return e;
 }
 
-// ---- CTA-wide helpers -------------------------------------------------------
-__device__ __forceinline__ double cta_sum(double v, double* sh) {
-    v = warp_sum(v);
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double t = 0;
-    for (int w = 0; w < int(blockDim.x / 32); ++w) t += sh[w];
-    return t;
+// ---- the coarsest level's CG -------------------------------------------------
+
+// Sum (double-float) and a vote over the first `nwarps` warps of the CTA,
+// returned to each of their threads: a shuffle tree per warp, one barrier of
+// those warps, and the same tree over the warps' results in every warp, so
+// no second barrier broadcasts it.  sh: one slot per warp; two calls in a row
+// must use different slots (the barrier of the second then separates the
+// readers of the first from its next writers).  A CG iteration is bound by the latency of
+// its two sums.  In FP64, with every warp adding all warps' doubles, GB300's
+// FP64 rate bound them: a PCG iteration of a 216^2 scene (27^2 coarsest
+// cells) took 70.7 us, of a 488^2 one (61^2) 76.7, and now 48 and 59.  A
+// double-float holds 48 bits of a sum that is rounded to 24: over 2700 random
+// sums of 9 to 9375 products its rounded value was the FP64 sum's every time.
+struct CgSlot {
+    float4 w[32];
+};
+__device__ __forceinline__ void cg_bar(uint32_t nwarps) {
+    asm volatile("bar.sync 1, %0;" ::"r"(nwarps * 32u) : "memory");
 }
-__device__ __forceinline__ float cta_max(float v, float* sh) {
-    v = warp_maxf(v);
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    float t = 0.0f;
-    for (int w = 0; w < int(blockDim.x / 32); ++w) t = fmaxf(t, sh[w]);
-    return t;
+// any: whether it holds in any thread (kAny).
+template <bool kAny>
+__device__ __forceinline__ float cg_reduce(F2 v, bool& any, CgSlot& sh, uint32_t nwarps) {
+    v = warp_sum(v);
+    if (kAny) any = __any_sync(0xffffffffu, any);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) sh.w[warp] = make_float4(v.hi, v.lo, kAny && any ? 1.0f : 0.0f, 0.0f);
+    cg_bar(nwarps);
+    const float4 q = lane < nwarps ? sh.w[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    v = warp_sum(F2{q.x, q.y});
+    if (kAny) any = __any_sync(0xffffffffu, q.z != 0.0f);
+    return float(f2_value(v));
 }
 
-// solve_coarse_exact's FP32 sums (:627-629, :660, :681-687): a[c] * b[c]
-// added one fluid cell after another in ascending order, by one thread.
-__device__ __forceinline__ float serial_dot(const uint32_t* bits, uint32_t w, uint32_t cells, const float* a,
-                                            const float* b) {
+// The reference solver mode's sums (solve_coarse_exact, :627-629, :660,
+// :681-687): the products, staged in fluid order, added one after another by
+// one thread.  prod holds `n` products rounded up to a multiple of 8 with
+// zeros behind them (a sum that starts at +0 is never -0, so adding +0
+// changes nothing).  Loads run two groups ahead of the add chain, whose
+// latency is all that is left.
+__device__ __forceinline__ float serial_sum8(const float* prod, uint32_t n) {
     float s = 0.0f;
-    for (uint32_t r = 0; r < cells; ++r)
-        if (bit_at(bits, r)) s = s + a[r + w] * b[r + w];
+    float a[8], b[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[k] = n > 0 ? prod[k] : 0.0f;
+    for (uint32_t i = 0; i < n; i += 8) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) b[k] = i + 8 < n ? prod[i + 8 + k] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s = s + a[k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a[k] = b[k];
+    }
     return s;
 }
-// Sum of a CTA: FP64 over the threads' parts (fast), or the serial FP32 sum
-// in the reference's order by thread 0 (exact; the vectors must be written
-// and visible to the CTA).
-__device__ __forceinline__ float cta_dot(bool exact, double part, const uint32_t* bits, uint32_t w, uint32_t cells,
-                                         const float* a, const float* b, double* shd) {
-    if (!exact) return float(cta_sum(part, shd));
-    __shared__ float s_dot;
-    __syncthreads();
-    if (threadIdx.x == 0) s_dot = serial_dot(bits, w, cells, a, b);
-    __syncthreads();
-    return s_dot;
-}
 
-// Plain CG on the coarsest level (solve_coarse_exact, :618-704) by one CTA.
-// Arrays may live in global or shared memory.  exact: the dot products are
-// the reference's serial FP32 sums (reference solver mode); otherwise FP64
-// sums over the threads.
-static __device__ __noinline__ void cta_coarse_cg(const uint32_t* bits, uint32_t w, uint32_t cells, const float* diag, const float* px,
-                              const float* py, const float* res, float* err, float* cs, float* cap, float* cr,
-                              bool exact) {
-    __shared__ double shd[32];
-    __shared__ float shf[32];
-    const long long W = w;
-    uint32_t nf = 0;
-    double g = 0;
-    for (uint32_t r = threadIdx.x; r < cells; r += blockDim.x) {
-        if (!bit_at(bits, r)) continue;
-        uint32_t c = r + w;
-        float rv = res[c];
-        err[c] = 0.0f;
-        cr[c] = rv;
-        cs[c] = rv;
-        g += double(rv * rv);
-        nf++;
+// The level a CG runs on.  own: diag, px, py and cs lie in this CTA's shared
+// memory and may be overwritten.
+struct CgArrays {
+    const uint32_t* bits;
+    uint32_t w, cells;
+    float *diag, *px, *py;
+    const float* res;
+    float *err, *cs, *cap, *cr;
+    bool own;
+};
+constexpr uint32_t kCgMaxK = 10;  // cells per thread held in registers
+
+// Plain CG on the coarsest level (solve_coarse_exact, :618-704) by the first
+// `nwarps` warps of a CTA.  Cell k of a thread is threadIdx.x + k * threads.
+// exact: the dot products are the reference's serial FP32 sums (reference
+// solver mode).
+//   K == 1: a cell's coefficients, vectors and the neighbours that count in
+//     registers, the directions in cs.
+//   K > 1:  the vectors of K cells in registers; diag, px and py (own) are
+//     first zeroed wherever the reference skips a term, so the loops run over
+//     all cells without a test (a term of zero leaves a sum as it was).
+//   K == 0: everything in memory (levels of more than kCgMaxK cells per
+//     thread).
+struct CgShared {
+    CgSlot slot[2];
+    float dot;
+    uint32_t pre[32 * kCgMaxK];  // exact: fluid cells before each mask word
+};
+template <int K>
+static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& sh, uint32_t nwarps, bool exact) {
+    const CgArrays A = arrays;  // in registers: a barrier makes the compiler read memory again
+    const uint32_t threads = nwarps * 32u;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t W = A.w, cells = A.cells;
+    const uint32_t nwords = (cells + 31u) >> 5;
+    uint32_t nfl = 0;  // fluid cells of the level
+    for (uint32_t k = lane; k < nwords; k += 32) nfl += uint32_t(__popc(A.bits[k]));
+    nfl = __reduce_add_sync(0xffffffffu, nfl);
+    if (K > 0 && exact) {
+        for (uint32_t word = threadIdx.x; word < nwords; word += threads) {
+            uint32_t c = 0;
+            for (uint32_t k = 0; k < word; ++k) c += uint32_t(__popc(A.bits[k]));
+            sh.pre[word] = c;
+        }
     }
-    float gamma = cta_dot(exact, g, bits, w, cells, cr, cr, shd);
-    uint32_t nfl = uint32_t(cta_sum(double(nf), shd));
-    if (gamma < 1e-12f) return;
-    uint32_t max_it = min(nfl, 100u);
+    // neighbours that count (right, left, up, down), bit 4: the cell is fluid
+    auto links = [&](uint32_t r) -> uint32_t {
+        if (r >= cells || !bit_at(A.bits, r)) return 0u;
+        const long long q = r;
+        return 16u | (fluid_raw(A.bits, q + 1, cells) ? 1u : 0u) | (fluid_raw(A.bits, q - 1, cells) ? 2u : 0u) |
+               (fluid_raw(A.bits, q + W, cells) ? 4u : 0u) | (fluid_raw(A.bits, q - (long long)W, cells) ? 8u : 0u);
+    };
+    auto apply = [&](uint32_t c, uint32_t nb, float d, float sc, float pxc, float pxl, float pyc, float pyd) {
+        // (all four loads first: they lie inside the padded array)
+        const float sr = A.cs[c + 1], sl = A.cs[c - 1], su = A.cs[c + W], sd = A.cs[c - W];
+        float v = d * sc;
+        float t = __fmaf_rn(pxc, sr, v);
+        v = (nb & 1u) ? t : v;
+        t = __fmaf_rn(pxl, sl, v);
+        v = (nb & 2u) ? t : v;
+        t = __fmaf_rn(pyc, su, v);
+        v = (nb & 4u) ? t : v;
+        t = __fmaf_rn(pyd, sd, v);
+        v = (nb & 8u) ? t : v;
+        return v;
+    };
+    // exact sums: the fluid cells' products are staged at cap in fluid order
+    auto stage = [&](uint32_t r, float q) {
+        const uint32_t word = r >> 5, m = A.bits[word];
+        if ((m >> lane) & 1u) A.cap[sh.pre[word] + uint32_t(__popc(m & ((1u << lane) - 1u)))] = q;
+    };
+    auto serial = [&]() {
+        if (nfl + threadIdx.x < ((nfl + 7u) & ~7u)) A.cap[nfl + threadIdx.x] = 0.0f;
+        cg_bar(nwarps);
+        if (threadIdx.x == 0) sh.dot = serial_sum8(A.cap, nfl);
+        cg_bar(nwarps);
+        return sh.dot;
+    };
+    // ... or added up by thread 0 itself where the cells are in memory
+    auto serial_cells = [&](const float* a, const float* b) {
+        cg_bar(nwarps);
+        if (threadIdx.x == 0) {
+            float s = 0.0f;
+            for (uint32_t r = 0; r < cells; ++r)
+                if (bit_at(A.bits, r)) s = s + a[r + W] * b[r + W];
+            sh.dot = s;
+        }
+        cg_bar(nwarps);
+        return sh.dot;
+    };
+    constexpr int KR = K > 0 ? K : 1;
+    uint32_t nb = 0;
+    float d = 0.0f, pxc = 0.0f, pxl = 0.0f, pyc = 0.0f, pyd = 0.0f;  // K == 1
+    float rv[KR], x[KR], av[KR];
+#pragma unroll
+    for (int k = 0; k < KR; ++k) rv[k] = x[k] = av[k] = 0.0f;
+    F2 g{0.0f, 0.0f};
+    bool more = false;
+    if constexpr (K == 1) {
+        if (exact) cg_bar(nwarps);  // sh.pre
+        nb = links(threadIdx.x);
+        if (nb) {
+            const uint32_t c = threadIdx.x + W;
+            d = A.diag[c];
+            pxc = A.px[c];
+            pxl = A.px[c - 1];
+            pyc = A.py[c];
+            pyd = A.py[c - W];
+            rv[0] = A.res[c];
+            A.cs[c] = rv[0];
+        }
+        const float q = rv[0] * rv[0];
+        if (exact && nb) stage(threadIdx.x, q);
+        g = F2{q, 0.0f};
+    } else if constexpr (K > 1) {
+        for (uint32_t c = threadIdx.x; c < cells + 2u * W; c += threads) {
+            const long long r = (long long)c - W;
+            const bool f = fluid_raw(A.bits, r, cells) != 0;
+            if (!f || !fluid_raw(A.bits, r + 1, cells)) A.px[c] = 0.0f;
+            if (!f || !fluid_raw(A.bits, r + W, cells)) A.py[c] = 0.0f;
+            if (!f) A.diag[c] = 0.0f;
+            A.cs[c] = f ? A.res[c] : 0.0f;
+        }
+        cg_bar(nwarps);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+            if (r >= cells) continue;
+            rv[k] = A.cs[r + W];
+            const float q = rv[k] * rv[k];
+            if (exact) stage(r, q);
+            g = f2_add(g, q);
+        }
+    } else {
+        for (uint32_t r = threadIdx.x; r < cells; r += threads) {
+            if (!bit_at(A.bits, r)) continue;
+            const uint32_t c = r + W;
+            const float q = A.res[c];
+            A.err[c] = 0.0f;
+            A.cr[c] = q;
+            A.cs[c] = q;
+            g = f2_add(g, q * q);
+        }
+    }
+    float gamma;
+    if (exact)
+        gamma = K > 0 ? serial() : serial_cells(A.cr, A.cr);
+    else
+        gamma = cg_reduce<false>(g, more, sh.slot[0], nwarps);
+    const uint32_t max_it = gamma < 1e-12f ? 0u : min(nfl, 100u);
     for (uint32_t it = 0; it < max_it; ++it) {
-        __syncthreads();
-        double d = 0;
-        for (uint32_t r = threadIdx.x; r < cells; r += blockDim.x) {
-            if (!bit_at(bits, r)) continue;
-            uint32_t c = r + w;
-            float v = diag[c] * cs[c];
-            if (fluid_raw(bits, (long long)r + 1, cells)) v = __fmaf_rn(px[c], cs[c + 1], v);
-            if (fluid_raw(bits, (long long)r - 1, cells)) v = __fmaf_rn(px[c - 1], cs[c - 1], v);
-            if (fluid_raw(bits, (long long)r + W, cells)) v = __fmaf_rn(py[c], cs[c + w], v);
-            if (fluid_raw(bits, (long long)r - W, cells)) v = __fmaf_rn(py[c - w], cs[c - w], v);
-            cap[c] = v;
-            d += double(cs[c] * v);
-        }
-        float delta = cta_dot(exact, d, bits, w, cells, cs, cap, shd);
-        if (fabsf(delta) < 1e-5f) break;
-        float alpha = gamma / delta;
-        float me = 0.0f;
-        for (uint32_t r = threadIdx.x; r < cells; r += blockDim.x) {
-            if (!bit_at(bits, r)) continue;
-            uint32_t c = r + w;
-            err[c] = err[c] + alpha * cs[c];
-            float nr = cr[c] - alpha * cap[c];
-            cr[c] = nr;
-            me = fmaxf(me, fabsf(nr));
-        }
-        if (cta_max(me, shf) < 1e-6f) break;
-        double ng = 0;
-        for (uint32_t r = threadIdx.x; r < cells; r += blockDim.x) {
-            if (!bit_at(bits, r)) continue;
-            uint32_t c = r + w;
-            ng += double(cr[c] * cr[c]);
-        }
-        float new_gamma = cta_dot(exact, ng, bits, w, cells, cr, cr, shd);
-        float beta = new_gamma / gamma;
-        gamma = new_gamma;
-        for (uint32_t r = threadIdx.x; r < cells; r += blockDim.x) {
-            if (!bit_at(bits, r)) continue;
-            uint32_t c = r + w;
-            cs[c] = cr[c] + (beta * cs[c]);
-        }
-    }
-    __syncthreads();
-}
-
-// The same CG run by one warp (shuffles only, no block barriers) for a
-// coarsest level of at most 32 * kWarpCgCells cells; the other warps wait.
-constexpr uint32_t kWarpCgCells = 8;
-static __device__ __noinline__ void warp_coarse_cg(const uint32_t* bits, uint32_t w, uint32_t cells, const float* diag, const float* px,
-                               const float* py, const float* res, float* err, float* cs, float* cap, float* cr,
-                               bool exact) {
-    if (threadIdx.x < 32) {
-        const long long W = w;
-        const uint32_t lane = threadIdx.x;
-        auto wsum = [](double v) {
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            return v;
-        };
-        // FP64 over the lanes, or the reference's serial FP32 sum by lane 0
-        auto wdot = [&](double part, const float* a, const float* b) {
-            if (!exact) return float(wsum(part));
-            __syncwarp();
-            float v = lane == 0 ? serial_dot(bits, w, cells, a, b) : 0.0f;
-            return __shfl_sync(0xffffffffu, v, 0);
-        };
-        double g = 0, nf = 0;
-        for (uint32_t r = lane; r < cells; r += 32) {
-            if (!bit_at(bits, r)) continue;
-            uint32_t c = r + w;
-            float rv = res[c];
-            err[c] = 0.0f;
-            cr[c] = rv;
-            cs[c] = rv;
-            g += double(rv * rv);
-            nf += 1.0;
-        }
-        float gamma = wdot(g, cr, cr);
-        uint32_t nfl = uint32_t(wsum(nf));
-        if (!(gamma < 1e-12f)) {
-            uint32_t max_it = min(nfl, 100u);
-            for (uint32_t it = 0; it < max_it; ++it) {
-                __syncwarp();
-                double d = 0;
-                for (uint32_t r = lane; r < cells; r += 32) {
-                    if (!bit_at(bits, r)) continue;
-                    uint32_t c = r + w;
-                    float v = diag[c] * cs[c];
-                    if (fluid_raw(bits, (long long)r + 1, cells)) v = __fmaf_rn(px[c], cs[c + 1], v);
-                    if (fluid_raw(bits, (long long)r - 1, cells)) v = __fmaf_rn(px[c - 1], cs[c - 1], v);
-                    if (fluid_raw(bits, (long long)r + W, cells)) v = __fmaf_rn(py[c], cs[c + w], v);
-                    if (fluid_raw(bits, (long long)r - W, cells)) v = __fmaf_rn(py[c - w], cs[c - w], v);
-                    cap[c] = v;
-                    d += double(cs[c] * v);
-                }
-                float delta = wdot(d, cs, cap);
-                if (fabsf(delta) < 1e-5f) break;
-                float alpha = gamma / delta;
-                float me = 0.0f;
-                for (uint32_t r = lane; r < cells; r += 32) {
-                    if (!bit_at(bits, r)) continue;
-                    uint32_t c = r + w;
-                    err[c] = err[c] + alpha * cs[c];
-                    float nr = cr[c] - alpha * cap[c];
-                    cr[c] = nr;
-                    me = fmaxf(me, fabsf(nr));
-                }
-                if (warp_maxf(me) < 1e-6f) break;
-                double ng = 0;
-                for (uint32_t r = lane; r < cells; r += 32) {
-                    if (!bit_at(bits, r)) continue;
-                    uint32_t c = r + w;
-                    ng += double(cr[c] * cr[c]);
-                }
-                float new_gamma = wdot(ng, cr, cr);
-                float beta = new_gamma / gamma;
-                gamma = new_gamma;
-                __syncwarp();
-                for (uint32_t r = lane; r < cells; r += 32) {
-                    if (!bit_at(bits, r)) continue;
-                    uint32_t c = r + w;
-                    cs[c] = cr[c] + (beta * cs[c]);
-                }
+        // (the directions are visible: a barrier follows their update)
+        F2 dsum{0.0f, 0.0f};
+        if constexpr (K == 1) {
+            float q = 0.0f;
+            if (nb) {
+                const uint32_t c = threadIdx.x + W;
+                const float sc = A.cs[c];
+                av[0] = apply(c, nb, d, sc, pxc, pxl, pyc, pyd);
+                q = sc * av[0];
+                if (exact) stage(threadIdx.x, q);
+            }
+            dsum = F2{q, 0.0f};
+        } else if constexpr (K > 1) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+                if (r >= cells) continue;
+                const uint32_t c = r + W;
+                const float sc = A.cs[c];
+                float v = A.diag[c] * sc;
+                v = __fmaf_rn(A.px[c], A.cs[c + 1], v);
+                v = __fmaf_rn(A.px[c - 1], A.cs[c - 1], v);
+                v = __fmaf_rn(A.py[c], A.cs[c + W], v);
+                v = __fmaf_rn(A.py[c - W], A.cs[c - W], v);
+                av[k] = v;
+                const float q = sc * v;
+                if (exact) stage(r, q);
+                dsum = f2_add(dsum, q);
+            }
+        } else {
+            for (uint32_t r = threadIdx.x; r < cells; r += threads) {
+                const uint32_t n = links(r);
+                if (!n) continue;
+                const uint32_t c = r + W;
+                const float sc = A.cs[c];
+                const float v = apply(c, n, A.diag[c], sc, A.px[c], A.px[c - 1], A.py[c], A.py[c - W]);
+                A.cap[c] = v;
+                dsum = f2_add(dsum, sc * v);
             }
         }
+        float delta;
+        if (exact)
+            delta = K > 0 ? serial() : serial_cells(A.cs, A.cap);
+        else
+            delta = cg_reduce<false>(dsum, more, sh.slot[1], nwarps);
+        if (fabsf(delta) < 1e-5f) break;
+        const float alpha = gamma / delta;
+        more = false;  // some |r| is not below the exit (max|r| < 1e-6)
+        F2 ng{0.0f, 0.0f};
+        if constexpr (K > 0) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+                if (r >= cells) continue;
+                x[k] = x[k] + alpha * A.cs[r + W];
+                rv[k] = rv[k] - alpha * av[k];
+                more = more || fabsf(rv[k]) >= 1e-6f;
+                const float q = rv[k] * rv[k];
+                if (exact) stage(r, q);
+                ng = K == 1 ? F2{q, 0.0f} : f2_add(ng, q);
+            }
+        } else {
+            for (uint32_t r = threadIdx.x; r < cells; r += threads) {
+                if (!bit_at(A.bits, r)) continue;
+                const uint32_t c = r + W;
+                A.err[c] = A.err[c] + alpha * A.cs[c];
+                const float nr = A.cr[c] - alpha * A.cap[c];
+                A.cr[c] = nr;
+                more = more || fabsf(nr) >= 1e-6f;
+                ng = f2_add(ng, nr * nr);
+            }
+        }
+        // the exit's test and the next r.r in one reduction (the latter is
+        // dropped when the former ends the loop)
+        float new_gamma = cg_reduce<true>(ng, more, sh.slot[0], nwarps);
+        if (!more) break;
+        if (exact) new_gamma = K > 0 ? serial() : serial_cells(A.cr, A.cr);
+        const float beta = new_gamma / gamma;
+        gamma = new_gamma;
+        if constexpr (K > 0) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+                if (r >= cells || (K == 1 && !nb)) continue;
+                A.cs[r + W] = rv[k] + (beta * A.cs[r + W]);
+            }
+        } else {
+            for (uint32_t r = threadIdx.x; r < cells; r += threads) {
+                if (!bit_at(A.bits, r)) continue;
+                const uint32_t c = r + W;
+                A.cs[c] = A.cr[c] + (beta * A.cs[c]);
+            }
+        }
+        cg_bar(nwarps);
+    }
+    if constexpr (K > 0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+            if (r < cells && bit_at(A.bits, r)) A.err[r + W] = x[k];
+        }
+    }
+}
+
+// The same CG for a level of at most 32 cells (a grid whose sides halve down
+// to 4 x 4), a cell per lane of one warp, all vectors in registers and the
+// neighbours' directions by shuffle.  The sums are FP64 over the lanes (one
+// warp's five adds are a shorter chain than the double-float's), or, exact,
+// serial over the lanes; a lane that is not fluid adds +0.
+static __device__ __noinline__ void cg_one_warp(const CgArrays& A, bool exact) {
+    const uint32_t lane = threadIdx.x, W = A.w, cells = A.cells, c = lane + W;
+    const uint32_t m = A.bits[0] & (cells < 32u ? (1u << cells) - 1u : 0xffffffffu);
+    const bool on = (m >> lane) & 1u;
+    auto fluid = [&](uint32_t l) { return on && l < 32u && ((m >> l) & 1u); };
+    const bool fr = fluid(lane + 1u), fl = fluid(lane - 1u), fu = fluid(lane + W), fd = fluid(lane - W);
+    float d = 0.0f, r = 0.0f, pr = 0.0f, pl = 0.0f, pu = 0.0f, pd = 0.0f, x = 0.0f;
+    if (on) {
+        d = A.diag[c];
+        r = A.res[c];
+        pr = fr ? A.px[c] : 0.0f;
+        pl = fl ? A.px[c - 1] : 0.0f;
+        pu = fu ? A.py[c] : 0.0f;
+        pd = fd ? A.py[c - W] : 0.0f;
+    }
+    auto dot = [&](float q) {
+        if (!exact) return float(warp_sum(double(q)));
+        float t = 0.0f;
+#pragma unroll 8
+        for (int l = 0; l < 32; ++l) t = t + __shfl_sync(0xffffffffu, q, l);
+        return t;
+    };
+    float s = r;
+    float gamma = dot(r * r);
+    const uint32_t max_it = gamma < 1e-12f ? 0u : min(uint32_t(__popc(m)), 100u);
+    for (uint32_t it = 0; it < max_it; ++it) {
+        const float sr = __shfl_sync(0xffffffffu, s, lane + 1u), sl = __shfl_sync(0xffffffffu, s, lane - 1u);
+        const float su = __shfl_sync(0xffffffffu, s, lane + W), sd = __shfl_sync(0xffffffffu, s, lane - W);
+        float v = d * s;
+        v = fr ? __fmaf_rn(pr, sr, v) : v;
+        v = fl ? __fmaf_rn(pl, sl, v) : v;
+        v = fu ? __fmaf_rn(pu, su, v) : v;
+        v = fd ? __fmaf_rn(pd, sd, v) : v;
+        const float delta = dot(s * v);
+        if (fabsf(delta) < 1e-5f) break;
+        const float alpha = gamma / delta;
+        x = x + alpha * s;
+        r = r - alpha * v;
+        if (!__any_sync(0xffffffffu, fabsf(r) >= 1e-6f)) break;
+        const float new_gamma = dot(r * r);
+        const float beta = new_gamma / gamma;
+        gamma = new_gamma;
+        s = r + (beta * s);
+    }
+    if (on) A.err[c] = x;
+}
+
+// A level of up to 32 cells takes one warp, up to 1024 one cell per thread of as many warps as that needs; above, all threads hold 4,
+// 6 or 10 cells each; beyond 10240 cells (or without shared-memory copies to
+// overwrite) the cells stay in memory.
+static __device__ __forceinline__ void cta_coarse_cg(const CgArrays& A, bool exact) {
+    __shared__ CgShared sh;
+    const uint32_t need = (A.cells + 31u) >> 5, all = blockDim.x >> 5;
+    const uint32_t nwarps = need < all ? need : all;
+    if ((threadIdx.x >> 5) < nwarps) {
+        if (need <= 1u)
+            cg_one_warp(A, exact);
+        else if (need <= all)
+            cg_warps<1>(A, sh, nwarps, exact);
+        else if (A.own && need <= 4u * all)
+            cg_warps<4>(A, sh, nwarps, exact);
+        else if (A.own && need <= 6u * all)
+            cg_warps<6>(A, sh, nwarps, exact);
+        else if (A.own && need <= kCgMaxK * all)
+            cg_warps<int(kCgMaxK)>(A, sh, nwarps, exact);
+        else
+            cg_warps<0>(A, sh, nwarps, exact);
     }
     __syncthreads();
 }
@@ -602,12 +790,9 @@ __device__ __forceinline__ void cta_tail(const TailParams& tp, uint32_t* sm, boo
     {
         SmemLevel L = smem_level(sm, tp.lv[tp.n - 1]);
         float* fs = reinterpret_cast<float*>(sm);
-        if (L.cells <= 32 * kWarpCgCells)
-            warp_coarse_cg(L.bits, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, fs + tp.o_cs, fs + tp.o_cap,
-                           fs + tp.o_cr, tp.exact != 0);
-        else
-            cta_coarse_cg(L.bits, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, fs + tp.o_cs, fs + tp.o_cap,
-                          fs + tp.o_cr, tp.exact != 0);
+        cta_coarse_cg(CgArrays{L.bits, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, fs + tp.o_cs, fs + tp.o_cap,
+                               fs + tp.o_cr, true},
+                      tp.exact != 0);
     }
     for (int l = tp.n - 2; l >= 0; --l) {
         SmemLevel f = smem_level(sm, tp.lv[l]);
