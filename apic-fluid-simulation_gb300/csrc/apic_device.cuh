@@ -432,27 +432,31 @@ __device__ __forceinline__ double sum_partials(const float2* part, uint32_t n) {
     return s_tot;
 }
 
-// Sum and maximum of n float4 partials (x, y: F2 sum; z: maximum).
+// Sum and maximum of n float4 partials (x, y: F2 sum; z: maximum), by the
+// first kThreads threads of a block of at least that many (the order of the
+// sum does not depend on the block's size).
 template <int kThreads>
 __device__ __forceinline__ void sum_max_partials(const float4* part, uint32_t n, double* sum, float* mx) {
     __shared__ F2 s_sp[kThreads / 32];
     __shared__ float s_mp[kThreads / 32];
     __shared__ double s_tot;
     __shared__ float s_max;
-    F2 t{0.0f, 0.0f};
-    float m = 0.0f;
-#pragma unroll 4
-    for (uint32_t b = threadIdx.x; b < n; b += kThreads) {
-        const float4 q = __ldcg(part + b);
-        t = f2_add(t, F2{q.x, q.y});
-        m = fmaxf(m, q.z);
-    }
-    t = warp_sum(t);
-    m = warp_maxf(m);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        s_sp[warp] = t;
-        s_mp[warp] = m;
+    if (warp < kThreads / 32) {
+        F2 t{0.0f, 0.0f};
+        float m = 0.0f;
+#pragma unroll 4
+        for (uint32_t b = threadIdx.x; b < n; b += kThreads) {
+            const float4 q = __ldcg(part + b);
+            t = f2_add(t, F2{q.x, q.y});
+            m = fmaxf(m, q.z);
+        }
+        t = warp_sum(t);
+        m = warp_maxf(m);
+        if (lane == 0) {
+            s_sp[warp] = t;
+            s_mp[warp] = m;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {

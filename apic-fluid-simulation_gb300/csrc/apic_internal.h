@@ -34,6 +34,11 @@ constexpr int kMaxLevels = 20;        // base + coarse levels
 constexpr int kSegBlock = APIC_SEG_BLOCK;  // threads per block of segment kernels
 constexpr int kSegWarps = kSegBlock / 32;
 constexpr int kMaxRedBlocks = 152 * (2048 / kSegBlock);  // one full wave on 152 SMs: grid of reduction kernels
+// Tiles of the V-cycle's grid-wide kernels (tiles.cuh): cells, threads, and the
+// most CTAs of a launch (four per SM on 152 SMs).
+constexpr uint32_t kTileX = 32, kTileY = 16;
+constexpr int kTileBlock = 256;
+constexpr uint32_t kMaxTileBlocks = 152 * 4;
 constexpr int kSortTile = 2048;       // keys per block in the radix sort
 constexpr int kSortThreads = 256;
 constexpr int kMaxDigitBits = 10;     // widest radix-sort digit (1024 buckets)
@@ -87,6 +92,8 @@ struct Ctl {
     uint32_t pad_count;     // duplicates padding the base list to a multiple of 8
     uint32_t red_counter;   // last-block-done counter of the reductions
     uint32_t pcg_on;        // the PCG loop goes on (a batched solve gates its phases on it)
+    uint32_t tile_count[kMaxLevels];  // tiles of a level that hold fluid
+    uint32_t res_sel;       // base residual's current buffer: 0 Level::res, 1 Level::res2
     float b_rz;             // batched solve: the iteration's r.z sum (from the last V-cycle's parts)
     float b_sap;            // batched solve: the iteration's s.Ap sum
 };
@@ -111,6 +118,12 @@ struct Level {
     float* py = nullptr;
     float* res = nullptr;
     float* err = nullptr;
+    // levels with a coarser one (tiles.cuh): the error between the V-cycle's
+    // down and up kernels, and the ascending list of tiles that hold fluid
+    float* pre = nullptr;
+    uint32_t* tiles = nullptr;
+    uint32_t tiles_x = 0, ntiles = 0;
+    float* res2 = nullptr;  // base level: the residual's second buffer (Ctl::res_sel)
 };
 
 // Particle field order, matching apic_field ids 0..8.
@@ -251,6 +264,20 @@ struct Scene {
     RenderBuffers* render = nullptr;          // splatting buffers (allocated on the first frame)
 };
 
+// The exit test of a PCG iteration's residual and the loop's decision, run by
+// the first kernel after the update (pcg::residual_exit, pcg::loop_decision).
+struct ExitArgs {
+    int on = 0;  // 0: no test here
+    const float4* part = nullptr;
+    uint32_t nparts = 0;
+    int mode = 0;
+    float solve_error = 0.0f;
+    cudaGraphConditionalHandle h = 0;
+    uint32_t cap = 0;
+    int dyn_cap = 0;
+    int set_cond = 0;
+};
+
 // ---- launchers (each enqueues on s.stream) --------------------------------
 // sort.cu
 cudaError_t launch_sort(Scene& s);
@@ -320,22 +347,24 @@ cudaError_t launch_post_forces(Scene& s);
 cudaError_t launch_extrapolate(Scene& s);
 cudaError_t launch_smoothed_view(Scene& s, float* out);
 cudaError_t launch_level_lists(Scene& s, int level);
+cudaError_t launch_tile_lists(Scene& s);  // every level's fluid tiles
 // solver.cu: the solve is recorded into graphs (apic_graph.h: build_solve)
 // solver.cu: the same solve launched kernel by kernel with host loop control
 // (profiling runs, so every kernel is a separate launch)
 cudaError_t run_solve_eager(Scene& s);
 // vcycle.cu
 void plan_vcycle(Scene& s);     // pick the coarse levels that run in one CTA / one cluster
+// level l takes its first red sweep from the kernel that restricts into it
+// (the cluster's first level; the tile kernels form it themselves)
+bool vcycle_wants_red(const Scene& s, int l);
 // vcycle_dsm.cu
 void plan_vcycle_dsm(Scene& s);
-void launch_vcycle_dsm(Scene& s, cudaStream_t st);
-// z = M^-1 r on s.stream; base_red_done: the base level's first red sweep
-// was already written (by k_pcg_update); rz_mode >= 0: the last kernel also
-// reduces r.z and finishes the PCG iteration for that solver mode (returns
-// false when this V-cycle form cannot, and the caller must).
-// residual_exit: the first kernel also runs the PCG residual's exit test
-// (k_smooth_exit; with base_red_done, rz_mode = the solver mode).
-bool enqueue_vcycle(Scene& s, bool base_red_done = false, int rz_mode = -1, bool residual_exit = false);
+void launch_vcycle_dsm(Scene& s, cudaStream_t st, const ExitArgs& exit);
+ExitArgs exit_args(const Scene& s, int mode);
+// z = M^-1 r on s.stream, in an iteration after the base level's down kernel
+// has run inside the update (base_done): the first kernel here runs the exit
+// test, and with a coarser level the last one stores the parts of r.z.
+void enqueue_vcycle(Scene& s, bool base_done = false, const ExitArgs& exit = ExitArgs());
 // runtime.cu
 cudaError_t launch_plan_first(Scene& s);
 cudaError_t launch_advance(Scene& s);
@@ -396,5 +425,9 @@ inline cudaError_t launch(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 bloc
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 uint32_t seg_grid(uint32_t words);     // blocks for a segment kernel over `words` words
+// blocks for a tile kernel on a level, and for its base level's block partials
+inline uint32_t tile_grid(const Level& L) {
+    return L.ntiles < kMaxTileBlocks ? (L.ntiles ? L.ntiles : 1u) : kMaxTileBlocks;
+}
 
 }  // namespace apic

@@ -24,7 +24,7 @@
 //
 // The V-cycle of a batched solve runs the coarse tail (the levels that fit in
 // one CTA's shared memory) as one CTA per scene, and the levels above it with
-// the segment kernels; the single-scene form may hold some of those levels
+// the tile kernels; the single-scene form may hold some of those levels
 // in a cluster's distributed shared memory instead, which computes the same
 // values.
 #include <cuda_runtime.h>
@@ -202,6 +202,7 @@ BScene make_bscene(Scene& s) {
         t.lv[l] = s.lv[l];
         t.grid[l] = seg_grid(s.lv[l].words);
     }
+    t.tgrid = tile_grid(s.lv[0]);
     t.ctl = s.ctl;
     t.search = s.search;
     t.ap = s.ap;
@@ -224,26 +225,14 @@ BScene make_bscene(Scene& s) {
 // every scene runs its own levels' kernels in its own order; a launch covers
 // the scenes that have that kernel at that point.
 void bat_vcycle(const BatchRun& r, int max_tail, int gate, bool in_iteration) {
-    if (!in_iteration) {
-        bat_smooth(r, 0, gate, 0, 1);
-        bat_smooth(r, 0, gate, 1, 1);
-    } else {
-        bat_smooth_exit(r);  // k_pcg_update ran the red sweep
-    }
-    for (int l = 1; l <= max_tail; ++l) {
-        bat_restrict(r, l, gate);
-        if (l < max_tail) bat_smooth(r, l, gate, 1, 1);  // no scene smooths its deepest level here
-    }
+    if (!in_iteration) bat_down(r, 0, gate);  // else bat_update_down did
+    for (int l = 1; l < max_tail; ++l) bat_down(r, l, gate);
     bat_tail(r, gate);
-    for (int l = max_tail - 1; l >= 1; --l) {
-        bat_prolong_black(r, l, gate, 0);
-        bat_prolong_red(r, l, gate, 0);
-    }
-    bat_prolong_black(r, 0, gate, 1);
+    for (int l = max_tail - 1; l >= 1; --l) bat_up(r, l, gate, 0);
     if (in_iteration)
-        bat_prolong_red_rz(r);
+        bat_up_rz(r);
     else
-        bat_prolong_red(r, 0, gate, 1);
+        bat_up(r, 0, gate, 1);
 }
 
 // build_pcg over the batch: setup, then WHILE(some scene's PCG goes on).
@@ -264,7 +253,8 @@ cudaError_t bat_pcg(Batch& b, const BatchRun& r, GraphCursor& c, int setup_gate,
     e = capture_on(r.st, body, [&]() {
         bat_spmv_dot(r);
         bat_sap(r);
-        bat_pcg_update(r, into_corr);
+        bat_update_down(r, into_corr);
+        bat_exit(r);
         bat_vcycle(r, b.max_tail, kGatePcg, true);
         bat_round_end(r, hp);
         return cudaGetLastError();

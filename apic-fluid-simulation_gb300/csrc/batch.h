@@ -37,6 +37,7 @@ enum : int {
 struct BScene {
     Level lv[kMaxLevels];
     uint32_t grid[kMaxLevels];  // seg_grid of each level: the scene's own launch size
+    uint32_t tgrid;             // tile_grid of the base level
     Ctl* ctl;
     float *search, *ap, *corr, *pressure;
     double *b64, *p64, *partials;
@@ -77,36 +78,38 @@ inline __host__ __device__ float2* bs_part_rz(const BScene& s) {
 // segment, since the others' partials are zero and a zero adds nothing to
 // the sums those partials feed (products and squares; a zero total stops
 // the solve whatever its sign), block_group consecutive blocks per item.
+// kKindTiles0 does the same with the tile blocks of the base level's down and
+// up kernels in an iteration.
 // Phases whose every cell is computed independently of the others in the
-// launch (sweeps of one colour, restriction, prolongation, copies) take one
-// item per chunk of chunk_segs segments of the level: kind_chunk(l) for the
-// levels the segment kernels smooth (l = 0, and l < tail_first),
-// kind_rchunk(l) for the restriction into level l (l <= tail_first), and
-// kKindExit: the base level's chunks after one item for the exit test.  The
-// chunk counts follow the segment lists of the substep (ctl->seg_count).
+// launch take chunks: kKindChunk, one item per chunk_segs segments of the
+// base level, and kind_tiles(l), one item per tile_chunk tiles of level l
+// (those the tile kernels smooth: l = 0 and l < tail_first).  The counts
+// follow the lists of the substep (ctl->seg_count, ctl->tile_count).
 // chunk_segs and block_group are the batch's shape (chosen by its tuner).
 using Shape = BatchShape;
-enum : int { kKindBase = 0, kKindExit = 1, kKindBlocks = 2 };
-inline __host__ __device__ int kind_chunk(int l) { return 3 + 2 * l; }
-inline __host__ __device__ int kind_rchunk(int l) { return 4 + 2 * l; }
-inline __host__ __device__ uint32_t kinds_for(int max_tail) { return uint32_t(2 * max_tail + 5); }
+enum : int { kKindBase = 0, kKindBlocks = 1, kKindChunk = 2, kKindTiles0 = 3 };
+inline __host__ __device__ int kind_tiles(int l) { return 4 + l; }
+inline __host__ __device__ uint32_t kinds_for(int max_tail) { return uint32_t(max_tail + 5); }
+// a tile holds as many cells as 16 segments
+inline __host__ __device__ uint32_t tile_chunk(Shape sh) { return sh.chunk_segs > 16u ? sh.chunk_segs / 16u : 1u; }
 #ifdef __CUDACC__
 // Blocks of the scene's base-level launch that hold a segment (at least one).
 __device__ __forceinline__ uint32_t busy_blocks(const BScene& s) {
     const uint32_t b = (s.ctl->seg_count[0] + kSegWarps - 1) / kSegWarps;
     return b < 1u ? 1u : (b < s.grid[0] ? b : s.grid[0]);
 }
+// ... of its base level's tile launch that hold a tile (at least one).
+__device__ __forceinline__ uint32_t busy_tile_blocks(const BScene& s) {
+    const uint32_t b = s.ctl->tile_count[0];
+    return b < 1u ? 1u : (b < s.tgrid ? b : s.tgrid);
+}
 __device__ __forceinline__ uint32_t kind_items(const BScene& s, int kind, Shape sh) {
     if (kind == kKindBase) return s.grid[0];
     if (kind == kKindBlocks) return (busy_blocks(s) + sh.block_group - 1) / sh.block_group;
-    const uint32_t* nseg = s.ctl->seg_count;
-    const uint32_t cs = sh.chunk_segs;
-    if (kind == kKindExit) return 1u + (nseg[0] + cs - 1) / cs;
-    const uint32_t l = uint32_t(kind - 3) >> 1;
-    const bool restrict_into = ((kind - 3) & 1) != 0;
-    if (restrict_into) return (l >= 1 && l <= s.tail_first) ? (nseg[l] + cs - 1) / cs : 0u;
-    if (l == 0) return max(1u, (nseg[0] + cs - 1) / cs);  // chunk 0 always exists
-    return l < s.tail_first ? (nseg[l] + cs - 1) / cs : 0u;
+    if (kind == kKindTiles0) return (busy_tile_blocks(s) + sh.block_group - 1) / sh.block_group;
+    if (kind == kKindChunk) return max(1u, (s.ctl->seg_count[0] + sh.chunk_segs - 1) / sh.chunk_segs);
+    const uint32_t l = uint32_t(kind - 4), n = tile_chunk(sh);
+    return l < s.tail_first ? (s.ctl->tile_count[l] + n - 1) / n : 0u;
 }
 
 // A chunk item's segments: [c cs, min(nseg, (c + 1) cs)), warp w of the CTA
@@ -122,6 +125,9 @@ __device__ __forceinline__ Chunk chunk_of(uint32_t c, uint32_t nseg, Shape sh) {
 // The blocks of a block-group item.
 __device__ __forceinline__ uint32_t group_end(const BScene& s, uint32_t item, Shape sh) {
     return min(busy_blocks(s), (item + 1) * sh.block_group);
+}
+__device__ __forceinline__ uint32_t tile_group_end(const BScene& s, uint32_t item, Shape sh) {
+    return min(busy_tile_blocks(s), (item + 1) * sh.block_group);
 }
 #endif
 
@@ -314,18 +320,16 @@ void bat_pcg_cond(const BatchRun& r, cudaGraphConditionalHandle h, int gate);
 void bat_round_end(const BatchRun& r, cudaGraphConditionalHandle h);
 void bat_sap(const BatchRun& r);
 void bat_spmv_dot(const BatchRun& r);
-void bat_pcg_update(const BatchRun& r, int into_corr);
+void bat_update_down(const BatchRun& r, int into_corr);
+void bat_exit(const BatchRun& r);
 void bat_mixed_accumulate(const BatchRun& r, int gate, int finalize);
 void bat_refine_end(const BatchRun& r);
 void bat_finish_solve(const BatchRun& r);
 void bat_pressure_to64(const BatchRun& r, int gate);
 // ---- V-cycle launchers (vcycle.cu) ----
-void bat_smooth_exit(const BatchRun& r);
-void bat_smooth(const BatchRun& r, int l, int gate, int color, int init);
-void bat_restrict(const BatchRun& r, int l, int gate);
-void bat_prolong_black(const BatchRun& r, int l, int gate, int base);
-void bat_prolong_red(const BatchRun& r, int l, int gate, int base);
-void bat_prolong_red_rz(const BatchRun& r);
+void bat_down(const BatchRun& r, int l, int gate);
+void bat_up(const BatchRun& r, int l, int gate, int base);
+void bat_up_rz(const BatchRun& r);
 void bat_tail(const BatchRun& r, int gate);
 void bat_prepare_tail();
 

@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kSegBlock) k_smooth_density(const uint32_t* __
 
 __global__ void __launch_bounds__(kSegBlock) k_laplacian(const uint32_t* __restrict__ fluid,
                                                           const uint32_t* __restrict__ obstacle,
-                                                          const uint32_t* __restrict__ seg, const Ctl* __restrict__ ctl,
+                                                          const uint32_t* __restrict__ seg, Ctl* __restrict__ ctl,
                                                           uint32_t W, uint32_t cells, float dx,
                                                           const float* __restrict__ u, const float* __restrict__ v,
                                                           const float* __restrict__ sm, const float* __restrict__ dens,
@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(kSegBlock) k_laplacian(const uint32_t* __restr
     const uint32_t nseg = ctl->seg_count[0];
     const int lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->res_sel = 0;  // res is written here
     const float target = 9.0f;
     const float noise = target * 1.15f;
     const float corr = 0.1f;
@@ -399,6 +400,40 @@ __global__ void __launch_bounds__(kOneThreads) k_coarsen_tail(TailLevels t, Ctl*
         compact_one(c.fluid, c.words, c.seg, l, ctl);
         __syncthreads();
     }
+}
+
+// The ascending list of a level's tiles that hold fluid, one CTA per level
+// (blockIdx.x): thread t of a round takes tile 1024 * round + t and ORs the
+// 32 bits of its rows.
+struct TileLists {
+    int n;
+    Level lv[kMaxLevels];
+};
+__global__ void __launch_bounds__(kOneThreads) k_tile_lists(TileLists t, Ctl* __restrict__ ctl) {
+    pdl_wait();
+    const Level& L = t.lv[blockIdx.x];
+    uint32_t count = 0;
+    for (uint32_t i0 = 0; i0 < L.ntiles; i0 += kOneThreads) {
+        const uint32_t i = i0 + threadIdx.x;
+        uint32_t any = 0;
+        if (i < L.ntiles) {
+            const uint32_t x0 = (i % L.tiles_x) * kTileX, y0 = (i / L.tiles_x) * kTileY;
+            const uint32_t rows = min(kTileY, L.h - y0), n = min(kTileX, L.w - x0);
+            const uint32_t mask = n >= 32u ? 0xffffffffu : (1u << n) - 1u;
+#pragma unroll 4
+            for (uint32_t y = 0; y < rows; ++y) {
+                const uint32_t raw = (y0 + y) * L.w + x0, sh = raw & 31u;
+                uint32_t bits = L.fluid[raw >> 5] >> sh;
+                if (sh && (raw >> 5) + 1u < L.words) bits |= L.fluid[(raw >> 5) + 1u] << (32u - sh);
+                any |= bits & mask;
+            }
+        }
+        uint32_t tot;
+        const uint32_t off = scan_1024(any ? 1u : 0u, &tot);
+        if (any) L.tiles[count + off] = i;
+        count += tot;
+    }
+    if (threadIdx.x == 0) ctl->tile_count[blockIdx.x] = count;
 }
 
 __global__ void __launch_bounds__(256) k_gradient(uint32_t uf, uint32_t vf, int W, int H, float inv_dx,
@@ -610,6 +645,16 @@ static cudaError_t compact_level(Scene& s, int level, const uint32_t* obstacle) 
     return cudaGetLastError();
 }
 
+// Every level that the V-cycle's tile kernels may work on (those with a
+// coarser one).
+cudaError_t launch_tile_lists(Scene& s) {
+    TileLists t;
+    t.n = s.nlevels - 1;
+    if (t.n < 1) return cudaSuccess;
+    for (int l = 0; l < t.n; ++l) t.lv[l] = s.lv[l];
+    launch(s.use_pdl, k_tile_lists, t.n, kOneThreads, 0, s.stream, t, s.ctl);
+    return cudaGetLastError();
+}
 cudaError_t launch_base_lists(Scene& s) { return compact_level(s, 0, s.obstacle); }
 cudaError_t launch_level_lists(Scene& s, int level) { return compact_level(s, level, nullptr); }
 
@@ -643,7 +688,7 @@ cudaError_t launch_multilevel(Scene& s) {
         for (int k = 0; k < s.nlevels; ++k) t.lv[k] = s.lv[k];
         launch(s.use_pdl, k_coarsen_tail, 1, kOneThreads, 0, s.stream, t, s.ctl);
     }
-    return cudaGetLastError();
+    return launch_tile_lists(s);
 }
 
 cudaError_t launch_gradient(Scene& s, bool post) {

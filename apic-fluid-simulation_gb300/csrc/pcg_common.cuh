@@ -57,57 +57,6 @@ __device__ __forceinline__ F2 ph_start(const Level& B, uint32_t nseg, uint32_t w
     return acc;
 }
 
-// Ap = A s (FMA chain of :1833-1846); returns s.Ap.
-__device__ __forceinline__ F2 ph_spmv(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps,
-                                      const float* s, float* ap) {
-    F2 acc{0.0f, 0.0f};
-    const long long W = B.w;
-    APIC_BASE_ALL(B, nseg, warp, nwarps) {
-        const long long raw = raw_;
-        const uint32_t c = raw_ + B.w;
-        const bool fr = fluid_raw(B.fluid, raw + 1, B.cells), fl = fluid_raw(B.fluid, raw - 1, B.cells);
-        const bool fu = fluid_raw(B.fluid, raw + W, B.cells), fd = fluid_raw(B.fluid, raw - W, B.cells);
-        const float sc = s[c], sr = s[c + 1], sl = s[c - 1], su = s[c + W], sd = s[c - W];
-        const float pxc = B.px[c], pxl = B.px[c - 1], pyc = B.py[c], pyd = B.py[c - W];
-        float v = B.diag[c] * sc;
-        float t = __fmaf_rn(pxc, sr, v);
-        v = fr ? t : v;
-        t = __fmaf_rn(pxl, sl, v);
-        v = fl ? t : v;
-        t = __fmaf_rn(pyc, su, v);
-        v = fu ? t : v;
-        t = __fmaf_rn(pyd, sd, v);
-        v = fd ? t : v;
-        if (!fluid_) continue;
-        ap[c] = v;
-        acc = f2_add(acc, v * sc);
-    }
-    return acc;
-}
-
-// x += alpha s (x = pressure in cell layout, or a padded vector);
-// r = fma(-alpha, Ap, r) (:1910-1928).  Returns max|r| and sum r^2 (each
-// square exact, summed in double-float).
-__device__ __forceinline__ void ph_update(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps, float alpha,
-                                          float* x, int x_padded, const float* s, const float* ap, float* max_r,
-                                          F2* r2) {
-    float mx = 0.0f;
-    F2 acc{0.0f, 0.0f};
-    APIC_BASE_ALL(B, nseg, warp, nwarps) {
-        const uint32_t c = raw_ + B.w;
-        const uint32_t xi = x_padded ? c : raw_;
-        const float nx = x[xi] + alpha * s[c];
-        const float nr = __fmaf_rn(-alpha, ap[c], B.res[c]);
-        if (!fluid_) continue;
-        x[xi] = nx;
-        B.res[c] = nr;
-        mx = fmaxf(mx, fabsf(nr));
-        acc = f2_add(acc, f2_square(nr));
-    }
-    *max_r = mx;
-    *r2 = acc;
-}
-
 // ---- graph-path forms with the search update folded in -----------------------
 // The search direction of an iteration, s' = z + beta s (:1945-1954), is not
 // written by a kernel of its own: the SpMV evaluates it at the five stencil
@@ -153,7 +102,8 @@ __device__ __forceinline__ F2 ph_spmv_search(const Level& B, uint32_t nseg, uint
     return acc;
 }
 
-// x += alpha s', r = fma(-alpha, Ap, r) (:1910-1928), s = s'; and on red
+// (grids without a coarser level; the others update in the base level's down
+// kernel, tiles.cuh)  x += alpha s', r = fma(-alpha, Ap, r) (:1910-1928), s = s'; and on red
 // cells the preconditioner's first sweep from zero error, which needs only
 // the cell's new residual: z = 0 + omega (r / diag - 0) (smooth_level
 // :487-507 with every neighbour still zero).  Returns max|r| and sum r^2.
@@ -224,7 +174,10 @@ __device__ __forceinline__ void loop_decision(Ctl* ctl, int mode, cudaGraphCondi
 // block, after the caller's dependency wait.
 __device__ __forceinline__ void residual_exit(Ctl* ctl, const float4* part, uint32_t n, int mode, float solve_error) {
     if (ctl->delta_stop) {  // s.Ap was unusable: no update, no residual parts
-        if (threadIdx.x == 0) ctl->pcg_done = 1;
+        if (threadIdx.x == 0) {
+            ctl->pcg_done = 1;
+            ctl->res_sel ^= 1u;  // the update left the residual where it was
+        }
         return;
     }
     double tot;
@@ -242,6 +195,33 @@ __device__ __forceinline__ void residual_exit(Ctl* ctl, const float4* part, uint
     }
 }
 
+// Base residual: the buffer that holds it now.
+__device__ __forceinline__ const float* cur_res(const Level& B, const Ctl* ctl) {
+    return ctl->res_sel && B.res2 ? B.res2 : B.res;
+}
+
+// The exit test and loop decision in every CTA of a kernel that runs after
+// the update and whose CTAs all go on or all return (a cluster, a single
+// CTA): each sums the parts itself, to the same verdict, and `writer`'s
+// thread 0 records it.  True: the solve is done.
+__device__ __forceinline__ bool exit_verdict(Ctl* ctl, const ExitArgs& a, bool writer) {
+    double tot;
+    float t;
+    sum_max_partials<kSegBlock>(a.part, a.nparts, &tot, &t);
+    const double rel = ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0;
+    const bool stop = ctl->delta_stop != 0;
+    const bool done =
+        stop || (a.mode == APIC_SOLVER_REFERENCE ? t < a.solve_error : rel <= ctl->target_rel);
+    if (writer && threadIdx.x == 0) {
+        if (stop) ctl->res_sel ^= 1u;  // the update left the residual where it was
+        else if (a.mode == APIC_SOLVER_REFERENCE) ctl->max_r_bits = __float_as_uint(t);
+        else ctl->rnorm2 = tot;
+        if (done) ctl->pcg_done = 1;
+        loop_decision(ctl, a.mode, a.h, a.cap, a.dyn_cap, a.set_cond);
+    }
+    return done;
+}
+
 // r.z after the preconditioner (:1936).
 __device__ __forceinline__ F2 ph_rz(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps) {
     F2 acc{0.0f, 0.0f};
@@ -251,16 +231,6 @@ __device__ __forceinline__ F2 ph_rz(const Level& B, uint32_t nseg, uint32_t warp
         if (fluid_) acc = f2_add(acc, rz);
     }
     return acc;
-}
-
-// s = z + beta s (:1945-1954).
-__device__ __forceinline__ void ph_search(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps, float beta,
-                                          float* s) {
-    APIC_BASE_ALL(B, nseg, warp, nwarps) {
-        const uint32_t c = raw_ + B.w;
-        const float v = B.err[c] + (beta * s[c]);
-        if (fluid_) s[c] = v;
-    }
 }
 
 // ---- FP64 refinement (APIC_SOLVER_REL_MIXED) ---------------------------------

@@ -299,6 +299,7 @@ void free_scene(Scene& s) {
         Level& L = s.lv[l];
         dfree(L.fluid, st); dfree(L.seg, st); dfree(L.diag, st); dfree(L.inv_diag, st); dfree(L.px, st);
         dfree(L.py, st); dfree(L.res, st); dfree(L.err, st);
+        dfree(L.pre, st); dfree(L.tiles, st); dfree(L.res2, st);
     }
     free_render(s);
     dfree(s.vec_stage, st);
@@ -701,6 +702,12 @@ int apic::create_scene(uint32_t width, uint32_t height, float cell_size, const a
         AL(L.fluid, L.words); AL(L.seg, L.words);
         AL(L.diag, L.padded); AL(L.inv_diag, L.padded); AL(L.px, L.padded); AL(L.py, L.padded);
         AL(L.res, L.padded); AL(L.err, L.padded);
+        if (l + 1 < s.nlevels) {
+            L.tiles_x = div_up(L.w, kTileX);
+            L.ntiles = L.tiles_x * div_up(L.h, kTileY);
+            AL(L.pre, L.padded); AL(L.tiles, L.ntiles);
+            if (l == 0) AL(L.res2, L.padded);
+        }
     }
     {
         Level& C = s.lv[s.nlevels - 1];
@@ -1036,7 +1043,7 @@ FieldDesc describe(apic_handle* h, int id, const PartPtrs* pp) {
         case APIC_F_OBSTACLE_BITS: M(s.obstacle, even_words(s.cells)); return d;
         case APIC_F_U_OPEN_BITS: M(s.u_open, s.u_open_words); return d;
         case APIC_F_V_OPEN_BITS: M(s.v_open, s.v_open_words); return d;
-        case APIC_F_RESIDUAL: F(s.lv[0].res, padded); return d;
+        case APIC_F_RESIDUAL: F(s.ctl_host->res_sel && s.lv[0].res2 ? s.lv[0].res2 : s.lv[0].res, padded); return d;
         case APIC_F_DIAG: F(s.lv[0].diag, padded); return d;
         case APIC_F_INV_DIAG: F(s.lv[0].inv_diag, padded); return d;
         case APIC_F_PLUS_X: F(s.lv[0].px, padded); return d;
@@ -1104,6 +1111,10 @@ int apic_read_field(apic_handle* h, int field, void* dst, uint64_t bytes) {
     Scene& s = h->s;
     CK(cudaStreamSynchronize(s.stream));
     PartPtrs pp = read_ptrs(s);
+    if (field == APIC_F_RESIDUAL) {  // which of its two buffers is current
+        int rc = sync_ctl(s);
+        if (rc) return rc;
+    }
     FieldDesc d = describe(h, field, &pp);
     if (!d.ok) return fail(APIC_ERR_INVALID_ARG, "unknown field " + std::to_string(field));
     if (field == APIC_F_FLUID_LIST) {
@@ -1131,6 +1142,10 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
     Scene& s = h->s;
     CK(cudaStreamSynchronize(s.stream));
     PartPtrs pp = read_ptrs(s);
+    if (field == APIC_F_RESIDUAL) {  // a solve starts from the first buffer
+        CK(cudaMemset(&s.ctl->res_sel, 0, sizeof(uint32_t)));
+        s.ctl_host->res_sel = 0;
+    }
     FieldDesc d = describe(h, field, &pp);
     if (!d.ok || field == APIC_F_FLUID_LIST || field == APIC_F_SORT_KEYS || field == APIC_F_SORT_VALS)
         return fail(APIC_ERR_INVALID_ARG, "field not writable: " + std::to_string(field));
@@ -1147,10 +1162,12 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
     }
     if (field == APIC_F_FLUID_BITS) {
         CK(launch_base_lists(s));
+        CK(launch_tile_lists(s));
         CK(cudaStreamSynchronize(s.stream));
     }
     if (field >= APIC_F_MG_FLUID_BITS && field % APIC_F_MG_LEVEL_STRIDE == APIC_F_MG_FLUID_BITS) {
         CK(launch_level_lists(s, field / APIC_F_MG_LEVEL_STRIDE + 1));
+        CK(launch_tile_lists(s));
         CK(cudaStreamSynchronize(s.stream));
     }
     if (field == APIC_F_EXT_FORCE_U || field == APIC_F_EXT_FORCE_V) s.has_ext = true;

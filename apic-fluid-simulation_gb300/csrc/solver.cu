@@ -31,6 +31,7 @@
 #include "apic_internal.h"
 #include "batch.h"
 #include "pcg_common.cuh"
+#include "tiles.cuh"
 
 namespace apic {
 namespace {
@@ -51,6 +52,7 @@ __device__ __forceinline__ void pcg_reset(Ctl* ctl) {
     ctl->beta_valid = 0;
     ctl->delta_stop = 0;
     ctl->rnorm2 = 0.0;
+    ctl->res_sel = 0;  // a solve's right-hand side is in the first buffer
 }
 
 __global__ void k_pcg_begin(Ctl* ctl, int stamp) {
@@ -107,6 +109,9 @@ __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nse
         beta = ng / ctl->gamma;
         if (bk.id == 0 && threadIdx.x == 0) ctl->beta = beta;
     }
+    // the buffer this iteration's update writes the residual to (read by the
+    // kernels after this one)
+    if (bk.id == 0 && threadIdx.x == 0) ctl->res_sel = (ctl->pcg_iters + 1u) & 1u;
     F2 acc = pcg::ph_spmv_search(B, nseg, blk_warp(bk), blk_nwarps(bk), s, beta, bv, ap, w0);
     block_store<kSegBlock>(bk, acc, part);
 }
@@ -121,38 +126,41 @@ __global__ void __launch_bounds__(kSegBlock) k_spmv_dot(Level B, const float* s,
 }
 
 // delta (the sum of k_spmv_dot's parts, formed by every block) gives alpha or
-// the exit (src/apic.rs:1899-1906, applied by the next kernel); then
-// p += alpha s', r = fma(-alpha, Ap, r)
-// (:1907-1932), s = s', the V-cycle's first red sweep on the base level, and
-// this block's part of ||r||^2 and max|r|, whose exit test runs in the next
-// kernel (k_smooth_conv).
+// the exit (src/apic.rs:1899-1906, applied by the next kernel).  False: the
+// block has nothing to do.
 // rz_sum, sap_sum: the parts' sums formed once beforehand (batched solves).
-__device__ __forceinline__ void kb_pcg_update(Blk bk, const Level& B, uint32_t nseg, uint32_t w0, float* p,
-                                              int p_padded, float* s, const float* ap, Ctl* ctl, const float2* sap,
-                                              uint32_t nsap, float4* part, int mode, const float* exact_parts,
-                                              const uint32_t* seg_pre, const float2* rz, uint32_t nrz,
-                                              const float* rz_sum = nullptr, const float* sap_sum = nullptr) {
-    if (ctl->pcg_done) return;
+struct StepArgs {
+    const float2* sap;
+    uint32_t nsap;
+    int mode;
+    const float* exact_parts;
+    const uint32_t* seg_pre;
+    const float2* rz;
+    uint32_t nrz;
+};
+__device__ __forceinline__ bool pcg_alpha(Blk bk, Ctl* ctl, const StepArgs& a, float* alpha_out,
+                                          const float* rz_sum = nullptr, const float* sap_sum = nullptr) {
+    if (ctl->pcg_done) return false;
     // this iteration's gamma: from the solve's start, or (relative modes) the
     // previous iteration's r.z parts, which k_spmv_dot summed the same way
     float gamma = ctl->gamma;
-    if (mode != APIC_SOLVER_REFERENCE && ctl->beta_valid) {
-        gamma = rz_sum ? *rz_sum : float(sum_partials<kSegBlock>(rz, nrz));
+    if (a.mode != APIC_SOLVER_REFERENCE && ctl->beta_valid) {
+        gamma = rz_sum ? *rz_sum : float(sum_partials<kSegBlock>(a.rz, a.nrz));
         if (!(gamma != 0.0f)) {
             if (bk.id == 0 && threadIdx.x == 0) ctl->pcg_done = 1;
-            return;
+            return false;
         }
     }
     float delta;
-    if (mode == APIC_SOLVER_REFERENCE) {
+    if (a.mode == APIC_SOLVER_REFERENCE) {
         // the chunk sums of k_delta_exact, added in chunk order from zero
-        const uint32_t nchunks = (seg_pre[ctl->seg_count[0]] + kDeltaChunk - 1) / kDeltaChunk;
+        const uint32_t nchunks = (a.seg_pre[ctl->seg_count[0]] + kDeltaChunk - 1) / kDeltaChunk;
         delta = 0.0f;
-        for (uint32_t c = 0; c < nchunks; ++c) delta = delta + exact_parts[c];
+        for (uint32_t c = 0; c < nchunks; ++c) delta = delta + a.exact_parts[c];
     } else {
-        delta = sap_sum ? *sap_sum : float(sum_partials<kSegBlock>(sap, nsap));
+        delta = sap_sum ? *sap_sum : float(sum_partials<kSegBlock>(a.sap, a.nsap));
     }
-    const bool stop = mode == APIC_SOLVER_REFERENCE ? fabsf(delta) < kSafety : (!(delta != 0.0f) || !isfinite(delta));
+    const bool stop = a.mode == APIC_SOLVER_REFERENCE ? fabsf(delta) < kSafety : (!(delta != 0.0f) || !isfinite(delta));
     const float alpha = gamma / delta;
     // every block reads pcg_done on entry, so the stop is recorded aside and
     // the next kernel turns it into pcg_done
@@ -162,33 +170,77 @@ __device__ __forceinline__ void kb_pcg_update(Blk bk, const Level& B, uint32_t n
         ctl->delta_stop = stop ? 1u : 0u;
         if (!stop) ctl->alpha = alpha;
     }
-    if (stop) return;
-    float mx;
-    F2 acc;
-    pcg::ph_update_search(B, nseg, blk_warp(bk), blk_nwarps(bk), alpha, ctl->beta, ctl->beta_valid != 0, p, p_padded,
-                          s, ap, &mx, &acc, w0);
-    block_store<kSegBlock>(bk, acc, mx, part);
-}
-__global__ void __launch_bounds__(kSegBlock) k_pcg_update(Level B, float* p, int p_padded, float* s,
-                                                          const float* ap, Ctl* ctl, const float2* sap,
-                                                          uint32_t nsap, float4* part, int mode,
-                                                          const float* exact_parts, const uint32_t* seg_pre,
-                                                          const float2* rz, uint32_t nrz) {
-    const uint32_t nseg = ctl->seg_count[0];
-    const uint32_t w0 = gwarp() < nseg ? B.seg[gwarp()] : 0xFFFFFFFFu;
-    pdl_wait();
-    kb_pcg_update(hw_blk(), B, nseg, w0, p, p_padded, s, ap, ctl, sap, nsap, part, mode, exact_parts, seg_pre, rz,
-                  nrz);
+    *alpha_out = alpha;
+    return !stop;
 }
 
-// Stand-alone exit test (paths whose V-cycle does not start with the base
-// level's black sweep).
-__global__ void __launch_bounds__(kSegBlock) k_residual_exit(Ctl* ctl, const float4* part, uint32_t n, int mode,
-                                                             float solve_error, cudaGraphConditionalHandle h,
-                                                             uint32_t cap, int dyn_cap, int set_cond) {
+// The update (p += alpha s', r = fma(-alpha, Ap, r), s = s', :1907-1932) in
+// the base level's down kernel (tiles.cuh), and this block's part of ||r||^2
+// and max|r|, whose exit test runs in the next kernel.  Block b takes the
+// tiles b, b + n, ...  A tile's constants are read before the wait for the
+// previous kernel and its vectors before alpha is formed from the parts.
+__device__ __forceinline__ tile::Update update_args(const Level& B, const Ctl* ctl, float* p, int p_padded, float* s,
+                                                    const float* ap) {
+    const bool second = ctl->res_sel != 0;  // the residual goes there
+    return tile::Update{second ? B.res : B.res2, ap, B.err, s, p, p_padded, second ? B.res2 : B.res};
+}
+// (after the dependency wait; g: the first tile's constants, if the block has one)
+__device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Level& C, tile::Shared& sh,
+                                               tile::DownRegs& g, uint32_t count, uint32_t id, float* p, int p_padded,
+                                               float* s, const float* ap, Ctl* ctl, const StepArgs& a, float4* part,
+                                               bool with_red, const float* rz_sum = nullptr,
+                                               const float* sap_sum = nullptr) {
+    if (ctl->pcg_done) return;
+    const tile::Update u = update_args(B, ctl, p, p_padded, s, ap);
+    if (bk.id < count) tile::down_load<true>(B, u.res, u, g);
+    float alpha;
+    if (!pcg_alpha(bk, ctl, a, &alpha, rz_sum, sap_sum)) return;
+    const float beta = ctl->beta;
+    const bool beta_valid = ctl->beta_valid != 0;
+    float mx = 0.0f;
+    F2 acc{0.0f, 0.0f};
+    for (uint32_t i = bk.id; i < count; i += bk.n) {
+        if (i != bk.id) {
+            id = B.tiles[i];
+            __syncthreads();  // the tile before this one has been read
+            tile::down_load_const(B, id, g);
+            tile::down_load<true>(B, u.res, u, g);
+        }
+        tile::down_tile<true>(sh, B, C, id, g, u, alpha, beta, beta_valid, with_red, &acc, &mx);
+    }
+    block_store<kSegBlock>(bk, acc, mx, part);
+}
+__global__ void __launch_bounds__(kTileBlock, 4) k_update_down(Level B, Level C, float* p, int p_padded, float* s,
+                                                                 const float* ap, Ctl* ctl, StepArgs a, float4* part,
+                                                                 int with_red) {
+    __shared__ tile::Shared sh;
+    const uint32_t count = ctl->tile_count[0];
+    const uint32_t id = blockIdx.x < count ? B.tiles[blockIdx.x] : 0u;
+    tile::DownRegs g;
+    if (blockIdx.x < count) tile::down_load_const(B, id, g);
     pdl_wait();
-    if (!ctl->pcg_done) pcg::residual_exit(ctl, part, n, mode, solve_error);
-    if (threadIdx.x == 0) pcg::loop_decision(ctl, mode, h, cap, dyn_cap, set_cond);
+    kb_update_down(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part, with_red != 0);
+}
+
+// The update alone, and the base level's first red sweep (grids without a
+// coarser level).
+__global__ void __launch_bounds__(kSegBlock) k_pcg_update(Level B, float* p, int p_padded, float* s,
+                                                          const float* ap, Ctl* ctl, StepArgs a, float4* part) {
+    pdl_wait();
+    float alpha;
+    if (!pcg_alpha(hw_blk(), ctl, a, &alpha)) return;
+    float mx;
+    F2 acc;
+    pcg::ph_update_search(B, ctl->seg_count[0], gwarp(), gnwarps(), alpha, ctl->beta, ctl->beta_valid != 0, p,
+                          p_padded, s, ap, &mx, &acc);
+    block_store<kSegBlock>(hw_blk(), acc, mx, part);
+}
+
+// Stand-alone exit test (grids without a coarser level).
+__global__ void __launch_bounds__(kSegBlock) k_residual_exit(Ctl* ctl, ExitArgs a) {
+    pdl_wait();
+    if (!ctl->pcg_done) pcg::residual_exit(ctl, a.part, a.nparts, a.mode, a.solve_error);
+    if (threadIdx.x == 0) pcg::loop_decision(ctl, a.mode, a.h, a.cap, a.dyn_cap, a.set_cond);
 }
 
 // This block's part of gamma' = r.z (src/apic.rs:1934-1943); the next
@@ -233,6 +285,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
     if (ctl->pcg_done) return;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t nseg = ctl->seg_count[0];
+    const float* __restrict__ res = pcg::cur_res(B, ctl);
     const uint32_t full = (B.cells / 8u) * 8u;
     const uint32_t nbatch = (nseg + kGammaBatch - 1) / kGammaBatch;
     // warps 1..31 stage batch b into buffer b % 2
@@ -243,7 +296,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
             const uint32_t w = B.seg[k0 + q];
             const uint32_t raw = w * 32u + lane;
             const bool on = ((B.fluid[w] >> lane) & 1u) && raw < full;
-            buf[q * 32u + lane] = on ? B.res[raw + B.w] * B.err[raw + B.w] : 0.0f;
+            buf[q * 32u + lane] = on ? res[raw + B.w] * B.err[raw + B.w] : 0.0f;
         }
     };
     float acc = 0.0f;
@@ -273,7 +326,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
     if (t != 0) return;
     float g = ((lanes[0] + lanes[2]) + (lanes[1] + lanes[3])) + ((lanes[4] + lanes[6]) + (lanes[5] + lanes[7]));
     for (uint32_t raw = full; raw < B.cells; ++raw)
-        if (bit_at(B.fluid, raw)) g = g + B.res[raw + B.w] * B.err[raw + B.w];
+        if (bit_at(B.fluid, raw)) g = g + res[raw + B.w] * B.err[raw + B.w];
     if (start) {
         ctl->gamma = g;
         ctl->dgamma = double(g);
@@ -400,6 +453,7 @@ __global__ void __launch_bounds__(kSegBlock) k_mixed_init(Level B, double* b64, 
 // True relative residual of p64 (flags: see pcg::ph_true_residual).
 __device__ __forceinline__ void kb_true_residual(Blk bk, const Level& B, const double* b64, const double* p64,
                                                  float* x, Ctl* ctl, double* partials, int flags) {
+    if ((flags & 1) && bk.id == 0 && threadIdx.x == 0) ctl->res_sel = 0;
     double rr = pcg::ph_true_residual(B, ctl->seg_count[0], blk_warp(bk), blk_nwarps(bk), b64, p64, x, flags);
     double tot;
     if (block_sum_last<kSegBlock>(bk, rr, partials, &ctl->red_counter, &tot) && threadIdx.x == 0)
@@ -594,7 +648,7 @@ __global__ void __launch_bounds__(kSegBlock) k_bat_round_end(const BScene* __res
     const BScene& S = tab[blockIdx.x - 1];
     Ctl* ctl = S.ctl;
     if (!bat_gate(ctl, kGatePcg) || ctl->pcg_done) return;
-    const float rz = float(sum_partials<kSegBlock>(bs_part_rz(S), busy_blocks(S)));
+    const float rz = float(sum_partials<kSegBlock>(bs_part_rz(S), busy_tile_blocks(S)));
     if (threadIdx.x == 0) ctl->b_rz = rz;
 }
 
@@ -618,7 +672,7 @@ __global__ void __launch_bounds__(kSegBlock) k_bat_mixed_init(const BScene* __re
 
 __global__ void __launch_bounds__(kSegBlock) k_bat_clear_pressure(const BScene* __restrict__ tab, BListRef L,
                                                                   int gate) {
-    bat_for_items(L, kind_chunk(0), false, [&](uint32_t sc, uint32_t lb, Shape sh) {
+    bat_for_items(L, kKindChunk, false, [&](uint32_t sc, uint32_t lb, Shape sh) {
         const BScene& S = tab[sc];
         if (!bat_gate(S.ctl, gate)) return;
         const Chunk ch = chunk_of(lb, S.ctl->seg_count[0], sh);
@@ -657,26 +711,41 @@ __global__ void __launch_bounds__(kSegBlock, 8) k_bat_spmv_dot(const BScene* __r
     });
 }
 
-__global__ void __launch_bounds__(kSegBlock, 8) k_bat_pcg_update(const BScene* __restrict__ tab, BListRef L,
-                                                              int into_corr) {
-    bat_for_items(L, kKindBlocks, true, [&](uint32_t sc, uint32_t item, Shape sh) {
+__global__ void __launch_bounds__(kTileBlock, 4) k_bat_update_down(const BScene* __restrict__ tab, BListRef L,
+                                                                     int into_corr) {
+    __shared__ tile::Shared sh;
+    bat_for_items(L, kKindTiles0, true, [&](uint32_t sc, uint32_t item, Shape shp) {
         const BScene& S = tab[sc];
         Ctl* ctl = S.ctl;
         if (!bat_gate(ctl, kGatePcg)) return;
-        const uint32_t nseg = ctl->seg_count[0], end = group_end(S, item, sh);
-        for (uint32_t b = item * sh.block_group; b < end; ++b) {
-            kb_pcg_update(Blk{b, S.grid[0]}, S.lv[0], nseg, 0xFFFFFFFFu, into_corr ? S.corr : S.pressure, into_corr,
-                          S.search, S.ap, ctl, bs_part_sap(S), S.grid[0], bs_part_res(S), kRel, nullptr, nullptr,
-                          bs_part_rz(S), S.grid[0], &ctl->b_rz, &ctl->b_sap);
+        const uint32_t count = ctl->tile_count[0], end = tile_group_end(S, item, shp);
+        const StepArgs a{bs_part_sap(S), S.grid[0], kRel, nullptr, nullptr, bs_part_rz(S), S.tgrid};
+        for (uint32_t b = item * shp.block_group; b < end; ++b) {
+            tile::DownRegs g;
+            const uint32_t id = b < count ? S.lv[0].tiles[b] : 0u;
+            if (b < count) tile::down_load_const(S.lv[0], id, g);
+            kb_update_down(Blk{b, S.tgrid}, S.lv[0], S.lv[1], sh, g, count, id, into_corr ? S.corr : S.pressure,
+                           into_corr, S.search, S.ap, ctl, a, bs_part_res(S), false, &ctl->b_rz, &ctl->b_sap);
             __syncthreads();
         }
     });
 }
 
+// The exit test and loop decision of every listed scene after its update
+// (k_bat_round_end then lists the scenes that go on).
+__global__ void __launch_bounds__(kSegBlock) k_bat_exit(const BScene* __restrict__ tab, uint32_t n) {
+    pdl_wait();
+    const BScene& S = tab[blockIdx.x];
+    Ctl* ctl = S.ctl;
+    if (!bat_gate(ctl, kGatePcg)) return;
+    if (!ctl->pcg_done) pcg::residual_exit(ctl, bs_part_res(S), busy_tile_blocks(S), APIC_SOLVER_REL_FP32, 0.0f);
+    if (threadIdx.x == 0) ctl->pcg_on = pcg::loop_continue(ctl, APIC_SOLVER_REL_FP32, 0u, 1) ? 1u : 0u;
+}
+
 // (k_mixed_accumulate: chunk 0 also counts the inner solve's iterations)
 __global__ void __launch_bounds__(kSegBlock) k_bat_mixed_accumulate(const BScene* __restrict__ tab, BListRef L,
                                                                     int gate, int finalize) {
-    bat_for_items(L, kind_chunk(0), false, [&](uint32_t sc, uint32_t lb, Shape sh) {
+    bat_for_items(L, kKindChunk, false, [&](uint32_t sc, uint32_t lb, Shape sh) {
         const BScene& S = tab[sc];
         Ctl* ctl = S.ctl;
         if (!bat_gate(ctl, gate)) return;
@@ -688,7 +757,7 @@ __global__ void __launch_bounds__(kSegBlock) k_bat_mixed_accumulate(const BScene
 
 __global__ void __launch_bounds__(kSegBlock) k_bat_pressure_to64(const BScene* __restrict__ tab, BListRef L,
                                                                  int gate) {
-    bat_for_items(L, kind_chunk(0), false, [&](uint32_t sc, uint32_t lb, Shape sh) {
+    bat_for_items(L, kKindChunk, false, [&](uint32_t sc, uint32_t lb, Shape sh) {
         const BScene& S = tab[sc];
         if (!bat_gate(S.ctl, gate)) return;
         const Chunk ch = chunk_of(lb, S.ctl->seg_count[0], sh);
@@ -742,10 +811,11 @@ void bat_spmv_dot(const BatchRun& r) {
     APIC_PGRID(k_bat_spmv_dot);
     k_bat_spmv_dot<<<g, kSegBlock, 0, r.st>>>(r.tab, r.list[kGatePcg]);
 }
-void bat_pcg_update(const BatchRun& r, int into_corr) {
-    APIC_PGRID(k_bat_pcg_update);
-    launch(r.pdl, k_bat_pcg_update, g, kSegBlock, 0, r.st, r.tab, r.list[kGatePcg], into_corr);
+void bat_update_down(const BatchRun& r, int into_corr) {
+    APIC_PGRID(k_bat_update_down);
+    launch(r.pdl, k_bat_update_down, g, kTileBlock, 0, r.st, r.tab, r.list[kGatePcg], into_corr);
 }
+void bat_exit(const BatchRun& r) { launch(r.pdl, k_bat_exit, r.nscenes, kSegBlock, 0, r.st, r.tab, r.nscenes); }
 void bat_mixed_accumulate(const BatchRun& r, int gate, int finalize) {
     APIC_PGRID(k_bat_mixed_accumulate);
     launch(false, k_bat_mixed_accumulate, g, kSegBlock, 0, r.st, r.tab, r.list[gate], gate, finalize);
@@ -758,32 +828,49 @@ void bat_pressure_to64(const BatchRun& r, int gate) {
 }
 #undef APIC_PGRID
 
+ExitArgs exit_args(const Scene& s, int mode) {
+    ExitArgs a;
+    a.on = 1;
+    a.part = part_res(s);
+    a.nparts = s.nlevels >= 2 ? tile_grid(s.lv[0]) : seg_grid(s.lv[0].words);
+    a.mode = mode;
+    a.solve_error = s.props.solve_error;
+    a.h = s.pcg_h;
+    a.cap = s.pcg_cap;
+    a.dyn_cap = s.pcg_dyn_cap;
+    a.set_cond = s.pcg_set_cond ? 1 : 0;
+    return a;
+}
+
 // One PCG iteration (src/apic.rs:1899-1955); x receives alpha * s.  The
 // search update that ends the reference's iteration happens at the start of
-// the next one (inside k_spmv_dot / k_pcg_update), and k_pcg_update also
-// runs the V-cycle's first base-level sweep.
+// the next one (inside k_spmv_dot / k_update_down).
 static void pcg_iteration(Scene& s, int mode, float* x, int p_padded) {
     const Level& B = s.lv[0];
-    uint32_t g = seg_grid(B.words);
+    const uint32_t g = seg_grid(B.words), tg = tile_grid(B);
     cudaStream_t st = s.stream;
-    const bool pdl = s.use_pdl;
+    const bool pdl = s.use_pdl, tiled = s.nlevels >= 2;
+    const uint32_t nrz = tiled ? tg : g;
     k_spmv_dot<<<g, kSegBlock, 0, st>>>(B, s.search, s.ap, s.ctl, part_sap(s), mode,
-                                         static_cast<const float2*>(part_rz(s)), g);
+                                         static_cast<const float2*>(part_rz(s)), nrz);
     if (mode == APIC_SOLVER_REFERENCE)
         launch(pdl, k_delta_exact, div_up(B.cells, kDeltaChunk), kDeltaThreads, 0, st, B,
                static_cast<const float*>(s.search), static_cast<const float*>(s.ap),
                static_cast<const uint32_t*>(s.seg_pre), s.ctl, s.exact_parts);
-    launch(pdl, k_pcg_update, g, kSegBlock, 0, st, B, x, p_padded, s.search, s.ap, s.ctl,
-           static_cast<const float2*>(part_sap(s)), g, part_res(s), mode, static_cast<const float*>(s.exact_parts),
-           static_cast<const uint32_t*>(s.seg_pre), static_cast<const float2*>(part_rz(s)), g);
-    // the residual's exit test runs inside the V-cycle's first kernel when
-    // that is the base level's black sweep, else on its own
-    const bool exit_in_vcycle = s.nlevels >= 2;
-    if (!exit_in_vcycle)
-        launch(pdl, k_residual_exit, 1, kSegBlock, 0, st, s.ctl, static_cast<const float4*>(part_res(s)), g, mode,
-               s.props.solve_error, s.pcg_h, s.pcg_cap, s.pcg_dyn_cap, s.pcg_set_cond ? 1 : 0);
-    // the V-cycle's last kernel also stores the parts of r.z (k_dot_rz's work)
-    if (!enqueue_vcycle(s, true, mode, exit_in_vcycle)) launch(pdl, k_dot_rz, g, kSegBlock, 0, st, B, s.ctl, part_rz(s));
+    const StepArgs a{part_sap(s), g, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
+    if (tiled) {
+        launch(pdl, k_update_down, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
+               static_cast<const float*>(s.ap), s.ctl, a, part_res(s), vcycle_wants_red(s, 1) ? 1 : 0);
+        // the V-cycle's next kernel runs the residual's exit test, its last
+        // one stores the parts of r.z
+        enqueue_vcycle(s, true, exit_args(s, mode));
+    } else {
+        launch(pdl, k_pcg_update, g, kSegBlock, 0, st, B, x, p_padded, s.search, static_cast<const float*>(s.ap),
+               s.ctl, a, part_res(s));
+        launch(pdl, k_residual_exit, 1, kSegBlock, 0, st, s.ctl, exit_args(s, mode));
+        enqueue_vcycle(s, true);
+        launch(pdl, k_dot_rz, g, kSegBlock, 0, st, B, s.ctl, part_rz(s));
+    }
     if (mode == APIC_SOLVER_REFERENCE)
         launch(pdl, k_gamma_exact, 1, kGammaThreads, kGammaSmem, st, B, s.ctl, 0, s.pcg_h, s.pcg_cap, s.pcg_dyn_cap,
                s.pcg_set_cond ? 1 : 0);

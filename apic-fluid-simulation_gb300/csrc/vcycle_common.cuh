@@ -611,104 +611,6 @@ __device__ __forceinline__ void ph_smooth(const Level& L, uint32_t nseg, uint32_
     }
 }
 
-// Restriction into coarse level c; with_red also runs c's first (red) sweep.
-__device__ __forceinline__ void ph_restrict(const Level& f, const Level& c, uint32_t nseg_c, uint32_t warp,
-                                            uint32_t nwarps, bool with_red, uint32_t w0 = kNoWord) {
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t s = warp, nxt = seg_first(c.seg, nseg_c, warp, w0); s < nseg_c; s += nwarps) {
-        const uint32_t word = nxt;
-        nxt = seg_next(c.seg, nseg_c, s + nwarps);
-        const uint32_t rc = word * 32 + lane;
-        if (rc >= c.cells) continue;
-        const bool fluid = (c.fluid[word] >> lane) & 1u;
-        const uint32_t cp = rc + c.w;
-        uint32_t cx, cy;
-        raw_xy(rc, c.w, c.wshift, cx, cy);
-        const float r = restrict_cell_all(f.fluid, f.w, f.cells, f.diag, f.px, f.py, f.res, f.err, cx, cy);
-        const float inv = c.inv_diag[cp];
-        if (!fluid) continue;
-        c.res[cp] = r;
-        if (with_red && ((cx + cy) & 1u) == 0u) c.err[cp] = inv != 0.0f ? 0.0f + (kOmega * (r * inv - 0.0f)) : 0.0f;
-    }
-}
-
-// Prolongation from c fused with f's reverse sweep of one colour: black (1)
-// reads red neighbours as prolonged values, red (0) reads final black ones.
-// last / extra: the base level's duplicated last fluid cell (else ~0u / 0).
-__device__ __forceinline__ void ph_prolong(const Level& c, const Level& f, uint32_t nseg_f, uint32_t warp,
-                                           uint32_t nwarps, int color, uint32_t last, uint32_t extra,
-                                           uint32_t w0 = kNoWord) {
-    const uint32_t lane = threadIdx.x & 31;
-    const float* fe = f.err;
-    const float* ce = c.err;
-    const uint32_t fw = f.w, cw = c.w;
-    const long long fcells = f.cells;
-    const int fs = f.wshift;
-    // coarse error under fine raw index rf; rf outside the grid (a neighbour
-    // whose value a select drops) is clamped so the load stays in bounds
-    auto coarse_e = [=](long long rf) {
-        const uint32_t r = uint32_t(rf < 0 ? 0 : (rf >= fcells ? fcells - 1 : rf));
-        uint32_t x, y;
-        raw_xy(r, fw, fs, x, y);
-        return ce[(y >> 1) * cw + (x >> 1) + cw];
-    };
-    for (uint32_t s = warp, nxt = seg_first(f.seg, nseg_f, warp, w0); s < nseg_f; s += nwarps) {
-        const uint32_t word = nxt;
-        nxt = seg_next(f.seg, nseg_f, s + nwarps);
-        const uint32_t raw = word * 32 + lane;
-        if (raw >= f.cells || int(!red_at(raw, fw, fs)) != color) continue;
-        const bool fluid = (f.fluid[word] >> lane) & 1u;
-        const uint32_t p = raw + fw;
-        const float old = prolonged(fe[p], coarse_e(raw), p == last ? extra : 0u);
-        float v;
-        if (color == 1)
-            v = sor_cell_all(f.fluid, fw, f.cells, f.inv_diag, f.px, f.py, f.res, raw, p, old, true,
-                             [=](uint32_t q, long long rq) {
-                                 return prolonged(fe[q], coarse_e(rq), q == last ? extra : 0u);
-                             });
-        else
-            v = sor_cell_all(f.fluid, fw, f.cells, f.inv_diag, f.px, f.py, f.res, raw, p, old, true,
-                             [fe](uint32_t q, long long) { return fe[q]; });
-        if (fluid) f.err[p] = v;
-    }
-}
-
-// ph_prolong's red pass on the base level, also returning this thread's share
-// of r.z over every fluid cell: red cells' new z, black cells' z as the
-// black pass left it (final).  The products are those of pcg::ph_rz.
-__device__ __forceinline__ F2 ph_prolong_red_rz(const Level& c, const Level& f, uint32_t nseg_f, uint32_t warp,
-                                                uint32_t nwarps, uint32_t last, uint32_t extra,
-                                                uint32_t w0 = kNoWord) {
-    const uint32_t lane = threadIdx.x & 31;
-    const float* fe = f.err;
-    const float* ce = c.err;
-    const uint32_t fw = f.w, cw = c.w;
-    F2 acc{0.0f, 0.0f};
-    for (uint32_t s = warp, nxt = seg_first(f.seg, nseg_f, warp, w0); s < nseg_f; s += nwarps) {
-        const uint32_t word = nxt;
-        nxt = seg_next(f.seg, nseg_f, s + nwarps);
-        const uint32_t raw = word * 32 + lane;
-        if (raw >= f.cells) continue;
-        const bool fluid = (f.fluid[word] >> lane) & 1u;
-        const uint32_t p = raw + fw;
-        float z;
-        uint32_t x, y;
-        raw_xy(raw, fw, f.wshift, x, y);
-        if (((x + y) & 1u) == 0u) {
-            const float ec = ce[(y >> 1) * cw + (x >> 1) + cw];
-            const float old = prolonged(fe[p], ec, p == last ? extra : 0u);
-            z = sor_cell_all(f.fluid, fw, f.cells, f.inv_diag, f.px, f.py, f.res, raw, p, old, true,
-                             [fe](uint32_t q, long long) { return fe[q]; });
-            if (fluid) f.err[p] = z;
-        } else {
-            z = fe[p];
-        }
-        const float rz = f.res[p] * z;
-        if (fluid) acc = f2_add(acc, rz);
-    }
-    return acc;
-}
-
 // Asynchronous 4-byte copy global -> shared (cp.async, sm_80+): the copies
 // of a whole array set are issued back to back and complete together at
 // cp_async_wait_all, so loading costs about one L2 round trip instead of one

@@ -22,6 +22,7 @@
 
 #include "apic_device.cuh"
 #include "apic_internal.h"
+#include "pcg_common.cuh"
 #include "vcycle_common.cuh"
 
 namespace apic {
@@ -295,7 +296,7 @@ __device__ __forceinline__ void dsm_load_first(const DsmParams& p, uint8_t* sm, 
 }
 
 __global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_dsm(DsmParams p, TailParams tp, uint32_t dsm_off,
-                                                               uint32_t dsm_bytes, const Ctl* ctl) {
+                                                               uint32_t dsm_bytes, Ctl* ctl, ExitArgs exit) {
     extern __shared__ __align__(16) uint8_t smem[];
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t rank = cl.block_rank();
@@ -321,6 +322,12 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_dsm(DsmParams p, Tai
         return;
     }
     dsm_load_first(p, dsm, rank);
+    // the exit test where this is the first kernel after the update: every CTA
+    // comes to the same verdict (one that finds it recorded returns above)
+    if (exit.on && pcg::exit_verdict(ctl, exit, rank == 0)) {
+        cp_async_wait_all();
+        return;
+    }
     cp_async_wait_all();
     __syncthreads();
     cl.sync();
@@ -440,8 +447,8 @@ void plan_vcycle_dsm(Scene& s) {
 
 // Levels dsm_first .. dsm_tail-1 and the tail in one cluster launch.  On
 // entry dsm_first's residual and first red sweep are in global memory
-// (k_restrict_red); on exit its final error is.
-void launch_vcycle_dsm(Scene& s, cudaStream_t st) {
+// (the down kernel above it); on exit its final error is.
+void launch_vcycle_dsm(Scene& s, cudaStream_t st, const ExitArgs& exit) {
     DsmParams p = {};
     p.first = s.dsm_first;
     p.n = s.dsm_tail - s.dsm_first;
@@ -487,7 +494,7 @@ void launch_vcycle_dsm(Scene& s, cudaStream_t st) {
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = dsm_config(s.dsm_smem, st, attr, s.use_pdl);
     cudaLaunchKernelEx(&cfg, k_vcycle_dsm, p, tp, s.dsm_off, uint32_t(s.dsm_smem - s.dsm_off),
-                       static_cast<const Ctl*>(s.ctl));
+                       s.ctl, exit);
 }
 
 }  // namespace apic
