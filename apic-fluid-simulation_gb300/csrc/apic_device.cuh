@@ -408,11 +408,13 @@ __device__ __forceinline__ void block_store(Blk bk, F2 v, float mx, float4* part
     }
 }
 
-// Total of n partials, returned to every thread of the block.
+// Total of n partials, rounded to FP32 (by one thread: an FP64 conversion by
+// every warp of a full SM takes half a microsecond at GB300's FP64 rate),
+// returned to every thread of the block.
 template <int kThreads>
-__device__ __forceinline__ double sum_partials(const float2* part, uint32_t n) {
+__device__ __forceinline__ float sum_partials(const float2* part, uint32_t n) {
     __shared__ F2 s_sp[kThreads / 32];
-    __shared__ double s_tot;
+    __shared__ float s_tot;
     F2 t{0.0f, 0.0f};
 #pragma unroll 4
     for (uint32_t b = threadIdx.x; b < n; b += kThreads) {
@@ -426,7 +428,7 @@ __device__ __forceinline__ double sum_partials(const float2* part, uint32_t n) {
     if (threadIdx.x == 0) {
         F2 a{0.0f, 0.0f};
         for (int w = 0; w < kThreads / 32; ++w) a = f2_add(a, s_sp[w]);
-        s_tot = f2_value(a);
+        s_tot = float(f2_value(a));
     }
     __syncthreads();
     return s_tot;
@@ -434,13 +436,11 @@ __device__ __forceinline__ double sum_partials(const float2* part, uint32_t n) {
 
 // Sum and maximum of n float4 partials (x, y: F2 sum; z: maximum), by the
 // first kThreads threads of a block of at least that many (the order of the
-// sum does not depend on the block's size).
+// sum does not depend on the block's size); thread 0 receives them.
 template <int kThreads>
 __device__ __forceinline__ void sum_max_partials(const float4* part, uint32_t n, double* sum, float* mx) {
     __shared__ F2 s_sp[kThreads / 32];
     __shared__ float s_mp[kThreads / 32];
-    __shared__ double s_tot;
-    __shared__ float s_max;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < kThreads / 32) {
         F2 t{0.0f, 0.0f};
@@ -466,12 +466,9 @@ __device__ __forceinline__ void sum_max_partials(const float4* part, uint32_t n,
             a = f2_add(a, s_sp[w]);
             b = fmaxf(b, s_mp[w]);
         }
-        s_tot = f2_value(a);
-        s_max = b;
+        *sum = f2_value(a);
+        *mx = b;
     }
-    __syncthreads();
-    *sum = s_tot;
-    *mx = s_max;
 }
 
 // Same pattern for a maximum of non-negative values (exact in any order).

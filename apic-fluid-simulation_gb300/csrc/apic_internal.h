@@ -347,6 +347,7 @@ cudaError_t launch_post_forces(Scene& s);
 cudaError_t launch_extrapolate(Scene& s);
 cudaError_t launch_smoothed_view(Scene& s, float* out);
 cudaError_t launch_level_lists(Scene& s, int level);
+cudaError_t launch_mask_level(Scene& s, int level);  // zero a coarse level's coefficients outside its fluid
 cudaError_t launch_tile_lists(Scene& s);  // every level's fluid tiles
 // solver.cu: the solve is recorded into graphs (apic_graph.h: build_solve)
 // solver.cu: the same solve launched kernel by kernel with host loop control
@@ -354,9 +355,6 @@ cudaError_t launch_tile_lists(Scene& s);  // every level's fluid tiles
 cudaError_t run_solve_eager(Scene& s);
 // vcycle.cu
 void plan_vcycle(Scene& s);     // pick the coarse levels that run in one CTA / one cluster
-// level l takes its first red sweep from the kernel that restricts into it
-// (the cluster's first level; the tile kernels form it themselves)
-bool vcycle_wants_red(const Scene& s, int l);
 // vcycle_dsm.cu
 void plan_vcycle_dsm(Scene& s);
 void launch_vcycle_dsm(Scene& s, cudaStream_t st, const ExitArgs& exit);

@@ -326,7 +326,17 @@ __device__ __forceinline__ void coarsen_word(const Level& f, const Level& c, uin
     }
     const uint32_t ballot = __ballot_sync(0xffffffffu, on);
     if (lane == 0) c.fluid[word] = ballot;
-    if (!on) return;
+    if (!on) {
+        // zero coefficients outside the fluid: the V-cycle's shared-memory
+        // levels run over all their cells (vcycle_common.cuh)
+        if (raw < c.cells) {
+            c.diag[raw + c.w] = 0.0f;
+            c.inv_diag[raw + c.w] = 0.0f;
+            c.px[raw + c.w] = 0.0f;
+            c.py[raw + c.w] = 0.0f;
+        }
+        return;
+    }
     float diag = 0.0f, px = 0.0f, py = 0.0f;
     for (uint32_t dy = 0; dy < 2; ++dy)
         for (uint32_t dx = 0; dx < 2; ++dx) {
@@ -347,6 +357,17 @@ __device__ __forceinline__ void coarsen_word(const Level& f, const Level& c, uin
     c.inv_diag[cp] = fd > 1e-6f ? 1.0f / fd : 0.0f;
     c.px[cp] = px * 0.5f;
     c.py[cp] = py * 0.5f;
+}
+
+// The same zeros on a coarse level whose mask or coefficients a caller wrote
+// (padding included).
+__global__ void __launch_bounds__(256) k_mask_level(Level c) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.padded || fluid_raw(c.fluid, (long long)i - c.w, c.cells)) return;
+    c.diag[i] = 0.0f;
+    c.inv_diag[i] = 0.0f;
+    c.px[i] = 0.0f;
+    c.py[i] = 0.0f;
 }
 
 // One coarse level from its finer level: one warp per coarse mask word.
@@ -645,6 +666,10 @@ static cudaError_t compact_level(Scene& s, int level, const uint32_t* obstacle) 
     return cudaGetLastError();
 }
 
+cudaError_t launch_mask_level(Scene& s, int level) {
+    k_mask_level<<<div_up(s.lv[level].padded, 256), 256, 0, s.stream>>>(s.lv[level]);
+    return cudaGetLastError();
+}
 // Every level that the V-cycle's tile kernels may work on (those with a
 // coarser one).
 cudaError_t launch_tile_lists(Scene& s) {

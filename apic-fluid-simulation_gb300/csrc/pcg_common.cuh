@@ -205,21 +205,26 @@ __device__ __forceinline__ const float* cur_res(const Level& B, const Ctl* ctl) 
 // CTA): each sums the parts itself, to the same verdict, and `writer`'s
 // thread 0 records it.  True: the solve is done.
 __device__ __forceinline__ bool exit_verdict(Ctl* ctl, const ExitArgs& a, bool writer) {
+    __shared__ bool s_done;
     double tot;
     float t;
     sum_max_partials<kSegBlock>(a.part, a.nparts, &tot, &t);
-    const double rel = ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0;
-    const bool stop = ctl->delta_stop != 0;
-    const bool done =
-        stop || (a.mode == APIC_SOLVER_REFERENCE ? t < a.solve_error : rel <= ctl->target_rel);
-    if (writer && threadIdx.x == 0) {
-        if (stop) ctl->res_sel ^= 1u;  // the update left the residual where it was
-        else if (a.mode == APIC_SOLVER_REFERENCE) ctl->max_r_bits = __float_as_uint(t);
-        else ctl->rnorm2 = tot;
-        if (done) ctl->pcg_done = 1;
-        loop_decision(ctl, a.mode, a.h, a.cap, a.dyn_cap, a.set_cond);
+    if (threadIdx.x == 0) {
+        const bool stop = ctl->delta_stop != 0;
+        bool done = stop;
+        if (!stop && a.mode == APIC_SOLVER_REFERENCE) done = t < a.solve_error;
+        else if (!stop) done = (ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0) <= ctl->target_rel;
+        s_done = done;
+        if (writer) {
+            if (stop) ctl->res_sel ^= 1u;  // the update left the residual where it was
+            else if (a.mode == APIC_SOLVER_REFERENCE) ctl->max_r_bits = __float_as_uint(t);
+            else ctl->rnorm2 = tot;
+            if (done) ctl->pcg_done = 1;
+            loop_decision(ctl, a.mode, a.h, a.cap, a.dyn_cap, a.set_cond);
+        }
     }
-    return done;
+    __syncthreads();
+    return s_done;
 }
 
 // r.z after the preconditioner (:1936).

@@ -1184,9 +1184,13 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
         CK(launch_tile_lists(s));
         CK(cudaStreamSynchronize(s.stream));
     }
-    if (field >= APIC_F_MG_FLUID_BITS && field % APIC_F_MG_LEVEL_STRIDE == APIC_F_MG_FLUID_BITS) {
-        CK(launch_level_lists(s, field / APIC_F_MG_LEVEL_STRIDE + 1));
-        CK(launch_tile_lists(s));
+    if (field >= APIC_F_MG_FLUID_BITS) {
+        const int level = field / APIC_F_MG_LEVEL_STRIDE + 1;
+        CK(launch_mask_level(s, level));
+        if (field % APIC_F_MG_LEVEL_STRIDE == APIC_F_MG_FLUID_BITS) {
+            CK(launch_level_lists(s, level));
+            CK(launch_tile_lists(s));
+        }
         CK(cudaStreamSynchronize(s.stream));
     }
     if (field == APIC_F_EXT_FORCE_U || field == APIC_F_EXT_FORCE_V) s.has_ext = true;

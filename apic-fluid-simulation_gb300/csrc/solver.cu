@@ -104,7 +104,7 @@ __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nse
     float beta = ctl->beta;
     const bool bv = ctl->beta_valid != 0;
     if (mode != APIC_SOLVER_REFERENCE && bv) {
-        const float ng = rz_sum ? *rz_sum : float(sum_partials<kSegBlock>(rz, nrz));
+        const float ng = rz_sum ? *rz_sum : sum_partials<kSegBlock>(rz, nrz);
         if (!(ng != 0.0f)) return;
         beta = ng / ctl->gamma;
         if (bk.id == 0 && threadIdx.x == 0) ctl->beta = beta;
@@ -145,7 +145,7 @@ __device__ __forceinline__ bool pcg_alpha(Blk bk, Ctl* ctl, const StepArgs& a, f
     // previous iteration's r.z parts, which k_spmv_dot summed the same way
     float gamma = ctl->gamma;
     if (a.mode != APIC_SOLVER_REFERENCE && ctl->beta_valid) {
-        gamma = rz_sum ? *rz_sum : float(sum_partials<kSegBlock>(a.rz, a.nrz));
+        gamma = rz_sum ? *rz_sum : sum_partials<kSegBlock>(a.rz, a.nrz);
         if (!(gamma != 0.0f)) {
             if (bk.id == 0 && threadIdx.x == 0) ctl->pcg_done = 1;
             return false;
@@ -158,7 +158,7 @@ __device__ __forceinline__ bool pcg_alpha(Blk bk, Ctl* ctl, const StepArgs& a, f
         delta = 0.0f;
         for (uint32_t c = 0; c < nchunks; ++c) delta = delta + a.exact_parts[c];
     } else {
-        delta = sap_sum ? *sap_sum : float(sum_partials<kSegBlock>(a.sap, a.nsap));
+        delta = sap_sum ? *sap_sum : sum_partials<kSegBlock>(a.sap, a.nsap);
     }
     const bool stop = a.mode == APIC_SOLVER_REFERENCE ? fabsf(delta) < kSafety : (!(delta != 0.0f) || !isfinite(delta));
     const float alpha = gamma / delta;
@@ -188,7 +188,7 @@ __device__ __forceinline__ tile::Update update_args(const Level& B, const Ctl* c
 __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Level& C, tile::Shared& sh,
                                                tile::DownRegs& g, uint32_t count, uint32_t id, float* p, int p_padded,
                                                float* s, const float* ap, Ctl* ctl, const StepArgs& a, float4* part,
-                                               bool with_red, const float* rz_sum = nullptr,
+                                               const float* rz_sum = nullptr,
                                                const float* sap_sum = nullptr) {
     if (ctl->pcg_done) return;
     const tile::Update u = update_args(B, ctl, p, p_padded, s, ap);
@@ -206,20 +206,19 @@ __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Lev
             tile::down_load_const(B, id, g);
             tile::down_load<true>(B, u.res, u, g);
         }
-        tile::down_tile<true>(sh, B, C, id, g, u, alpha, beta, beta_valid, with_red, &acc, &mx);
+        tile::down_tile<true>(sh, B, C, id, g, u, alpha, beta, beta_valid, &acc, &mx);
     }
     block_store<kSegBlock>(bk, acc, mx, part);
 }
 __global__ void __launch_bounds__(kTileBlock, 4) k_update_down(Level B, Level C, float* p, int p_padded, float* s,
-                                                                 const float* ap, Ctl* ctl, StepArgs a, float4* part,
-                                                                 int with_red) {
+                                                                 const float* ap, Ctl* ctl, StepArgs a, float4* part) {
     __shared__ tile::Shared sh;
     const uint32_t count = ctl->tile_count[0];
     const uint32_t id = blockIdx.x < count ? B.tiles[blockIdx.x] : 0u;
     tile::DownRegs g;
     if (blockIdx.x < count) tile::down_load_const(B, id, g);
     pdl_wait();
-    kb_update_down(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part, with_red != 0);
+    kb_update_down(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part);
 }
 
 // The update alone, and the base level's first red sweep (grids without a
@@ -648,7 +647,7 @@ __global__ void __launch_bounds__(kSegBlock) k_bat_round_end(const BScene* __res
     const BScene& S = tab[blockIdx.x - 1];
     Ctl* ctl = S.ctl;
     if (!bat_gate(ctl, kGatePcg) || ctl->pcg_done) return;
-    const float rz = float(sum_partials<kSegBlock>(bs_part_rz(S), busy_tile_blocks(S)));
+    const float rz = sum_partials<kSegBlock>(bs_part_rz(S), busy_tile_blocks(S));
     if (threadIdx.x == 0) ctl->b_rz = rz;
 }
 
@@ -658,7 +657,7 @@ __global__ void __launch_bounds__(kSegBlock) k_bat_sap(const BScene* __restrict_
     const BScene& S = tab[blockIdx.x];
     Ctl* ctl = S.ctl;
     if (!bat_gate(ctl, kGatePcg) || ctl->pcg_done) return;
-    const float sap = float(sum_partials<kSegBlock>(bs_part_sap(S), busy_blocks(S)));
+    const float sap = sum_partials<kSegBlock>(bs_part_sap(S), busy_blocks(S));
     if (threadIdx.x == 0) ctl->b_sap = sap;
 }
 
@@ -725,7 +724,7 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_update_down(const BScene*
             const uint32_t id = b < count ? S.lv[0].tiles[b] : 0u;
             if (b < count) tile::down_load_const(S.lv[0], id, g);
             kb_update_down(Blk{b, S.tgrid}, S.lv[0], S.lv[1], sh, g, count, id, into_corr ? S.corr : S.pressure,
-                           into_corr, S.search, S.ap, ctl, a, bs_part_res(S), false, &ctl->b_rz, &ctl->b_sap);
+                           into_corr, S.search, S.ap, ctl, a, bs_part_res(S), &ctl->b_rz, &ctl->b_sap);
             __syncthreads();
         }
     });
@@ -860,7 +859,7 @@ static void pcg_iteration(Scene& s, int mode, float* x, int p_padded) {
     const StepArgs a{part_sap(s), g, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
     if (tiled) {
         launch(pdl, k_update_down, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
-               static_cast<const float*>(s.ap), s.ctl, a, part_res(s), vcycle_wants_red(s, 1) ? 1 : 0);
+               static_cast<const float*>(s.ap), s.ctl, a, part_res(s));
         // the V-cycle's next kernel runs the residual's exit test, its last
         // one stores the parts of r.z
         enqueue_vcycle(s, true, exit_args(s, mode));

@@ -153,13 +153,13 @@ __device__ __forceinline__ void down_load(const Level& f, const float* res, cons
     }
 }
 
-// Red sweep from zero error, black sweep, restriction into c; with_red: also
-// c's first red sweep.  kUpdate: first r = fma(-alpha, Ap, r), x += alpha s',
+// Red sweep from zero error, black sweep, restriction into c (whose first red
+// sweep is formed where its residual is read).  kUpdate: first r = fma(-alpha, Ap, r), x += alpha s',
 // s = s', and this thread's part of sum r^2 and max |r|.
 template <bool kUpdate>
 __device__ __forceinline__ void down_tile(Shared& t, const Level& f, const Level& c, uint32_t id, const DownRegs& g,
-                                          const Update& u, float alpha, float beta, bool beta_valid, bool with_red,
-                                          F2* acc, float* mx) {
+                                          const Update& u, float alpha, float beta, bool beta_valid, F2* acc,
+                                          float* mx) {
     int x0, y0;
     tile_origin(f, id, x0, y0);
     float r[kPer];
@@ -171,7 +171,7 @@ __device__ __forceinline__ void down_tile(Shared& t, const Level& f, const Level
         t.r[idx] = r[i];
         t.px[idx] = g.q[i].px;
         t.py[idx] = g.q[i].py;
-        t.e[idx] = (g.q[i].red && g.q[i].inv != 0.0f) ? 0.0f + (vc::kOmega * (r[i] * g.q[i].inv - 0.0f)) : 0.0f;
+        t.e[idx] = g.q[i].red ? vc::red_first(r[i], g.q[i].inv) : 0.0f;
     }
     __syncthreads();
 #pragma unroll
@@ -227,10 +227,6 @@ __device__ __forceinline__ void down_tile(Shared& t, const Level& f, const Level
         const uint32_t cx = uint32_t(x0 >> 1) + (threadIdx.x & 15u), cy = uint32_t(y0 >> 1) + (threadIdx.x >> 5);
         const uint32_t cp = cy * c.w + cx + c.w;
         c.res[cp] = sum;
-        if (with_red && ((cx + cy) & 1u) == 0u) {
-            const float inv = c.inv_diag[cp];
-            c.err[cp] = inv != 0.0f ? 0.0f + (vc::kOmega * (sum * inv - 0.0f)) : 0.0f;
-        }
     }
 }
 

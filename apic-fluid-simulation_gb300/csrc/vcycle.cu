@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kSegBlock) k_smooth(Level L, int li, const Ctl
 // update's exit test and the loop's decision, in an extra block beside the
 // sweeps; later kernels see its verdict.
 __device__ __forceinline__ void kb_down(Blk bk, const Level& f, const Level& c, tile::Shared& sh, tile::DownRegs& g,
-                                        uint32_t id, uint32_t end, const float* res, bool with_red) {
+                                        uint32_t id, uint32_t end, const float* res) {
     const tile::Update none{};
     for (uint32_t i = bk.id; i < end; i += bk.n) {
         if (i != bk.id) {
@@ -73,11 +73,10 @@ __device__ __forceinline__ void kb_down(Blk bk, const Level& f, const Level& c, 
             tile::down_load_const(f, id, g);
         }
         tile::down_load<false>(f, res, none, g);
-        tile::down_tile<false>(sh, f, c, id, g, none, 0.0f, 0.0f, false, with_red, nullptr, nullptr);
+        tile::down_tile<false>(sh, f, c, id, g, none, 0.0f, 0.0f, false, nullptr, nullptr);
     }
 }
-__global__ void __launch_bounds__(kTileBlock, 4) k_down(Level f, Level c, int lf, Ctl* ctl, int with_red,
-                                                          ExitArgs exit) {
+__global__ void __launch_bounds__(kTileBlock, 4) k_down(Level f, Level c, int lf, Ctl* ctl, ExitArgs exit) {
     __shared__ tile::Shared sh;
     const uint32_t extra = exit.on ? 1u : 0u;
     if (exit.on && blockIdx.x == 0) {
@@ -94,7 +93,7 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_down(Level f, Level c, int lf
     if (bk.id < count) tile::down_load_const(f, id, g);
     pdl_wait();
     if (ctl->pcg_done) return;
-    kb_down(bk, f, c, sh, g, id, count, lf == 0 ? pcg::cur_res(f, ctl) : f.res, with_red != 0);
+    kb_down(bk, f, c, sh, g, id, count, lf == 0 ? pcg::cur_res(f, ctl) : f.res);
 }
 
 // The prolongation from c and level f's black and red sweeps; kRz: the base
@@ -168,12 +167,16 @@ __global__ void __launch_bounds__(kTailThreads) k_coarse_solve(Level L, float* _
     cta_coarse_cg(A, exact != 0);
 }
 
-__global__ void __launch_bounds__(kTailThreads) k_vcycle_tail(TailParams tp, Ctl* ctl, ExitArgs exit) {
-    pdl_wait();
-    if (ctl->pcg_done) return;
-    if (exit.on && pcg::exit_verdict(ctl, exit, true)) return;
+__global__ void __launch_bounds__(kTailThreads) k_vcycle_tail(const __grid_constant__ TailParams tp, Ctl* ctl,
+                                                              ExitArgs exit) {
     extern __shared__ uint32_t sm[];
-    cta_tail(tp, sm, true);
+    cta_tail_issue_coeffs(tp, sm);  // while the previous kernel drains
+    pdl_wait();
+    if (ctl->pcg_done || (exit.on && pcg::exit_verdict(ctl, exit, true))) {
+        cp_async_wait_all();
+        return;
+    }
+    cta_tail(tp, sm);
 }
 
 size_t tail_level_bytes(const Level& L) { return 4ull * (L.words + 6ull * L.padded); }
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_down(const BScene* __rest
         tile::DownRegs g;
         tile::down_load_const(S.lv[lf], id, g);
         kb_down(Blk{i0, 1u}, S.lv[lf], S.lv[lf + 1], sh, g, id, end,
-                lf == 0 ? pcg::cur_res(S.lv[0], ctl) : S.lv[lf].res, false);
+                lf == 0 ? pcg::cur_res(S.lv[0], ctl) : S.lv[lf].res);
     });
 }
 
@@ -255,7 +258,8 @@ __global__ void __launch_bounds__(kTailThreads) k_bat_tail(const BScene* __restr
         uint32_t* dst = reinterpret_cast<uint32_t*>(&s_tp);
         for (uint32_t i = threadIdx.x; i < sizeof(TailParams) / 4; i += blockDim.x) dst[i] = src[i];
         __syncthreads();
-        cta_tail(s_tp, sm, true);
+        cta_tail_issue_coeffs(s_tp, sm);
+        cta_tail(s_tp, sm);
         __syncthreads();
     }
 }
@@ -304,11 +308,6 @@ void plan_vcycle(Scene& s) {
     plan_vcycle_dsm(s);
 }
 
-bool vcycle_wants_red(const Scene& s, int l) {
-    const bool dsm = s.use_dsm && s.dsm_first < s.dsm_tail && s.dsm_tail < s.nlevels;
-    return dsm && l == s.dsm_first;
-}
-
 // One V-cycle on s.stream: z = M^-1 r in lv[0].err.  Two kernels per level
 // (k_down, k_up) above the levels that the distributed-shared-memory cluster
 // or the shared-memory tail holds, or above the coarsest level's CG.
@@ -328,8 +327,7 @@ void enqueue_vcycle(Scene& s, bool base_done, const ExitArgs& exit_in) {
     const bool dsm = s.use_dsm && s.dsm_first < s.dsm_tail && s.dsm_tail < s.nlevels;
     ExitArgs exit = exit_in;
     auto down = [&](int l) {
-        launch(pdl, k_down, tile_grid(L[l]) + (exit.on ? 1u : 0u), kTileBlock, 0, st, L[l], L[l + 1], l, s.ctl,
-               vcycle_wants_red(s, l + 1) ? 1 : 0, exit);
+        launch(pdl, k_down, tile_grid(L[l]) + (exit.on ? 1u : 0u), kTileBlock, 0, st, L[l], L[l + 1], l, s.ctl, exit);
         exit.on = 0;
     };
     if (!base_done) down(0);

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include "apic_device.cuh"
 #include "apic_internal.h"
 
@@ -22,63 +24,11 @@ constexpr size_t kTailSmemBudget = 200 * 1024;
 // ---- per-cell arithmetic shared by the global and the shared-memory kernels
 
 // One SOR update (src/apic.rs:487-507) of padded cell c with raw index raw.
-// nb(padded, raw) returns a neighbour's current error; neighbours that are not
-// fluid are skipped (their reference contribution is zero).
-template <class NB>
-__device__ __forceinline__ float sor_cell(const uint32_t* bits, uint32_t w, uint32_t cells, const float* inv_d,
-                                          const float* px, const float* py, const float* res, long long raw,
-                                          uint32_t c, float old, bool neighbours, NB nb) {
-    float inv = inv_d[c];
-    if (inv == 0.0f) return old;
-    float sum = res[c];
-    if (neighbours) {
-        const long long W = w;
-        if (fluid_raw(bits, raw + 1, cells)) sum = __fmaf_rn(-px[c], nb(c + 1, raw + 1), sum);
-        if (fluid_raw(bits, raw + W, cells)) sum = __fmaf_rn(-py[c], nb(c + w, raw + W), sum);
-        if (fluid_raw(bits, raw - 1, cells)) sum = __fmaf_rn(-px[c - 1], nb(c - 1, raw - 1), sum);
-        if (fluid_raw(bits, raw - W, cells)) sum = __fmaf_rn(-py[c - w], nb(c - w, raw - W), sum);
-    }
-    float gs = sum * inv;
-    return old + (kOmega * (gs - old));
-}
-
-// Coarse residual of coarse cell (cx, cy) from its fine children (:549-583).
-// E(padded, raw) gives the fine error of a fluid cell.
-template <class E>
-__device__ __forceinline__ float restrict_cell_fn(const uint32_t* fb, uint32_t fw, uint32_t fcells, const float* fd,
-                                                  const float* fpx, const float* fpy, const float* fr, E fe,
-                                                  uint32_t cx, uint32_t cy) {
-    float sum = 0.0f;
-    const long long W = fw;
-    for (uint32_t dy = 0; dy < 2; ++dy)
-        for (uint32_t dx = 0; dx < 2; ++dx) {
-            long long rf = (long long)(cy * 2 + dy) * fw + (cx * 2 + dx);
-            if (!fluid_raw(fb, rf, fcells)) continue;
-            uint32_t pf = uint32_t(rf) + fw;
-            float b = fr[pf];
-            float ax = fd[pf] * fe(pf, rf);
-            if (fluid_raw(fb, rf + 1, fcells)) ax += fpx[pf] * fe(pf + 1, rf + 1);
-            if (fluid_raw(fb, rf + W, fcells)) ax += fpy[pf] * fe(pf + fw, rf + W);
-            if (fluid_raw(fb, rf - 1, fcells)) ax += fpx[pf - 1] * fe(pf - 1, rf - 1);
-            if (fluid_raw(fb, rf - W, fcells)) ax += fpy[pf - fw] * fe(pf - fw, rf - W);
-            sum += b - ax;
-        }
-    return sum;
-}
-
-__device__ __forceinline__ float restrict_cell(const uint32_t* fb, uint32_t fw, uint32_t fcells, const float* fd,
-                                               const float* fpx, const float* fpy, const float* fr, const float* fe,
-                                               uint32_t cx, uint32_t cy) {
-    return restrict_cell_fn(fb, fw, fcells, fd, fpx, fpy, fr, [fe](uint32_t p, long long) { return fe[p]; }, cx, cy);
-}
-
-// Branch-free forms of sor_cell / restrict_cell for the sweeps whose
-// neighbour values are plain loads.  Every load is issued up front, without
-// waiting for the fluid tests: all neighbours of a cell with raw index in
-// [0, cells) have padded indices inside [0, cells + 2w), the extent of every
-// level array.  Non-fluid neighbours (and children) are then dropped by
-// selects, which yields the same floats as skipping them.  nb / fe must be
-// safe to call for any such neighbour.
+// Every load is issued up front, without waiting for the fluid tests: all
+// neighbours of a cell with raw index in [0, cells) have padded indices
+// inside [0, cells + 2w), the extent of every level array.  Non-fluid
+// neighbours are then dropped by selects, which yields the same floats as
+// skipping them.  nb must be safe to call for any such neighbour.
 template <class NB>
 __device__ __forceinline__ float sor_cell_all(const uint32_t* bits, uint32_t w, uint32_t cells, const float* inv_d,
                                               const float* px, const float* py, const float* res, long long raw,
@@ -104,38 +54,6 @@ __device__ __forceinline__ float sor_cell_all(const uint32_t* bits, uint32_t w, 
     const float nv = old + (kOmega * (gs - old));
     return inv == 0.0f ? old : nv;
 }
-
-// Coarse residual of coarse cell (cx, cy) (any cell of the coarse grid).
-__device__ __forceinline__ float restrict_cell_all(const uint32_t* fb, uint32_t fw, uint32_t fcells, const float* fd,
-                                                   const float* fpx, const float* fpy, const float* fr,
-                                                   const float* fe, uint32_t cx, uint32_t cy) {
-    float sum = 0.0f;
-    const long long W = fw;
-#pragma unroll
-    for (uint32_t dy = 0; dy < 2; ++dy)
-#pragma unroll
-        for (uint32_t dx = 0; dx < 2; ++dx) {
-            const long long rf = (long long)(cy * 2 + dy) * fw + (cx * 2 + dx);
-            const uint32_t pf = uint32_t(rf) + fw;
-            const bool f0 = fluid_raw(fb, rf, fcells);
-            const bool fr_ = fluid_raw(fb, rf + 1, fcells), fu = fluid_raw(fb, rf + W, fcells);
-            const bool fl = fluid_raw(fb, rf - 1, fcells), fdn = fluid_raw(fb, rf - W, fcells);
-            const float b = fr[pf];
-            float ax = fd[pf] * fe[pf];
-            float t = ax + fpx[pf] * fe[pf + 1];
-            ax = fr_ ? t : ax;
-            t = ax + fpy[pf] * fe[pf + fw];
-            ax = fu ? t : ax;
-            t = ax + fpx[pf - 1] * fe[pf - 1];
-            ax = fl ? t : ax;
-            t = ax + fpy[pf - fw] * fe[pf - fw];
-            ax = fdn ? t : ax;
-            t = sum + (b - ax);
-            sum = f0 ? t : sum;
-        }
-    return sum;
-}
-
 
 // e + ec, plus ec again `reps` times (the padded base list, :611-615).
 __device__ __forceinline__ float prolonged(float e, float ec, uint32_t reps) {
@@ -475,7 +393,13 @@ static __device__ __noinline__ void cg_one_warp(const CgArrays& A, bool exact) {
         pd = fd ? A.py[c - W] : 0.0f;
     }
     auto dot = [&](float q) {
-        if (!exact) return float(warp_sum(double(q)));
+        if (!exact) {
+            double t = double(q);
+            if (cells > 16u) t += __shfl_xor_sync(0xffffffffu, t, 16);  // (else the upper lanes hold zeros)
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            return __shfl_sync(0xffffffffu, float(t), 0);
+        }
         float t = 0.0f;
 #pragma unroll 8
         for (int l = 0; l < 32; ++l) t = t + __shfl_sync(0xffffffffu, q, l);
@@ -532,57 +456,177 @@ static __device__ __forceinline__ void cta_coarse_cg(const CgArrays& A, bool exa
 
 // ---- the coarse tail in shared memory ----------------------------------------
 struct TailLevel {
-    uint32_t w, h, cells, words, padded;
-    int wshift;   // log2 w, or -1 when w is not a power of two
     const uint32_t* fluid;
     const float *diag, *inv, *px, *py;
     float* res;   // global residual (read for the first tail level)
     float* err;   // global error (written back for the first tail level)
-    uint32_t o_bits, o_diag, o_inv, o_px, o_py, o_res, o_err;  // shared offsets, 4-byte units
 };
 struct TailParams {
     int n;                      // tail levels; lv[n - 1] is the coarsest
     int exact;                  // coarsest CG with the reference's serial FP32 sums
-    uint32_t o_cs, o_cap, o_cr;  // coarse CG vectors
+    uint32_t w, h;              // of the first level
+    int wshift;                 // log2 w, or -1 when w is not a power of two
     TailLevel lv[kMaxLevels];
 };
 
+// One level in the tail's shared memory (32-bit words): mask words, then
+// diagonal, inverse diagonal, couplings, residual and error, each `padded`
+// long.  A level follows from the one before it by arithmetic alone (sides
+// halve, offsets add up): a load of its sizes and offsets from the kernel's
+// parameters missed the constant cache at each phase (0.25 us of 0.4).
 struct SmemLevel {
-    uint32_t w, h, cells;
+    uint32_t w, h, cells, words, padded;
     int wshift;
     uint32_t* bits;
     float *diag, *inv, *px, *py, *res, *err;
 };
-
-__device__ __forceinline__ SmemLevel smem_level(uint32_t* sm, const TailLevel& t) {
-    float* f = reinterpret_cast<float*>(sm);
-    return SmemLevel{t.w,          t.h,          t.cells,      t.wshift,     sm + t.o_bits, f + t.o_diag,
-                     f + t.o_inv,  f + t.o_px,   f + t.o_py,   f + t.o_res,  f + t.o_err};
+inline __host__ __device__ uint32_t tail_words(uint32_t cells) { return (cells + 63u) / 64u * 2u; }
+inline __host__ __device__ uint32_t tail_padded(uint32_t w, uint32_t cells) { return (cells + 2u * w + 7u) & ~7u; }
+__device__ __forceinline__ SmemLevel smem_at(uint32_t* at, uint32_t w, uint32_t h, int wshift) {
+    SmemLevel L;
+    L.w = w;
+    L.h = h;
+    L.cells = w * h;
+    L.words = tail_words(L.cells);
+    L.padded = tail_padded(w, L.cells);
+    L.wshift = wshift;
+    L.bits = at;
+    L.diag = reinterpret_cast<float*>(at + L.words);
+    L.inv = L.diag + L.padded;
+    L.px = L.inv + L.padded;
+    L.py = L.px + L.padded;
+    L.res = L.py + L.padded;
+    L.err = L.res + L.padded;
+    return L;
+}
+__device__ __forceinline__ SmemLevel smem_first(const TailParams& tp, uint32_t* sm) {
+    return smem_at(sm, tp.w, tp.h, tp.wshift);
+}
+__device__ __forceinline__ SmemLevel smem_coarser(const SmemLevel& f) {
+    return smem_at(f.bits + f.words + 6u * f.padded, f.w >> 1, f.h >> 1, f.wshift > 0 ? f.wshift - 1 : -1);
+}
+__device__ __forceinline__ SmemLevel smem_finer(const SmemLevel& c) {
+    const uint32_t w = c.w << 1, h = c.h << 1;
+    return smem_at(c.bits - tail_words(w * h) - 6u * tail_padded(w, w * h), w, h, c.wshift >= 0 ? c.wshift + 1 : -1);
 }
 
-// One colour sweep of a shared-memory level (w even: every level that is
-// swept has a coarser one).  Thread t visits the colour's cells k = t,
-// t + blockDim.x, ... directly, row by row, and skips the cells outside the
-// fluid mask (their result is never stored).
-__device__ __forceinline__ void cta_sweep(const SmemLevel& L, int color, int init) {
-    const float* e = L.err;
+// ---- phases on levels in shared memory ---------------------------------------
+// The coarse levels' coefficients are zero at every cell outside the fluid
+// (the multigrid setup writes them so), so on a level held by a CTA (the
+// tail, below) or by a cluster in bands of rows (vcycle_dsm.cu) a phase runs
+// over all cells without a test.  A neighbour that the reference skips enters
+// with a zero coupling, which leaves a sum as it was; a cell whose inverse
+// diagonal is zero keeps its old value, as in the reference.  A level takes
+// four phases a V-cycle: black sweep (the red one is formed with the residual,
+// red_first), restriction; prolongation fused into the black and into the red
+// reverse sweep.  What bounds a phase is its instructions (32 warps on four
+// schedulers) and then its barrier, so index arithmetic and tests went first.
+
+// The first red sweep of a cell from zero error (its own residual is all it takes).
+__device__ __forceinline__ float red_first(float r, float inv) {
+    return inv != 0.0f ? 0.0f + (kOmega * (r * inv - 0.0f)) : 0.0f;
+}
+// One SOR update; er, eu, el, ed: the neighbours' errors in the reference's order.
+__device__ __forceinline__ float sor_masked(float inv, float sum, float pxc, float pyc, float pxl, float pyd, float er,
+                                            float eu, float el, float ed, float old) {
+    sum = __fmaf_rn(-pxc, er, sum);
+    sum = __fmaf_rn(-pyc, eu, sum);
+    sum = __fmaf_rn(-pxl, el, sum);
+    sum = __fmaf_rn(-pyd, ed, sum);
+    const float gs = sum * inv;
+    const float nv = old + (kOmega * (gs - old));
+    return inv == 0.0f ? old : nv;
+}
+// b - A e of the cell at index i of arrays with rows of w (restrict :549-583).
+__device__ __forceinline__ float left_over(const float* r, const float* d, const float* px, const float* py,
+                                           const float* e, int i, int id, int w) {
+    float ax = d[id] * e[i];
+    ax = ax + px[i] * e[i + 1];
+    ax = ax + py[i] * e[i + w];
+    ax = ax + px[i - 1] * e[i - 1];
+    ax = ax + py[i - w] * e[i - w];
+    return r[i] - ax;
+}
+// The errors around a cell under prolongation: its coarse cell's error c0,
+// that of the coarse cell beside it in x and in y (the other two neighbours
+// lie under c0).
+struct CoarseAround {
+    float c0, h, v;
+};
+__device__ __forceinline__ CoarseAround coarse_around(const float* ce, int cc, int cw, bool x_odd, bool y_odd) {
+    return CoarseAround{ce[cc], ce[cc + (x_odd ? 1 : -1)], ce[cc + (y_odd ? cw : -cw)]};
+}
+
+// k-th cell of one colour of a level with rows of w = 2 * half: its row and column.
+__device__ __forceinline__ void colour_cell(uint32_t k, uint32_t half, int hshift, uint32_t color, uint32_t& x,
+                                            uint32_t& y) {
+    uint32_t kk;
+    raw_xy(k, half, hshift, kk, y);
+    x = 2u * kk + ((y + color) & 1u);
+}
+
+// The tail's phases (padded layout; w even on every level that is swept).
+__device__ __forceinline__ void cta_black(const SmemLevel& L) {
     const uint32_t half = L.w >> 1;
-    const int hs = L.wshift > 0 ? L.wshift - 1 : -1;
-    const uint32_t n = L.h * half;
-    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
-        uint32_t kk, row;
-        raw_xy(k, half, hs, kk, row);
-        const uint32_t r = row * L.w + 2u * kk + ((row + uint32_t(color)) & 1u);
-        if (!bit_at(L.bits, r)) continue;
-        const uint32_t c = r + L.w;
-        const float old = init ? 0.0f : e[c];
-        L.err[c] = sor_cell_all(L.bits, L.w, L.cells, L.inv, L.px, L.py, L.res, r, c, old, !(init && color == 0),
-                                [e](uint32_t p, long long) { return e[p]; });
+    const int hs = L.wshift > 0 ? L.wshift - 1 : -1, w = int(L.w);
+    for (uint32_t k = threadIdx.x; k < L.h * half; k += blockDim.x) {
+        uint32_t x, y;
+        colour_cell(k, half, hs, 1u, x, y);
+        const int c = int((y + 1u) * L.w + x);
+        L.err[c] = sor_masked(L.inv[c], L.res[c], L.px[c], L.py[c], L.px[c - 1], L.py[c - w], L.err[c + 1],
+                              L.err[c + w], L.err[c - 1], L.err[c - w], 0.0f);
     }
     __syncthreads();
 }
-
-
+// Two threads per coarse cell, one per row of its children; the even one adds
+// the four in the reference's order.
+__device__ __forceinline__ void cta_restrict(const SmemLevel& f, const SmemLevel& c) {
+    const uint32_t n = (2u * c.cells + 31u) & ~31u;  // whole warps take part in the shuffles
+    const int w = int(f.w);
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t q = i >> 1, dy = i & 1u;
+        float d0 = 0.0f, d1 = 0.0f;
+        uint32_t cx = 0, cy = 0;
+        if (q < c.cells) {
+            raw_xy(q, c.w, c.wshift, cx, cy);
+            const int p = int((2u * cy + dy + 1u) * f.w + 2u * cx);
+            d0 = left_over(f.res, f.diag, f.px, f.py, f.err, p, p, w);
+            d1 = left_over(f.res, f.diag, f.px, f.py, f.err, p + 1, p + 1, w);
+        }
+        const float d2 = __shfl_down_sync(0xffffffffu, d0, 1), d3 = __shfl_down_sync(0xffffffffu, d1, 1);
+        if (dy == 0 && q < c.cells) {
+            const float sum = (((0.0f + d0) + d1) + d2) + d3;
+            const uint32_t p = q + c.w;
+            c.res[p] = sum;
+            c.err[p] = ((cx + cy) & 1u) == 0u ? red_first(sum, c.inv[p]) : 0.0f;
+        }
+    }
+    __syncthreads();
+}
+template <int kColor>
+__device__ __forceinline__ void cta_up(const SmemLevel& f, const SmemLevel& c) {
+    const uint32_t half = f.w >> 1;
+    const int hs = f.wshift > 0 ? f.wshift - 1 : -1, w = int(f.w);
+    for (uint32_t k = threadIdx.x; k < f.h * half; k += blockDim.x) {
+        uint32_t x, y;
+        colour_cell(k, half, hs, kColor, x, y);
+        const int p = int((y + 1u) * f.w + x), cc = int(((y >> 1) + 1u) * c.w + (x >> 1));
+        const bool xo = x & 1u, yo = y & 1u;
+        float er = f.err[p + 1], eu = f.err[p + w], el = f.err[p - 1], ed = f.err[p - w], old = f.err[p];
+        if (kColor == 1) {
+            const CoarseAround a = coarse_around(c.err, cc, int(c.w), xo, yo);
+            old = old + a.c0;
+            er = er + (xo ? a.h : a.c0);
+            el = el + (xo ? a.c0 : a.h);
+            eu = eu + (yo ? a.v : a.c0);
+            ed = ed + (yo ? a.c0 : a.v);
+        } else {
+            old = old + c.err[cc];
+        }
+        f.err[p] = sor_masked(f.inv[p], f.res[p], f.px[p], f.py[p], f.px[p - 1], f.py[p - w], er, eu, el, ed, old);
+    }
+    __syncthreads();
+}
 
 // ---- sweep phases over a level's segment list -------------------------------
 // `warp` / `nwarps`: this warp's index in the grid and the grid's warp count.
@@ -627,125 +671,90 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 
 // Start copying every tail level's mask and coefficients into shared memory
-// (complete after cp_async_wait_all).  The whole tail region is zeroed first:
-// cells outside the fluid mask are never written, and with the stale shared
-// memory of earlier kernels left in place the cluster-launched solve reached
-// NaN (after other scenes had run in the process; the read that carried it
-// was not located), while zeroed memory gives the same results as before.
+// (complete after cp_async_wait_all), and zero the vectors (their padding is
+// read beside the level's edge).
 __device__ __forceinline__ void cta_tail_issue_coeffs(const TailParams& tp, uint32_t* sm) {
-    if (tp.n > 0) {
-        const uint32_t words = tp.o_cr + tp.lv[tp.n - 1].padded;
-        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) sm[i] = 0u;
-        __syncthreads();  // zeroes land before any copy into the same words
-    }
+    SmemLevel L = smem_first(tp, sm);
     for (int l = 0; l < tp.n; ++l) {
         const TailLevel& t = tp.lv[l];
-        SmemLevel L = smem_level(sm, t);
-        for (uint32_t i = threadIdx.x; i < t.words; i += blockDim.x) cp_async4(L.bits + i, t.fluid + i);
-        for (uint32_t i = threadIdx.x; i < t.padded; i += blockDim.x) {
+        for (uint32_t i = threadIdx.x; i < L.words; i += blockDim.x) cp_async4(L.bits + i, t.fluid + i);
+        for (uint32_t i = threadIdx.x; i < L.padded; i += blockDim.x) {
             cp_async4(L.diag + i, t.diag + i);
             cp_async4(L.inv + i, t.inv + i);
             cp_async4(L.px + i, t.px + i);
             cp_async4(L.py + i, t.py + i);
+            L.err[i] = 0.0f;
+            if (l > 0) L.res[i] = 0.0f;
         }
+        L = smem_coarser(L);
     }
 }
 
-// Copy every tail level's mask and coefficients into shared memory.
-__device__ __forceinline__ void cta_tail_load_coeffs(const TailParams& tp, uint32_t* sm) {
-    cta_tail_issue_coeffs(tp, sm);
+// The V-cycle on the tail's levels by one CTA: the first level's residual and
+// first red sweep are in shared memory, its final error stays there.
+__device__ __forceinline__ void cta_tail_levels(const TailParams& tp, uint32_t* sm) {
+    const int n = tp.n;
+    SmemLevel f = smem_first(tp, sm);
+    for (int l = 0; l + 1 < n; ++l) {
+        const SmemLevel c = smem_coarser(f);
+        cta_black(f);
+        cta_restrict(f, c);
+        f = c;
+    }
+    float* cg = reinterpret_cast<float*>(f.bits + f.words + 6u * f.padded);  // three vectors behind the last level
+    cta_coarse_cg(CgArrays{f.bits, f.w, f.cells, f.diag, f.px, f.py, f.res, f.err, cg, cg + f.padded,
+                           cg + 2u * f.padded, true},
+                  tp.exact != 0);
+    for (int l = n - 2; l >= 0; --l) {
+        const SmemLevel c = f;
+        f = smem_finer(c);
+        cta_up<1>(f, c);
+        cta_up<0>(f, c);
+    }
+}
+
+// The coarse tail by one CTA, from the first level's residual in global
+// memory to its error there.  The coefficients' copies were issued before
+// (cta_tail_issue_coeffs).
+__device__ __forceinline__ void cta_tail(const TailParams& tp, uint32_t* sm) {
+    const SmemLevel L = smem_first(tp, sm);
+    const float* res = tp.lv[0].res;
+    float* err = tp.lv[0].err;
+    for (uint32_t i = threadIdx.x; i < L.padded; i += blockDim.x) cp_async4(L.res + i, res + i);
     cp_async_wait_all();
     __syncthreads();
-}
-
-// The coarse tail (levels held in shared memory) by one CTA.  load_coeffs:
-// copy masks and coefficients first (otherwise they are already resident);
-// the first level's residual is always copied in and its error copied out.
-// load_coeffs false: the coefficients are resident or their copies were
-// issued earlier by this CTA (cta_tail_issue_coeffs); the wait below covers
-// those too.  global_io false: the first level's residual is already in
-// shared memory and its error stays there (a cluster's other CTAs exchange
-// them through distributed shared memory).
-__device__ __forceinline__ void cta_tail(const TailParams& tp, uint32_t* sm, bool load_coeffs,
-                                         bool global_io = true) {
-    if (load_coeffs) cta_tail_issue_coeffs(tp, sm);
-    if (global_io) {
-        const TailLevel& t = tp.lv[0];
-        SmemLevel L = smem_level(sm, t);
-        for (uint32_t i = threadIdx.x; i < t.padded; i += blockDim.x) cp_async4(L.res + i, t.res + i);
+    // (only the fluid cells' residual was written)
+    for (uint32_t i = threadIdx.x; i < L.padded; i += blockDim.x) {
+        const long long r = (long long)i - L.w;
+        if (!fluid_raw(L.bits, r, L.cells)) L.res[i] = 0.0f;
+        else if (red_at(uint32_t(r), L.w, L.wshift)) L.err[i] = red_first(L.res[i], L.inv[i]);
     }
-    cp_async_wait_all();
     __syncthreads();
-    for (int l = 0; l + 1 < tp.n; ++l) {
-        SmemLevel f = smem_level(sm, tp.lv[l]);
-        SmemLevel c = smem_level(sm, tp.lv[l + 1]);
-        cta_sweep(f, 0, 1);
-        cta_sweep(f, 1, 1);
-        for (uint32_t rc = threadIdx.x; rc < c.cells; rc += blockDim.x) {
-            if (!bit_at(c.bits, rc)) continue;
-            uint32_t cx, cy;
-            raw_xy(rc, c.w, c.wshift, cx, cy);
-            c.res[rc + c.w] = restrict_cell_all(f.bits, f.w, f.cells, f.diag, f.px, f.py, f.res, f.err, cx, cy);
-        }
-        __syncthreads();
-    }
-    {
-        SmemLevel L = smem_level(sm, tp.lv[tp.n - 1]);
-        float* fs = reinterpret_cast<float*>(sm);
-        cta_coarse_cg(CgArrays{L.bits, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, fs + tp.o_cs, fs + tp.o_cap,
-                               fs + tp.o_cr, true},
-                      tp.exact != 0);
-    }
-    for (int l = tp.n - 2; l >= 0; --l) {
-        SmemLevel f = smem_level(sm, tp.lv[l]);
-        SmemLevel c = smem_level(sm, tp.lv[l + 1]);
-        for (uint32_t r = threadIdx.x; r < f.cells; r += blockDim.x)
-            if (bit_at(f.bits, r)) {
-                uint32_t x, y;
-                raw_xy(r, f.w, f.wshift, x, y);
-                f.err[r + f.w] = f.err[r + f.w] + c.err[(y >> 1) * c.w + (x >> 1) + c.w];
-            }
-        __syncthreads();
-        cta_sweep(f, 1, 0);
-        cta_sweep(f, 0, 0);
-    }
-    if (!global_io) {
-        __syncthreads();
-        return;
-    }
-    const TailLevel& t = tp.lv[0];
-    SmemLevel L = smem_level(sm, t);
-    for (uint32_t r = threadIdx.x; r < t.cells; r += blockDim.x)
-        if (bit_at(L.bits, r)) t.err[r + t.w] = L.err[r + t.w];
+    cta_tail_levels(tp, sm);
+    for (uint32_t r = threadIdx.x; r < L.cells; r += blockDim.x)
+        if (bit_at(L.bits, r)) err[r + L.w] = L.err[r + L.w];
 }
 
-// Host: tail parameters for levels [first, s.nlevels) laid out in shared memory.
+// Host: tail parameters for levels [first, s.nlevels), and the 32-bit words
+// they take in shared memory (the CG's three vectors last).
 inline TailParams make_tail_params(const Scene& s, int first, uint32_t* words_out) {
     TailParams tp;
+    std::memset(&tp, 0, sizeof(tp));
     tp.n = s.nlevels - first;
     tp.exact = coarse_cg_exact(s) ? 1 : 0;
     uint32_t off = 0;
     for (int k = 0; k < tp.n; ++k) {
         const Level& v = s.lv[first + k];
-        TailLevel& t = tp.lv[k];
-        t.w = v.w; t.h = v.h; t.cells = v.cells; t.words = v.words; t.padded = v.padded;
-        t.wshift = -1;
-        for (int k = 0; k < 31; ++k)
-            if ((1u << k) == v.w) t.wshift = k;
-        t.fluid = v.fluid; t.diag = v.diag; t.inv = v.inv_diag; t.px = v.px; t.py = v.py;
-        t.res = v.res; t.err = v.err;
-        t.o_bits = off; off += v.words;
-        t.o_diag = off; off += v.padded;
-        t.o_inv = off; off += v.padded;
-        t.o_px = off; off += v.padded;
-        t.o_py = off; off += v.padded;
-        t.o_res = off; off += v.padded;
-        t.o_err = off; off += v.padded;
+        if (k == 0) {
+            tp.w = v.w;
+            tp.h = v.h;
+            tp.wshift = v.wshift;
+        }
+        tp.lv[k] = TailLevel{v.fluid, v.diag, v.inv_diag, v.px, v.py, v.res, v.err};
+        off += tail_words(v.cells) + 6 * tail_padded(v.w, v.cells);
     }
-    uint32_t cp = s.lv[s.nlevels - 1].padded;
-    tp.o_cs = off; off += cp;
-    tp.o_cap = off; off += cp;
-    tp.o_cr = off; off += cp;
+    const Level& last = s.lv[s.nlevels - 1];
+    off += 3 * tail_padded(last.w, last.cells);
     *words_out = off;
     return tp;
 }

@@ -2,21 +2,25 @@
 //
 // The same V-cycle arithmetic as vcycle.cu (smooth_level src/apic.rs:471-535,
 // restrict :537-594, prolongate :596-616, solve_coarse_exact :618-704), with
-// the levels between the base kernels and the coarse tail held in the shared
-// memory of one 16-CTA thread-block cluster.  CTA r owns rows
-// [r*R, (r+1)*R) of every such level (R = height / 16): their error and
-// residual, and their mask and coefficients plus one halo row on each side.
-// A stencil read that falls in another CTA's rows goes to that CTA's shared
-// memory (distributed shared memory, a few hundred cycles instead of an L2
-// round trip); phases are separated by cluster barriers, whose release /
-// acquire order makes every CTA's writes visible to the others.  CTA 0 then
-// runs the coarse tail (levels of fewer than 64 rows) exactly as
-// k_vcycle_tail does, through global memory.
+// the levels between the grid-wide kernels and the coarse tail held in the
+// shared memory of one 16-CTA thread-block cluster.  CTA r owns rows
+// [r R, (r+1) R) of every such level (R = height / 16) and holds two more rows
+// on each side: with them it smooths its band and the row next to it by
+// itself, computing the neighbour's values again from the same inputs with
+// the same operations.  What it cannot compute, the neighbours push into its
+// halo rows as they form it (distributed shared memory, stores only): the
+// coarse residual of the restriction, the boundary rows' final errors.  So a
+// level costs one cluster barrier going down and one going up, and no phase
+// waits for another CTA's shared memory.  CTA 0 runs the coarse tail (levels
+// of fewer than kDsmTailRows rows) between the two halves; the restriction
+// into it writes there directly and it pushes every band its rows.
 //
-// A phase over a level costs a few hundred cycles of shared-memory latency
-// plus one cluster barrier, where the same phase as a kernel (or a phase of
-// k_vcycle_mid on L2-resident arrays) costs an L2 round trip per dependent
-// load plus a launch.
+// Bound by the latency of its phases and barriers (some 190 KB per CTA never
+// leave the SMs).  The form before this one read neighbours' rows in place,
+// tested fluid bits per neighbour, took a cluster barrier per sweep and read
+// every level's layout from the kernel's parameters; a PCG iteration with it
+// took 43.2 us at 128^2 (64^2 in the cluster), 51.2 at 256^2, 69.6 at 1024^2
+// (256^2 to 64^2 in the cluster), now 32.6, 37.4 and 58.1.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -34,347 +38,329 @@ constexpr uint32_t kDsmCtas = 16;
 constexpr uint32_t kDsmTailRows = 64;
 constexpr int kDsmMaxLevels = 6;
 constexpr size_t kDsmSmemBudget = 220 * 1024;
+constexpr int kDsmHalo = 2;
+constexpr int kDsmPad = 4;  // floats before and after a level's rows (reads one past a row's ends)
 
-// Host-computed layout of one distributed level (byte offsets into the
-// dynamic shared memory, identical in every CTA).  Widths are multiples of
-// 32, so every row starts on a mask word.
+// One distributed level; widths are multiples of 32.
 struct DsmLevel {
-    int w, h, cells, R;
-    int rw_shift, half_shift;  // log2(R*w), log2(w/2), or -1 when not a power of two
     const uint32_t* fluid;
     const float *diag, *inv, *px, *py;  // global, padded layout
-    float *res, *err;                   // global, padded layout
-    uint32_t o_fl, o_diag, o_inv, o_px, o_py, o_res, o_err;
 };
-
 struct DsmParams {
-    int n;  // distributed levels; lv[0] is V-cycle level `first`
-    int first;
+    int n;       // distributed levels, finest first
+    int w, R;    // of the finest
+    int hshift;  // log2(w / 2), or -1 when it is not a power of two
+    int cells;
+    const float* res;  // of the finest, global, padded layout
+    float* err;
+    const float* tinv;        // the first tail level's inverse diagonal, global
     DsmLevel lv[kDsmMaxLevels];
-    // the first tail level (coarse level of lv[n-1]), in global memory
-    int tw, tcells;
-    const uint32_t* tfluid;
-    float* tres;
-    const float* terr;
 };
 
-// This CTA's view of a distributed level.  Coefficients and mask bits are
-// indexed by li = (y - y0 + 1) * w + x (rows y0-1 .. y0+R; rows outside the
-// grid hold zero bits), error and residual by (y - y0) * w + x.  A raw index
-// r = y * w + x moves to li by r - lo + w.
-struct View {
-    int w, h, cells, R, y0, lo, rw;
-    int rw_shift, half_shift;
-    const uint32_t* flw;
-    const float *diag, *inv, *px, *py;
-    float *res, *err;
+// A distributed level in this CTA's shared memory: five arrays of rows -2 ..
+// R + 1 (row 0 is the band's first) with kDsmPad floats before and after,
+// indexed by row * w + x, then the diagonal's rows 0 .. R - 1.  As in the flat
+// index of the reference, the cell after a row's last one is the next row's
+// first.  The levels lie one after another, each half the width and rows of
+// the one before; behind the last, the tail's error around the band (rows -1
+// .. R / 2 of its width) and its inverse diagonal under it.
+struct Band {
+    int w, R, hshift;
+    float* at;  // the level's first float
+    float *e, *r, *inv, *px, *py, *d;
 };
-
-__device__ __forceinline__ View view_of(const DsmLevel& L, uint8_t* sm, uint32_t rank) {
-    View v;
-    v.w = L.w;
-    v.h = L.h;
-    v.cells = L.cells;
-    v.R = L.R;
-    v.y0 = int(rank) * L.R;
-    v.lo = v.y0 * L.w;
-    v.rw = L.R * L.w;
-    v.rw_shift = L.rw_shift;
-    v.half_shift = L.half_shift;
-    v.flw = reinterpret_cast<const uint32_t*>(sm + L.o_fl);
-    v.diag = reinterpret_cast<const float*>(sm + L.o_diag);
-    v.inv = reinterpret_cast<const float*>(sm + L.o_inv);
-    v.px = reinterpret_cast<const float*>(sm + L.o_px);
-    v.py = reinterpret_cast<const float*>(sm + L.o_py);
-    v.res = reinterpret_cast<float*>(sm + L.o_res);
-    v.err = reinterpret_cast<float*>(sm + L.o_err);
-    return v;
+__device__ __forceinline__ int band_floats(int w, int R) { return (R + 2 * kDsmHalo) * w + 2 * kDsmPad; }
+__device__ __forceinline__ Band band_at(float* at, int w, int R, int hshift) {
+    const int n = band_floats(w, R);
+    float* e = at + kDsmPad + kDsmHalo * w;
+    return Band{w, R, hshift, at, e, e + n, e + 2 * n, e + 3 * n, e + 4 * n, at + 5 * n};
+}
+__device__ __forceinline__ Band band_coarser(const Band& f) {
+    return band_at(f.d + f.R * f.w, f.w >> 1, f.R >> 1, f.hshift > 0 ? f.hshift - 1 : -1);
+}
+__device__ __forceinline__ Band band_finer(const Band& c) {
+    const int w = c.w << 1, R = c.R << 1;
+    return band_at(c.at - 5 * band_floats(w, R) - R * w, w, R, c.hshift >= 0 ? c.hshift + 1 : -1);
 }
 
-__device__ __forceinline__ bool flb(const View& v, int li) { return (v.flw[li >> 5] >> (li & 31)) & 1u; }
-
-// Error at raw index r of this level: own rows from this CTA's shared
-// memory, other rows from the owning CTA's (rank r / (R*w)); 0 outside the
-// grid (the callers drop non-fluid values).
-__device__ __forceinline__ float err_raw(const View& v, const cg::cluster_group& cl, int r) {
-    const int rel = r - v.lo;
-    if (rel >= 0 && rel < v.rw) return v.err[rel];
-    if (r < 0 || r >= v.cells) return 0.0f;
-    const int rank = v.rw_shift >= 0 ? (r >> v.rw_shift) : (r / v.rw);
-    const float* remote = cl.map_shared_rank(v.err, rank);
-    return remote[r - rank * v.rw];
+// The neighbours' views of an array in this CTA's shared memory.
+struct Peers {
+    float *below, *above;  // rank - 1, rank + 1 (this CTA's own where there is none)
+    bool has_below, has_above;
+};
+__device__ __forceinline__ Peers peers_of(const cg::cluster_group& cl, float* p, uint32_t rank) {
+    const bool b = rank > 0, a = rank + 1 < kDsmCtas;
+    return Peers{cl.map_shared_rank(p, b ? rank - 1 : rank), cl.map_shared_rank(p, a ? rank + 1 : rank), b, a};
 }
 
-// (x, y) of the i-th cell of an area `half` cells wide.
-__device__ __forceinline__ void split(int i, int half, int shift, int& row, int& col) {
-    if (shift >= 0) {
-        row = i >> shift;
-        col = i & (half - 1);
+// Cell k of one colour in rows first, first + 1, ...
+__device__ __forceinline__ void band_cell(const Band& b, int k, int first, int color, int& row, int& x) {
+    const int half = b.w >> 1;
+    int q;
+    if (b.hshift >= 0) {
+        q = k >> b.hshift;
+        k &= half - 1;
     } else {
-        row = i / half;
-        col = i - row * half;
+        q = k / half;
+        k -= q * half;
+    }
+    row = first + q;
+    x = 2 * k + ((row + color) & 1);  // (a band starts on an even row)
+}
+
+// Black sweep after the red one, on the band and a row on each side.
+__device__ __forceinline__ void dsm_black(const Band& b) {
+    const int n = (b.R + 2) * (b.w >> 1), w = b.w;
+    for (int k = threadIdx.x; k < n; k += kTailThreads) {
+        int row, x;
+        band_cell(b, k, -1, 1, row, x);
+        const int i = row * w + x;
+        b.e[i] = sor_masked(b.inv[i], b.r[i], b.px[i], b.py[i], b.px[i - 1], b.py[i - w], b.e[i + 1], b.e[i + w],
+                            b.e[i - 1], b.e[i - w], 0.0f);
     }
 }
 
-// One SOR update of own cell (x, y): sor_cell_all's arithmetic and neighbour
-// order (raw+1, raw+w, raw-1, raw-w, where raw +- 1 wraps between rows as
-// the reference's flat index does).  nb(r, xn, yn) gives a neighbour's error.
-template <class NB>
-__device__ __forceinline__ float sor_dsm(const View& v, int x, int y, float old, bool neighbours, NB nb) {
-    const int li = (y - v.y0 + 1) * v.w + x;
-    const int raw = y * v.w + x;
-    const int W = v.w;
-    const float inv = v.inv[li];
-    float sum = v.res[li - W];
-    if (neighbours) {
-        const bool fr = flb(v, li + 1), fu = flb(v, li + W), fl = flb(v, li - 1), fd = flb(v, li - W);
-        const float pxc = v.px[li], pyc = v.py[li], pxl = v.px[li - 1], pyd = v.py[li - W];
-        const bool xr = x + 1 < W, xl = x > 0;
-        const float er = nb(raw + 1, xr ? x + 1 : 0, xr ? y : y + 1);
-        const float eu = nb(raw + W, x, y + 1);
-        const float el = nb(raw - 1, xl ? x - 1 : W - 1, xl ? y : y - 1);
-        const float ed = nb(raw - W, x, y - 1);
-        float t = __fmaf_rn(-pxc, er, sum);
-        sum = fr ? t : sum;
-        t = __fmaf_rn(-pyc, eu, sum);
-        sum = fu ? t : sum;
-        t = __fmaf_rn(-pxl, el, sum);
-        sum = fl ? t : sum;
-        t = __fmaf_rn(-pyd, ed, sum);
-        sum = fd ? t : sum;
-    }
-    const float gs = sum * inv;
-    const float nv = old + (kOmega * (gs - old));
-    return inv == 0.0f ? old : nv;
-}
-
-// One colour sweep over own cells (init: the level's error was zero-filled).
-__device__ __forceinline__ void dsm_sweep(const View& v, const cg::cluster_group& cl, int color, bool init) {
-    const int half = v.w >> 1;
-    const int n = v.R * half;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        int row, k;
-        split(i, half, v.half_shift, row, k);
-        const int y = v.y0 + row;
-        const int x = 2 * k + ((y + color) & 1);
-        const int o = row * v.w + x;
-        if (!flb(v, o + v.w)) continue;  // only fluid cells store
-        const float old = init ? 0.0f : v.err[o];
-        v.err[o] = sor_dsm(v, x, y, old, !(init && color == 0), [&](int r, int, int) { return err_raw(v, cl, r); });
-    }
-}
-
-// Restriction of fine view f into the coarse cells of this CTA's coarse rows
-// (their children are this CTA's fine rows): restrict_cell_all's arithmetic.
-// Coarse view c (with_red: also its first red sweep) or, when c is null, the
-// first tail level's residual in CTA 0's shared memory (tail_res, padded
-// layout, mapped into this CTA's address space).
-__device__ __forceinline__ void dsm_restrict(const View& f, const cg::cluster_group& cl, const View* c,
-                                             const DsmParams& p, float* tail_res, uint32_t rank, bool with_red) {
-    const int wc = f.w >> 1;
-    const int rc = f.R >> 1;
-    const int yc0 = int(rank) * rc;
-    const int n = rc * wc;
-    const int W = f.w;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        int row, cx;
-        split(i, wc, f.half_shift, row, cx);
-        const int cy = yc0 + row;
-        const int craw = cy * wc + cx;
-        // only fluid coarse cells store
-        if (c ? !flb(*c, craw - c->lo + wc) : !bit_at(p.tfluid, uint32_t(craw))) continue;
-        float sum = 0.0f;
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-            for (int dx = 0; dx < 2; ++dx) {
-                const int rf = (cy * 2 + dy) * W + (cx * 2 + dx);
-                const int li = rf - f.lo + W;
-                const bool f0 = flb(f, li);
-                const bool fr = flb(f, li + 1), fu = flb(f, li + W), fl = flb(f, li - 1), fd = flb(f, li - W);
-                const float b = f.res[li - W];
-                float ax = f.diag[li] * f.err[li - W];
-                float t = ax + f.px[li] * err_raw(f, cl, rf + 1);
-                ax = fr ? t : ax;
-                t = ax + f.py[li] * err_raw(f, cl, rf + W);
-                ax = fu ? t : ax;
-                t = ax + f.px[li - 1] * err_raw(f, cl, rf - 1);
-                ax = fl ? t : ax;
-                t = ax + f.py[li - W] * err_raw(f, cl, rf - W);
-                ax = fd ? t : ax;
-                t = sum + (b - ax);
-                sum = f0 ? t : sum;
-            }
-        if (c) {
-            const int co = craw - c->lo;
-            c->res[co] = sum;
-            if (with_red && ((cx + cy) & 1) == 0) {
-                const float inv = c->inv[co + wc];
-                c->err[co] = inv != 0.0f ? 0.0f + (kOmega * (sum * inv - 0.0f)) : 0.0f;
-            }
+// Restriction of the band into its coarse rows, two threads per coarse cell
+// (one per row of children); put(coarse row, x, sum) stores the residual.
+template <class Put>
+__device__ __forceinline__ void dsm_restrict(const Band& f, Put put) {
+    const int cw = f.w >> 1, n = f.R * cw, w = f.w;  // a multiple of 32: whole warps
+    for (int k = threadIdx.x; k < n; k += kTailThreads) {
+        const int q = k >> 1, dy = k & 1;
+        int row, x;
+        if (f.hshift >= 0) {
+            row = q >> f.hshift;
+            x = q & (cw - 1);
         } else {
-            tail_res[craw + wc] = sum;  // CTA 0's shared memory
+            row = q / cw;
+            x = q - row * cw;
+        }
+        const int i = (2 * row + dy) * w + 2 * x;
+        const float d0 = left_over(f.r, f.d, f.px, f.py, f.e, i, i, w);
+        const float d1 = left_over(f.r, f.d, f.px, f.py, f.e, i + 1, i + 1, w);
+        const float d2 = __shfl_down_sync(0xffffffffu, d0, 1), d3 = __shfl_down_sync(0xffffffffu, d1, 1);
+        if (dy == 0) put(row, x, (((0.0f + d0) + d1) + d2) + d3);
+    }
+}
+
+// Reverse sweep of one colour with the prolongation from ce (rows of w / 2,
+// rows -1 .. R / 2): black on the band and a row on each side, red on the
+// band.  done(row, x, value) for every cell.
+template <int kColor, class Done>
+__device__ __forceinline__ void dsm_up(const Band& f, const float* ce, Done done) {
+    const int first = kColor == 1 ? -1 : 0, rows = kColor == 1 ? f.R + 2 : f.R;
+    const int n = rows * (f.w >> 1), w = f.w, cw = f.w >> 1;
+    for (int k = threadIdx.x; k < n; k += kTailThreads) {
+        int row, x;
+        band_cell(f, k, first, kColor, row, x);
+        const int i = row * w + x, cc = (row >> 1) * cw + (x >> 1);
+        float er = f.e[i + 1], eu = f.e[i + w], el = f.e[i - 1], ed = f.e[i - w], old = f.e[i];
+        if (kColor == 1) {
+            const bool xo = x & 1, yo = row & 1;
+            const CoarseAround a = coarse_around(ce, cc, cw, xo, yo);
+            old = old + a.c0;
+            er = er + (xo ? a.h : a.c0);
+            el = el + (xo ? a.c0 : a.h);
+            eu = eu + (yo ? a.v : a.c0);
+            ed = ed + (yo ? a.c0 : a.v);
+        } else {
+            old = old + ce[cc];
+        }
+        const float z = sor_masked(f.inv[i], f.r[i], f.px[i], f.py[i], f.px[i - 1], f.py[i - w], er, eu, el, ed, old);
+        f.e[i] = z;
+        done(row, x, z);
+    }
+}
+
+// Start copying the coefficients of a band and its halo (zero outside the
+// fluid; rows outside the grid are zeroed here) and zero its vectors.
+__device__ __forceinline__ void dsm_issue_coeffs(const DsmLevel& L, const Band& b, uint32_t rank) {
+    const int rows = b.R + 2 * kDsmHalo, n4 = rows * b.w / 4, n = band_floats(b.w, b.R);
+    const int base = (int(rank) * b.R - kDsmHalo) * b.w;  // raw index of the first halo row
+    const int cells = int(kDsmCtas) * b.R * b.w;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (threadIdx.x < 2 * kDsmPad) {  // before and after the rows
+        const int i = int(threadIdx.x) < kDsmPad ? int(threadIdx.x) : int(threadIdx.x) + rows * b.w;
+        for (int k = 0; k < 5; ++k) b.at[k * n + i] = 0.0f;
+    }
+    for (int j = threadIdx.x; j < n4; j += kTailThreads) {
+        const int raw = base + 4 * j;
+        float* to = b.at + kDsmPad + 4 * j;  // e; r, inv, px, py follow every n floats
+        *reinterpret_cast<float4*>(to) = zero;
+        *reinterpret_cast<float4*>(to + n) = zero;
+        if (raw >= 0 && raw < cells) {
+            const size_t g = size_t(raw) + b.w;
+            cp_async16(to + 2 * n, L.inv + g);
+            cp_async16(to + 3 * n, L.px + g);
+            cp_async16(to + 4 * n, L.py + g);
+            const int own = 4 * j - kDsmHalo * b.w;
+            if (own >= 0 && own < b.R * b.w) cp_async16(b.d + own, L.diag + g);
+        } else {
+            *reinterpret_cast<float4*>(to + 2 * n) = zero;
+            *reinterpret_cast<float4*>(to + 3 * n) = zero;
+            *reinterpret_cast<float4*>(to + 4 * n) = zero;
         }
     }
 }
 
-// Prolongation from the coarse level into own fine cells of one colour,
-// fused with that colour's post-sweep (ph_prolong's arithmetic).  Coarse
-// error from view c, or (c null) from the first tail level's error in CTA 0's
-// shared memory (tail_err, padded layout).
-__device__ __forceinline__ void dsm_prolong(const View& f, const cg::cluster_group& cl, const View* c,
-                                            const float* tail_err, int color) {
-    const int wc = f.w >> 1;
-    // coarse error under fine cell (x, y); outside the grid (a neighbour
-    // whose value a select drops) reads 0
-    auto coarse_e = [&](int x, int y) -> float {
-        if (y < 0 || y >= f.h) return 0.0f;
-        const int craw = (y >> 1) * wc + (x >> 1);
-        return c ? err_raw(*c, cl, craw) : tail_err[craw + wc];
-    };
-    const int half = f.w >> 1;
-    const int n = f.R * half;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        int row, k;
-        split(i, half, f.half_shift, row, k);
-        const int y = f.y0 + row;
-        const int x = 2 * k + ((y + color) & 1);
-        const int o = row * f.w + x;
-        if (!flb(f, o + f.w)) continue;  // only fluid cells store
-        const float old = prolonged(f.err[o], coarse_e(x, y), 0u);
-        float z;
-        if (color == 1)
-            z = sor_dsm(f, x, y, old, true, [&](int r, int xn, int yn) {
-                return prolonged(err_raw(f, cl, r), coarse_e(xn, yn), 0u);
-            });
-        else
-            z = sor_dsm(f, x, y, old, true, [&](int r, int, int) { return err_raw(f, cl, r); });
-        f.err[o] = z;
-    }
-}
-
-// Start copying this CTA's rows (plus halo) of every distributed level's mask
-// and coefficients into shared memory (they do not change during a solve).
-__device__ __forceinline__ void dsm_load_coeffs(const DsmParams& p, uint8_t* sm, uint32_t rank) {
-    for (int k = 0; k < p.n; ++k) {
-        const DsmLevel& L = p.lv[k];
-        const View v = view_of(L, sm, rank);
-        const int base = v.lo - L.w;  // raw index of local index 0
-        const int nh = (L.R + 2) * L.w;
-        // mask words of rows y0-1 .. y0+R (zero outside the grid)
-        uint32_t* flw = reinterpret_cast<uint32_t*>(sm + L.o_fl);
-        const int words = L.cells >> 5;
-        for (int j = threadIdx.x; j < (nh >> 5); j += blockDim.x) {
-            const int g = (base >> 5) + j;  // base is a multiple of 32 (w is)
-            if (g >= 0 && g < words) cp_async4(flw + j, L.fluid + g);
-            else flw[j] = 0u;
-        }
-        // 16-byte copies: base + w = y0 * w is a multiple of 32 floats and
-        // the arrays start 256-byte aligned; padded index base + i + w lies
-        // in [0, cells + 2w) for rows -1 .. h
-        for (int i = 4 * threadIdx.x; i < nh; i += 4 * blockDim.x) {
-            const size_t g = size_t(base + i + L.w);
-            cp_async16(const_cast<float*>(v.diag) + i, L.diag + g);
-            cp_async16(const_cast<float*>(v.inv) + i, L.inv + g);
-            cp_async16(const_cast<float*>(v.px) + i, L.px + g);
-            cp_async16(const_cast<float*>(v.py) + i, L.py + g);
-        }
-    }
-}
-
-// Start copying the first level's residual and first red sweep (written by
-// the kernel before this one).
-__device__ __forceinline__ void dsm_load_first(const DsmParams& p, uint8_t* sm, uint32_t rank) {
-    const DsmLevel& L = p.lv[0];
-    const View v = view_of(L, sm, rank);
-    const int no = L.R * L.w;
-    for (int i = 4 * threadIdx.x; i < no; i += 4 * blockDim.x) {
-        const size_t g = size_t(v.lo + i + L.w);
-        cp_async16(v.res + i, L.res + g);
-        cp_async16(v.err + i, L.err + g);
-    }
-}
-
-__global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_dsm(DsmParams p, TailParams tp, uint32_t dsm_off,
-                                                               uint32_t dsm_bytes, Ctl* ctl, ExitArgs exit) {
+__global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_dsm(const __grid_constant__ DsmParams p,
+                                                               const __grid_constant__ TailParams tp, uint32_t dsm_off,
+                                                               Ctl* ctl, ExitArgs exit) {
     extern __shared__ __align__(16) uint8_t smem[];
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t rank = cl.block_rank();
-    uint8_t* dsm = smem + dsm_off;
+    float* dsm = reinterpret_cast<float*>(smem + dsm_off);
     uint32_t* tail_sm = reinterpret_cast<uint32_t*>(smem);
-    // the first tail level's residual and error live in CTA 0's shared memory
-    float* tail_res = cl.map_shared_rank(reinterpret_cast<float*>(tail_sm) + tp.lv[0].o_res, 0);
-    const float* tail_err = cl.map_shared_rank(reinterpret_cast<float*>(tail_sm) + tp.lv[0].o_err, 0);
-    // Zero the distributed levels first (error and residual of cells outside
-    // the fluid mask are never written): with stale shared memory from
-    // earlier kernels in place the V-cycle reached NaN on scenes with fluid in
-    // every band (noise masks, 512^2), like the coarse tail did; the read
-    // that carried the stale value was not located.
-    for (uint32_t i = threadIdx.x; i < dsm_bytes / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(dsm)[i] = 0u;
-    __syncthreads();
+    const int n = p.n;
+    const Band first = band_at(dsm, p.w, p.R, p.hshift);
     // masks and coefficients were written by the multigrid setup, before the
-    // solve: their copies start while the previous kernel drains
-    if (rank == 0) cta_tail_issue_coeffs(tp, tail_sm);
-    dsm_load_coeffs(p, dsm, rank);
-    pdl_wait();
-    if (ctl->pcg_done) {  // the same value in every CTA: all reach every barrier
-        cp_async_wait_all();
-        return;
+    // solve: their copies start before the wait for the previous kernel
+    Band b = first;
+    for (int k = 0; k < n; ++k) {
+        if (k > 0) b = band_coarser(b);
+        dsm_issue_coeffs(p.lv[k], b, rank);
     }
-    dsm_load_first(p, dsm, rank);
-    // the exit test where this is the first kernel after the update: every CTA
-    // comes to the same verdict (one that finds it recorded returns above)
-    if (exit.on && pcg::exit_verdict(ctl, exit, rank == 0)) {
-        cp_async_wait_all();
-        return;
+    const Band last = b;
+    const int tw = last.w >> 1, tail_rows = last.R >> 1;
+    float* te = last.d + last.R * last.w;                 // the tail's error around the band
+    float* ti = te + (tail_rows + 2) * tw + 2 * kDsmPad;  // its inverse diagonal under it
+    for (int i = threadIdx.x; i < (tail_rows + 2) * tw + 2 * kDsmPad; i += kTailThreads) te[i] = 0.0f;
+    for (int i = threadIdx.x; i < tail_rows * tw; i += kTailThreads)
+        cp_async4(ti + i, p.tinv + (int(rank) * tail_rows + 1) * tw + i);
+    if (rank == 0) cta_tail_issue_coeffs(tp, tail_sm);
+    const int rows = first.R + 2 * kDsmHalo, n2 = rows * first.w / 2;
+    const int base = (int(rank) * first.R - kDsmHalo) * first.w;
+    uint32_t mask = 0;  // fluid bits of this thread's pairs of the finest level (at most 16 pairs: 220 KB)
+    for (int j = threadIdx.x, k = 0; j < n2; j += kTailThreads, k += 2) {
+        const int raw = base + 2 * j;
+        if (raw >= 0 && raw < p.cells) mask |= ((p.lv[0].fluid[raw >> 5] >> (raw & 31)) & 3u) << k;
+    }
+    __syncthreads();
+    // no CTA writes into another's shared memory before that one has zeroed
+    // it; waited for only before the first such write
+    cl.barrier_arrive();
+    pdl_wait();
+    // (the same value, and the same verdict, in every CTA)
+    bool done = ctl->pcg_done != 0;
+    if (!done) {
+        // the finest level's residual (written by the kernel before), halo included
+        for (int j = threadIdx.x; j < n2 / 2; j += kTailThreads) {
+            const int raw = base + 4 * j;
+            if (raw >= 0 && raw < p.cells)
+                cp_async16(first.r - kDsmHalo * first.w + 4 * j, p.res + size_t(raw) + first.w);
+        }
+        // the exit test where this is the first kernel after the update
+        done = exit.on && pcg::exit_verdict(ctl, exit, rank == 0);
     }
     cp_async_wait_all();
     __syncthreads();
-    cl.sync();
+    if (!done) {  // mask it (only the fluid cells' was written); its first red sweep
+        for (int j = threadIdx.x, k = 0; j < n2; j += kTailThreads, k += 2) {
+            const int i = 2 * j - kDsmHalo * first.w;
+            float2 r = *reinterpret_cast<const float2*>(first.r + i);
+            if (!((mask >> k) & 1u)) r.x = 0.0f;
+            if (!((mask >> k) & 2u)) r.y = 0.0f;
+            *reinterpret_cast<float2*>(first.r + i) = r;
+            // the red one of the pair: the first on even rows
+            const bool odd = ((2 * j) / first.w) & 1;
+            const float2 inv = *reinterpret_cast<const float2*>(first.inv + i);
+            *reinterpret_cast<float2*>(first.e + i) =
+                odd ? make_float2(0.0f, red_first(r.y, inv.y)) : make_float2(red_first(r.x, inv.x), 0.0f);
+        }
+    }
+    __syncthreads();
+    cl.barrier_wait();
+    if (done) return;
 
-    // views are rebuilt from the kernel parameters where needed (an array
-    // of them would live in local memory)
-    const int n = p.n;
+    Band f = first;
     for (int k = 0; k < n; ++k) {
-        const View f = view_of(p.lv[k], dsm, rank);
-        dsm_sweep(f, cl, 1, true);  // black sweep; red came with the residual
-        cl.sync();
+        dsm_black(f);
+        __syncthreads();
         if (k + 1 < n) {
-            const View c = view_of(p.lv[k + 1], dsm, rank);
-            dsm_restrict(f, cl, &c, p, tail_res, rank, true);
+            // the coarse band's residual and red sweep, and what the
+            // neighbours' halos need of them: red errors two rows out, the
+            // black cells' residual one row out
+            const Band c = band_coarser(f);
+            const Peers pe = peers_of(cl, c.e, rank), pr = peers_of(cl, c.r, rank);
+            dsm_restrict(f, [&](int row, int x, float sum) {
+                const int i = row * c.w + x;
+                const bool red = ((row + x) & 1) == 0;
+                const float e = red ? red_first(sum, c.inv[i]) : 0.0f;
+                c.r[i] = sum;
+                c.e[i] = e;
+                if (row < kDsmHalo && pe.has_below) {
+                    const int q = (c.R + row) * c.w + x;
+                    if (red) pe.below[q] = e;
+                    else if (row == 0) pr.below[q] = sum;
+                }
+                if (row >= c.R - kDsmHalo && pe.has_above) {
+                    const int q = (row - c.R) * c.w + x;
+                    if (red) pe.above[q] = e;
+                    else if (row == c.R - 1) pr.above[q] = sum;
+                }
+            });
+            f = c;
         } else {
-            dsm_restrict(f, cl, nullptr, p, tail_res, rank, false);
+            const SmemLevel t = smem_first(tp, tail_sm);
+            float* tr = cl.map_shared_rank(t.res, 0);
+            float* tz = cl.map_shared_rank(t.err, 0);
+            const int row0 = int(rank) * tail_rows;
+            dsm_restrict(f, [&](int row, int x, float sum) {
+                const int y = row0 + row, q = (y + 1) * tw + x;
+                tr[q] = sum;
+                tz[q] = ((x + y) & 1) == 0 ? red_first(sum, ti[row * tw + x]) : 0.0f;
+            });
         }
         cl.sync();
     }
-    if (rank == 0) cta_tail(tp, tail_sm, false, false);
+    if (rank == 0) {
+        cta_tail_levels(tp, tail_sm);
+        // every band's rows of the tail's error, and one on each side
+        const float* err = smem_first(tp, tail_sm).err;
+        const int per = (tail_rows + 2) * tw;
+        for (int i = threadIdx.x; i < per * int(kDsmCtas); i += kTailThreads) {
+            const int to = i / per, j = i - to * per;
+            // row -1 of the band of CTA `to` is row to * tail_rows of the padded layout
+            cl.map_shared_rank(te, to)[kDsmPad + j] = err[to * tail_rows * tw + j];
+        }
+    }
     cl.sync();
-    for (int k = n - 1; k >= 0; --k) {
-        const View f = view_of(p.lv[k], dsm, rank);
-        if (k + 1 < n) {
-            const View c = view_of(p.lv[k + 1], dsm, rank);
-            dsm_prolong(f, cl, &c, tail_err, 1);
-            cl.sync();
-            dsm_prolong(f, cl, &c, tail_err, 0);
-        } else {
-            dsm_prolong(f, cl, nullptr, tail_err, 1);
-            cl.sync();
-            dsm_prolong(f, cl, nullptr, tail_err, 0);
+    const float* ce = te + kDsmPad + tw;
+    for (int k = n - 1; k >= 1; --k) {
+        dsm_up<1>(f, ce, [](int, int, float) {});
+        __syncthreads();
+        // The finer level reads the coarse rows beside its own: the
+        // neighbours have those rows' black cells and are sent the red
+        // ones, into the residual's halo (whose red cells nothing reads),
+        // since they may still be sweeping with the errors they hold.
+        const Peers pr = peers_of(cl, f.r, rank);
+        dsm_up<0>(f, ce, [&](int row, int x, float z) {
+            if (row == 0 && pr.has_below) pr.below[f.R * f.w + x] = z;
+            if (row == f.R - 1 && pr.has_above) pr.above[-f.w + x] = z;
+        });
+        cl.sync();
+        for (int i = threadIdx.x; i < f.w; i += kTailThreads) {  // half a row's red cells on each side
+            const int half = f.w >> 1, row = i < half ? -1 : f.R;
+            const int q = row * f.w + 2 * (i < half ? i : i - half) + (row & 1);
+            f.e[q] = f.r[q];
         }
-        cl.sync();  // the next (finer) level reads this one's final error
+        __syncthreads();
+        ce = f.e;
+        f = band_finer(f);
     }
-    // the first level's final error, for the global prolongation above it
-    const DsmLevel& L0 = p.lv[0];
-    const View v0 = view_of(L0, dsm, rank);
-    const int no = L0.R * L0.w;
-    for (int i = threadIdx.x; i < no; i += blockDim.x)
-        if (flb(v0, i + L0.w)) L0.err[size_t(v0.lo + i + L0.w)] = v0.err[i];
+    // the finest level's final error goes to global memory
+    float* out = p.err + (int(rank) * f.R + 1) * f.w;
+    dsm_up<1>(f, ce, [&](int row, int x, float z) {
+        if (row >= 0 && row < f.R) out[row * f.w + x] = z;
+    });
+    __syncthreads();
+    dsm_up<0>(f, ce, [&](int row, int x, float z) { out[row * f.w + x] = z; });
 }
 
-size_t dsm_level_bytes(const Level& L, uint32_t R) {
-    const size_t nh = size_t(R + 2) * L.w, no = size_t(R) * L.w;
-    auto up16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-    return up16(nh / 8) + 4 * up16(4 * nh) + 2 * up16(4 * no);
+// Floats of one distributed level.
+size_t dsm_level_floats(const Level& L, uint32_t R) {
+    const size_t band = size_t(R + 2 * kDsmHalo) * L.w + 2 * kDsmPad;
+    return 5 * band + size_t(R) * L.w;
 }
 
 int log2_exact(uint32_t v) {
@@ -417,15 +403,18 @@ void plan_vcycle_dsm(Scene& s) {
     int d = 1;
     while (d < s.nlevels && s.lv[d].h >= kDsmTailRows) ++d;
     if (d >= s.nlevels || d < 2) return;
-    uint32_t tail_words = 0;
-    make_tail_params(s, d, &tail_words);
-    const size_t off = (size_t(tail_words) * 4 + 15) & ~size_t(15);
+    uint32_t tail_size = 0;
+    make_tail_params(s, d, &tail_size);
+    const size_t off = (size_t(tail_size) * 4 + 15) & ~size_t(15);
     size_t bytes = off;
     int m = d;
     for (int l = d - 1; l >= 1 && d - l <= kDsmMaxLevels; --l) {
         const Level& L = s.lv[l];
-        if (L.h % kDsmCtas != 0 || (L.w % 32u) || ((L.h / kDsmCtas) & 1u)) break;
-        const size_t b = bytes + dsm_level_bytes(L, L.h / kDsmCtas);
+        const uint32_t R = L.h / kDsmCtas;
+        if (L.h % kDsmCtas != 0 || (L.w % 32u) || (R & 1u)) break;
+        size_t b = bytes + 4 * dsm_level_floats(L, R);
+        // the tail's error around a band, its inverse diagonal under it
+        if (l == d - 1) b += 4 * (size_t(R + 2) * (L.w / 2) + 2 * kDsmPad);
         if (b > kDsmSmemBudget) break;
         bytes = b;
         m = l;
@@ -446,55 +435,28 @@ void plan_vcycle_dsm(Scene& s) {
 }
 
 // Levels dsm_first .. dsm_tail-1 and the tail in one cluster launch.  On
-// entry dsm_first's residual and first red sweep are in global memory
-// (the down kernel above it); on exit its final error is.
+// entry dsm_first's residual is in global memory (the down kernel above it);
+// on exit its final error is.
 void launch_vcycle_dsm(Scene& s, cudaStream_t st, const ExitArgs& exit) {
     DsmParams p = {};
-    p.first = s.dsm_first;
     p.n = s.dsm_tail - s.dsm_first;
-    uint32_t tail_words = 0;
-    TailParams tp = make_tail_params(s, s.dsm_tail, &tail_words);
-    size_t o = 0;  // level offsets are relative to the distributed region
-    auto take = [&](size_t bytes) {
-        const uint32_t at = uint32_t(o);
-        o += (bytes + 15) & ~size_t(15);
-        return at;
-    };
+    uint32_t tail_size = 0;
+    TailParams tp = make_tail_params(s, s.dsm_tail, &tail_size);
+    const Level& F = s.lv[s.dsm_first];
+    p.w = int(F.w);
+    p.R = int(F.h / kDsmCtas);
+    p.hshift = log2_exact(F.w / 2);
+    p.cells = int(F.cells);
+    p.res = F.res;
+    p.err = F.err;
+    p.tinv = s.lv[s.dsm_tail].inv_diag;
     for (int k = 0; k < p.n; ++k) {
         const Level& L = s.lv[s.dsm_first + k];
-        DsmLevel& d = p.lv[k];
-        d.w = int(L.w);
-        d.h = int(L.h);
-        d.cells = int(L.cells);
-        d.R = int(L.h / kDsmCtas);
-        d.rw_shift = log2_exact(uint32_t(d.R) * L.w);
-        d.half_shift = log2_exact(L.w / 2);
-        d.fluid = L.fluid;
-        d.diag = L.diag;
-        d.inv = L.inv_diag;
-        d.px = L.px;
-        d.py = L.py;
-        d.res = L.res;
-        d.err = L.err;
-        const size_t nh = size_t(d.R + 2) * L.w, no = size_t(d.R) * L.w;
-        d.o_fl = take(nh / 8);
-        d.o_diag = take(4 * nh);
-        d.o_inv = take(4 * nh);
-        d.o_px = take(4 * nh);
-        d.o_py = take(4 * nh);
-        d.o_res = take(4 * no);
-        d.o_err = take(4 * no);
+        p.lv[k] = DsmLevel{L.fluid, L.diag, L.inv_diag, L.px, L.py};
     }
-    const Level& T = s.lv[s.dsm_tail];
-    p.tw = int(T.w);
-    p.tcells = int(T.cells);
-    p.tfluid = T.fluid;
-    p.tres = T.res;
-    p.terr = T.err;
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = dsm_config(s.dsm_smem, st, attr, s.use_pdl);
-    cudaLaunchKernelEx(&cfg, k_vcycle_dsm, p, tp, s.dsm_off, uint32_t(s.dsm_smem - s.dsm_off),
-                       s.ctl, exit);
+    cudaLaunchKernelEx(&cfg, k_vcycle_dsm, p, tp, s.dsm_off, s.ctl, exit);
 }
 
 }  // namespace apic
