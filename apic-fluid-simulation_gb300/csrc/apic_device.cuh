@@ -26,6 +26,15 @@ __device__ __forceinline__ float rclamp(float x, float lo, float hi) {
     return x;
 }
 
+// Grid coordinate p / dx.  A power-of-two cell size divides by multiplying
+// with its reciprocal, which is exact (the same product rounds the same way),
+// instead of the 20-odd instructions of an IEEE division; inv is 0 for any
+// other size (exact_reciprocal).
+struct CellSize {
+    float dx, inv;
+};
+__device__ __forceinline__ float over_dx(float p, CellSize c) { return c.inv != 0.0f ? p * c.inv : p / c.dx; }
+
 // temporal_kernel_w_t, src/apic.rs:31-46.
 __device__ __forceinline__ float temporal_w(float tau) {
     float ts = tau - 0.5f;

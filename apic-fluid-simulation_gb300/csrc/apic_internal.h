@@ -20,6 +20,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <string>
 
@@ -400,6 +401,13 @@ int update_prepare(apic_handle* h);       // build the update graph ahead of the
 cudaStream_t scene_stream(apic_handle* h);
 
 // helpers shared by the launchers
+// 1 / dx where dx is a power of two whose reciprocal is a normal number (a
+// division by dx is then exactly a multiplication by it), else 0.
+inline float exact_reciprocal(float dx) {
+    int e = 0;
+    if (!(dx > 0.0f) || std::frexp(dx, &e) != 0.5f || e < -124 || e > 126) return 0.0f;
+    return 1.0f / dx;
+}
 inline uint32_t div_up(uint64_t a, uint64_t b) { return uint32_t((a + b - 1) / b); }
 
 // Launch kern on st.  pdl: programmatic dependent launch, so the kernel's

@@ -64,11 +64,11 @@ cudaError_t scratch_for_current_context(uint32_t** out) {
 
 // Morton key of each particle's clamped cell and its slot (src/apic.rs:1049-1064).
 __global__ void k_keys_from_positions(const float* __restrict__ px, const float* __restrict__ py, uint32_t n,
-                                      float dx, float max_x, float max_y, uint32_t* __restrict__ keys,
+                                      CellSize cs, float max_x, float max_y, uint32_t* __restrict__ keys,
                                       uint32_t* __restrict__ vals) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float gx = px[i] / dx, gy = py[i] / dx;
+    float gx = over_dx(px[i], cs), gy = over_dx(py[i], cs);
     uint32_t cx = uint32_t(trunc_x86(fmin_x86(fmax_x86(gx, 0.0f), max_x)));
     uint32_t cy = uint32_t(trunc_x86(fmin_x86(fmax_x86(gy, 0.0f), max_y)));
     keys[i] = morton(cx, cy);
@@ -106,7 +106,8 @@ extern "C" int apic_morton_sort_noalloc(const float* pos_x, const float* pos_y, 
     uint32_t* hist = scratch + 2ull * kNoAllocMaxKeys;
     uint32_t* scan_tmp = hist + kHistWords;
     float max_x = float(width - 1), max_y = float(height - 1);
-    k_keys_from_positions<<<div_up(n, 256), 256, 0, st>>>(pos_x, pos_y, n, cell_size, max_x, max_y, keys_out,
+    k_keys_from_positions<<<div_up(n, 256), 256, 0, st>>>(pos_x, pos_y, n, CellSize{cell_size, exact_reciprocal(cell_size)},
+                                                          max_x, max_y, keys_out,
                                                           vals_out);
     e = radix_sort_pairs_in(keys_out, vals_out, keys_alt, vals_alt, hist, scan_tmp, n,
                             morton_key_bits(width, height), st);

@@ -101,7 +101,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_u32(uint32_t v, uint32_
 // Four particles per thread with 16-byte loads and stores (the arrays hold
 // npad, a multiple of 8, lanes; keys of lanes n .. npad-1 are never read).
 __global__ void __launch_bounds__(256) k_p2g_bin_keys(const PartPtrs* __restrict__ pp, uint32_t n, int W, int H,
-                                                      float dx, uint32_t* __restrict__ keys,
+                                                      CellSize cs, uint32_t* __restrict__ keys,
                                                       uint32_t* __restrict__ vals, uint32_t* __restrict__ fluid) {
     pdl_wait();
     const uint32_t i0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) k_p2g_bin_keys(const PartPtrs* __restrict
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const bool live = i0 + uint32_t(q) < n;
-        const float gx = xs[q] / dx, gy = ys[q] / dx;
+        const float gx = over_dx(xs[q], cs), gy = over_dx(ys[q], cs);
         const int cx0 = max(min(trunc_x86(floorf(gx - 0.5f)), W - 1), 0);
         const int cy0 = max(min(trunc_x86(floorf(gy - 0.5f)), H - 1), 0);
         k[q] = uint32_t(cy0) * uint32_t(W) + uint32_t(cx0);
@@ -162,13 +162,14 @@ struct P2gRec {
 struct P2gBase {
     float gx, gy, wt;
 };
-__device__ __forceinline__ P2gBase p2g_base(const PartPtrs* __restrict__ pp, uint32_t slot, float dx, float prev_dt) {
+__device__ __forceinline__ P2gBase p2g_base(const PartPtrs* __restrict__ pp, uint32_t slot, CellSize cs,
+                                            float prev_dt) {
     const float tr = pp->f[TR][slot];
     const float tau = (-tr) / prev_dt;
     P2gBase b;
     b.wt = temporal_w(tau);
-    b.gx = pp->f[PX][slot] / dx;
-    b.gy = pp->f[PY][slot] / dx;
+    b.gx = over_dx(pp->f[PX][slot], cs);
+    b.gy = over_dx(pp->f[PY][slot], cs);
     return b;
 }
 
@@ -253,7 +254,8 @@ struct GlobalRecs {
     const uint32_t* vals;  // sorted slots
     const PartPtrs* pp;
     int grid, W, H;
-    float dx, prev_dt;
+    CellSize cs;
+    float prev_dt;
     uint32_t* status;
     uint32_t n, npad;  // sorted pairs, particle lanes (the checked build tests against them)
     __device__ __forceinline__ uint32_t slot_at(int p) const {
@@ -263,7 +265,7 @@ struct GlobalRecs {
     __device__ __forceinline__ P2gRec rec(int p) const {
         P2gRec r;
         const uint32_t sl = slot_at(p);
-        if (!p2g_record(pp, sl, p2g_base(pp, sl, dx, prev_dt), grid, W, H, dx, r)) atomicOr(status, kStatusP2gLayout);
+        if (!p2g_record(pp, sl, p2g_base(pp, sl, cs, prev_dt), grid, W, H, cs.dx, r)) atomicOr(status, kStatusP2gLayout);
         return r;
     }
     __device__ __forceinline__ uint32_t code_at(int p) const { return rec(p).code; }
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(kGatherThreads, 2) k_p2g_gather(const PartPtrs
                                                                   const uint32_t* __restrict__ vals,
                                                                   const uint32_t* __restrict__ lo,
                                                                   const uint32_t* __restrict__ hi, int W, int H,
-                                                                  float dx, Ctl* __restrict__ ctl, GatherOut o,
+                                                                  CellSize cs, Ctl* __restrict__ ctl, GatherOut o,
                                                                   uint32_t n, uint32_t npad) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* s_slot = reinterpret_cast<uint32_t*>(smem);
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(kGatherThreads, 2) k_p2g_gather(const PartPtrs
         // more particles than the stage holds even for one row: every face
         // reads its runs from global memory and computes the records it needs
         for (int g = 0; g < 3; ++g) {
-            GlobalRecs R{vals, pp, g, W, H, dx, prev_dt, &ctl->status, n, npad};
+            GlobalRecs R{vals, pp, g, W, H, cs, prev_dt, &ctl->status, n, npad};
             auto bin = [&](int x, int y, int& b, int& e) {
                 const uint32_t c = uint32_t(y) * uint32_t(W) + uint32_t(x);
                 b = int(lo[c]);
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(kGatherThreads, 2) k_p2g_gather(const PartPtrs
             __syncthreads();
         }
         for (uint32_t p = threadIdx.x; p < P; p += kGatherThreads) {
-            const P2gBase bs = p2g_base(pp, s_slot[p] & ~kLastInRun, dx, prev_dt);
+            const P2gBase bs = p2g_base(pp, s_slot[p] & ~kLastInRun, cs, prev_dt);
             s_gx[p] = bs.gx;
             s_gy[p] = bs.gy;
             s_wt[p] = bs.wt;
@@ -576,7 +578,7 @@ __global__ void __launch_bounds__(kGatherThreads, 2) k_p2g_gather(const PartPtrs
             for (uint32_t p = threadIdx.x; p < P; p += kGatherThreads) {
                 P2gRec rec;
                 const P2gBase bs{s_gx[p], s_gy[p], s_wt[p]};
-                if (!p2g_record(pp, s_slot[p] & ~kLastInRun, bs, g, W, H, dx, rec)) bad = true;
+                if (!p2g_record(pp, s_slot[p] & ~kLastInRun, bs, g, W, H, cs.dx, rec)) bad = true;
                 s_code[p] = rec.code;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -624,24 +626,93 @@ __device__ __forceinline__ void add_partials(const P2gRec& rec, float (&pv)[NQ],
     }
 }
 
+// A particle whose three stencils lie inside their grids, so that no index is
+// clamped: its u corners start at column 0 or 1 of the six positions, its v
+// corners at row 0 or 1, its density corners are the four positions.  Every
+// position then takes at most one corner, by a select, where the general form
+// tests each corner against each position (24 tests a grid).
+__device__ __forceinline__ bool p2g_inside(const P2gBase& b, int W, int H) {
+    const float cx = floorf(b.gx - 0.5f), cy = floorf(b.gy - 0.5f);
+    return cx >= 0.0f && cx <= float(W - 2) && cy >= 0.0f && cy <= float(H - 2);
+}
+struct P2gRaw {
+    float px, py, tr, vx, cux, cuy, vy, cvx, cvy;
+};
+__device__ __forceinline__ P2gRaw p2g_raw(const PartPtrs* __restrict__ pp, uint32_t slot) {
+    return P2gRaw{pp->f[PX][slot],  pp->f[PY][slot],  pp->f[TR][slot],  pp->f[VX][slot], pp->f[CUX][slot],
+                  pp->f[CUY][slot], pp->f[VY][slot], pp->f[CVX][slot], pp->f[CVY][slot]};
+}
+__device__ __forceinline__ P2gBase p2g_base(const P2gRaw& r, CellSize cs, float prev_dt) {
+    const float tau = (-r.tr) / prev_dt;
+    return P2gBase{over_dx(r.px, cs), over_dx(r.py, cs), temporal_w(tau)};
+}
+__device__ __forceinline__ void p2g_add_inside(const P2gRaw& p, const P2gBase& b, int W, int H, float dx,
+                                               float (&uv)[6], float (&uw)[6], float (&vv)[6], float (&vw)[6],
+                                               float (&dw)[4]) {
+    Stencil su, sv;
+    u_stencil(b.gx, b.gy, W, H, dx, su);
+    v_stencil(b.gx, b.gy, W, H, dx, sv);
+    const float cgx = b.gx - 0.5f, cgy = b.gy - 0.5f;
+    const float cbx = floorf(cgx), cby = floorf(cgy);
+    const bool sx = floorf(b.gx) != cbx, sy = floorf(b.gy) != cby;
+    float w[4], v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        w[k] = su.w[k] * b.wt;
+        v[k] = (p.vx + p.cux * su.ox[k] + p.cuy * su.oy[k]) * w[k];
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        uv[3 * r + 0] = uv[3 * r + 0] + (sx ? 0.0f : v[2 * r]);
+        uv[3 * r + 1] = uv[3 * r + 1] + (sx ? v[2 * r] : v[2 * r + 1]);
+        uv[3 * r + 2] = uv[3 * r + 2] + (sx ? v[2 * r + 1] : 0.0f);
+        uw[3 * r + 0] = uw[3 * r + 0] + (sx ? 0.0f : w[2 * r]);
+        uw[3 * r + 1] = uw[3 * r + 1] + (sx ? w[2 * r] : w[2 * r + 1]);
+        uw[3 * r + 2] = uw[3 * r + 2] + (sx ? w[2 * r + 1] : 0.0f);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        w[k] = sv.w[k] * b.wt;
+        v[k] = (p.vy + p.cvx * sv.ox[k] + p.cvy * sv.oy[k]) * w[k];
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        vv[c] = vv[c] + (sy ? 0.0f : v[c]);
+        vv[2 + c] = vv[2 + c] + (sy ? v[c] : v[2 + c]);
+        vv[4 + c] = vv[4 + c] + (sy ? v[2 + c] : 0.0f);
+        vw[c] = vw[c] + (sy ? 0.0f : w[c]);
+        vw[2 + c] = vw[2 + c] + (sy ? w[c] : w[2 + c]);
+        vw[4 + c] = vw[4 + c] + (sy ? w[2 + c] : 0.0f);
+    }
+    const float ctx = cgx - cbx, cty = cgy - cby;
+    dw[0] = dw[0] + ((1.0f - ctx) * (1.0f - cty)) * b.wt;
+    dw[1] = dw[1] + (ctx * (1.0f - cty)) * b.wt;
+    dw[2] = dw[2] + ((1.0f - ctx) * cty) * b.wt;
+    dw[3] = dw[3] + (ctx * cty) * b.wt;
+}
+
 // One thread per region cell (352 threads for 340 cells, then the tile's 256
-// cells' faces), two CTAs per SM: the per-cell loops are load-latency bound.
+// cells' faces), two CTAs per SM.  The per-cell loops wait on loads: slot,
+// then nine fields, then some 230 instructions.  The slot two particles ahead
+// and the fields one ahead are in flight meanwhile (80 registers; three CTAs
+// with 56 and spills were faster without the fields ahead, are slower with
+// them: 460 against 352 us).  1024^2 dam break (1.0 M particles) 73 -> 53 us,
+// 2048^2 noise (8.3 M) 589 -> 352 us, of which the selects of
+// p2g_add_inside and the exact reciprocal took 17 and 182.
 constexpr int kCellThreads = 352;
-// kMinB 3 (56 registers, some spilled) for grids of more than 2 M cells
-// (4096^2: 3.56 vs 3.79 ms per P2G stage), 2 below.
-template <int kMinB>
-__global__ void __launch_bounds__(kCellThreads, kMinB) k_p2g_cells(const PartPtrs* __restrict__ pp,
-                                                                 const uint32_t* __restrict__ vals,
-                                                                 const uint32_t* __restrict__ lo,
-                                                                 const uint32_t* __restrict__ hi, int W, int H,
-                                                                 float dx, Ctl* __restrict__ ctl, GatherOut o,
-                                                                 uint32_t n, uint32_t npad) {
+__global__ void __launch_bounds__(kCellThreads, 2) k_p2g_cells(const PartPtrs* __restrict__ pp,
+                                                             const uint32_t* __restrict__ vals,
+                                                             const uint32_t* __restrict__ lo,
+                                                             const uint32_t* __restrict__ hi, int W, int H,
+                                                             CellSize cs, Ctl* __restrict__ ctl, GatherOut o,
+                                                             uint32_t n, uint32_t npad) {
     __shared__ CellPartials sp;
+    const float dx = cs.dx;
     const int x0 = blockIdx.x * kGatherTW, y0 = blockIdx.y * kGatherTH;
     const int rx0 = x0 - 2, ry0 = y0 - 2;
     pdl_wait();
     const float prev_dt = ctl->prev_dt;
-    bool bad = false;
+    bool bad = false, some = false;
     for (int rc = threadIdx.x; rc < kCellRegion; rc += kCellThreads) {
         const int x = rx0 + rc % kRegionW, y = ry0 + rc / kRegionW;
         uint32_t b = 0, e = 0;
@@ -651,20 +722,31 @@ __global__ void __launch_bounds__(kCellThreads, kMinB) k_p2g_cells(const PartPtr
             e = hi[c];
         }
         float uv[6] = {}, uw[6] = {}, vv[6] = {}, vw[6] = {}, dv[4] = {}, dw[4] = {};
-        // the next particle's slot is loaded while this one's fields are
+        // two particles ahead the slot is loaded, one ahead the fields
         if (!APIC_IN_BOUNDS(e, uint64_t(n) + 1u, &ctl->status)) e = b;
-        uint32_t next = b < e ? vals[b] : 0u;
+        auto slot_at = [&](uint32_t p) {
+            const uint32_t sl = p < e ? vals[p] : 0u;
+            return APIC_IN_BOUNDS(sl, npad, &ctl->status) ? sl : 0u;
+        };
+        uint32_t slot = slot_at(b), next = slot_at(b + 1);
+        P2gRaw raw = b < e ? p2g_raw(pp, slot) : P2gRaw{};
         for (uint32_t p = b; p < e; ++p) {
-            const uint32_t slot = next;
-            if (p + 1 < e) next = vals[p + 1];
-            if (!APIC_IN_BOUNDS(slot, npad, &ctl->status)) continue;
-            const P2gBase bs = p2g_base(pp, slot, dx, prev_dt);
+            const P2gRaw cur = raw;
+            const uint32_t here = slot;
+            slot = next;
+            if (p + 1 < e) raw = p2g_raw(pp, slot);
+            next = slot_at(p + 2);
+            const P2gBase bs = p2g_base(cur, cs, prev_dt);
+            if (p2g_inside(bs, W, H)) {
+                p2g_add_inside(cur, bs, W, H, dx, uv, uw, vv, vw, dw);
+                continue;
+            }
             P2gRec rec;
-            if (!p2g_record(pp, slot, bs, kGridU, W, H, dx, rec)) bad = true;
+            if (!p2g_record(pp, here, bs, kGridU, W, H, dx, rec)) bad = true;
             add_partials<6, true>(rec, uv, uw);
-            if (!p2g_record(pp, slot, bs, kGridV, W, H, dx, rec)) bad = true;
+            if (!p2g_record(pp, here, bs, kGridV, W, H, dx, rec)) bad = true;
             add_partials<6, true>(rec, vv, vw);
-            if (!p2g_record(pp, slot, bs, kGridD, W, H, dx, rec)) bad = true;
+            if (!p2g_record(pp, here, bs, kGridD, W, H, dx, rec)) bad = true;
             add_partials<4, false>(rec, dv, dw);
         }
 #pragma unroll
@@ -677,9 +759,10 @@ __global__ void __launch_bounds__(kCellThreads, kMinB) k_p2g_cells(const PartPtr
 #pragma unroll
         for (int q = 0; q < 4; ++q) sp.dw[q][rc] = dw[q];
         sp.has[rc] = e > b;
+        some = e > b;
     }
     if (bad) atomicOr(&ctl->status, kStatusP2gLayout);
-    __syncthreads();
+    some = __syncthreads_or(some) != 0;  // (a region without particles: zeros, no sums)
     if (threadIdx.x >= kGatherThreads) return;
     const int tx = threadIdx.x % kGatherTW, ty = threadIdx.x / kGatherTW;
     const int i = x0 + tx, j = y0 + ty;
@@ -687,7 +770,7 @@ __global__ void __launch_bounds__(kCellThreads, kMinB) k_p2g_cells(const PartPtr
     // region index of cell (x, y), or -1 when it holds no particle (or lies
     // outside the grid)
     auto cell = [&](int x, int y) -> int {
-        if (x < 0 || y < 0 || x >= W || y >= H) return -1;
+        if (!some || x < 0 || y < 0 || x >= W || y >= H) return -1;
         const int rc = (y - ry0) * kRegionW + (x - rx0);
         return sp.has[rc] ? rc : -1;
     };
@@ -923,6 +1006,8 @@ static int bin_key_bits(const Scene& s) {
     return b;
 }
 
+static CellSize cell_size(const Scene& s) { return CellSize{s.dx, exact_reciprocal(s.dx)}; }
+
 // P2G stage; bin_lo / bin_hi and the base fluid mask must be zero (the
 // caller clears them), every accumulator entry is written.
 cudaError_t launch_p2g(Scene& s) {
@@ -933,7 +1018,7 @@ cudaError_t launch_p2g(Scene& s) {
     const uint32_t* svals = s.bin_vals;
     if (s.n > 0) {
         launch(s.use_pdl, k_p2g_bin_keys, div_up(s.n, 1024), 256, 0, s.stream, static_cast<const PartPtrs*>(s.pp), s.n,
-               int(s.W), int(s.H), s.dx, s.bin_keys, s.bin_vals, s.lv[0].fluid);
+               int(s.W), int(s.H), cell_size(s), s.bin_keys, s.bin_vals, s.lv[0].fluid);
         uint32_t *kres, *vres;
         e = radix_sort_pairs(s.bin_keys, s.bin_vals, s.bin_keys_alt, s.bin_vals_alt, s.sort_hist, s.sort_scan_tmp, s.n,
                              bin_key_bits(s), s.stream, s.use_pdl, &kres, &vres, &s.ctl->status);
@@ -947,12 +1032,11 @@ cudaError_t launch_p2g(Scene& s) {
     if (ref)
         launch(s.use_pdl && s.n > 0, k_p2g_gather<true>, grid, kGatherThreads, kGatherSmem, s.stream,
                static_cast<const PartPtrs*>(s.pp), svals, static_cast<const uint32_t*>(s.bin_lo),
-               static_cast<const uint32_t*>(s.bin_hi), int(s.W), int(s.H), s.dx, s.ctl, o, s.n, s.npad);
+               static_cast<const uint32_t*>(s.bin_hi), int(s.W), int(s.H), cell_size(s), s.ctl, o, s.n, s.npad);
     else
-        launch(s.use_pdl && s.n > 0, s.cells > (2u << 20) ? k_p2g_cells<3> : k_p2g_cells<2>, grid, kCellThreads, 0,
-               s.stream,
+        launch(s.use_pdl && s.n > 0, k_p2g_cells, grid, kCellThreads, 0, s.stream,
                static_cast<const PartPtrs*>(s.pp), svals, static_cast<const uint32_t*>(s.bin_lo),
-               static_cast<const uint32_t*>(s.bin_hi), int(s.W), int(s.H), s.dx, s.ctl, o, s.n, s.npad);
+               static_cast<const uint32_t*>(s.bin_hi), int(s.W), int(s.H), cell_size(s), s.ctl, o, s.n, s.npad);
     return cudaGetLastError();
 }
 

@@ -33,7 +33,7 @@ constexpr int kScanBlock = 1024;                  // elements per scan block
 // Four particles per thread with 16-byte loads and stores: the particle
 // arrays and the pair buffers hold npad (a multiple of 8) lanes, so lanes
 // n .. npad-1 get keys too, which the sort of n pairs never reads.
-__global__ void __launch_bounds__(256) k_morton_keys(const PartPtrs* __restrict__ pp, uint32_t n, float dx, float max_x,
+__global__ void __launch_bounds__(256) k_morton_keys(const PartPtrs* __restrict__ pp, uint32_t n, CellSize cs, float max_x,
                                                      float max_y, uint32_t* __restrict__ keys,
                                                      uint32_t* __restrict__ vals) {
     pdl_wait();
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) k_morton_keys(const PartPtrs* __restrict_
     uint32_t k[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const float gx = xs[q] / dx, gy = ys[q] / dx;  // Vec2x8 / f32x8: per-component division
+        const float gx = over_dx(xs[q], cs), gy = over_dx(ys[q], cs);  // Vec2x8 / f32x8: per-component division
         const uint32_t cx = uint32_t(trunc_x86(fmin_x86(fmax_x86(gx, 0.0f), max_x)));
         const uint32_t cy = uint32_t(trunc_x86(fmin_x86(fmax_x86(gy, 0.0f), max_y)));
         k[q] = morton(cx, cy);
@@ -319,7 +319,8 @@ bool radix_sort_in_alt(int bits) {
 cudaError_t launch_sort(Scene& s) {
     if (s.n == 0) return cudaSuccess;
     float max_x = float(s.W > 0 ? s.W - 1 : 0), max_y = float(s.H > 0 ? s.H - 1 : 0);
-    launch(s.use_pdl, k_morton_keys, div_up(s.n, 1024), 256, 0, s.stream, s.pp, s.n, s.dx, max_x, max_y, s.keys,
+    launch(s.use_pdl, k_morton_keys, div_up(s.n, 1024), 256, 0, s.stream, s.pp, s.n,
+           CellSize{s.dx, exact_reciprocal(s.dx)}, max_x, max_y, s.keys,
            s.vals);
     // the sorted pairs stay where the last pass wrote them (no copy back)
     uint32_t *k_res, *v_res;
