@@ -142,54 +142,122 @@ __global__ void k_tile_ranges(const uint32_t* __restrict__ keys, uint32_t m, uin
 __device__ __forceinline__ uint32_t blend8(float c, float a, uint32_t dst, const float* d8) {
     const float d = d8[dst];
     const float o = c * a + d * (1.0f - a);
-    const float q = o * 255.0f + 0.5f;
-    return q >= 255.0f ? 255u : (q > 0.0f ? uint32_t(q) : 0u);
+    // (finite: the conversion saturates below zero)
+    return __float2uint_rz(fminf(o * 255.0f + 0.5f, 255.0f));
 }
 
 // One CTA per 16 x 16 tile, one thread per pixel: blend the tile's quads in
-// particle order.
+// particle order.  The kernel is bound by instructions, so a thread should
+// meet only the quads that cover its pixel, a warp should have few idle lanes
+// while it blends, and warps should not wait for each other (particles are
+// Morton-sorted: a stretch of the tile's list covers a corner of the tile).
+// So each warp owns 8 x 4 pixels and goes through the tile's list by itself:
+// it lists the quads that touch its pixels, with the columns and rows they
+// cover (the exact comparisons, a bit each), up to kWindow of them; then every
+// lane collects the listed quads that cover its pixel in bit masks, and the
+// lanes walk their masks side by side, each blending another quad.  The disc's
+// texels have their clamped border around them, so a bilinear sample is four
+// loads from one address.  1920 x 1080, 1.1 M particles (4 to a pixel, 144
+// blends a pixel): 995 us when every pixel tested every quad of the tile and
+// a warp blended one quad at a time (14 lanes of 32 active), 340 us now (27).
+constexpr uint32_t kWindow = 512;
+constexpr uint32_t kRasterGroups = 4;  // 32-quad groups of the list loaded at once
 __global__ void __launch_bounds__(kTileThreads) k_splat_raster(const uint32_t* __restrict__ vals,
                                                               const uint32_t* __restrict__ start,
                                                               const uint32_t* __restrict__ end,
                                                               const float4* __restrict__ quad, RenderParamsDev p,
                                                               uint32_t* __restrict__ frame) {
-    __shared__ float tex[kTex * kTex];
+    constexpr uint32_t kWarps = kTileThreads / 32;
+    __shared__ float tex[(kTex + 2) * (kTex + 2)];
     __shared__ float d8[256];
-    __shared__ float4 ent[kTileThreads];
-    for (int t = threadIdx.x; t < kTex * kTex; t += kTileThreads)
-        tex[t] = float(circle_alpha(t % kTex, t / kTex)) / 255.0f;
+    __shared__ uint32_t list[kWarps][kWindow];            // quads that touch the warp's pixels
+    __shared__ uint16_t cover[kWarps][kWindow];           // bit k: column k of the 8; bit 8 + k: row k of the 4
+    __shared__ uint32_t masks[kWarps][kWindow / 32][32];  // per lane: which of them cover its pixel
+    for (int t = threadIdx.x; t < (kTex + 2) * (kTex + 2); t += kTileThreads) {
+        const int x = min(max(t % (kTex + 2) - 1, 0), kTex - 1), y = min(max(t / (kTex + 2) - 1, 0), kTex - 1);
+        tex[t] = float(circle_alpha(x, y)) / 255.0f;
+    }
     d8[threadIdx.x] = float(threadIdx.x) / 255.0f;
+    __syncthreads();
     const uint32_t tile = blockIdx.x;
-    const uint32_t px = (tile % p.ntx) * kTile + (threadIdx.x % kTile);
-    const uint32_t py = (tile / p.ntx) * kTile + (threadIdx.x / kTile);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t px0 = (tile % p.ntx) * kTile + (warp & 1u) * 8u, py0 = (tile / p.ntx) * kTile + (warp >> 1) * 4u;
+    const uint32_t px = px0 + (lane & 7u), py = py0 + (lane >> 3);
+    const uint32_t mine = (1u << (lane & 7u)) | (0x100u << (lane >> 3));
     const float cx = float(px) + 0.5f, cy = float(py) + 0.5f;
     uint32_t dr = p.bg & 0xFFu, dg = (p.bg >> 8) & 0xFFu, db = (p.bg >> 16) & 0xFFu;
     const uint32_t b0 = start[tile], b1 = end[tile];
-    __syncthreads();
-    for (uint32_t base = b0; base < b1; base += kTileThreads) {
-        const uint32_t j = base + threadIdx.x;
-        if (j < b1) ent[threadIdx.x] = quad[vals[j]];
-        __syncthreads();
-        const uint32_t cnt = min(kTileThreads, b1 - base);
-        for (uint32_t e = 0; e < cnt; ++e) {
-            const float4 q = ent[e];
-            if (!(q.x <= cx && cx < q.x + p.size && q.y <= cy && cy < q.y + p.size)) continue;
-            const float u = (cx - q.x) * p.tex_scale - 0.5f;
-            const float v = (cy - q.y) * p.tex_scale - 0.5f;
+    uint32_t n = 0;
+    for (uint32_t base = b0; base < b1; base += 32u * kRasterGroups) {
+        uint32_t id[kRasterGroups];
+        float4 q[kRasterGroups];
+#pragma unroll
+        for (uint32_t g = 0; g < kRasterGroups; ++g) {
+            const uint32_t j = base + 32u * g + lane;
+            id[g] = j < b1 ? vals[j] : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (uint32_t g = 0; g < kRasterGroups; ++g)
+            q[g] = id[g] != 0xFFFFFFFFu ? quad[id[g]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (uint32_t g = 0; g < kRasterGroups; ++g) {
+            uint32_t m = 0;
+            const float x1 = q[g].x + p.size, y1 = q[g].y + p.size;
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) {
+                const float x = float(px0 + k) + 0.5f;
+                if (q[g].x <= x && x < x1) m |= 1u << k;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                const float y = float(py0 + k) + 0.5f;
+                if (q[g].y <= y && y < y1) m |= 0x100u << k;
+            }
+            const bool hit = id[g] != 0xFFFFFFFFu && (m & 0xFFu) && (m & 0xF00u);
+            const uint32_t votes = __ballot_sync(0xffffffffu, hit);
+            if (hit) {
+                const uint32_t at = n + uint32_t(__popc(votes & ((1u << lane) - 1u)));
+                list[warp][at] = id[g];
+                cover[warp][at] = uint16_t(m);
+            }
+            n += uint32_t(__popc(votes));
+        }
+        // (the next groups add at most 32 * kRasterGroups)
+        if (n + 32u * kRasterGroups <= kWindow && base + 32u * kRasterGroups < b1) continue;
+        __syncwarp();
+        const uint32_t words = (n + 31u) / 32u;
+        for (uint32_t w = 0; w < words; ++w) {
+            const uint32_t left = min(32u, n - 32u * w);
+            uint32_t todo = 0;
+            for (uint32_t k = 0; k < left; ++k)
+                if ((cover[warp][32u * w + k] & mine) == mine) todo |= 1u << k;
+            masks[warp][w][lane] = todo;
+        }
+        uint32_t w = 0, todo = words ? masks[warp][0][lane] : 0u;  // (a lane reads its own words)
+        for (;;) {
+            while (!todo && ++w < words) todo = masks[warp][w][lane];
+            if (!todo) break;
+            const uint32_t k = 32u * w + uint32_t(__ffs(int(todo))) - 1u;
+            todo &= todo - 1u;
+            const float4 e = quad[list[warp][k]];
+            const float u = (cx - e.x) * p.tex_scale - 0.5f;
+            const float v = (cy - e.y) * p.tex_scale - 0.5f;
             const float fu = floorf(u), fv = floorf(v);
             const float wu = u - fu, wv = v - fv;
-            const int iu = int(fu), iv = int(fv);
-            const int u0 = min(max(iu, 0), kTex - 1), u1 = min(max(iu + 1, 0), kTex - 1);
-            const int v0 = min(max(iv, 0), kTex - 1), v1 = min(max(iv + 1, 0), kTex - 1);
-            const float top = tex[v0 * kTex + u0] * (1.0f - wu) + tex[v0 * kTex + u1] * wu;
-            const float bot = tex[v1 * kTex + u0] * (1.0f - wu) + tex[v1 * kTex + u1] * wu;
+            // a covered pixel samples from -0.5 to 31.5: texels -1 .. 32 (clamped
+            // all the same, so that no rounding can reach outside the table)
+            const int iu = min(max(int(fu), -1), kTex - 1), iv = min(max(int(fv), -1), kTex - 1);
+            const float* t = tex + (iv + 1) * (kTex + 2) + iu + 1;
+            const float top = t[0] * (1.0f - wu) + t[1] * wu;
+            const float bot = t[kTex + 2] * (1.0f - wu) + t[kTex + 3] * wu;
             const float a = top * (1.0f - wv) + bot * wv;
-            const float r = q.z;
+            const float r = e.z;
             dr = blend8(r, a, dr, d8);
             dg = blend8(0.5f, a, dg, d8);
             db = blend8(1.0f - r * 0.5f, a, db, d8);
         }
-        __syncthreads();
+        __syncwarp();  // the list is filled again
+        n = 0;
     }
     if (px < p.width && py < p.height) frame[size_t(py) * p.width + px] = dr | (dg << 8) | (db << 16) | (0xFFu << 24);
 }
