@@ -211,6 +211,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+// Zero the digit counts and tile counters in front of a radix sort's scratch
+// (kSortHeadWords; block 0, in the kernel that makes the keys).
+__device__ __forceinline__ void clear_sort_head(uint32_t* head) {
+    if (blockIdx.x != 0) return;
+    for (uint32_t i = threadIdx.x; i < kSortHeadWords; i += blockDim.x) head[i] = 0u;
+}
+
 // ---- block coordinates ----
 // A block's index within its scene's grid and that grid's size in blocks.  A
 // launch for one scene uses the hardware's values; a launch over many scenes

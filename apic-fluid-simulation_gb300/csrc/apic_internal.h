@@ -40,9 +40,9 @@ constexpr int kMaxRedBlocks = 152 * (2048 / kSegBlock);  // one full wave on 152
 constexpr uint32_t kTileX = 32, kTileY = 16;
 constexpr int kTileBlock = 256;
 constexpr uint32_t kMaxTileBlocks = 152 * 4;
-constexpr int kSortTile = 2048;       // keys per block in the radix sort
-constexpr int kSortThreads = 256;
+constexpr uint32_t kManyTiles = 2048;  // up to 1024^2 one CTA lists a level's tiles from the mask itself
 constexpr int kMaxDigitBits = 10;     // widest radix-sort digit (1024 buckets)
+constexpr uint32_t kSortHeadWords = 3072 + 32;  // digit counts and tile counters of a sort, in front of its scratch
 
 // Device-resident control block of one scene.
 struct Ctl {
@@ -104,6 +104,7 @@ enum : uint32_t {
     kStatusBadStep = 2u,
     kStatusP2gLayout = 8u,  // a particle's staggered stencil left the bins P2G searches (never expected)
     kStatusBounds = 16u,    // checked build (APIC_BOUNDS_CHECK): an index left its buffer
+    kStatusSortWait = 32u,  // a bounded wait of the radix sort gave up (never expected)
 };
 
 struct Level {
@@ -123,6 +124,7 @@ struct Level {
     // down and up kernels, and the ascending list of tiles that hold fluid
     float* pre = nullptr;
     uint32_t* tiles = nullptr;
+    uint32_t* tile_flags = nullptr;  // levels of more than kManyTiles tiles: which hold fluid, a bit each
     uint32_t tiles_x = 0, ntiles = 0;
     float* res2 = nullptr;  // base level: the residual's second buffer (Ctl::res_sel)
 };
@@ -185,8 +187,7 @@ struct Scene {
     uint32_t* vals = nullptr;
     uint32_t* keys_alt = nullptr;
     uint32_t* vals_alt = nullptr;
-    uint32_t* sort_hist = nullptr;         // sort_hist_words(n)
-    uint32_t* sort_scan_tmp = nullptr;
+    uint32_t* sort_scratch = nullptr;      // sort_scratch_words(scene, n)
     // P2G binning: (cell of the density stencil's base, slot) pairs sorted by
     // cell, and each cell's run [bin_lo, bin_hi) in the sorted pairs
     uint32_t *bin_keys = nullptr, *bin_vals = nullptr, *bin_keys_alt = nullptr, *bin_vals_alt = nullptr;
@@ -282,8 +283,6 @@ struct ExitArgs {
 // ---- launchers (each enqueues on s.stream) --------------------------------
 // sort.cu
 cudaError_t launch_sort(Scene& s);
-// Exclusive scan of data[0..n) in place; tmp holds div_up(n, 1024) words.
-cudaError_t exclusive_scan_u32(uint32_t* data, uint32_t n, uint32_t* tmp, cudaStream_t st);
 // Block partials of the PCG loop's split reductions, in Scene::partials after
 // the 2 * kMaxRedBlocks doubles of the single-kernel reductions: s.Ap (one
 // float2 per block), the residual's sum of squares and max (one float4) and
@@ -309,19 +308,22 @@ inline bool coarse_cg_exact(const Scene& s) { return s.solver_mode == APIC_SOLVE
 cudaError_t render_frame(Scene& s, const RenderParamsDev& p, RenderResult* out);
 const uint32_t* render_frame_ptr(const Scene& s, uint32_t* width, uint32_t* height);
 void free_render(Scene& s);
-cudaError_t radix_sort_pairs_in(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* hist,
-                                uint32_t* scan_tmp, uint32_t n, int bits, cudaStream_t st);
-// Stable LSD sort with digits of up to kMaxDigitBits bits; the sorted pairs
-// stay where the last pass wrote them (*keys_out / *vals_out: keys/vals or
-// keys_alt/vals_alt).  hist: sort_hist_words(n), scan_tmp: sort_scan_words(n).
-// status: where the checked build (APIC_BOUNDS_CHECK) records an index outside
-// its buffer (may be null).
-cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* hist,
-                             uint32_t* scan_tmp, uint32_t n, int bits, cudaStream_t st, bool pdl,
-                             uint32_t** keys_out, uint32_t** vals_out, uint32_t* status = nullptr);
+// Stable LSD sort of n pairs with digits of up to kMaxDigitBits bits; the
+// sorted pairs stay where the last pass wrote them (*keys_out / *vals_out:
+// keys/vals or keys_alt/vals_alt).  iota >= 0: the values are the pair's index
+// >> iota (vals is only a buffer then).  scratch: sort_scratch_words, its head
+// zeroed (clear_sort_head).  status: where a bounded wait that gave up or an
+// index outside the buffers is recorded (may be null).
+cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* scratch,
+                             uint32_t n, int bits, int iota, cudaStream_t st, bool pdl, uint32_t** keys_out,
+                             uint32_t** vals_out, uint32_t* status = nullptr);
+cudaError_t radix_sort_pairs_digits(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
+                                    uint32_t* scratch, uint32_t n, int bits, int dbits, cudaStream_t st);
 bool radix_sort_in_alt(int bits);     // radix_sort_pairs over `bits` bits ends in the alt buffers
-uint32_t sort_hist_words(uint32_t n);
-uint32_t sort_scan_words(uint32_t n);
+int sort_digit_bits(int bits);        // ... its digit width
+uint32_t sort_scratch_words(uint32_t n, int bits, int dbits);
+uint32_t sort_scratch_words(const Scene& s, uint32_t n);  // enough for the scene's two sorts
+int bin_key_bits(const Scene& s);
 bool sort_result_in_alt(const Scene& s);  // where launch_sort leaves the Morton-sorted pairs
 int morton_key_bits(uint32_t width, uint32_t height);
 // runtime.cu: record the calling thread's last error text (apic_last_error)

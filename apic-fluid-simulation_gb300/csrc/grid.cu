@@ -425,30 +425,39 @@ __global__ void __launch_bounds__(kOneThreads) k_coarsen_tail(TailLevels t, Ctl*
 
 // The ascending list of a level's tiles that hold fluid, one CTA per level
 // (blockIdx.x): thread t of a round takes tile 1024 * round + t and ORs the
-// 32 bits of its rows.
+// 32 bits of its rows, or, on a large level, reads the flag that a grid-wide
+// kernel formed (4096^2, 32768 tiles: 200 us by one CTA alone).
 struct TileLists {
     int n;
     Level lv[kMaxLevels];
 };
+__device__ __forceinline__ bool tile_holds_fluid(const Level& L, uint32_t i) {
+    const uint32_t x0 = (i % L.tiles_x) * kTileX, y0 = (i / L.tiles_x) * kTileY;
+    const uint32_t rows = min(kTileY, L.h - y0), n = min(kTileX, L.w - x0);
+    const uint32_t mask = n >= 32u ? 0xffffffffu : (1u << n) - 1u;
+    uint32_t any = 0;
+#pragma unroll 8
+    for (uint32_t y = 0; y < rows; ++y) {
+        const uint32_t raw = (y0 + y) * L.w + x0, sh = raw & 31u;
+        uint32_t bits = L.fluid[raw >> 5] >> sh;
+        if (sh && (raw >> 5) + 1u < L.words) bits |= L.fluid[(raw >> 5) + 1u] << (32u - sh);
+        any |= bits & mask;
+    }
+    return any != 0;
+}
+__global__ void __launch_bounds__(256) k_tile_flags(Level L) {
+    pdl_wait();
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    const uint32_t votes = __ballot_sync(0xffffffffu, i < L.ntiles && tile_holds_fluid(L, i));
+    if ((threadIdx.x & 31u) == 0 && i < L.ntiles) L.tile_flags[i >> 5] = votes;
+}
 __global__ void __launch_bounds__(kOneThreads) k_tile_lists(TileLists t, Ctl* __restrict__ ctl) {
     pdl_wait();
     const Level& L = t.lv[blockIdx.x];
     uint32_t count = 0;
     for (uint32_t i0 = 0; i0 < L.ntiles; i0 += kOneThreads) {
         const uint32_t i = i0 + threadIdx.x;
-        uint32_t any = 0;
-        if (i < L.ntiles) {
-            const uint32_t x0 = (i % L.tiles_x) * kTileX, y0 = (i / L.tiles_x) * kTileY;
-            const uint32_t rows = min(kTileY, L.h - y0), n = min(kTileX, L.w - x0);
-            const uint32_t mask = n >= 32u ? 0xffffffffu : (1u << n) - 1u;
-#pragma unroll 4
-            for (uint32_t y = 0; y < rows; ++y) {
-                const uint32_t raw = (y0 + y) * L.w + x0, sh = raw & 31u;
-                uint32_t bits = L.fluid[raw >> 5] >> sh;
-                if (sh && (raw >> 5) + 1u < L.words) bits |= L.fluid[(raw >> 5) + 1u] << (32u - sh);
-                any |= bits & mask;
-            }
-        }
+        const bool any = i < L.ntiles && (L.tile_flags ? (L.tile_flags[i >> 5] >> (i & 31u)) & 1u : tile_holds_fluid(L, i));
         uint32_t tot;
         const uint32_t off = scan_1024(any ? 1u : 0u, &tot);
         if (any) L.tiles[count + off] = i;
@@ -676,7 +685,11 @@ cudaError_t launch_tile_lists(Scene& s) {
     TileLists t;
     t.n = s.nlevels - 1;
     if (t.n < 1) return cudaSuccess;
-    for (int l = 0; l < t.n; ++l) t.lv[l] = s.lv[l];
+    for (int l = 0; l < t.n; ++l) {
+        t.lv[l] = s.lv[l];
+        if (s.lv[l].tile_flags)
+            launch(s.use_pdl, k_tile_flags, div_up(s.lv[l].ntiles, 256), 256, 0, s.stream, s.lv[l]);
+    }
     launch(s.use_pdl, k_tile_lists, t.n, kOneThreads, 0, s.stream, t, s.ctl);
     return cudaGetLastError();
 }

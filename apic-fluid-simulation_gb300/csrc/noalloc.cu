@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "apic_device.cuh"
@@ -22,11 +23,12 @@ namespace {
 
 // Largest particle count the scratch array supports.
 constexpr uint32_t kNoAllocMaxKeys = 1u << 20;  // 1,048,576 particles
-constexpr uint32_t kNoAllocBlocks = kNoAllocMaxKeys / kSortTile;
-constexpr uint32_t kHistWords = 256u * kNoAllocBlocks;
-constexpr uint32_t kScanWords = (kHistWords + 1023u) / 1024u + 1u;
-// layout: alternate keys | alternate slots | digit histogram | scan partials
-constexpr size_t kScratchWords = 2ull * kNoAllocMaxKeys + kHistWords + kScanWords;  // ~8.5 MiB
+// The sort's scratch for the most keys: 512 tiles at 20 bits of key (two
+// passes of 10 bits over 256 tiles of 4096 keys), less for more bits, whose
+// digits are 8 bits wide (up to four passes).
+constexpr uint32_t kSortWords = kSortHeadWords + 2u * 256u * 1024u;
+// layout: alternate keys | alternate slots | the sort's scratch
+constexpr size_t kScratchWords = 2ull * kNoAllocMaxKeys + kSortWords;  // ~10 MiB
 
 static __device__ __align__(256) uint32_t g_sort_scratch[kScratchWords];
 
@@ -65,14 +67,15 @@ cudaError_t scratch_for_current_context(uint32_t** out) {
 // Morton key of each particle's clamped cell and its slot (src/apic.rs:1049-1064).
 __global__ void k_keys_from_positions(const float* __restrict__ px, const float* __restrict__ py, uint32_t n,
                                       CellSize cs, float max_x, float max_y, uint32_t* __restrict__ keys,
-                                      uint32_t* __restrict__ vals) {
+                                      uint32_t* __restrict__ vals, uint32_t* __restrict__ head) {
+    clear_sort_head(head);
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float gx = over_dx(px[i], cs), gy = over_dx(py[i], cs);
     uint32_t cx = uint32_t(trunc_x86(fmin_x86(fmax_x86(gx, 0.0f), max_x)));
     uint32_t cy = uint32_t(trunc_x86(fmin_x86(fmax_x86(gy, 0.0f), max_y)));
     keys[i] = morton(cx, cy);
-    vals[i] = i;
+    if (vals) vals[i] = i;
 }
 
 int reject(int code, const char* msg) {
@@ -101,16 +104,23 @@ extern "C" int apic_morton_sort_noalloc(const float* pos_x, const float* pos_y, 
     cudaError_t e = scratch_for_current_context(&scratch);
     if (e != cudaSuccess) return reject(APIC_ERR_CUDA, cudaGetErrorString(e));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint32_t* keys_alt = scratch;
-    uint32_t* vals_alt = scratch + kNoAllocMaxKeys;
-    uint32_t* hist = scratch + 2ull * kNoAllocMaxKeys;
-    uint32_t* scan_tmp = hist + kHistWords;
+    uint32_t* head = scratch + 2ull * kNoAllocMaxKeys;
+    const int bits = morton_key_bits(width, height);
+    const int dbits = bits <= 2 * kMaxDigitBits ? sort_digit_bits(bits) : 8;
+    const int passes = dbits > 0 ? (bits + dbits - 1) / dbits : 0;
+    // the keys start where an even number of passes ends in the caller's buffers
+    uint32_t *k0 = keys_out, *v0 = vals_out, *k1 = scratch, *v1 = scratch + kNoAllocMaxKeys;
+    if (passes % 2 == 1) {
+        std::swap(k0, k1);
+        std::swap(v0, v1);
+    }
+    if (sort_scratch_words(n, bits, dbits) > kSortWords)  // (not reached: see kSortWords)
+        return reject(APIC_ERR_UNSUPPORTED, "apic_morton_sort_noalloc: sort scratch too small");
     float max_x = float(width - 1), max_y = float(height - 1);
-    k_keys_from_positions<<<div_up(n, 256), 256, 0, st>>>(pos_x, pos_y, n, CellSize{cell_size, exact_reciprocal(cell_size)},
-                                                          max_x, max_y, keys_out,
-                                                          vals_out);
-    e = radix_sort_pairs_in(keys_out, vals_out, keys_alt, vals_alt, hist, scan_tmp, n,
-                            morton_key_bits(width, height), st);
+    k_keys_from_positions<<<div_up(n, 256), 256, 0, st>>>(pos_x, pos_y, n,
+                                                          CellSize{cell_size, exact_reciprocal(cell_size)}, max_x,
+                                                          max_y, k0, passes == 0 ? v0 : nullptr, head);
+    e = radix_sort_pairs_digits(k0, v0, k1, v1, head, n, bits, dbits, st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return reject(APIC_ERR_CUDA, cudaGetErrorString(e));
     return APIC_OK;

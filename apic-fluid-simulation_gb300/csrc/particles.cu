@@ -102,8 +102,9 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_u32(uint32_t v, uint32_
 // npad, a multiple of 8, lanes; keys of lanes n .. npad-1 are never read).
 __global__ void __launch_bounds__(256) k_p2g_bin_keys(const PartPtrs* __restrict__ pp, uint32_t n, int W, int H,
                                                       CellSize cs, uint32_t* __restrict__ keys,
-                                                      uint32_t* __restrict__ vals, uint32_t* __restrict__ fluid) {
+                                                      uint32_t* __restrict__ fluid, uint32_t* __restrict__ head) {
     pdl_wait();
+    clear_sort_head(head);
     const uint32_t i0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
     const bool any = i0 < n;
     float4 px = make_float4(0.0f, 0.0f, 0.0f, 0.0f), py = px;
@@ -130,10 +131,7 @@ __global__ void __launch_bounds__(256) k_p2g_bin_keys(const PartPtrs* __restrict
         const uint32_t m = __reduce_or_sync(peers, bit);
         if (live && (peers & ((1u << lane) - 1u)) == 0) atomicOr(fluid + word, m);
     }
-    if (any) {
-        *reinterpret_cast<uint4*>(keys + i0) = make_uint4(k[0], k[1], k[2], k[3]);
-        *reinterpret_cast<uint4*>(vals + i0) = make_uint4(i0, i0 + 1, i0 + 2, i0 + 3);
-    }
+    if (any) *reinterpret_cast<uint4*>(keys + i0) = make_uint4(k[0], k[1], k[2], k[3]);
 }
 
 __global__ void __launch_bounds__(256) k_p2g_bounds(const uint32_t* __restrict__ keys, uint32_t n,
@@ -998,14 +996,6 @@ __global__ void k_swap_tables(PartPtrs* pp) {
 
 }  // namespace
 
-// Bit length of the largest P2G bin key (row-major cell index).
-static int bin_key_bits(const Scene& s) {
-    uint32_t mx = s.cells > 0 ? s.cells - 1 : 0;
-    int b = 0;
-    while (b < 32 && (mx >> b)) ++b;
-    return b;
-}
-
 static CellSize cell_size(const Scene& s) { return CellSize{s.dx, exact_reciprocal(s.dx)}; }
 
 // P2G stage; bin_lo / bin_hi and the base fluid mask must be zero (the
@@ -1018,10 +1008,10 @@ cudaError_t launch_p2g(Scene& s) {
     const uint32_t* svals = s.bin_vals;
     if (s.n > 0) {
         launch(s.use_pdl, k_p2g_bin_keys, div_up(s.n, 1024), 256, 0, s.stream, static_cast<const PartPtrs*>(s.pp), s.n,
-               int(s.W), int(s.H), cell_size(s), s.bin_keys, s.bin_vals, s.lv[0].fluid);
+               int(s.W), int(s.H), cell_size(s), s.bin_keys, s.lv[0].fluid, s.sort_scratch);
         uint32_t *kres, *vres;
-        e = radix_sort_pairs(s.bin_keys, s.bin_vals, s.bin_keys_alt, s.bin_vals_alt, s.sort_hist, s.sort_scan_tmp, s.n,
-                             bin_key_bits(s), s.stream, s.use_pdl, &kres, &vres, &s.ctl->status);
+        e = radix_sort_pairs(s.bin_keys, s.bin_vals, s.bin_keys_alt, s.bin_vals_alt, s.sort_scratch, s.n,
+                             bin_key_bits(s), 0, s.stream, s.use_pdl, &kres, &vres, &s.ctl->status);
         if (e != cudaSuccess) return e;
         launch(s.use_pdl, k_p2g_bounds, div_up(s.n, 256), 256, 0, s.stream, static_cast<const uint32_t*>(kres), s.n,
                s.bin_lo, s.bin_hi, s.cells, &s.ctl->status);

@@ -70,7 +70,8 @@ __device__ __forceinline__ uint32_t circle_alpha(int x, int y) {
 // `ntiles`, which sorts after every real tile.
 __global__ void __launch_bounds__(256) k_splat_bin(const PartPtrs* __restrict__ pp, uint32_t n, RenderParamsDev p,
                                                    float4* __restrict__ quad, uint32_t* __restrict__ keys,
-                                                   uint32_t* __restrict__ vals, RenderCounters* __restrict__ cnt) {
+                                                   RenderCounters* __restrict__ cnt, uint32_t* __restrict__ head) {
+    clear_sort_head(head);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < n;
     float x = 0.0f, y = 0.0f, vx = 0.0f, vy = 0.0f;
@@ -124,7 +125,6 @@ __global__ void __launch_bounds__(256) k_splat_bin(const PartPtrs* __restrict__ 
         }
     }
     *reinterpret_cast<uint4*>(keys + size_t(i) * 4) = make_uint4(k0, k1, k2, k3);
-    *reinterpret_cast<uint4*>(vals + size_t(i) * 4) = make_uint4(i, i, i, i);
 }
 
 // First and one-past-last sorted pair of every tile (both zeroed before).
@@ -290,8 +290,8 @@ struct RenderBuffers {
     size_t quad_cap = 0;
     uint32_t *keys = nullptr, *vals = nullptr, *keys_alt = nullptr, *vals_alt = nullptr;
     size_t keys_cap = 0, vals_cap = 0, keys_alt_cap = 0, vals_alt_cap = 0;
-    uint32_t *hist = nullptr, *scan_tmp = nullptr;
-    size_t hist_cap = 0, scan_cap = 0;
+    uint32_t* scratch = nullptr;
+    size_t scratch_cap = 0;
     uint32_t *start = nullptr, *end = nullptr;
     size_t start_cap = 0, end_cap = 0;
     RenderCounters* cnt = nullptr;
@@ -301,7 +301,7 @@ struct RenderBuffers {
 void free_render(Scene& s) {
     RenderBuffers* b = s.render;
     if (!b) return;
-    void* ptrs[] = {b->frame, b->quad, b->keys, b->vals, b->keys_alt, b->vals_alt, b->hist, b->scan_tmp,
+    void* ptrs[] = {b->frame, b->quad, b->keys, b->vals, b->keys_alt, b->vals_alt, b->scratch,
                     b->start, b->end, b->cnt};
     for (void* q : ptrs)
         if (q) cudaFree(q);
@@ -315,8 +315,7 @@ cudaError_t render_frame(Scene& s, const RenderParamsDev& p, RenderResult* out) 
     RenderBuffers& b = *s.render;
     const size_t pixels = size_t(p.width) * p.height;
     const size_t m = size_t(s.n) * 4;
-    const uint32_t sort_blocks = div_up(m, kSortTile);
-    const size_t hist_words = size_t(256) * (sort_blocks ? sort_blocks : 1);
+    const int bits = bit_length(p.ntiles);
     cudaError_t e;
     if ((e = grow(&b.frame, &b.frame_cap, pixels)) != cudaSuccess) return e;
     if ((e = grow(&b.quad, &b.quad_cap, size_t(s.n ? s.n : 1))) != cudaSuccess) return e;
@@ -324,8 +323,8 @@ cudaError_t render_frame(Scene& s, const RenderParamsDev& p, RenderResult* out) 
     if ((e = grow(&b.vals, &b.vals_cap, m ? m : 1)) != cudaSuccess) return e;
     if ((e = grow(&b.keys_alt, &b.keys_alt_cap, m ? m : 1)) != cudaSuccess) return e;
     if ((e = grow(&b.vals_alt, &b.vals_alt_cap, m ? m : 1)) != cudaSuccess) return e;
-    if ((e = grow(&b.hist, &b.hist_cap, hist_words)) != cudaSuccess) return e;
-    if ((e = grow(&b.scan_tmp, &b.scan_cap, size_t(div_up(hist_words, 1024)) + 1)) != cudaSuccess) return e;
+    if ((e = grow(&b.scratch, &b.scratch_cap, sort_scratch_words(uint32_t(m), bits, sort_digit_bits(bits)))) != cudaSuccess)
+        return e;
     if ((e = grow(&b.start, &b.start_cap, size_t(p.ntiles))) != cudaSuccess) return e;
     if ((e = grow(&b.end, &b.end_cap, size_t(p.ntiles))) != cudaSuccess) return e;
     if (!b.cnt && (e = cudaMalloc(&b.cnt, sizeof(RenderCounters))) != cudaSuccess) return e;
@@ -340,14 +339,16 @@ cudaError_t render_frame(Scene& s, const RenderParamsDev& p, RenderResult* out) 
         return e;
     cudaMemsetAsync(b.start, 0, sizeof(uint32_t) * p.ntiles, st);
     cudaMemsetAsync(b.end, 0, sizeof(uint32_t) * p.ntiles, st);
+    uint32_t *keys = b.keys, *vals = b.vals;
     if (s.n) {
-        k_splat_bin<<<div_up(s.n, 256), 256, 0, st>>>(s.pp, s.n, p, b.quad, b.keys, b.vals, b.cnt);
-        if ((e = radix_sort_pairs_in(b.keys, b.vals, b.keys_alt, b.vals_alt, b.hist, b.scan_tmp, uint32_t(m),
-                                     bit_length(p.ntiles), st)) != cudaSuccess)
+        k_splat_bin<<<div_up(s.n, 256), 256, 0, st>>>(s.pp, s.n, p, b.quad, b.keys, b.cnt, b.scratch);
+        // (pair 4 i + k belongs to particle i)
+        if ((e = radix_sort_pairs(b.keys, b.vals, b.keys_alt, b.vals_alt, b.scratch, uint32_t(m), bits, 2, st, true,
+                                  &keys, &vals)) != cudaSuccess)
             return e;
-        k_tile_ranges<<<div_up(m, 256), 256, 0, st>>>(b.keys, uint32_t(m), p.ntiles, b.start, b.end);
+        k_tile_ranges<<<div_up(m, 256), 256, 0, st>>>(keys, uint32_t(m), p.ntiles, b.start, b.end);
     }
-    k_splat_raster<<<p.ntiles, kTileThreads, 0, st>>>(b.vals, b.start, b.end, b.quad, p, b.frame);
+    k_splat_raster<<<p.ntiles, kTileThreads, 0, st>>>(vals, b.start, b.end, b.quad, p, b.frame);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(b.cnt_host, b.cnt, sizeof(RenderCounters), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
         return e;
@@ -356,9 +357,9 @@ cudaError_t render_frame(Scene& s, const RenderParamsDev& p, RenderResult* out) 
     out->nan = b.cnt_host->nan;
     out->oob = b.cnt_host->oob;
     out->picked = b.cnt_host->pick == ~0ull ? -1 : int64_t(b.cnt_host->pick & 0xFFFFFFFFull);
-    // bin + ranges + raster, and per 8-bit sort pass: histogram, three scan
-    // kernels, scatter
-    out->kernels = s.n ? 3u + 5u * uint32_t((bit_length(p.ntiles) + 7) / 8) : 1u;
+    // bin + ranges + raster, the sort's counts and its passes
+    const uint32_t digit = uint32_t(sort_digit_bits(bits));
+    out->kernels = s.n ? 4u + (uint32_t(bits) + digit - 1u) / digit : 1u;
     return cudaSuccess;
 }
 

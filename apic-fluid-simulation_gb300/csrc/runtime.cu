@@ -235,7 +235,7 @@ void free_particles(Scene& s) {
     for (int f = 0; f < NPF; ++f) { dfree(s.part[f], st); dfree(s.part_alt[f], st); }
     dfree(s.keys, st); dfree(s.vals, st); dfree(s.keys_alt, st); dfree(s.vals_alt, st);
     dfree(s.bin_keys, st); dfree(s.bin_vals, st); dfree(s.bin_keys_alt, st); dfree(s.bin_vals_alt, st);
-    dfree(s.sort_hist, st); dfree(s.sort_scan_tmp, st);
+    dfree(s.sort_scratch, st);
     s.part_cap = 0;
 }
 
@@ -304,7 +304,7 @@ void free_scene(Scene& s) {
         Level& L = s.lv[l];
         dfree(L.fluid, st); dfree(L.seg, st); dfree(L.diag, st); dfree(L.inv_diag, st); dfree(L.px, st);
         dfree(L.py, st); dfree(L.res, st); dfree(L.err, st);
-        dfree(L.pre, st); dfree(L.tiles, st); dfree(L.res2, st);
+        dfree(L.pre, st); dfree(L.tiles, st); dfree(L.tile_flags, st); dfree(L.res2, st);
     }
     free_render(s);
     dfree(s.vec_stage, st);
@@ -377,8 +377,7 @@ int alloc_particles(Scene& s, uint32_t npad, uint32_t n) {
     CK(dalloc(&s.keys_alt, npad, st)); CK(dalloc(&s.vals_alt, npad, st));
     CK(dalloc(&s.bin_keys, npad, st)); CK(dalloc(&s.bin_vals, npad, st));
     CK(dalloc(&s.bin_keys_alt, npad, st)); CK(dalloc(&s.bin_vals_alt, npad, st));
-    CK(dalloc(&s.sort_hist, sort_hist_words(n), st));
-    CK(dalloc(&s.sort_scan_tmp, sort_scan_words(n), st));
+    CK(dalloc(&s.sort_scratch, sort_scratch_words(s, n), st));
     s.part_cap = npad;
     return APIC_OK;
 }
@@ -399,9 +398,8 @@ int load_particles(apic_handle* h, uint32_t n, const float* px, const float* py,
     if (rc != APIC_OK) return rc;
     // sort scratch may need to grow when n grows within the same capacity
     if (n != s.n) {
-        dfree(s.sort_hist, s.stream); dfree(s.sort_scan_tmp, s.stream);
-        CK(dalloc(&s.sort_hist, sort_hist_words(n), s.stream));
-        CK(dalloc(&s.sort_scan_tmp, sort_scan_words(n), s.stream));
+        dfree(s.sort_scratch, s.stream);
+        CK(dalloc(&s.sort_scratch, sort_scratch_words(s, n), s.stream));
     }
     // a new particle set: the next mixed solve starts from zero pressure
     if (s.p64) CK(cudaMemsetAsync(s.p64, 0, sizeof(double) * (uint64_t(s.cells) + 2ull * s.W), s.stream));
@@ -722,6 +720,7 @@ int apic::create_scene(uint32_t width, uint32_t height, float cell_size, const a
             L.tiles_x = div_up(L.w, kTileX);
             L.ntiles = L.tiles_x * div_up(L.h, kTileY);
             AL(L.pre, L.padded); AL(L.tiles, L.ntiles);
+            if (L.ntiles > kManyTiles) AL(L.tile_flags, div_up(L.ntiles, 32));
             if (l == 0) AL(L.res2, L.padded);
         }
     }
@@ -887,6 +886,7 @@ int update_finish(apic_handle* h) {
                                   uint64_t(c.pcg_iters_total) * s.kn_pcg + uint64_t(c.refinements_total) * s.kn_refine;
     if (c.status & kStatusBounds)
         return fail(APIC_ERR_CUDA, "bounds check: an index left its buffer (build with APIC_BOUNDS_CHECK)");
+    if (c.status & kStatusSortWait) return fail(APIC_ERR_TIMEOUT, "radix sort: a bounded device wait gave up");
     if (c.status & kStatusP2gLayout)
         return fail(APIC_ERR_CUDA, "P2G: a particle's stencil left the cells its faces gather from (internal error)");
     if (c.status & kStatusBadStep) return fail(APIC_ERR_NONFINITE, "substep size is not positive (non-finite velocities)");

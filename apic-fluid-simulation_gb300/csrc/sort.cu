@@ -8,16 +8,24 @@
 // to rdst; this sort is stable (equal keys keep ascending `val`), which is the
 // order the oracle defines.
 //
-// Per pass over one digit of up to 10 bits: a histogram kernel (warp match +
-// shared counters), a device-wide exclusive scan of the digit-major
-// histogram, and a scatter kernel that ranks keys stably inside its tile with
-// __match_any_sync and writes them through a shared-memory stage.  Only the
-// bits below the bit length of the largest possible key are sorted: higher
-// bits are zero for every key, so their passes would be identities.  The
-// digit width is chosen per sort for the fewest passes (20-bit keys of a
-// 1024^2 grid: two 10-bit passes), and the sorted pairs stay in the buffer
-// the last pass wrote.
+// One kernel counts every digit of the keys (k_sort_prepare); then a pass over
+// one digit of up to 10 bits is one kernel (k_sort_pass) that reads each pair
+// once and writes it once.  A tile ranks its keys stably with
+// __match_any_sync, publishes its count of each digit value, and finds its
+// place behind the tiles before it by adding up what they published
+// ("decoupled look-back", Merrill and Garland, "Single-pass Parallel Prefix
+// Scan with Decoupled Look-back", 2016, and its use in radix sorting by
+// Adinets and Merrill, "Onesweep", 2022): a tile that knows its own place
+// publishes the running total, so later tiles stop there.  Tiles take their
+// numbers from a counter as they start, so a tile only waits for tiles that
+// are running or done; the wait is bounded all the same.  Only the bits below
+// the bit length of the largest possible key are sorted: higher bits are zero
+// for every key, so their passes would be identities.  The digit width is
+// chosen per sort for the fewest passes (20-bit keys of a 1024^2 grid: two
+// 10-bit passes), and the sorted pairs stay in the buffer the last pass wrote.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "apic_device.cuh"
 #include "apic_internal.h"
@@ -26,17 +34,27 @@ namespace apic {
 
 namespace {
 
-constexpr int kItems = kSortTile / kSortThreads;  // 8 keys per thread
 constexpr uint32_t kMaxBuckets = 1u << kMaxDigitBits;
-constexpr int kScanBlock = 1024;                  // elements per scan block
+constexpr int kSortThreads = 512;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr uint32_t kMaxPasses = 4;
+// Scratch words in front of the tiles' published counts: every digit's
+// histogram (passes * buckets <= 3072) and a tile counter per pass.
+constexpr uint32_t kSortHead = kSortHeadWords;
+// A published count: the tile's own, with bit 31 the total up to and with it.
+constexpr uint32_t kNotReady = 0xFFFFFFFFu, kInclusive = 0x80000000u;
+constexpr int kLookback = 8;             // earlier tiles read at once
+constexpr uint32_t kSpinLimit = 1u << 22;  // rounds of reads before a wait gives up (seconds)
 
 // Four particles per thread with 16-byte loads and stores: the particle
-// arrays and the pair buffers hold npad (a multiple of 8) lanes, so lanes
-// n .. npad-1 get keys too, which the sort of n pairs never reads.
+// arrays and the key buffers hold npad (a multiple of 8) lanes, so lanes
+// n .. npad-1 get keys too, which the sort of n pairs never reads.  (The
+// slots need no array: the first pass makes them up.)
 __global__ void __launch_bounds__(256) k_morton_keys(const PartPtrs* __restrict__ pp, uint32_t n, CellSize cs, float max_x,
                                                      float max_y, uint32_t* __restrict__ keys,
-                                                     uint32_t* __restrict__ vals) {
+                                                     uint32_t* __restrict__ head) {
     pdl_wait();
+    clear_sort_head(head);
     const uint32_t i0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
     if (i0 >= n) return;
     const float4 px = *reinterpret_cast<const float4*>(pp->f[PX] + i0);
@@ -51,201 +69,269 @@ __global__ void __launch_bounds__(256) k_morton_keys(const PartPtrs* __restrict_
         k[q] = morton(cx, cy);
     }
     *reinterpret_cast<uint4*>(keys + i0) = make_uint4(k[0], k[1], k[2], k[3]);
-    *reinterpret_cast<uint4*>(vals + i0) = make_uint4(i0, i0 + 1, i0 + 2, i0 + 3);
 }
 
-// Per-tile digit histogram of a `dbits`-bit digit (dbits <= kMaxDigitBits),
-// written digit-major: hist[d * nblocks + b].
-__global__ void __launch_bounds__(kSortThreads) k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n,
-                                                             int shift, int dbits, uint32_t* __restrict__ hist) {
+// Counts of every digit value of every pass, and the published counts' start
+// value.  Keys come in nearly sorted order: a thread takes eight consecutive
+// ones and adds a run of equal digits at once, and a warp whose threads all
+// end with the same digit (the high ones) adds it once (a key at a time,
+// 8.3 M keys took 43 us).
+constexpr uint32_t kCountKeys = 8;
+__global__ void __launch_bounds__(kSortThreads) k_sort_prepare(const uint32_t* __restrict__ keys, uint32_t n,
+                                                               int passes, int dbits, uint32_t* __restrict__ head,
+                                                               uint32_t state_words) {
+    __shared__ uint32_t h[kMaxBuckets * 3];
     pdl_wait();
-    __shared__ uint32_t h[kMaxBuckets];
-    const uint32_t nbk = 1u << dbits, mask = nbk - 1u;
-    for (uint32_t d = threadIdx.x; d < nbk; d += kSortThreads) h[d] = 0;
+    const uint32_t nbk = 1u << dbits, mask = nbk - 1u, lane = threadIdx.x & 31u;
+    for (uint32_t d = threadIdx.x; d < uint32_t(passes) * nbk; d += kSortThreads) h[d] = 0;
+    uint4* state = reinterpret_cast<uint4*>(head + kSortHead);
+    for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < (state_words + 3u) / 4u;
+         i += gridDim.x * kSortThreads)
+        state[i] = make_uint4(kNotReady, kNotReady, kNotReady, kNotReady);
     __syncthreads();
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t base = blockIdx.x * kSortTile + warp * (kSortTile / kSortThreads * 32);
-    for (int r = 0; r < kItems; ++r) {
-        uint32_t i = base + r * 32 + lane;
-        uint32_t d = i < n ? (keys[i] >> shift) & mask : kMaxBuckets;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        if (d < kMaxBuckets && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&h[d], uint32_t(__popc(peers)));
-    }
-    __syncthreads();
-    for (uint32_t d = threadIdx.x; d < nbk; d += kSortThreads) hist[d * gridDim.x + blockIdx.x] = h[d];
-}
-
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total);
-
-// Stable scatter of one tile; offs = exclusive scan of hist.  Keys are ranked
-// inside the tile with __match_any_sync (per-warp running counters, then a
-// prefix over warps and over digits), staged in shared memory in the tile's
-// sorted order, and written out so that consecutive threads write the
-// consecutive positions of one digit's run.
-__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const uint32_t* __restrict__ keys,
-                                                                const uint32_t* __restrict__ vals, uint32_t n,
-                                                                int shift, int dbits,
-                                                                const uint32_t* __restrict__ offs,
-                                                                uint32_t* __restrict__ okeys,
-                                                                uint32_t* __restrict__ ovals,
-                                                                uint32_t* __restrict__ status) {
-    pdl_wait();
-    __shared__ uint16_t wh[kSortThreads / 32][kMaxBuckets];  // per-warp counts, then offsets
-    __shared__ uint32_t boff[kMaxBuckets];                   // global start of this tile's digit d
-    __shared__ uint32_t lstart[kMaxBuckets];                 // tile-local start of digit d
-    __shared__ uint32_t sk[kSortTile], sv[kSortTile];
-    const uint32_t nbk = 1u << dbits, mask = nbk - 1u;
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t d = threadIdx.x; d < nbk; d += kSortThreads) {
-        for (int w = 0; w < kSortThreads / 32; ++w) wh[w][d] = 0;
-        boff[d] = offs[d * gridDim.x + blockIdx.x];
-    }
-    __syncthreads();
-    const uint32_t tile0 = blockIdx.x * kSortTile;
-    uint32_t base = tile0 + warp * (kItems * 32);
-    uint32_t k[kItems], v[kItems], rk[kItems];
-    uint32_t lt = (1u << lane) - 1u;
-    for (int r = 0; r < kItems; ++r) {
-        uint32_t i = base + r * 32 + lane;
-        bool ok = i < n;
-        k[r] = ok ? keys[i] : 0u;
-        v[r] = ok ? vals[i] : 0u;
-        uint32_t d = ok ? (k[r] >> shift) & mask : kMaxBuckets;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        uint32_t before = ok ? wh[warp][d] : 0u;
-        __syncwarp();
-        if (ok && (peers & lt) == 0) wh[warp][d] = uint16_t(before + uint32_t(__popc(peers)));
-        __syncwarp();
-        rk[r] = before + uint32_t(__popc(peers & lt));
-    }
-    __syncthreads();
-    // per digit: warp offsets inside the digit, and the digit's tile count;
-    // then the tile-local start of each digit (digits split evenly over threads)
-    const uint32_t per = (nbk + kSortThreads - 1) / kSortThreads;
-    const uint32_t d0 = min(threadIdx.x * per, nbk), d1 = min(d0 + per, nbk);
-    uint32_t mine = 0;
-    for (uint32_t d = d0; d < d1; ++d) {
-        uint32_t run = 0;
-        for (int w = 0; w < kSortThreads / 32; ++w) {
-            uint32_t c = wh[w][d];
-            wh[w][d] = uint16_t(run);
-            run += c;
+    const bool aligned = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;  // a caller's buffer may not be
+    const uint64_t step = uint64_t(gridDim.x) * kSortThreads * kCountKeys;
+    // (whole warps stay in the loop: the vote below is the warp's)
+    for (uint64_t w0 = (uint64_t(blockIdx.x) * kSortThreads + (threadIdx.x & ~31u)) * kCountKeys; w0 < n; w0 += step) {
+        const uint64_t i0 = w0 + lane * kCountKeys;
+        uint32_t k[kCountKeys];
+        uint32_t live = 0;
+        if (i0 + kCountKeys <= n && aligned) {
+            const uint4 a = *reinterpret_cast<const uint4*>(keys + i0), b = *reinterpret_cast<const uint4*>(keys + i0 + 4);
+            k[0] = a.x; k[1] = a.y; k[2] = a.z; k[3] = a.w;
+            k[4] = b.x; k[5] = b.y; k[6] = b.z; k[7] = b.w;
+            live = kCountKeys;
+        } else {
+#pragma unroll
+            for (uint32_t j = 0; j < kCountKeys; ++j) {
+                const bool ok = i0 + j < n;
+                k[j] = ok ? keys[i0 + j] : 0u;
+                live += ok ? 1u : 0u;
+            }
         }
-        lstart[d] = run;
-        mine += run;
-    }
-    uint32_t tot;
-    uint32_t ex = block_exclusive_scan(mine, &tot);
-    for (uint32_t d = d0; d < d1; ++d) {
-        uint32_t c = lstart[d];
-        lstart[d] = ex;
-        ex += c;
+        for (int p = 0; p < passes; ++p) {
+            uint32_t* hp = h + uint32_t(p) * nbk;
+            uint32_t cur = (k[0] >> (p * dbits)) & mask, run = live > 0 ? 1u : 0u;
+#pragma unroll
+            for (uint32_t j = 1; j < kCountKeys; ++j) {
+                const uint32_t d = (k[j] >> (p * dbits)) & mask;
+                if (j < live && d != cur) {
+                    atomicAdd(&hp[cur], run);
+                    cur = d;
+                    run = 0;
+                }
+                run += j < live ? 1u : 0u;
+            }
+            int same;
+            __match_all_sync(0xffffffffu, cur, &same);
+            if (same) {
+                const uint32_t all = __reduce_add_sync(0xffffffffu, run);
+                if (lane == 0) atomicAdd(&hp[cur], all);
+            } else if (run) {
+                atomicAdd(&hp[cur], run);
+            }
+        }
     }
     __syncthreads();
+    for (uint32_t d = threadIdx.x; d < uint32_t(passes) * nbk; d += kSortThreads)
+        if (h[d]) atomicAdd(&head[d], h[d]);
+}
+
+__device__ __forceinline__ uint32_t load_published(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void publish(uint32_t* p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// One stable pass.  Bound by instructions (some 130 per 32 pairs) and by the
+// waits between its steps, with 16 warps per CTA and two CTAs per SM: 1.05 M
+// pairs 18 us, 8.3 M 59 us, where a histogram, three scan kernels and a
+// scatter took 36 and 87.  kItems keys per thread; a thread looks after kPer
+// consecutive digit values (two when there are 1024, else one).  iota >= 0:
+// the values are the pair's index >> iota, not read from vals.  Shared
+// memory (dynamic): per-warp counts of each digit (16 bits), their tile-wide
+// start and global offset, the tile's pairs in sorted order.
+template <int kItems, int kPer>
+__global__ void __launch_bounds__(kSortThreads) k_sort_pass(const uint32_t* __restrict__ keys,
+                                                            const uint32_t* __restrict__ vals, uint32_t n, int shift,
+                                                            int dbits, int pass, int iota, uint32_t* __restrict__ head,
+                                                            uint32_t* __restrict__ okeys, uint32_t* __restrict__ ovals,
+                                                            uint32_t* __restrict__ status) {
+    constexpr uint32_t kTileKeys = uint32_t(kItems) * kSortThreads;
+    extern __shared__ uint32_t sm[];
+    const uint32_t nbk = 1u << dbits, mask = nbk - 1u;
+    uint16_t* wh = reinterpret_cast<uint16_t*>(sm);              // [warp][digit]
+    uint32_t* lstart = sm + kSortWarps * nbk / 2u;               // [digit]
+    uint32_t* goff = lstart + nbk;                               // [digit]
+    uint32_t* sk = goff + nbk;
+    uint32_t* sv = sk + kTileKeys;
+    __shared__ uint32_t s_tile;
+    __shared__ unsigned long long s_scan[kSortWarps];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint32_t i = threadIdx.x; i < kSortWarps * nbk / 2u; i += kSortThreads) sm[i] = 0u;
+    pdl_wait();
+    if (threadIdx.x == 0) s_tile = atomicAdd(head + 3072 + pass, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile, ntiles = gridDim.x;
+    const uint32_t tile0 = tile * kTileKeys, base = tile0 + warp * (32u * kItems);
+    uint32_t k[kItems], v[kItems], rk[kItems];
+#pragma unroll
     for (int r = 0; r < kItems; ++r) {
-        uint32_t i = base + r * 32 + lane;
-        if (i >= n) continue;
-        uint32_t d = (k[r] >> shift) & mask;
-        uint32_t lp = lstart[d] + wh[warp][d] + rk[r];
-        sk[lp] = k[r];
-        sv[lp] = v[r];
+        const uint32_t i = base + uint32_t(r) * 32u + lane;
+        k[r] = i < n ? keys[i] : 0u;
+        v[r] = iota >= 0 ? i >> iota : (i < n ? vals[i] : 0u);
+    }
+    const uint32_t d0 = threadIdx.x * uint32_t(kPer);
+    const bool owner = d0 < nbk;
+    uint32_t total_all[kPer];  // of this thread's digits over all tiles
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) total_all[j] = owner ? head[uint32_t(pass) * nbk + d0 + uint32_t(j)] : 0u;
+    uint16_t* mine = wh + warp * nbk;
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+        const bool ok = base + uint32_t(r) * 32u + lane < n;
+        const uint32_t d = ok ? (k[r] >> shift) & mask : kMaxBuckets;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = ok ? mine[d] : 0u, below = uint32_t(__popc(peers & ((1u << lane) - 1u)));
+        __syncwarp();
+        if (ok && below == 0) mine[d] = uint16_t(before + uint32_t(__popc(peers)));
+        __syncwarp();
+        rk[r] = before + below;
     }
     __syncthreads();
-    const uint32_t cnt = n - tile0 < uint32_t(kSortTile) ? n - tile0 : uint32_t(kSortTile);
-    for (uint32_t q = threadIdx.x; q < cnt; q += kSortThreads) {
-        uint32_t key = sk[q];
-        uint32_t d = (key >> shift) & mask;
-        uint32_t pos = boff[d] + (q - lstart[d]);
-        if (!APIC_IN_BOUNDS(pos, n, status)) continue;
+    // this thread's digits: the warps' places within the digit, the tile's count
+    uint32_t* state = head + kSortHead + (size_t(pass) * ntiles + tile) * nbk;
+    uint32_t cnt[kPer];
+    unsigned long long both = 0;  // count in the tile | count over all tiles << 32
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        uint32_t run = 0;
+        if (owner) {
+            for (int w = 0; w < kSortWarps; ++w) {
+                const uint32_t c = wh[uint32_t(w) * nbk + d0 + uint32_t(j)];
+                wh[uint32_t(w) * nbk + d0 + uint32_t(j)] = uint16_t(run);
+                run += c;
+            }
+            publish(state + d0 + j, tile == 0 ? run | kInclusive : run);
+        }
+        cnt[j] = run;
+        both += (static_cast<unsigned long long>(total_all[j]) << 32) | run;
+    }
+    // exclusive sums over the digits of both
+    unsigned long long x = both;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= uint32_t(o)) x += y;
+    }
+    if (lane == 31) s_scan[warp] = x;
+    __syncthreads();
+    unsigned long long ex = x - both;
+    for (uint32_t w = 0; w < warp; ++w) ex += s_scan[w];
+    uint32_t local[kPer], global[kPer];
+    {
+        uint32_t l = uint32_t(ex), g = uint32_t(ex >> 32);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            local[j] = l;
+            global[j] = g;
+            if (owner) lstart[d0 + j] = l;
+            l += cnt[j];
+            g += total_all[j];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+        if (base + uint32_t(r) * 32u + lane >= n) continue;
+        const uint32_t d = (k[r] >> shift) & mask;
+        const uint32_t at = lstart[d] + mine[d] + rk[r];
+        sk[at] = k[r];
+        sv[at] = v[r];
+    }
+    // look back: add up what the tiles before this one published, kLookback of
+    // them at a time, until one has its running total
+    bool lost = false;
+    if (owner && tile > 0) {
+        uint32_t sum[kPer], left[kPer];  // left: tiles still to add (0: done)
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            sum[j] = 0;
+            left[j] = tile;
+        }
+        uint32_t spins = 0;
+        for (;;) {
+            bool open = false;
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                if (left[j] == 0) continue;
+                const uint32_t* at = state + d0 + j - size_t(tile) * nbk;  // tile 0's
+                uint32_t q[kLookback];
+#pragma unroll
+                for (int b = 0; b < kLookback; ++b)
+                    q[b] = left[j] > uint32_t(b) ? load_published(at + size_t(left[j] - 1u - uint32_t(b)) * nbk)
+                                                 : kNotReady;
+                bool go = true;
+#pragma unroll
+                for (int b = 0; b < kLookback; ++b) {
+                    if (!go || q[b] == kNotReady) {
+                        go = false;
+                        continue;
+                    }
+                    sum[j] += q[b] & ~kInclusive;
+                    left[j] -= 1u;
+                    if (q[b] & kInclusive) {
+                        left[j] = 0;
+                        go = false;
+                    }
+                }
+                open = open || left[j] != 0;
+            }
+            if (!open) break;
+            if (++spins > kSpinLimit) {
+                lost = true;
+                break;
+            }
+        }
+        if (!lost) {
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                publish(state + d0 + j, (sum[j] + cnt[j]) | kInclusive);
+                global[j] += sum[j];
+            }
+        }
+    }
+    if (owner) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) goff[d0 + j] = global[j] - local[j];
+    }
+    if (__syncthreads_or(lost)) {  // (never expected) leave the output alone
+        if (threadIdx.x == 0 && status) atomicOr(status, kStatusSortWait);
+        return;
+    }
+    const uint32_t here = min(kTileKeys, n - tile0);
+    for (uint32_t q = threadIdx.x; q < here; q += kSortThreads) {
+        const uint32_t key = sk[q], pos = goff[(key >> shift) & mask] + q;
+        if (pos >= n) {  // (scratch overwritten by an overlapping call)
+            if (status) atomicOr(status, kStatusBounds);
+            continue;
+        }
         okeys[pos] = key;
         ovals[pos] = sv[q];
     }
 }
 
-// ---- device-wide exclusive scan of u32 (three kernels, no inter-block waits)
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
-    __shared__ uint32_t sw[32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) sw[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t s = lane < int(blockDim.x / 32) ? sw[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        sw[lane] = s;
-    }
-    __syncthreads();
-    uint32_t pre = warp > 0 ? sw[warp - 1] : 0u;
-    *total = sw[blockDim.x / 32 - 1];
-    __syncthreads();
-    return pre + x - v;
-}
-
-__global__ void __launch_bounds__(256) k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n,
-                                                     uint32_t* __restrict__ bsum) {
-    pdl_wait();
-    uint32_t b0 = blockIdx.x * kScanBlock;
-    uint32_t s = 0;
-    for (int k = 0; k < kScanBlock / 256; ++k) {
-        uint32_t i = b0 + k * 256 + threadIdx.x;
-        if (i < n) s += in[i];
-    }
-    __shared__ uint32_t red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) bsum[blockIdx.x] = red[0];
-}
-
-__global__ void __launch_bounds__(1024) k_scan_blocksums(uint32_t* __restrict__ bsum, uint32_t nb) {
-    pdl_wait();
-    uint32_t carry = 0;
-    for (uint32_t c = 0; c < nb; c += 1024) {
-        uint32_t i = c + threadIdx.x;
-        uint32_t v = i < nb ? bsum[i] : 0u;
-        uint32_t tot;
-        uint32_t ex = block_exclusive_scan(v, &tot);
-        if (i < nb) bsum[i] = carry + ex;
-        carry += tot;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_scan_down(uint32_t* __restrict__ data, uint32_t n,
-                                                   const uint32_t* __restrict__ bsum) {
-    pdl_wait();
-    uint32_t b0 = blockIdx.x * kScanBlock;
-    uint32_t carry = bsum[blockIdx.x];
-    for (int k = 0; k < kScanBlock / 256; ++k) {
-        uint32_t i = b0 + k * 256 + threadIdx.x;
-        uint32_t v = i < n ? data[i] : 0u;
-        uint32_t tot;
-        uint32_t ex = block_exclusive_scan(v, &tot);
-        if (i < n) data[i] = carry + ex;
-        carry += tot;
-    }
-}
-
 }  // namespace
 
-cudaError_t exclusive_scan_u32(uint32_t* data, uint32_t n, uint32_t* tmp, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    uint32_t nb = div_up(n, kScanBlock);
-    launch(st != nullptr, k_scan_reduce, nb, 256, 0, st, data, n, tmp);
-    launch(st != nullptr, k_scan_blocksums, 1, 1024, 0, st, tmp, nb);
-    launch(st != nullptr, k_scan_down, nb, 256, 0, st, data, n, tmp);
-    return cudaGetLastError();
+// Bit length of the largest P2G bin key (row-major cell index).
+int bin_key_bits(const Scene& s) {
+    uint32_t mx = s.cells > 0 ? s.cells - 1 : 0;
+    int b = 0;
+    while (b < 32 && (mx >> b)) ++b;
+    return b;
 }
 
 static int key_bits(const Scene& s) {
@@ -274,58 +360,80 @@ static int digit_bits(int bits) {
     return (bits + passes - 1) / passes;
 }
 
-static cudaError_t lsd_passes(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
-                              uint32_t* hist, uint32_t* scan_tmp, uint32_t n, int bits, int dbits, cudaStream_t st,
-                              bool pdl, uint32_t** keys_out, uint32_t** vals_out, uint32_t* status) {
-    uint32_t nb = div_up(n, kSortTile);
-    uint32_t* k_in = keys;
-    uint32_t* v_in = vals;
-    uint32_t* k_out = keys_alt;
-    uint32_t* v_out = vals_alt;
-    for (int shift = 0; dbits > 0 && shift < bits; shift += dbits) {
-        launch(pdl, k_sort_hist, nb, kSortThreads, 0, st, static_cast<const uint32_t*>(k_in), n, shift, dbits, hist);
-        cudaError_t e = exclusive_scan_u32(hist, (1u << dbits) * nb, scan_tmp, st);
-        if (e != cudaSuccess) return e;
-        launch(pdl, k_sort_scatter, nb, kSortThreads, 0, st, static_cast<const uint32_t*>(k_in),
-               static_cast<const uint32_t*>(v_in), n, shift, dbits, static_cast<const uint32_t*>(hist), k_out, v_out,
-               status);
+// Tile size of a sort: small sorts take small tiles, for which the look-back
+// is short and more SMs work; from 256 K pairs on 4096 pairs a tile.
+static int tile_items(uint32_t n) { return n <= 65536u ? 2 : n <= 262144u ? 4 : 8; }
+static uint32_t sort_tiles(uint32_t n) { return div_up(n, uint32_t(tile_items(n)) * kSortThreads); }
+static int sort_passes(int bits, int dbits) { return dbits > 0 ? (bits + dbits - 1) / dbits : 0; }
+static size_t pass_smem(int items, int dbits) {
+    const size_t nbk = size_t(1) << dbits;
+    return kSortWarps * nbk * 2 + 2 * nbk * 4 + 2 * size_t(items) * kSortThreads * 4;
+}
+
+template <int kItems>
+static cudaError_t sort_pass(bool pdl, uint32_t tiles, cudaStream_t st, const uint32_t* k, const uint32_t* v,
+                             uint32_t n, int shift, int dbits, int pass, int iota, uint32_t* head, uint32_t* ok,
+                             uint32_t* ov, uint32_t* status) {
+    auto kern = dbits > 9 ? k_sort_pass<kItems, 2> : k_sort_pass<kItems, 1>;
+    const size_t smem = pass_smem(kItems, dbits);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    return launch(pdl, kern, tiles, kSortThreads, smem, st, k, v, n, shift, dbits, pass, iota, head, ok, ov, status);
+}
+
+static cudaError_t lsd_passes(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* head,
+                              uint32_t n, int bits, int dbits, int iota, cudaStream_t st, bool pdl,
+                              uint32_t** keys_out, uint32_t** vals_out, uint32_t* status) {
+    uint32_t *k_in = keys, *v_in = vals, *k_out = keys_alt, *v_out = vals_alt;
+    const int passes = sort_passes(bits, dbits), items = tile_items(n);
+    const uint32_t tiles = sort_tiles(n);
+    cudaError_t e = cudaSuccess;
+    if (passes > 0)
+        e = launch(pdl, k_sort_prepare, std::min(div_up(n, kSortThreads * kCountKeys), 304u), kSortThreads, 0, st,
+                   static_cast<const uint32_t*>(k_in), n, passes, dbits, head,
+                   uint32_t(passes) * tiles << dbits);
+    for (int p = 0; p < passes && e == cudaSuccess; ++p) {
+        auto pass = items == 2 ? sort_pass<2> : items == 4 ? sort_pass<4> : sort_pass<8>;
+        e = pass(pdl, tiles, st, k_in, v_in, n, p * dbits, dbits, p, p == 0 ? iota : -1, head, k_out, v_out, status);
         std::swap(k_in, k_out);
         std::swap(v_in, v_out);
     }
     *keys_out = k_in;
     *vals_out = v_in;
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-uint32_t sort_hist_words(uint32_t n) { return kMaxBuckets * div_up(n > 0 ? n : 1, kSortTile); }
-uint32_t sort_scan_words(uint32_t n) { return div_up(sort_hist_words(n), 1024) + 1; }
+uint32_t sort_scratch_words(uint32_t n, int bits, int dbits) {
+    if (n == 0) return kSortHead;
+    return kSortHead + uint32_t(((size_t(sort_passes(bits, dbits)) * sort_tiles(n) << dbits) + 3) & ~size_t(3));
+}
+uint32_t sort_scratch_words(const Scene& s, uint32_t n) {
+    const int m = key_bits(s), b = bin_key_bits(s);
+    return std::max(sort_scratch_words(n, m, digit_bits(m)), sort_scratch_words(n, b, digit_bits(b)));
+}
 
-cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* hist,
-                             uint32_t* scan_tmp, uint32_t n, int bits, cudaStream_t st, bool pdl,
-                             uint32_t** keys_out, uint32_t** vals_out, uint32_t* status) {
+cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* scratch,
+                             uint32_t n, int bits, int iota, cudaStream_t st, bool pdl, uint32_t** keys_out,
+                             uint32_t** vals_out, uint32_t* status) {
     *keys_out = keys;
     *vals_out = vals;
     if (n == 0) return cudaSuccess;
-    return lsd_passes(keys, vals, keys_alt, vals_alt, hist, scan_tmp, n, bits, digit_bits(bits), st, pdl, keys_out,
+    return lsd_passes(keys, vals, keys_alt, vals_alt, scratch, n, bits, digit_bits(bits), iota, st, pdl, keys_out,
                       vals_out, status);
 }
 
-bool radix_sort_in_alt(int bits) {
-    int d = digit_bits(bits);
-    int passes = d > 0 ? (bits + d - 1) / d : 0;
-    return passes % 2 == 1;
-}
+bool radix_sort_in_alt(int bits) { return sort_passes(bits, digit_bits(bits)) % 2 == 1; }
+int sort_digit_bits(int bits) { return digit_bits(bits); }
 
 cudaError_t launch_sort(Scene& s) {
     if (s.n == 0) return cudaSuccess;
     float max_x = float(s.W > 0 ? s.W - 1 : 0), max_y = float(s.H > 0 ? s.H - 1 : 0);
     launch(s.use_pdl, k_morton_keys, div_up(s.n, 1024), 256, 0, s.stream, s.pp, s.n,
-           CellSize{s.dx, exact_reciprocal(s.dx)}, max_x, max_y, s.keys,
-           s.vals);
+           CellSize{s.dx, exact_reciprocal(s.dx)}, max_x, max_y, s.keys, s.sort_scratch);
     // the sorted pairs stay where the last pass wrote them (no copy back)
     uint32_t *k_res, *v_res;
-    cudaError_t e = radix_sort_pairs(s.keys, s.vals, s.keys_alt, s.vals_alt, s.sort_hist, s.sort_scan_tmp, s.n,
-                                     key_bits(s), s.stream, s.use_pdl, &k_res, &v_res, &s.ctl->status);
+    cudaError_t e = radix_sort_pairs(s.keys, s.vals, s.keys_alt, s.vals_alt, s.sort_scratch, s.n, key_bits(s), 0,
+                                     s.stream, s.use_pdl, &k_res, &v_res, &s.ctl->status);
     if (e != cudaSuccess) return e;
     return launch_permute(s, v_res);
 }
@@ -334,22 +442,12 @@ cudaError_t launch_sort(Scene& s) {
 // passes is fixed by the grid size).
 bool sort_result_in_alt(const Scene& s) { return radix_sort_in_alt(key_bits(s)); }
 
-// Stable LSD sort of (keys, vals)[0..n) over the low `bits` key bits in 8-bit
-// digits, with all intermediate storage supplied by the caller:
-// keys_alt/vals_alt (n words each), hist (256 * ceil(n / 2048) words) and
-// scan_tmp (ceil(hist / 1024) words).  The sorted pairs end in keys/vals.
-cudaError_t radix_sort_pairs_in(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* hist,
-                                uint32_t* scan_tmp, uint32_t n, int bits, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
+// The same sort with digits of the caller's choice (noalloc.cu).
+cudaError_t radix_sort_pairs_digits(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
+                                    uint32_t* scratch, uint32_t n, int bits, int dbits, cudaStream_t st) {
     uint32_t *k_res, *v_res;
-    cudaError_t e = lsd_passes(keys, vals, keys_alt, vals_alt, hist, scan_tmp, n, bits, bits > 0 ? 8 : 0, st,
-                               st != nullptr, &k_res, &v_res, nullptr);
-    if (e != cudaSuccess) return e;
-    if (k_res != keys) {
-        cudaMemcpyAsync(keys, k_res, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(vals, v_res, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
-    }
-    return cudaGetLastError();
+    return lsd_passes(keys, vals, keys_alt, vals_alt, scratch, n, bits, dbits, 0, st, st != nullptr, &k_res, &v_res,
+                      nullptr);
 }
 
 // Bit length of the largest Morton key of a width x height grid.

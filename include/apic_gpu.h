@@ -313,7 +313,7 @@ int apic_get_stream(apic_handle* h, void** stream_out);
  * another runtime or a fixed budget.  pos_x/pos_y: n device floats;
  * keys_out/vals_out: n device u32 (sorted keys; original slot of each).
  * Every intermediate buffer lives in one fixed device array inside the
- * library (about 8.5 MiB, held by every GPU that loads it until exit), so n is
+ * library (about 10 MiB, held by every GPU that loads it until exit), so n is
  * limited to 1,048,576; larger n, or a width or height above 65536 (the
  * Morton code interleaves 16 bits per axis), returns APIC_ERR_INVALID_ARG.
  * The first call in a CUDA context (normally: the first on a device) looks up
