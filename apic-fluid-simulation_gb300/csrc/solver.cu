@@ -257,6 +257,36 @@ __global__ void __launch_bounds__(kSegBlock) k_dot_rz(Level B, Ctl* ctl, float2*
 // Krylov reductions in exactly the reference's order; the solve is then
 // bit-identical to the oracle's.
 
+// acc + v[0].x + v[0].y + ... + v[n - 1].w, one addition after another, with
+// the loads kAhead vectors ahead of the add chain.
+template <uint32_t kAhead>
+__device__ __forceinline__ float add_in_order(const float4* v, uint32_t n, float acc) {
+    float4 a[kAhead];
+#pragma unroll
+    for (uint32_t k = 0; k < kAhead; ++k) a[k] = k < n ? v[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    uint32_t i = 0;
+    for (; i + kAhead <= n; i += kAhead) {
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            const float4 q = a[k];
+            a[k] = i + kAhead + k < n ? v[i + kAhead + k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            acc = acc + q.x;
+            acc = acc + q.y;
+            acc = acc + q.z;
+            acc = acc + q.w;
+        }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kAhead; ++k) {
+        if (i + k >= n) break;
+        acc = acc + a[k].x;
+        acc = acc + a[k].y;
+        acc = acc + a[k].z;
+        acc = acc + a[k].w;
+    }
+    return acc;
+}
+
 // gamma = dot_product(residual[W..W+cells], error[W..W+cells]) (:11-29): eight
 // lane sums, lane = raw index mod 8, each added in ascending order; then
 // wide's reduce_add pairing ((l0 + l2) + (l1 + l3)) + ((l4 + l6) + (l5 + l7));
@@ -268,18 +298,24 @@ __global__ void __launch_bounds__(kSegBlock) k_dot_rz(Level B, Ctl* ctl, float2*
 // products of a batch of segments (32 raw cells each, zero where not fluid)
 // in shared memory while threads 0..7 add the previous batch's products of
 // their lane in order (two stage buffers); only those eight add chains are
-// serial.
+// serial.  A lane's products of a segment (raw cells t, t + 8, t + 16, t + 24)
+// lie side by side in its own row of the stage, so a thread takes a segment
+// with one 16-byte load and has the next eight in flight: the four dependent
+// adds are all that a segment costs (1024^2 grid, 514605 fluid cells: a solve
+// of one such pass 402 -> 302 us).
 // start: the solve's first gamma (sets gamma and the SAFTY exit,
 // :1887-1892), else the iteration's new gamma.
 constexpr int kGammaThreads = 1024;
-constexpr uint32_t kGammaBatch = 512;  // segments staged per round (64 KB)
-constexpr size_t kGammaSmem = 2 * size_t(kGammaBatch) * 32 * sizeof(float);
+constexpr uint32_t kGammaBatch = 512;               // segments staged per round
+constexpr uint32_t kGammaRow = 4 * kGammaBatch + 4;  // a lane's row (the rows start four banks apart)
+constexpr uint32_t kGammaAhead = 8;                 // segments loaded ahead of the adds
+constexpr size_t kGammaSmem = 2 * 8 * size_t(kGammaRow) * sizeof(float);
 // The iteration's form (start 0) also finishes the iteration (beta, or the
 // SAFTY exit) and, when set_cond, sets the loop condition.
 __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl, int start,
                                                                cudaGraphConditionalHandle h, uint32_t cap,
                                                                int dyn_cap, int set_cond) {
-    extern __shared__ float stage[];  // two buffers of kGammaBatch segments
+    extern __shared__ __align__(16) float stage[];  // two buffers of eight rows
     pdl_wait();
     if (ctl->pcg_done) return;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -289,13 +325,14 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
     const uint32_t nbatch = (nseg + kGammaBatch - 1) / kGammaBatch;
     // warps 1..31 stage batch b into buffer b % 2
     auto fill = [&](uint32_t b) {
-        float* buf = stage + (b & 1u) * kGammaBatch * 32u;
+        float* buf = stage + (b & 1u) * 8u * kGammaRow + (lane & 7u) * kGammaRow + (lane >> 3);
         const uint32_t k0 = b * kGammaBatch, nb = min(kGammaBatch, nseg - k0);
+#pragma unroll 4
         for (uint32_t q = warp - 1; q < nb; q += kGammaThreads / 32 - 1) {
             const uint32_t w = B.seg[k0 + q];
             const uint32_t raw = w * 32u + lane;
             const bool on = ((B.fluid[w] >> lane) & 1u) && raw < full;
-            buf[q * 32u + lane] = on ? res[raw + B.w] * B.err[raw + B.w] : 0.0f;
+            buf[4u * q] = on ? res[raw + B.w] * B.err[raw + B.w] : 0.0f;
         }
     };
     float acc = 0.0f;
@@ -304,15 +341,9 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
     for (uint32_t b = 0; b < nbatch; ++b) {
         if (warp == 0) {
             if (t < 8) {
-                const float* buf = stage + (b & 1u) * kGammaBatch * 32u;
+                const float4* row = reinterpret_cast<const float4*>(stage + (b & 1u) * 8u * kGammaRow + t * kGammaRow);
                 const uint32_t nb = min(kGammaBatch, nseg - b * kGammaBatch);
-                for (uint32_t q = 0; q < nb; ++q) {
-                    const float* p = buf + q * 32u + t;
-                    acc = acc + p[0];
-                    acc = acc + p[8];
-                    acc = acc + p[16];
-                    acc = acc + p[24];
-                }
+                acc = add_in_order<kGammaAhead>(row, nb, acc);
             }
         } else if (b + 1 < nbatch) {
             fill(b + 1);
@@ -380,15 +411,20 @@ __global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, ui
 // in ascending order, in chunks of 8192 cells each summed serially from zero
 // (rayon's par_chunks(8192)); k_pcg_update then adds the chunk sums in chunk
 // order.  s' is the iteration's search direction, z + beta s (k_spmv_dot
-// evaluates the same expression).  One block per chunk: its warps stage the
-// chunk's products in fluid order in shared memory (positions from
-// seg_pre), then one thread adds them in order.
-constexpr int kDeltaThreads = 256;
+// evaluates the same expression).  One block per chunk: warps 1..15 stage the
+// products in fluid order in shared memory (positions from seg_pre), a
+// stretch of segments at a time, while thread 0 adds those staged before, in
+// order, the loads ahead of its add chain: a chunk costs its 8192 dependent
+// adds.  (Staged as a whole first, and added with each product's load in the
+// chain, a PCG iteration of a 256^2 grid with 30657 fluid cells took 117 us;
+// with this and the r.z sum's rows it takes 82.)
+constexpr int kDeltaThreads = 512;
+constexpr uint32_t kDeltaStretch = 60;  // segments staged at a time (15 warps, four each)
 __global__ void __launch_bounds__(kDeltaThreads) k_delta_exact(Level B, const float* __restrict__ s,
                                                                const float* __restrict__ ap,
                                                                const uint32_t* __restrict__ seg_pre, Ctl* ctl,
                                                                float* __restrict__ parts) {
-    __shared__ float prod[kDeltaChunk];
+    __shared__ __align__(16) float prod[kDeltaChunk];
     __shared__ uint32_t s_k0, s_k1;
     pdl_wait();
     if (ctl->pcg_done) return;
@@ -398,40 +434,58 @@ __global__ void __launch_bounds__(kDeltaThreads) k_delta_exact(Level B, const fl
     const uint32_t f0 = c * kDeltaChunk;
     if (f0 >= nfluid) return;
     const uint32_t f1 = min(f0 + kDeltaChunk, nfluid);
-    if (threadIdx.x == 0) {
-        // segments [k0, k1) hold fluid cells f0 .. f1-1 (every segment holds at least one)
-        uint32_t lo = 0, hi = nseg;  // last k with seg_pre[k] <= f0
-        while (hi - lo > 1) {
+    if (threadIdx.x < 2) {
+        // segments [k0, k1) hold fluid cells f0 .. f1-1 (every segment holds
+        // at least one): the last k with seg_pre[k] <= f0, the first with
+        // seg_pre[k] >= f1
+        const uint32_t want = threadIdx.x == 0 ? f0 + 1u : f1;
+        uint32_t lo = 0, hi = nseg;
+        while (lo < hi) {
             const uint32_t mid = (lo + hi) / 2;
-            if (seg_pre[mid] <= f0) lo = mid; else hi = mid;
+            if (seg_pre[mid] < want) lo = mid + 1; else hi = mid;
         }
-        s_k0 = lo;
-        uint32_t lo2 = lo, hi2 = nseg;  // first k with seg_pre[k] >= f1
-        while (lo2 < hi2) {
-            const uint32_t mid = (lo2 + hi2) / 2;
-            if (seg_pre[mid] < f1) lo2 = mid + 1; else hi2 = mid;
-        }
-        s_k1 = lo2;
+        if (threadIdx.x == 0) s_k0 = lo - 1u;
+        else s_k1 = lo;
     }
     __syncthreads();
     const float beta = ctl->beta;
     const bool beta_valid = ctl->beta_valid != 0;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t k = s_k0 + warp; k < s_k1; k += kDeltaThreads / 32) {
-        const uint32_t w = B.seg[k];
-        const uint32_t m = B.fluid[w];
-        if (!((m >> lane) & 1u)) continue;
-        const uint32_t pos = seg_pre[k] + uint32_t(__popc(m & ((1u << lane) - 1u)));
-        if (pos < f0 || pos >= f1) continue;
-        const uint32_t cidx = w * 32u + lane + B.w;
-        prod[pos - f0] = ap[cidx] * pcg::search_at(B.err, s, beta, beta_valid, cidx);
-    }
+    const uint32_t k0 = s_k0, k1 = s_k1;
+    auto stage = [&](uint32_t from) {
+        const uint32_t end = min(from + kDeltaStretch, k1);
+#pragma unroll 4
+        for (uint32_t k = from + warp - 1u; k < end; k += kDeltaThreads / 32 - 1) {
+            const uint32_t w = B.seg[k];
+            const uint32_t m = B.fluid[w];
+            if (!((m >> lane) & 1u)) continue;
+            const uint32_t pos = seg_pre[k] + uint32_t(__popc(m & ((1u << lane) - 1u)));
+            if (pos < f0 || pos >= f1) continue;
+            const uint32_t cidx = w * 32u + lane + B.w;
+            prod[pos - f0] = ap[cidx] * pcg::search_at(B.err, s, beta, beta_valid, cidx);
+        }
+    };
+    if (warp != 0) stage(k0);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float sum = 0.0f;
-        for (uint32_t i = 0; i < f1 - f0; ++i) sum = sum + prod[i];
-        parts[c] = sum;
+    float sum = 0.0f;
+    uint32_t done = 0;  // products added (thread 0)
+    for (uint32_t k = k0; k < k1; k += kDeltaStretch) {
+        if (warp != 0) {
+            if (k + kDeltaStretch < k1) stage(k + kDeltaStretch);
+        } else if (threadIdx.x == 0) {
+            // staged so far; the last stretch adds what is left, the others
+            // whole vectors
+            const uint32_t next = min(k + kDeltaStretch, k1);
+            const uint32_t have = min(seg_pre[next], f1) - f0;
+            const uint32_t n4 = (have - done) / 4u;
+            sum = add_in_order<8>(reinterpret_cast<const float4*>(prod + done), n4, sum);
+            done += 4u * n4;
+            if (next == k1)
+                for (; done < have; ++done) sum = sum + prod[done];
+        }
+        __syncthreads();
     }
+    if (threadIdx.x == 0) parts[c] = sum;
 }
 
 // ---- FP64 refinement helpers (APIC_SOLVER_REL_MIXED) ----------------------

@@ -401,8 +401,10 @@ static __device__ __noinline__ void cg_one_warp(const CgArrays& A, bool exact) {
             return __shfl_sync(0xffffffffu, float(t), 0);
         }
         float t = 0.0f;
-#pragma unroll 8
-        for (int l = 0; l < 32; ++l) t = t + __shfl_sync(0xffffffffu, q, l);
+        for (uint32_t l0 = 0; l0 < cells; l0 += 8) {  // (lanes beyond the level hold zeros)
+#pragma unroll
+            for (uint32_t l = 0; l < 8; ++l) t = t + __shfl_sync(0xffffffffu, q, int(l0 + l));
+        }
         return t;
     };
     float s = r;
