@@ -375,8 +375,12 @@ static cudaError_t sort_pass(bool pdl, uint32_t tiles, cudaStream_t st, const ui
                              uint32_t n, int shift, int dbits, int pass, int iota, uint32_t* head, uint32_t* ok,
                              uint32_t* ov, uint32_t* status) {
     auto kern = dbits > 9 ? k_sort_pass<kItems, 2> : k_sort_pass<kItems, 1>;
+    // the limit is the kernel's largest, not this pass's: scenes are prepared on
+    // several threads, and a limit that changes under another thread's graph
+    // breaks that graph
     const size_t smem = pass_smem(kItems, dbits);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(pass_smem(kItems, dbits > 9 ? kMaxDigitBits : 9)));
     if (e != cudaSuccess) return e;
     return launch(pdl, kern, tiles, kSortThreads, smem, st, k, v, n, shift, dbits, pass, iota, head, ok, ov, status);
 }
