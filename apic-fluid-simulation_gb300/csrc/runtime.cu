@@ -412,7 +412,7 @@ int load_particles(apic_handle* h, uint32_t n, const float* px, const float* py,
         } else {
             CK(cudaMemcpyAsync(s.part[f], src, sizeof(float) * n, cudaMemcpyHostToDevice, s.stream));
             float pad[8];
-            std::fill(pad, pad + 8, pad_last ? src[n - 1] : 0.0f);
+            std::fill(pad, pad + 8, pad_last && n > 0 ? src[n - 1] : 0.0f);
             if (npad > n)
                 CK(cudaMemcpyAsync(s.part[f] + n, pad, sizeof(float) * (npad - n), cudaMemcpyHostToDevice, s.stream));
         }
