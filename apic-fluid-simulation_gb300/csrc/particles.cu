@@ -42,13 +42,11 @@ namespace {
 //                   for every particle; fluid bits (an OR: order-free)
 //   radix sort      stable, so each cell's particles stay in slot order
 //   k_p2g_bounds    each cell's run [lo, hi) in the sorted pairs
-//   k_p2g_gather    per 32 x 8 tile of cells: stage the particles of the
-//                   tile's cells and a two-cell halo below and to the left in
-//                   shared memory (in bands of rows when they do not fit),
-//                   compute their stencil contributions once per grid, then
-//                   let each face merge the runs of the (up to six) cells
-//                   whose particles can reach it by slot and fold the
-//                   contributions in (chunk, corner, lane) order.
+//   k_p2g_gather    per grid and 16 x 8 tile of faces: stage the
+//                   contributions of the particles that reach the tile, in
+//                   one run per stencil base and in slot order, then let each
+//                   face merge the runs of its four bases and fold them in
+//                   (chunk, corner, lane) order.
 //
 // Which cells can reach a face follows from the clamped index arithmetic
 // (u_index / v_index, :1029-1041): the u stencil's rows equal the density
@@ -59,14 +57,9 @@ namespace {
 // x in [i-1, i], y in [j-1, j].  A particle whose corners fall outside those
 // offsets (impossible by the arithmetic above, checked anyway) raises
 // kStatusP2gLayout.
-constexpr int kGatherTW = 32, kGatherTH = 8;           // tile of cells, one thread per cell
+constexpr int kGatherTW = 32, kGatherTH = 8;           // tile of cells (cell order), one thread per cell
 constexpr int kGatherThreads = kGatherTW * kGatherTH;
 constexpr int kRegionW = kGatherTW + 2, kRegionH = kGatherTH + 2;
-constexpr int kRegionBins = kRegionW * kRegionH;       // 340 cells whose particles a tile reads
-constexpr int kGatherCap = 2048;                       // staged particles per tile (more: read from global)
-// slot, corner code, 4 values, 4 weights, and the grid position and temporal
-// weight that every grid's contributions share
-constexpr size_t kGatherSmem = size_t(kGatherCap) * (4 + 4 + 8 * 4 + 3 * 4) + size_t(kRegionBins) * 8 + 64;
 
 enum { kGridU = 0, kGridV = 1, kGridD = 2 };
 
@@ -232,364 +225,441 @@ __device__ __forceinline__ bool p2g_record(const PartPtrs* __restrict__ pp, uint
     return ok;
 }
 
-// Records staged in shared memory (fast path) or computed from global memory
-// when they are needed (regions with more particles than the stage holds).
-// A staged slot carries kLastInRun in bit 31 when it is the last particle of
-// its cell's run (slots are below 2^31).
-constexpr uint32_t kLastInRun = 0x80000000u;
-struct StagedRecs {
-    static constexpr bool kStaged = true;
-    const uint32_t* slot;
-    const uint32_t* code;
-    const float* val;  // [4][kGatherCap]
-    const float* w;    // [4][kGatherCap]
-    __device__ __forceinline__ uint32_t code_at(int p) const { return code[p]; }
-    __device__ __forceinline__ float val_at(int k, int p) const { return val[k * kGatherCap + p]; }
-    __device__ __forceinline__ float w_at(int k, int p) const { return w[k * kGatherCap + p]; }
-};
-struct GlobalRecs {
-    static constexpr bool kStaged = false;
-    const uint32_t* vals;  // sorted slots
-    const PartPtrs* pp;
-    int grid, W, H;
-    CellSize cs;
-    float prev_dt;
-    uint32_t* status;
-    uint32_t n, npad;  // sorted pairs, particle lanes (the checked build tests against them)
-    __device__ __forceinline__ uint32_t slot_at(int p) const {
-        const uint32_t sl = APIC_IN_BOUNDS(uint32_t(p), n, status) ? vals[p] : 0u;
-        return APIC_IN_BOUNDS(sl, npad, status) ? sl : 0u;
-    }
-    __device__ __forceinline__ P2gRec rec(int p) const {
-        P2gRec r;
-        const uint32_t sl = slot_at(p);
-        if (!p2g_record(pp, sl, p2g_base(pp, sl, cs, prev_dt), grid, W, H, cs.dx, r)) atomicOr(status, kStatusP2gLayout);
-        return r;
-    }
-    __device__ __forceinline__ uint32_t code_at(int p) const { return rec(p).code; }
-    __device__ __forceinline__ float val_at(int k, int p) const { return rec(p).val[k]; }
-    __device__ __forceinline__ float w_at(int k, int p) const { return rec(p).w[k]; }
-};
-
-// The fold of one face over its contributions in slot order.  Consecutive
-// contributions of one chunk form the chunk's groups: per corner k, the
-// lanes' contributions summed in lane order; at the end of the chunk the
-// groups are added to the face in corner order.
-struct FaceFold {
-    float acc_v = 0.0f, acc_w = 0.0f;
-    float gv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    uint32_t gm = 0, chunk = 0xFFFFFFFFu;
-    template <bool kVal, class Recs>
-    __device__ __forceinline__ void add(const Recs& R, uint32_t slot, int p, uint32_t hit) {
-        if ((slot >> 3) != chunk) {
-            flush<kVal>();
-            chunk = slot >> 3;
-        }
-        // only the corners that land here are read (usually one)
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (hit & (1u << k)) {
-                if (kVal) gv[k] = gv[k] + R.val_at(k, p);
-                gw[k] = gw[k] + R.w_at(k, p);
-            }
-        gm |= hit;
-    }
-    template <bool kVal>
-    __device__ __forceinline__ void flush() {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (gm & (1u << k)) {
-                if (kVal) acc_v = acc_v + gv[k];
-                acc_w = acc_w + gw[k];
-            }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) { gv[k] = 0.0f; gw[k] = 0.0f; }
-        gm = 0;
-    }
-};
-
-// Fold of one face: merge NR slot-ordered runs [b, e) by slot; run r's
-// records reach this face through the corners in bits 4r .. 4r + 3 of their
-// code.
-//
-// Staged form: each run's head is one 64-bit key (slot << 32 | position << 5
-// | last-in-run << 4 | run), so the merge step is a minimum over NR keys and
-// the head's successor is the next staged position unless the head ends its
-// run.  Global form: positions and ends in registers.
-template <int NR, bool kVal, bool kRef, class Recs>
-__device__ __forceinline__ void fold_face(const Recs& R, int (&b)[NR], const int (&e)[NR], float& out_v,
-                                          float& out_w) {
-    if constexpr (!kRef) {
-        // cell order: the runs one after another, slots ascending in each,
-        // the corners that land here in corner order
-        float av = 0.0f, aw = 0.0f;
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-            for (int p = b[r]; p < e[r]; ++p) {
-                if constexpr (Recs::kStaged) {
-                    const uint32_t hit = (R.code_at(p) >> (4 * r)) & 0xFu;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (hit & (1u << k)) {
-                            if (kVal) av = av + R.val_at(k, p);
-                            aw = aw + R.w_at(k, p);
-                        }
-                } else {
-                    const P2gRec rr = R.rec(p);
-                    const uint32_t hit = (rr.code >> (4 * r)) & 0xFu;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (hit & (1u << k)) {
-                            if (kVal) av = av + rr.val[k];
-                            aw = aw + rr.w[k];
-                        }
-                }
-            }
-        out_v = av;
-        out_w = aw;
-        return;
-    }
-    FaceFold f;
-    if constexpr (Recs::kStaged) {
-        auto key_at = [&](uint32_t p, uint32_t r) {
-            const uint32_t sw = R.slot[p];
-            return (uint64_t(sw & ~kLastInRun) << 32) | (uint64_t(p) << 5) | (uint64_t(sw >> 31) << 4) | uint64_t(r);
-        };
-        uint64_t key[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) key[r] = b[r] < e[r] ? key_at(uint32_t(b[r]), uint32_t(r)) : ~0ull;
-        for (;;) {
-            uint64_t best = key[0];
-#pragma unroll
-            for (int r = 1; r < NR; ++r) best = key[r] < best ? key[r] : best;
-            if (best == ~0ull) break;
-            const uint32_t m = uint32_t(best) & 0xFu;
-            const uint32_t p = uint32_t(best >> 5) & 0x07FFFFFFu;
-            const uint64_t nk = ((best >> 4) & 1u) ? ~0ull : key_at(p + 1u, m);
-#pragma unroll
-            for (int r = 0; r < NR; ++r) key[r] = uint32_t(r) == m ? nk : key[r];
-            const uint32_t hit = (R.code_at(int(p)) >> (4u * m)) & 0xFu;
-            if (hit) f.template add<kVal>(R, uint32_t(best >> 32), int(p), hit);
-        }
-    } else {
-        uint32_t hs[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) hs[r] = b[r] < e[r] ? R.slot_at(b[r]) : 0xFFFFFFFFu;
-        for (;;) {
-            uint32_t best = hs[0];
-            int m = 0;
-#pragma unroll
-            for (int r = 1; r < NR; ++r)
-                if (hs[r] < best) { best = hs[r]; m = r; }
-            if (best == 0xFFFFFFFFu) break;
-            int p = 0;
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (r == m) {
-                    p = b[r];
-                    b[r] = p + 1;
-                    hs[r] = b[r] < e[r] ? R.slot_at(b[r]) : 0xFFFFFFFFu;
-                }
-            const uint32_t hit = (R.code_at(p) >> (4 * m)) & 0xFu;
-            if (hit) f.template add<kVal>(R, best, p, hit);
-        }
-    }
-    f.template flush<kVal>();
-    out_v = f.acc_v;
-    out_w = f.acc_w;
+// A particle whose three stencils lie inside their grids, so that no index is
+// clamped: it reaches four different nodes of each grid, and its u base is
+// its density base or the column after it, its v base that or the row above.
+__device__ __forceinline__ bool p2g_inside(const P2gBase& b, int W, int H) {
+    const float cx = floorf(b.gx - 0.5f), cy = floorf(b.gy - 0.5f);
+    return cx >= 0.0f && cx <= float(W - 2) && cy >= 0.0f && cy <= float(H - 2);
 }
 
 struct GatherOut {
     float *acc_u, *acc_uw, *acc_v, *acc_vw, *dens;
 };
 
-// The faces and cells of this thread's cell (i, j) for one grid; bin(x, y)
-// gives a cell's run (empty outside the grid).  Run r of a face is the cell
-// at offset (rx, ry) with r = ry * nx + rx, the index p2g_record codes.
-template <bool kRef, class Recs, class Bin>
-__device__ __forceinline__ void fold_cell(const Recs& R, const Bin& bin, int grid, int i, int j, int W, int H,
-                                          const GatherOut& o) {
-    auto run = [&](int x, int y, int& b, int& e) {
-        if (x < 0 || x >= W || y < 0 || y >= H) { b = e = 0; return; }
-        bin(x, y, b, e);
+// ---- one face from global memory (any particles) ----
+// The face's cells' runs are merged by slot and each particle's record is
+// computed when its turn comes.  For tiles whose particles do not fit the
+// stage even for one row of faces, and for particles outside the inner cells
+// (the first substep after such a set was written: advection keeps particles
+// 1.001 cells from the walls).
+__device__ __noinline__ void fold_face_global(const PartPtrs* __restrict__ pp, const uint32_t* __restrict__ vals,
+                                              const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
+                                              int grid, int x, int y, int W, int H, CellSize cs, float prev_dt,
+                                              uint32_t* status, uint32_t n, uint32_t npad, float& out_v,
+                                              float& out_w) {
+    // the cell of run r lies at offset (r % nx, r / nx) below and to the left,
+    // the index by which p2g_record codes the corners
+    const int nx = grid == kGridU ? 3 : 2, nr = grid == kGridD ? 4 : 6;
+    uint32_t b[6], e[6], head[6];
+    auto slot_at = [&](uint32_t p) {
+        const uint32_t sl = APIC_IN_BOUNDS(p, n, status) ? vals[p] : 0u;
+        return APIC_IN_BOUNDS(sl, npad, status) ? sl : 0u;
     };
-    if (grid == kGridU) {
-        // u face (fi, j), and (W, j) from the last column's thread
-        for (int fi = i; fi <= (i == W - 1 ? W : i); ++fi) {
-            int b[6], e[6];
 #pragma unroll
-            for (int r = 0; r < 6; ++r) run(fi - r % 3, j - r / 3, b[r], e[r]);
-            float v, w;
-            fold_face<6, true, kRef>(R, b, e, v, w);
-            const uint32_t f = uint32_t(j) * uint32_t(W + 1) + uint32_t(fi);
-            o.acc_u[f] = v;
-            o.acc_uw[f] = w;
+    for (int r = 0; r < 6; ++r) {
+        const int cx = x - r % nx, cy = y - r / nx;
+        b[r] = e[r] = 0;
+        if (r < nr && cx >= 0 && cx < W && cy >= 0 && cy < H) {
+            const uint32_t c = uint32_t(cy) * uint32_t(W) + uint32_t(cx);
+            b[r] = lo[c];
+            e[r] = hi[c];
         }
-    } else if (grid == kGridV) {
-        for (int fj = j; fj <= (j == H - 1 ? H : j); ++fj) {
-            int b[6], e[6];
-#pragma unroll
-            for (int r = 0; r < 6; ++r) run(i - r % 2, fj - r / 2, b[r], e[r]);
-            float v, w;
-            fold_face<6, true, kRef>(R, b, e, v, w);
-            const uint32_t f = uint32_t(fj) * uint32_t(W) + uint32_t(i);
-            o.acc_v[f] = v;
-            o.acc_vw[f] = w;
-        }
-    } else {
-        int b[4], e[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) run(i - r % 2, j - r / 2, b[r], e[r]);
-        float v, w;
-        fold_face<4, false, kRef>(R, b, e, v, w);
-        o.dens[uint32_t(j) * uint32_t(W) + uint32_t(i)] = w;
+        head[r] = b[r] < e[r] ? slot_at(b[r]) : 0xFFFFFFFFu;
     }
+    // per chunk and corner the lanes' contributions in lane order; at the end
+    // of the chunk the corners' sums are added to the face in corner order
+    float av = 0.0f, aw = 0.0f, gv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    uint32_t chunk = 0xFFFFFFFFu;
+    bool bad = false;
+    auto flush = [&] {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {  // (no sum here is ever -0: a corner without terms adds nothing)
+            av = av + gv[k];
+            aw = aw + gw[k];
+            gv[k] = gw[k] = 0.0f;
+        }
+    };
+    for (;;) {
+        uint32_t slot = head[0];
+        int m = 0;
+#pragma unroll
+        for (int r = 1; r < 6; ++r)
+            if (head[r] < slot) { slot = head[r]; m = r; }
+        if (slot == 0xFFFFFFFFu) break;
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+            if (r == m) {
+                ++b[r];
+                head[r] = b[r] < e[r] ? slot_at(b[r]) : 0xFFFFFFFFu;
+            }
+        P2gRec rec;
+        if (!p2g_record(pp, slot, p2g_base(pp, slot, cs, prev_dt), grid, W, H, cs.dx, rec)) bad = true;
+        const uint32_t hit = (rec.code >> (4 * m)) & 0xFu;
+        if (!hit) continue;
+        if ((slot >> 3) != chunk) {
+            flush();
+            chunk = slot >> 3;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (hit & (1u << k)) {
+                if (grid != kGridD) gv[k] = gv[k] + rec.val[k];
+                gw[k] = gw[k] + rec.w[k];
+            }
+    }
+    flush();
+    if (bad) atomicOr(status, kStatusP2gLayout);
+    out_v = av;
+    out_w = aw;
 }
 
-// One CTA per 32 x 8 tile.  The region's cell counts are scanned once; when
-// the region holds more particles than the stage (dense scenes: the
-// reference's default block has 9 per cell), the tile is processed as 2, 4
-// or 8 bands of rows, each staging only its own region (band rows plus the
-// two-row halo); a single row whose region still overflows reads its records
-// from global memory.  kRef: the reference's order, else cell order
-// (APIC_OPT_P2G_ORDER).
-template <bool kRef>
-__global__ void __launch_bounds__(kGatherThreads, 2) k_p2g_gather(const PartPtrs* __restrict__ pp,
-                                                                  const uint32_t* __restrict__ vals,
-                                                                  const uint32_t* __restrict__ lo,
-                                                                  const uint32_t* __restrict__ hi, int W, int H,
-                                                                  CellSize cs, Ctl* __restrict__ ctl, GatherOut o,
-                                                                  uint32_t n, uint32_t npad) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t* s_slot = reinterpret_cast<uint32_t*>(smem);
-    uint32_t* s_code = s_slot + kGatherCap;
-    float* s_val = reinterpret_cast<float*>(s_code + kGatherCap);
-    float* s_w = s_val + 4 * kGatherCap;
-    float* s_gx = s_w + 4 * kGatherCap;
-    float* s_gy = s_gx + kGatherCap;
-    float* s_wt = s_gy + kGatherCap;
-    uint32_t* s_off = reinterpret_cast<uint32_t*>(s_wt + kGatherCap);  // kRegionBins + 1
-    uint32_t* s_glo = s_off + kRegionBins + 1;                            // kRegionBins
-    __shared__ uint32_t s_total, s_band;
-    __shared__ uint32_t s_rowg[kRegionH];
+// ---- the gather in the reference's order ----
+// One CTA per grid (u, v, density) and 16 x 8 tile of its faces.  A particle
+// inside the grids reaches a face through one corner, given by the offset of
+// its stencil base from the face, so a face's terms are those of four runs of
+// particles, one per base, corner k of the run at base (-(k & 1), -(k >> 1)).
+// The sorted pairs give the runs of the density bases; the u base is that or
+// the next column (s = 1), the v base that or the next row, so a u or v run is
+// the s = 0 particles of one cell and the s = 1 particles of the cell before it
+// on the line (a row of cells for u, a column for v).  A particle's place in
+// its run is a count of s bits in its own cell and a binary search by slot in
+// the other.  Within a run the chunk never falls, so merging the four heads by
+// (chunk, corner) yields the terms group by group in the reference's order:
+// some 40 instructions a term.  The stage holds two words and four (value,
+// weight) pairs a particle; a tile whose particles exceed it is done in bands
+// of rows.
+//
+// What bounds it is issue slots and the latency of the field loads together: a
+// particle's place and record (about 250 instructions a grid, on 1.2-1.3 times
+// the particles for the halo) and the merge (12 terms a particle).  Three CTAs
+// an SM are 24 warps; half of a CTA's threads have no face, they help to stage.
+// 4.6 million particles, nine a cell: 655 -> 392 us against one CTA per 32 x 8
+// tile and all grids whose faces merged six runs of unsplit cells; the stage
+// of a 64 x 64 grid, where 96 CTAs run instead of 16, 143 -> 42 us.
+constexpr int kFaceTW = 16, kFaceTH = 8, kFaceThreads = 256;
+constexpr int kFaceCap = 1760;  // staged particles (three CTAs per SM)
+constexpr size_t kFaceSmem = size_t(kFaceCap) * (4 + 4 + 4 * 8 + 1);
+constexpr int kFaceRegion = (kFaceTW + 1) * (kFaceTH + 2);  // cells, of v the most (u: 18 x 9)
+static_assert(kFaceRegion >= (kFaceTW + 2) * (kFaceTH + 1) && kFaceRegion <= kFaceThreads, "one thread per cell");
 
-    const int x0 = blockIdx.x * kGatherTW, y0 = blockIdx.y * kGatherTH;
-    const int rx0 = x0 - 2, ry0 = y0 - 2;
-    const int tx = threadIdx.x % kGatherTW, ty = threadIdx.x / kGatherTW;
-    const int i = x0 + tx, j = y0 + ty;
-    const bool cell = i < W && j < H;
-    pdl_wait();
+struct FaceShared {
+    uint32_t sums[kFaceThreads / 32];
+    uint32_t cnt[kFaceRegion], glo[kFaceRegion];  // particles of each cell, first sorted pair (row by row)
+    uint32_t off[kFaceRegion + 1];                // the band's cells along its lines: first place,
+    uint32_t from[kFaceRegion];                   // sorted pair of place 0 of a row that starts with the cell,
+    uint32_t one[kFaceRegion + 1];                // and how many places before it hold s = 1
+    uint32_t bits[kFaceCap / 32 + 1], before[kFaceCap / 32 + 1];  // s of 32 places, s = 1 before them
+    uint32_t row_n[kFaceTH + 2];                  // particles of each row
+};
+
+// The sum over the block, to every thread.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* sums) {
+    const uint32_t lane = threadIdx.x & 31u;
+    v = __reduce_add_sync(0xffffffffu, v);
+    if (lane == 0) sums[threadIdx.x / 32u] = v;
+    __syncthreads();
+    return __reduce_add_sync(0xffffffffu, lane < kFaceThreads / 32 ? sums[lane] : 0u);
+}
+
+template <int G>
+__device__ __forceinline__ void gather_tile(const PartPtrs* __restrict__ pp, const uint32_t* __restrict__ vals,
+                                            const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi, int W,
+                                            int H, CellSize cs, Ctl* __restrict__ ctl, float* __restrict__ out_v,
+                                            float* __restrict__ out_w, uint32_t n, uint32_t npad, FaceShared& sh,
+                                            unsigned char* smem) {
+    constexpr int HX = G == kGridU ? 2 : 1, HY = G == kGridV ? 2 : 1;
+    constexpr int RW = kFaceTW + HX, RH = kFaceTH + HY;
+    const int FW = G == kGridU ? W + 1 : W, FH = G == kGridV ? H + 1 : H;
+    float2* rec = reinterpret_cast<float2*>(smem);                         // [4][kFaceCap]
+    uint32_t* cells = reinterpret_cast<uint32_t*>(rec + 4 * kFaceCap);     // by cell: slot | s << 31
+    uint32_t* runs = cells + kFaceCap;                                     // by run: slot & ~7 | last of its run
+    uint8_t* cell_of = reinterpret_cast<uint8_t*>(runs + kFaceCap);
+    const float *fpx = pp->f[PX], *fpy = pp->f[PY], *ftr = pp->f[TR];
+    const float* fvel = pp->f[G == kGridU ? VX : VY];
+    const float *fgx = pp->f[G == kGridU ? CUX : CVX], *fgy = pp->f[G == kGridU ? CUY : CVY];
+    const int x0 = blockIdx.x * kFaceTW, y0 = blockIdx.y * kFaceTH;
+    if (x0 >= FW || y0 >= FH) return;
+    const int rx0 = x0 - HX, ry0 = y0 - HY;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    const int tx = int(t) % kFaceTW, ty = int(t) / kFaceTW;
+    const int fx = x0 + tx, fy = y0 + ty;
+    const bool face = ty < kFaceTH && fx < FW && fy < FH;
+    const uint32_t f = uint32_t(fy) * uint32_t(FW) + uint32_t(fx);
     const float prev_dt = ctl->prev_dt;
 
-    // the region's runs: counts, their exclusive scan, first global position per row
-    if (threadIdx.x < kRegionH) s_rowg[threadIdx.x] = 0xFFFFFFFFu;
-    uint32_t cnt[2] = {0u, 0u};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int rb = 2 * threadIdx.x + h;
-        if (rb < kRegionBins) {
-            const int x = rx0 + rb % kRegionW, y = ry0 + rb / kRegionW;
-            uint32_t gl = 0, gh = 0;
-            if (x >= 0 && x < W && y >= 0 && y < H) {
-                const uint32_t c = uint32_t(y) * uint32_t(W) + uint32_t(x);
-                gl = lo[c];
-                gh = hi[c];
-            }
-            cnt[h] = gh - gl;
-            s_glo[rb] = gl;
+    // the region's cells
+    uint32_t cnt = 0;
+    if (t < RW * RH) {
+        const int x = rx0 + int(t) % RW, y = ry0 + int(t) / RW;
+        uint32_t gl = 0, gh = 0;
+        if (x >= 0 && x < W && y >= 0 && y < H) {
+            const uint32_t c = uint32_t(y) * uint32_t(W) + uint32_t(x);
+            gl = lo[c];
+            gh = hi[c];
+            if (!APIC_IN_BOUNDS(gh, uint64_t(n) + 1u, &ctl->status)) gh = gl;
         }
+        cnt = gh - gl;
+        sh.cnt[t] = cnt;
+        sh.glo[t] = gl;
     }
-    uint32_t tot;
-    const uint32_t ex = block_exclusive_scan_u32(cnt[0] + cnt[1], &tot);
-    if (2 * threadIdx.x < kRegionBins) s_off[2 * threadIdx.x] = ex;
-    if (2 * threadIdx.x + 1 < kRegionBins) s_off[2 * threadIdx.x + 1] = ex + cnt[0];
-    if (threadIdx.x == 0) { s_off[kRegionBins] = tot; s_total = tot; }
-    __syncthreads();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int rb = 2 * threadIdx.x + h;
-        if (rb < kRegionBins && cnt[h] > 0) atomicMin(&s_rowg[rb / kRegionW], s_glo[rb]);
-    }
-    if (threadIdx.x == 0) {
-        // the tallest band whose every region fits the stage (0: none)
-        uint32_t band = 0;
-        for (uint32_t th = kGatherTH; th >= 1 && !band; th >>= 1) {
-            bool fits = true;
-            for (uint32_t r0 = 0; r0 < uint32_t(kGatherTH); r0 += th)
-                fits = fits && s_off[(r0 + th + 2) * kRegionW] - s_off[r0 * kRegionW] <= uint32_t(kGatherCap);
-            if (fits) band = th;
-        }
-        s_band = band;
-    }
-    __syncthreads();
-    const uint32_t band = s_band;
-
-    if (band == 0) {
-        // more particles than the stage holds even for one row: every face
-        // reads its runs from global memory and computes the records it needs
-        for (int g = 0; g < 3; ++g) {
-            GlobalRecs R{vals, pp, g, W, H, cs, prev_dt, &ctl->status, n, npad};
-            auto bin = [&](int x, int y, int& b, int& e) {
-                const uint32_t c = uint32_t(y) * uint32_t(W) + uint32_t(x);
-                b = int(lo[c]);
-                e = int(hi[c]);
-            };
-            if (cell) fold_cell<kRef>(R, bin, g, i, j, W, H, o);
+    const uint32_t total = block_sum(cnt, sh.sums);
+    if (total == 0) {
+        if (face) {
+            if (G != kGridD) out_v[f] = 0.0f;
+            out_w[f] = 0.0f;
         }
         return;
     }
-    const StagedRecs R{s_slot, s_code, s_val, s_w};
-    for (uint32_t r0 = 0; r0 < uint32_t(kGatherTH); r0 += band) {
-        const uint32_t r1 = r0 + band + 2;  // region rows [r0, r1)
-        const uint32_t base = s_off[r0 * kRegionW];
-        const uint32_t P = s_off[r1 * kRegionW] - base;
-        // stage the slots: each region row is one contiguous range of the sorted pairs
-        for (uint32_t r = r0; r < r1; ++r) {
-            const uint32_t s0 = s_off[r * kRegionW] - base, s1 = s_off[(r + 1) * kRegionW] - base;
-            const uint32_t g0 = s_rowg[r];
-            for (uint32_t q = threadIdx.x; q < s1 - s0; q += kGatherThreads) {
-                const uint32_t sl = APIC_IN_BOUNDS(g0 + q, n, &ctl->status) ? vals[g0 + q] : 0u;
-                s_slot[s0 + q] = APIC_IN_BOUNDS(sl, npad, &ctl->status) ? sl : 0u;
+    // the tallest band whose every region fits the stage (0: none)
+    uint32_t band = kFaceTH;
+    if (total > uint32_t(kFaceCap)) {
+        for (uint32_t r = warp; r < RH; r += kFaceThreads / 32) {
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, lane < RW ? sh.cnt[r * RW + lane] : 0u);
+            if (lane == 0) sh.row_n[r] = sum;
+        }
+        __syncthreads();
+        for (band = kFaceTH / 2; band >= 1; band >>= 1) {
+            bool fits = true;
+            for (uint32_t r0 = 0; r0 < uint32_t(kFaceTH); r0 += band) {
+                uint32_t sum = 0;
+                for (uint32_t r = r0; r < r0 + band + HY; ++r) sum += sh.row_n[r];
+                fits = fits && sum <= uint32_t(kFaceCap);
+            }
+            if (fits) break;
+        }
+    }
+
+    for (uint32_t r0 = 0; r0 < uint32_t(kFaceTH); r0 += band ? band : uint32_t(kFaceTH)) {
+        const uint32_t nrow = (band ? band : uint32_t(kFaceTH)) + HY;  // region rows [r0, r0 + nrow)
+        const bool mine = face && uint32_t(ty) >= r0 && uint32_t(ty) < r0 + nrow - HY;
+        // cell (x, y) of the band's region along the lines
+        auto at = [&](uint32_t x, uint32_t y) { return G == kGridV ? x * nrow + y : y * RW + x; };
+        bool odd = band == 0;
+        uint32_t P = 0;
+        if (band) {
+            const uint32_t x = G == kGridV ? t / nrow : t % RW, y = G == kGridV ? t % nrow : t / RW;
+            const bool in = t < RW * nrow;
+            const uint32_t mine_n = in ? sh.cnt[(r0 + y) * RW + x] : 0u;
+            const uint32_t ex = block_exclusive_scan_u32(mine_n, &P);
+            if (in) {
+                sh.off[t] = ex;
+                sh.from[t] = sh.glo[(r0 + y) * RW + x] - ex;
+                for (uint32_t k = 0; k < mine_n; ++k) cell_of[ex + k] = uint8_t(t);
+            }
+            if (t == 0) sh.off[RW * nrow] = P;
+            if (P == 0) {  // (the same for every thread)
+                if (mine) {
+                    if (G != kGridD) out_v[f] = 0.0f;
+                    out_w[f] = 0.0f;
+                }
+                __syncthreads();
+                continue;
+            }
+            __syncthreads();
+            // each cell's particles in slot order, with s; three a thread in flight
+            for (uint32_t p0 = t; p0 - lane < P; p0 += 3 * kFaceThreads) {
+                uint32_t slot[3];
+                float px[3], py[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const uint32_t p = p0 + uint32_t(i) * kFaceThreads;
+                    slot[i] = 0;
+                    if (p < P) {
+                        const uint32_t g = sh.from[cell_of[p]] + p;
+                        if (APIC_IN_BOUNDS(g, n, &ctl->status)) slot[i] = vals[g];
+                        if (!APIC_IN_BOUNDS(slot[i], npad, &ctl->status)) slot[i] = 0;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    px[i] = fpx[slot[i]];
+                    py[i] = fpy[slot[i]];
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const uint32_t p = p0 + uint32_t(i) * kFaceThreads;
+                    if (p - lane >= P) break;  // (warps as a whole)
+                    const float gx = over_dx(px[i], cs), gy = over_dx(py[i], cs);
+                    odd = odd || (p < P && !p2g_inside(P2gBase{gx, gy, 0.0f}, W, H));
+                    const bool s = p < P && (G == kGridU   ? floorf(gx) != floorf(gx - 0.5f)
+                                             : G == kGridV ? floorf(gy) != floorf(gy - 0.5f)
+                                                           : false);
+                    if (p < P) cells[p] = slot[i] | (s ? 0x80000000u : 0u);
+                    if (G != kGridD) {
+                        const uint32_t b = __ballot_sync(0xffffffffu, s);
+                        if (lane == 0) sh.bits[p / 32u] = b;
+                    }
+                }
+            }
+            odd = __syncthreads_or(odd) != 0;
+        }
+        if (odd) {
+            float v, w;
+            if (mine) {
+                fold_face_global(pp, vals, lo, hi, G, fx, fy, W, H, cs, prev_dt, &ctl->status, n, npad, v, w);
+                if (G != kGridD) out_v[f] = v;
+                out_w[f] = w;
+            }
+            __syncthreads();
+            continue;
+        }
+        auto ones = [&](uint32_t p) {  // places before p with s = 1
+            return sh.before[p / 32u] + uint32_t(__popc(sh.bits[p / 32u] & ((1u << (p % 32u)) - 1u)));
+        };
+        if (G != kGridD) {
+            // the count of s = 1 before every word of places (each warp for
+            // itself), then before every cell
+            {
+                const uint32_t words = (P + 31u) / 32u;
+                const uint32_t a = 2u * lane < words ? __popc(sh.bits[2u * lane]) : 0u;
+                const uint32_t b = 2u * lane + 1u < words ? __popc(sh.bits[2u * lane + 1u]) : 0u;
+                uint32_t sum = a + b;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t up = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= uint32_t(o)) sum += up;
+                }
+                if (2u * lane <= words) sh.before[2u * lane] = sum - a - b;
+                if (2u * lane + 1u <= words) sh.before[2u * lane + 1u] = sum - b;
+                __syncwarp();
+            }
+            if (t <= RW * nrow) sh.one[t] = ones(sh.off[t]);
+            __syncthreads();
+        }
+        // the run of base c: the s = 1 particles of the cell before it on the
+        // line and the s = 0 particles of cell c, in slot order (the runs that
+        // a line starts or ends with reach no face of the tile)
+        auto run_begin = [&](uint32_t c) { return G == kGridD ? sh.off[c] : sh.off[c] - (sh.one[c] - sh.one[c - 1]); };
+        auto run_end = [&](uint32_t c) { return G == kGridD ? sh.off[c + 1] : sh.off[c + 1] - (sh.one[c + 1] - sh.one[c]); };
+        // (the next particle's fields are on their way while this one is placed)
+        struct Fields {
+            uint32_t own;
+            float px, py, tr, vel, gx, gy;
+        };
+        auto load = [&](uint32_t p) {
+            Fields r;
+            r.own = p < P ? cells[p] : 0u;
+            const uint32_t slot = r.own & 0x7FFFFFFFu;
+            r.px = fpx[slot];
+            r.py = fpy[slot];
+            r.tr = ftr[slot];
+            if (G != kGridD) {
+                r.vel = fvel[slot];
+                r.gx = fgx[slot];
+                r.gy = fgy[slot];
+            }
+            return r;
+        };
+        Fields ahead = load(t);
+        for (uint32_t p = t; p < P; p += kFaceThreads) {
+            const Fields cur = ahead;
+            ahead = load(p + kFaceThreads);
+            const uint32_t slot = cur.own & 0x7FFFFFFFu, s = cur.own >> 31;
+            P2gBase b;
+            b.gx = over_dx(cur.px, cs);
+            b.gy = over_dx(cur.py, cs);
+            uint32_t c = cell_of[p], place = p;
+            if (G != kGridD) {
+                const uint32_t pos = G == kGridU ? uint32_t(int(floorf(b.gx - 0.5f)) - rx0)
+                                                 : uint32_t(int(floorf(b.gy - 0.5f)) - ry0) - r0;
+                const uint32_t len = G == kGridU ? uint32_t(RW) : nrow;
+                if (pos + s == 0u || pos + s == len) continue;  // (a run that no face reads)
+                // its place: the cell's earlier particles with the same s, and the
+                // lower slots of the run's other cell with the other s
+                const uint32_t o = s ? c + 1u : c - 1u, ob = sh.off[o];
+                uint32_t at2 = ob, len2 = sh.off[o + 1] - ob;
+                while (len2 > 0) {
+                    const uint32_t half = len2 >> 1;
+                    const bool below = (cells[at2 + half] & 0x7FFFFFFFu) < slot;
+                    at2 = below ? at2 + half + 1u : at2;
+                    len2 = below ? len2 - half - 1u : half;
+                }
+                const uint32_t k1 = ones(p) - sh.one[c], o1 = ones(at2) - sh.one[o];
+                place = s ? k1 + (at2 - ob) - o1 : p - sh.off[c] - k1 + o1;
+                c += s;
+                place += run_begin(c);
+            }
+            runs[place] = (slot & ~7u) | (place + 1u == run_end(c) ? 1u : 0u);
+            b.wt = temporal_w((-cur.tr) / prev_dt);
+            if (G == kGridD) {
+                const float cgx = b.gx - 0.5f, cgy = b.gy - 0.5f;
+                const float ctx = cgx - floorf(cgx), cty = cgy - floorf(cgy);
+                float* rw = reinterpret_cast<float*>(rec);
+                rw[0 * kFaceCap + place] = ((1.0f - ctx) * (1.0f - cty)) * b.wt;
+                rw[1 * kFaceCap + place] = (ctx * (1.0f - cty)) * b.wt;
+                rw[2 * kFaceCap + place] = ((1.0f - ctx) * cty) * b.wt;
+                rw[3 * kFaceCap + place] = (ctx * cty) * b.wt;
+            } else {
+                Stencil st;
+                if (G == kGridU) u_stencil(b.gx, b.gy, W, H, cs.dx, st);
+                else v_stencil(b.gx, b.gy, W, H, cs.dx, st);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float w = st.w[k] * b.wt;
+                    rec[k * kFaceCap + place] = make_float2((cur.vel + cur.gx * st.ox[k] + cur.gy * st.oy[k]) * w, w);
+                }
             }
         }
         __syncthreads();
-        if constexpr (kRef) {
-            // mark each run's last particle (the merge reads it)
-            for (uint32_t rb = r0 * kRegionW + threadIdx.x; rb < r1 * kRegionW; rb += kGatherThreads)
-                if (s_off[rb + 1] > s_off[rb]) s_slot[s_off[rb + 1] - 1u - base] |= kLastInRun;
-            __syncthreads();
-        }
-        for (uint32_t p = threadIdx.x; p < P; p += kGatherThreads) {
-            const P2gBase bs = p2g_base(pp, s_slot[p] & ~kLastInRun, cs, prev_dt);
-            s_gx[p] = bs.gx;
-            s_gy[p] = bs.gy;
-            s_wt[p] = bs.wt;
-        }
-        auto bin = [&](int x, int y, int& b, int& e) {
-            const int rb = (y - ry0) * kRegionW + (x - rx0);
-            b = int(s_off[rb] - base);
-            e = int(s_off[rb + 1] - base);
-        };
-        const bool mine = cell && uint32_t(ty) >= r0 && uint32_t(ty) < r0 + band;
-        for (int g = 0; g < 3; ++g) {
-            bool bad = false;
-            for (uint32_t p = threadIdx.x; p < P; p += kGatherThreads) {
-                P2gRec rec;
-                const P2gBase bs{s_gx[p], s_gy[p], s_wt[p]};
-                if (!p2g_record(pp, s_slot[p] & ~kLastInRun, bs, g, W, H, cs.dx, rec)) bad = true;
-                s_code[p] = rec.code;
+        if (mine) {
+            uint32_t head[4], pos[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (g != kGridD) s_val[k * kGatherCap + p] = rec.val[k];
-                    s_w[k * kGatherCap + p] = rec.w[k];
+            for (uint32_t k = 0; k < 4; ++k) {
+                const uint32_t c = at(uint32_t(tx) + HX - (k & 1u), uint32_t(ty) - r0 + HY - (k >> 1));
+                const uint32_t b = run_begin(c);
+                pos[k] = b;
+                head[k] = b < run_end(c) ? runs[b] | (k << 1) : 0xFFFFFFFFu;
+            }
+            float av = 0.0f, aw = 0.0f, gv = 0.0f, gw = 0.0f;
+            uint32_t group = 0xFFFFFFFFu;
+            for (;;) {
+                const uint32_t best = min(min(head[0], head[1]), min(head[2], head[3]));
+                if (best == 0xFFFFFFFFu) break;
+                const uint32_t m = (best >> 1) & 3u;
+                const uint32_t p = m & 2u ? (m & 1u ? pos[3] : pos[2]) : (m & 1u ? pos[1] : pos[0]);
+                const uint32_t next = best & 1u ? 0xFFFFFFFFu : runs[p + 1u] | (best & 6u);
+                float2 r;
+                if (G == kGridD) r = make_float2(0.0f, reinterpret_cast<const float*>(rec)[m * kFaceCap + p]);
+                else r = rec[m * kFaceCap + p];
+                // a new (chunk, corner) group: the one before goes to the face
+                // (no sum here is ever -0, so adding an empty one changes nothing)
+                const bool fresh = (best >> 1) != group;
+                group = best >> 1;
+                if (G != kGridD) {
+                    av = fresh ? av + gv : av;
+                    gv = fresh ? r.x : gv + r.x;
+                }
+                aw = fresh ? aw + gw : aw;
+                gw = fresh ? r.y : gw + r.y;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    head[k] = k == m ? next : head[k];
+                    pos[k] = k == m ? p + 1u : pos[k];
                 }
             }
-            if (bad) atomicOr(&ctl->status, kStatusP2gLayout);
-            __syncthreads();
-            if (mine) fold_cell<kRef>(R, bin, g, i, j, W, H, o);
-            __syncthreads();
+            if (G != kGridD) out_v[f] = av + gv;
+            out_w[f] = aw + gw;
         }
+        __syncthreads();
     }
+}
+
+__global__ void __launch_bounds__(kFaceThreads, 3) k_p2g_gather(const PartPtrs* __restrict__ pp,
+                                                                const uint32_t* __restrict__ vals,
+                                                                const uint32_t* __restrict__ lo,
+                                                                const uint32_t* __restrict__ hi, int W, int H,
+                                                                CellSize cs, Ctl* __restrict__ ctl, GatherOut o,
+                                                                uint32_t n, uint32_t npad) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ FaceShared sh;
+    pdl_wait();
+    if (blockIdx.z == kGridU)
+        gather_tile<kGridU>(pp, vals, lo, hi, W, H, cs, ctl, o.acc_u, o.acc_uw, n, npad, sh, smem);
+    else if (blockIdx.z == kGridV)
+        gather_tile<kGridV>(pp, vals, lo, hi, W, H, cs, ctl, o.acc_v, o.acc_vw, n, npad, sh, smem);
+    else
+        gather_tile<kGridD>(pp, vals, lo, hi, W, H, cs, ctl, nullptr, o.dens, n, npad, sh, smem);
 }
 
 // Cell order (APIC_OPT_P2G_ORDER 2), one CTA per 32 x 8 tile.  Each cell of
@@ -624,15 +694,11 @@ __device__ __forceinline__ void add_partials(const P2gRec& rec, float (&pv)[NQ],
     }
 }
 
-// A particle whose three stencils lie inside their grids, so that no index is
-// clamped: its u corners start at column 0 or 1 of the six positions, its v
-// corners at row 0 or 1, its density corners are the four positions.  Every
-// position then takes at most one corner, by a select, where the general form
-// tests each corner against each position (24 tests a grid).
-__device__ __forceinline__ bool p2g_inside(const P2gBase& b, int W, int H) {
-    const float cx = floorf(b.gx - 0.5f), cy = floorf(b.gy - 0.5f);
-    return cx >= 0.0f && cx <= float(W - 2) && cy >= 0.0f && cy <= float(H - 2);
-}
+// For a particle inside (p2g_inside) the u corners start at column 0 or 1 of
+// the six positions, the v corners at row 0 or 1, the density corners are the
+// four positions.  Every position then takes at most one corner, by a select,
+// where the general form tests each corner against each position (24 tests a
+// grid).
 struct P2gRaw {
     float px, py, tr, vx, cux, cuy, vy, cvx, cvy;
 };
@@ -1002,8 +1068,8 @@ static CellSize cell_size(const Scene& s) { return CellSize{s.dx, exact_reciproc
 // caller clears them), every accumulator entry is written.
 cudaError_t launch_p2g(Scene& s) {
     const bool ref = p2g_reference_order(s);
-    cudaError_t e = cudaFuncSetAttribute(k_p2g_gather<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(kGatherSmem));
+    cudaError_t e = cudaFuncSetAttribute(k_p2g_gather, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(kFaceSmem));
     if (e != cudaSuccess) return e;
     const uint32_t* svals = s.bin_vals;
     if (s.n > 0) {
@@ -1018,9 +1084,11 @@ cudaError_t launch_p2g(Scene& s) {
         svals = vres;
     }
     GatherOut o{s.acc_u, s.acc_uw, s.acc_v, s.acc_vw, s.density};
-    dim3 grid(div_up(s.W, kGatherTW), div_up(s.H, kGatherTH));
+    const dim3 grid(div_up(s.W, kGatherTW), div_up(s.H, kGatherTH));
+    // a grid has up to (W + 1) x H or W x (H + 1) faces
+    const dim3 faces(div_up(s.W + 1, kFaceTW), div_up(s.H + 1, kFaceTH), 3);
     if (ref)
-        launch(s.use_pdl && s.n > 0, k_p2g_gather<true>, grid, kGatherThreads, kGatherSmem, s.stream,
+        launch(s.use_pdl && s.n > 0, k_p2g_gather, faces, kFaceThreads, kFaceSmem, s.stream,
                static_cast<const PartPtrs*>(s.pp), svals, static_cast<const uint32_t*>(s.bin_lo),
                static_cast<const uint32_t*>(s.bin_hi), int(s.W), int(s.H), cell_size(s), s.ctl, o, s.n, s.npad);
     else
