@@ -200,25 +200,35 @@ __device__ __forceinline__ const float* cur_res(const Level& B, const Ctl* ctl) 
     return ctl->res_sel && B.res2 ? B.res2 : B.res;
 }
 
-// The exit test and loop decision in every CTA of a kernel that runs after
-// the update and whose CTAs all go on or all return (a cluster, a single
-// CTA): each sums the parts itself, to the same verdict, and `writer`'s
-// thread 0 records it.  True: the solve is done.
-__device__ __forceinline__ bool exit_verdict(Ctl* ctl, const ExitArgs& a, bool writer) {
+// In every CTA of a kernel whose CTAs all go on or all return (a cluster, a
+// single CTA): whether the solve is over.  After an update (a.on) each CTA sums
+// the residual's parts itself, to the same verdict, and `writer`'s thread 0
+// records it and takes the loop decision, also where the update itself ended
+// the solve (else the loop would go on without end).  One thread reads
+// pcg_done: the writer may set it meanwhile, and a CTA's threads must agree.
+__device__ __forceinline__ bool solve_over(Ctl* ctl, const ExitArgs& a, bool writer) {
+    if (!a.on) return ctl->pcg_done != 0;
     __shared__ bool s_done;
-    double tot;
+    uint32_t was_done = 0, delta_stop = 0;
+    double bnorm2 = 0.0, target = 0.0, tot;
     float t;
+    if (threadIdx.x == 0) {  // (on their way during the sum)
+        was_done = ctl->pcg_done;
+        delta_stop = ctl->delta_stop;
+        bnorm2 = ctl->bnorm2;
+        target = ctl->target_rel;
+    }
     sum_max_partials<kSegBlock>(a.part, a.nparts, &tot, &t);
     if (threadIdx.x == 0) {
-        const bool stop = ctl->delta_stop != 0;
-        bool done = stop;
-        if (!stop && a.mode == APIC_SOLVER_REFERENCE) done = t < a.solve_error;
-        else if (!stop) done = (ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0) <= ctl->target_rel;
+        const bool before = was_done != 0, stop = !before && delta_stop != 0;
+        bool done = before || stop;
+        if (!done && a.mode == APIC_SOLVER_REFERENCE) done = t < a.solve_error;
+        else if (!done) done = (bnorm2 > 0.0 ? sqrt(tot / bnorm2) : 0.0) <= target;
         s_done = done;
         if (writer) {
             if (stop) ctl->res_sel ^= 1u;  // the update left the residual where it was
-            else if (a.mode == APIC_SOLVER_REFERENCE) ctl->max_r_bits = __float_as_uint(t);
-            else ctl->rnorm2 = tot;
+            else if (!before && a.mode == APIC_SOLVER_REFERENCE) ctl->max_r_bits = __float_as_uint(t);
+            else if (!before) ctl->rnorm2 = tot;
             if (done) ctl->pcg_done = 1;
             loop_decision(ctl, a.mode, a.h, a.cap, a.dyn_cap, a.set_cond);
         }

@@ -161,8 +161,7 @@ __global__ void __launch_bounds__(kTailThreads) k_coarse_solve(Level L, float* _
     }
     pdl_wait();
     cp_async_wait_all();
-    if (ctl->pcg_done) return;
-    if (exit.on && pcg::exit_verdict(ctl, exit, true)) return;
+    if (pcg::solve_over(ctl, exit, true)) return;
     __syncthreads();
     cta_coarse_cg(A, exact != 0);
 }
@@ -172,7 +171,7 @@ __global__ void __launch_bounds__(kTailThreads) k_vcycle_tail(const __grid_const
     extern __shared__ uint32_t sm[];
     cta_tail_issue_coeffs(tp, sm);  // while the previous kernel drains
     pdl_wait();
-    if (ctl->pcg_done || (exit.on && pcg::exit_verdict(ctl, exit, true))) {
+    if (pcg::solve_over(ctl, exit, true)) {
         cp_async_wait_all();
         return;
     }

@@ -240,18 +240,14 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_dsm(const __grid_con
     // it; waited for only before the first such write
     cl.barrier_arrive();
     pdl_wait();
-    // (the same value, and the same verdict, in every CTA)
-    bool done = ctl->pcg_done != 0;
-    if (!done) {
-        // the finest level's residual (written by the kernel before), halo included
-        for (int j = threadIdx.x; j < n2 / 2; j += kTailThreads) {
-            const int raw = base + 4 * j;
-            if (raw >= 0 && raw < p.cells)
-                cp_async16(first.r - kDsmHalo * first.w + 4 * j, p.res + size_t(raw) + first.w);
-        }
-        // the exit test where this is the first kernel after the update
-        done = exit.on && pcg::exit_verdict(ctl, exit, rank == 0);
+    // the finest level's residual (written by the kernel before), halo included
+    for (int j = threadIdx.x; j < n2 / 2; j += kTailThreads) {
+        const int raw = base + 4 * j;
+        if (raw >= 0 && raw < p.cells)
+            cp_async16(first.r - kDsmHalo * first.w + 4 * j, p.res + size_t(raw) + first.w);
     }
+    // (the same verdict in every CTA)
+    const bool done = pcg::solve_over(ctl, exit, rank == 0);
     cp_async_wait_all();
     __syncthreads();
     if (!done) {  // mask it (only the fluid cells' was written); its first red sweep
