@@ -424,30 +424,58 @@ __device__ __forceinline__ void block_store(Blk bk, F2 v, float mx, float4* part
     }
 }
 
-// Total of n partials, rounded to FP32 (by one thread: an FP64 conversion by
-// every warp of a full SM takes half a microsecond at GB300's FP64 rate),
-// returned to every thread of the block.
+// Totals of partials, rounded to FP32 (the high part of a normalised
+// double-float is its rounded value), to every thread: the parts of a thread
+// in ascending order, a shuffle tree per warp, the warps in order.  The loads
+// do not wait for anything, so a caller that may turn out to have nothing to
+// do sums first and asks then.
 template <int kThreads>
-__device__ __forceinline__ float sum_partials(const float2* part, uint32_t n) {
-    __shared__ F2 s_sp[kThreads / 32];
-    __shared__ float s_tot;
+__device__ __forceinline__ F2 lane_partials(const float2* part, uint32_t n) {
     F2 t{0.0f, 0.0f};
 #pragma unroll 4
     for (uint32_t b = threadIdx.x; b < n; b += kThreads) {
         const float2 q = __ldcg(part + b);
         t = f2_add(t, F2{q.x, q.y});
     }
-    t = warp_sum(t);
+    return t;
+}
+template <int kThreads>
+__device__ __forceinline__ float sum_partials(const float2* part, uint32_t n) {
+    __shared__ F2 s_sp[kThreads / 32];
+    __shared__ float s_tot;
+    const F2 t = warp_sum(lane_partials<kThreads>(part, n));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) s_sp[warp] = t;
     __syncthreads();
     if (threadIdx.x == 0) {
         F2 a{0.0f, 0.0f};
         for (int w = 0; w < kThreads / 32; ++w) a = f2_add(a, s_sp[w]);
-        s_tot = float(f2_value(a));
+        s_tot = a.hi;
     }
     __syncthreads();
     return s_tot;
+}
+// Two totals at once.
+template <int kThreads>
+__device__ __forceinline__ float2 sum_partials(const float2* part0, uint32_t n0, const float2* part1, uint32_t n1) {
+    __shared__ F2 s_sp2[2][kThreads / 32];
+    __shared__ float s_tot2[2];
+    F2 t0 = lane_partials<kThreads>(part0, n0), t1 = lane_partials<kThreads>(part1, n1);
+    t0 = warp_sum(t0);
+    t1 = warp_sum(t1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        s_sp2[0][warp] = t0;
+        s_sp2[1][warp] = t1;
+    }
+    __syncthreads();
+    if (lane == 0 && warp < 2) {
+        F2 a{0.0f, 0.0f};
+        for (int w = 0; w < kThreads / 32; ++w) a = f2_add(a, s_sp2[warp][w]);
+        s_tot2[warp] = a.hi;
+    }
+    __syncthreads();
+    return make_float2(s_tot2[0], s_tot2[1]);
 }
 
 // Sum and maximum of n float4 partials (x, y: F2 sum; z: maximum), by the

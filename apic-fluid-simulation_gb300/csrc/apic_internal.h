@@ -71,9 +71,10 @@ struct Ctl {
     unsigned long long solve_t0;  // %globaltimer at the start of the running solve (ns)
     unsigned long long solve_ns;  // summed solve time of this update (ns)
     uint32_t max_r_bits;    // max |r| (float bits)
-    uint32_t pcg_done;
+    uint32_t pcg_done;      // 1: ended by a test, kStoppedAtCap: by the iteration cap
     uint32_t pcg_iters;
     uint32_t pcg_iters_total;
+    uint32_t pcg_bodies;    // runs of the PCG loop's body (loop_body iterations each)
     uint32_t not_converged;
     uint32_t refinements;
     uint32_t inner_cap;     // iteration cap of the running (inner) solve
@@ -86,6 +87,7 @@ struct Ctl {
     double rnorm2;          // ||r||^2 of the recursive residual
     double true_rel;        // ||b - A p|| / ||b|| (FP64)
     double target_rel;      // tolerance of the running inner solve
+    double stop2;           // ||r||^2 at which the solve has reached it
     // fluid bookkeeping, per level (0 = base)
     uint32_t seg_count[kMaxLevels];
     uint32_t fluid_cells;   // base fluid cells (src/apic.rs:1461-1485)
@@ -99,6 +101,7 @@ struct Ctl {
     float b_sap;            // batched solve: the iteration's s.Ap sum
 };
 
+constexpr uint32_t kStoppedAtCap = 2u;  // Ctl::pcg_done
 enum : uint32_t {
     kStatusNonfinite = 1u,
     kStatusBadStep = 2u,
@@ -365,7 +368,8 @@ ExitArgs exit_args(const Scene& s, int mode);
 // z = M^-1 r on s.stream, in an iteration after the base level's down kernel
 // has run inside the update (base_done): the first kernel here runs the exit
 // test, and with a coarser level the last one stores the parts of r.z.
-void enqueue_vcycle(Scene& s, bool base_done = false, const ExitArgs& exit = ExitArgs());
+// sel: the base residual's buffer where it is known (0, 1), else -1.
+void enqueue_vcycle(Scene& s, bool base_done = false, const ExitArgs& exit = ExitArgs(), int sel = -1);
 // runtime.cu
 cudaError_t launch_plan_first(Scene& s);
 cudaError_t launch_advance(Scene& s);

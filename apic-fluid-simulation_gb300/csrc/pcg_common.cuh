@@ -153,13 +153,17 @@ __device__ __forceinline__ void finish_rz_reference(Ctl* ctl, float ng) {
 // converged, under the iteration cap; dyn_cap reads the remaining budget of a
 // refinement).  In the relative modes a continuing loop's next iteration
 // forms beta from the r.z parts that this iteration's V-cycle stores
-// (beta_valid); the reference mode's k_gamma_exact does that itself.  Run by
-// thread 0 of one block; loop_decision sets the graph's loop condition when
-// set_cond.
+// (beta_valid); the reference mode's k_gamma_exact does that itself.  A loop
+// that ends at the cap is marked in pcg_done too: the loop's body holds several
+// iterations, and those after the last must do nothing.  Run by thread 0 of
+// one block; loop_decision sets the graph's loop condition when set_cond.
 __device__ __forceinline__ bool loop_continue(Ctl* ctl, int mode, uint32_t cap, int dyn_cap) {
     const uint32_t c = dyn_cap ? ctl->inner_cap : cap;
     const bool cont = !ctl->pcg_done && ctl->pcg_iters < c;
-    if (cont && mode != APIC_SOLVER_REFERENCE) ctl->beta_valid = 1;
+    if (mode != APIC_SOLVER_REFERENCE) {
+        if (cont) ctl->beta_valid = 1;
+        else if (!ctl->pcg_done) ctl->pcg_done = kStoppedAtCap;
+    }
     return cont;
 }
 __device__ __forceinline__ void loop_decision(Ctl* ctl, int mode, cudaGraphConditionalHandle h, uint32_t cap,
@@ -189,10 +193,17 @@ __device__ __forceinline__ void residual_exit(Ctl* ctl, const float4* part, uint
             if (t < solve_error) ctl->pcg_done = 1;
         } else {
             ctl->rnorm2 = tot;
-            const double rel = ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0;
-            if (rel <= ctl->target_rel) ctl->pcg_done = 1;
+            if (tot <= ctl->stop2) ctl->pcg_done = 1;
         }
     }
+}
+
+// ||r||^2 at which a solve relative to ||b|| has converged; formed once, by
+// the thread that sets the target, so that the test in an iteration is a
+// comparison (a division and a square root in FP64 took 0.6 us of it).
+__device__ __forceinline__ void set_target(Ctl* ctl, double rel) {
+    ctl->target_rel = rel;
+    ctl->stop2 = ctl->bnorm2 > 0.0 ? rel * rel * ctl->bnorm2 : HUGE_VAL;
 }
 
 // Base residual: the buffer that holds it now.
@@ -209,27 +220,29 @@ __device__ __forceinline__ const float* cur_res(const Level& B, const Ctl* ctl) 
 __device__ __forceinline__ bool solve_over(Ctl* ctl, const ExitArgs& a, bool writer) {
     if (!a.on) return ctl->pcg_done != 0;
     __shared__ bool s_done;
-    uint32_t was_done = 0, delta_stop = 0;
-    double bnorm2 = 0.0, target = 0.0, tot;
+    uint32_t was_done = 0, delta_stop = 0, iters = 0, cap = 0;
+    double stop2 = 0.0, tot;
     float t;
     if (threadIdx.x == 0) {  // (on their way during the sum)
         was_done = ctl->pcg_done;
         delta_stop = ctl->delta_stop;
-        bnorm2 = ctl->bnorm2;
-        target = ctl->target_rel;
+        iters = ctl->pcg_iters;
+        cap = a.dyn_cap ? ctl->inner_cap : a.cap;
+        stop2 = ctl->stop2;
     }
     sum_max_partials<kSegBlock>(a.part, a.nparts, &tot, &t);
     if (threadIdx.x == 0) {
         const bool before = was_done != 0, stop = !before && delta_stop != 0;
         bool done = before || stop;
         if (!done && a.mode == APIC_SOLVER_REFERENCE) done = t < a.solve_error;
-        else if (!done) done = (bnorm2 > 0.0 ? sqrt(tot / bnorm2) : 0.0) <= target;
-        s_done = done;
+        else if (!done) done = tot <= stop2;
+        // (at the iteration cap every CTA returns, as the decision marks it)
+        s_done = done || (a.mode != APIC_SOLVER_REFERENCE && iters >= cap);
         if (writer) {
             if (stop) ctl->res_sel ^= 1u;  // the update left the residual where it was
             else if (!before && a.mode == APIC_SOLVER_REFERENCE) ctl->max_r_bits = __float_as_uint(t);
             else if (!before) ctl->rnorm2 = tot;
-            if (done) ctl->pcg_done = 1;
+            if (done && !before) ctl->pcg_done = 1;
             loop_decision(ctl, a.mode, a.h, a.cap, a.dyn_cap, a.set_cond);
         }
     }

@@ -54,6 +54,7 @@ __global__ void k_begin_update(Ctl* ctl, float frame_dt, uint32_t flags, uint32_
     ctl->flags = flags;
     ctl->substeps = 0;
     ctl->pcg_iters_total = 0;
+    ctl->pcg_bodies = 0;
     ctl->not_converged = 0;
     ctl->has_ext = has_ext;
     ctl->has_post = has_post;
@@ -883,7 +884,7 @@ int update_finish(apic_handle* h) {
         s.stats.kernel_launches = (c.sorted ? s.kn_bsort : 0u) + uint64_t(c.substeps) * s.kn_bstep;
     else if (!s.profiling)
         s.stats.kernel_launches = uint64_t(s.kn_top) + (c.sorted ? s.kn_sort : 0u) + uint64_t(c.substeps) * s.kn_loop +
-                                  uint64_t(c.pcg_iters_total) * s.kn_pcg + uint64_t(c.refinements_total) * s.kn_refine;
+                                  uint64_t(c.pcg_bodies) * s.kn_pcg + uint64_t(c.refinements_total) * s.kn_refine;
     if (c.status & kStatusBounds)
         return fail(APIC_ERR_CUDA, "bounds check: an index left its buffer (build with APIC_BOUNDS_CHECK)");
     if (c.status & kStatusSortWait) return fail(APIC_ERR_TIMEOUT, "radix sort: a bounded device wait gave up");

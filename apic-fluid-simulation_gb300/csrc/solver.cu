@@ -100,13 +100,15 @@ __global__ void __launch_bounds__(kSegBlock) k_pcg_start(Level B, float* s, Ctl*
 __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nseg, uint32_t w0, const float* s,
                                             float* ap, Ctl* ctl, float2* part, int mode, const float2* rz,
                                             uint32_t nrz, const float* rz_sum = nullptr) {
-    if (ctl->pcg_done) return;
+    const bool done = ctl->pcg_done != 0, bv = ctl->beta_valid != 0;
     float beta = ctl->beta;
-    const bool bv = ctl->beta_valid != 0;
+    const float gamma = ctl->gamma;
+    float ng = 0.0f;
+    if (mode != APIC_SOLVER_REFERENCE) ng = rz_sum ? *rz_sum : sum_partials<kSegBlock>(rz, nrz);
+    if (done) return;
     if (mode != APIC_SOLVER_REFERENCE && bv) {
-        const float ng = rz_sum ? *rz_sum : sum_partials<kSegBlock>(rz, nrz);
         if (!(ng != 0.0f)) return;
-        beta = ng / ctl->gamma;
+        beta = ng / gamma;
         if (bk.id == 0 && threadIdx.x == 0) ctl->beta = beta;
     }
     // the buffer this iteration's update writes the residual to (read by the
@@ -115,13 +117,15 @@ __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nse
     F2 acc = pcg::ph_spmv_search(B, nseg, blk_warp(bk), blk_nwarps(bk), s, beta, bv, ap, w0);
     block_store<kSegBlock>(bk, acc, part);
 }
+// first: of its loop body (counted).
 __global__ void __launch_bounds__(kSegBlock) k_spmv_dot(Level B, const float* s, float* ap, Ctl* ctl, float2* part,
-                                                        int mode, const float2* rz, uint32_t nrz) {
+                                                        int mode, const float2* rz, uint32_t nrz, int first) {
     // the base segment list is written by the substep's setup: load this
     // warp's first word before waiting on the previous kernel
     const uint32_t nseg = ctl->seg_count[0];
     const uint32_t w0 = gwarp() < nseg ? B.seg[gwarp()] : 0xFFFFFFFFu;
     pdl_wait();
+    if (first && blockIdx.x == 0 && threadIdx.x == 0) ctl->pcg_bodies++;
     kb_spmv_dot(hw_blk(), B, nseg, w0, s, ap, ctl, part, mode, rz, nrz);
 }
 
@@ -140,25 +144,28 @@ struct StepArgs {
 };
 __device__ __forceinline__ bool pcg_alpha(Blk bk, Ctl* ctl, const StepArgs& a, float* alpha_out,
                                           const float* rz_sum = nullptr, const float* sap_sum = nullptr) {
-    if (ctl->pcg_done) return false;
+    const bool done = ctl->pcg_done != 0, bv = ctl->beta_valid != 0;
     // this iteration's gamma: from the solve's start, or (relative modes) the
     // previous iteration's r.z parts, which k_spmv_dot summed the same way
-    float gamma = ctl->gamma;
-    if (a.mode != APIC_SOLVER_REFERENCE && ctl->beta_valid) {
-        gamma = rz_sum ? *rz_sum : sum_partials<kSegBlock>(a.rz, a.nrz);
-        if (!(gamma != 0.0f)) {
-            if (bk.id == 0 && threadIdx.x == 0) ctl->pcg_done = 1;
-            return false;
-        }
-    }
-    float delta;
+    float gamma = ctl->gamma, delta;
     if (a.mode == APIC_SOLVER_REFERENCE) {
+        if (done) return false;
         // the chunk sums of k_delta_exact, added in chunk order from zero
         const uint32_t nchunks = (a.seg_pre[ctl->seg_count[0]] + kDeltaChunk - 1) / kDeltaChunk;
         delta = 0.0f;
         for (uint32_t c = 0; c < nchunks; ++c) delta = delta + a.exact_parts[c];
     } else {
-        delta = sap_sum ? *sap_sum : sum_partials<kSegBlock>(a.sap, a.nsap);
+        const float2 sums =
+            rz_sum ? make_float2(*rz_sum, *sap_sum) : sum_partials<kSegBlock>(a.rz, a.nrz, a.sap, a.nsap);
+        if (done) return false;
+        delta = sums.y;
+        if (bv) {
+            gamma = sums.x;
+            if (!(gamma != 0.0f)) {
+                if (bk.id == 0 && threadIdx.x == 0) ctl->pcg_done = 1;
+                return false;
+            }
+        }
     }
     const bool stop = a.mode == APIC_SOLVER_REFERENCE ? fabsf(delta) < kSafety : (!(delta != 0.0f) || !isfinite(delta));
     const float alpha = gamma / delta;
@@ -179,24 +186,25 @@ __device__ __forceinline__ bool pcg_alpha(Blk bk, Ctl* ctl, const StepArgs& a, f
 // and max|r|, whose exit test runs in the next kernel.  Block b takes the
 // tiles b, b + n, ...  A tile's constants are read before the wait for the
 // previous kernel and its vectors before alpha is formed from the parts.
+// sel: the buffer the residual goes to (Ctl::res_sel, which alternates), or -1:
+// read it.
 __device__ __forceinline__ tile::Update update_args(const Level& B, const Ctl* ctl, float* p, int p_padded, float* s,
-                                                    const float* ap) {
-    const bool second = ctl->res_sel != 0;  // the residual goes there
+                                                    const float* ap, int sel) {
+    const bool second = sel >= 0 ? sel != 0 : ctl->res_sel != 0;
     return tile::Update{second ? B.res : B.res2, ap, B.err, s, p, p_padded, second ? B.res2 : B.res};
 }
 // (after the dependency wait; g: the first tile's constants, if the block has one)
 __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Level& C, tile::Shared& sh,
                                                tile::DownRegs& g, uint32_t count, uint32_t id, float* p, int p_padded,
                                                float* s, const float* ap, Ctl* ctl, const StepArgs& a, float4* part,
-                                               const float* rz_sum = nullptr,
+                                               int sel, const float* rz_sum = nullptr,
                                                const float* sap_sum = nullptr) {
-    if (ctl->pcg_done) return;
-    const tile::Update u = update_args(B, ctl, p, p_padded, s, ap);
+    const float beta = ctl->beta;
+    const bool beta_valid = ctl->beta_valid != 0;
+    const tile::Update u = update_args(B, ctl, p, p_padded, s, ap, sel);
     if (bk.id < count) tile::down_load<true>(B, u.res, u, g);
     float alpha;
     if (!pcg_alpha(bk, ctl, a, &alpha, rz_sum, sap_sum)) return;
-    const float beta = ctl->beta;
-    const bool beta_valid = ctl->beta_valid != 0;
     float mx = 0.0f;
     F2 acc{0.0f, 0.0f};
     for (uint32_t i = bk.id; i < count; i += bk.n) {
@@ -211,14 +219,15 @@ __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Lev
     block_store<kSegBlock>(bk, acc, mx, part);
 }
 __global__ void __launch_bounds__(kTileBlock, 4) k_update_down(Level B, Level C, float* p, int p_padded, float* s,
-                                                                 const float* ap, Ctl* ctl, StepArgs a, float4* part) {
+                                                                 const float* ap, Ctl* ctl, StepArgs a, float4* part,
+                                                                 int sel) {
     __shared__ tile::Shared sh;
     const uint32_t count = ctl->tile_count[0];
     const uint32_t id = blockIdx.x < count ? B.tiles[blockIdx.x] : 0u;
     tile::DownRegs g;
     if (blockIdx.x < count) tile::down_load_const(B, id, g);
     pdl_wait();
-    kb_update_down(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part);
+    kb_update_down(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part, sel);
 }
 
 // The update alone, and the base level's first red sweep (grids without a
@@ -365,7 +374,9 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
         pcg::finish_rz_reference(ctl, g);
         if (set_cond) {
             const uint32_t c = dyn_cap ? ctl->inner_cap : cap;
-            cudaGraphSetConditional(h, (!ctl->pcg_done && ctl->pcg_iters < c) ? 1u : 0u);
+            const bool cont = !ctl->pcg_done && ctl->pcg_iters < c;
+            if (!cont && !ctl->pcg_done) ctl->pcg_done = kStoppedAtCap;
+            cudaGraphSetConditional(h, cont ? 1u : 0u);
         }
     }
 }
@@ -553,12 +564,12 @@ __global__ void k_pcg_cond(const Ctl* __restrict__ ctl, cudaGraphConditionalHand
 __device__ __forceinline__ void finish_solve(Ctl* ctl, uint32_t cap) {
     ctl->solve_ns += global_ns() - ctl->solve_t0;
     ctl->pcg_iters_total += ctl->pcg_iters;
-    if (ctl->pcg_iters >= cap && !ctl->pcg_done) ctl->not_converged++;
+    if (ctl->pcg_iters >= cap && ctl->pcg_done != 1u) ctl->not_converged++;
 }
 __global__ void k_finish_solve(Ctl* ctl, uint32_t cap) { finish_solve(ctl, cap); }
 
 __device__ __forceinline__ void rel_begin(Ctl* ctl, double tol, uint32_t cap) {
-    ctl->target_rel = tol;
+    pcg::set_target(ctl, tol);
     ctl->inner_cap = cap;
     ctl->refinements = 0;
     ctl->used_iters = 0;
@@ -579,7 +590,7 @@ __device__ __forceinline__ bool refine_cond(Ctl* ctl, double tol, uint32_t cap) 
         ctl->refinements++;
         ctl->inner_cap = cap - ctl->used_iters;
         double t = kInnerReduction * ctl->true_rel;  // target relative to ||b||
-        ctl->target_rel = t > 0.5 * tol ? t : 0.5 * tol;
+        pcg::set_target(ctl, t > 0.5 * tol ? t : 0.5 * tol);
         pcg_reset(ctl);  // the inner solve that follows starts here
     }
     ctl->cond = cont ? 1u : 0u;
@@ -778,7 +789,7 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_update_down(const BScene*
             const uint32_t id = b < count ? S.lv[0].tiles[b] : 0u;
             if (b < count) tile::down_load_const(S.lv[0], id, g);
             kb_update_down(Blk{b, S.tgrid}, S.lv[0], S.lv[1], sh, g, count, id, into_corr ? S.corr : S.pressure,
-                           into_corr, S.search, S.ap, ctl, a, bs_part_res(S), &ctl->b_rz, &ctl->b_sap);
+                           into_corr, S.search, S.ap, ctl, a, bs_part_res(S), -1, &ctl->b_rz, &ctl->b_sap);
             __syncthreads();
         }
     });
@@ -898,14 +909,14 @@ ExitArgs exit_args(const Scene& s, int mode) {
 // One PCG iteration (src/apic.rs:1899-1955); x receives alpha * s.  The
 // search update that ends the reference's iteration happens at the start of
 // the next one (inside k_spmv_dot / k_update_down).
-static void pcg_iteration(Scene& s, int mode, float* x, int p_padded) {
+static void pcg_iteration(Scene& s, int mode, float* x, int p_padded, bool first, int sel) {
     const Level& B = s.lv[0];
     const uint32_t g = seg_grid(B.words), tg = tile_grid(B);
     cudaStream_t st = s.stream;
     const bool pdl = s.use_pdl, tiled = s.nlevels >= 2;
     const uint32_t nrz = tiled ? tg : g;
-    k_spmv_dot<<<g, kSegBlock, 0, st>>>(B, s.search, s.ap, s.ctl, part_sap(s), mode,
-                                         static_cast<const float2*>(part_rz(s)), nrz);
+    launch(pdl && !first, k_spmv_dot, g, kSegBlock, 0, st, B, static_cast<const float*>(s.search), s.ap, s.ctl,
+           part_sap(s), mode, static_cast<const float2*>(part_rz(s)), nrz, first ? 1 : 0);
     if (mode == APIC_SOLVER_REFERENCE)
         launch(pdl, k_delta_exact, div_up(B.cells, kDeltaChunk), kDeltaThreads, 0, st, B,
                static_cast<const float*>(s.search), static_cast<const float*>(s.ap),
@@ -913,10 +924,10 @@ static void pcg_iteration(Scene& s, int mode, float* x, int p_padded) {
     const StepArgs a{part_sap(s), g, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
     if (tiled) {
         launch(pdl, k_update_down, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
-               static_cast<const float*>(s.ap), s.ctl, a, part_res(s));
+               static_cast<const float*>(s.ap), s.ctl, a, part_res(s), sel);
         // the V-cycle's next kernel runs the residual's exit test, its last
         // one stores the parts of r.z
-        enqueue_vcycle(s, true, exit_args(s, mode));
+        enqueue_vcycle(s, true, exit_args(s, mode), sel);
     } else {
         launch(pdl, k_pcg_update, g, kSegBlock, 0, st, B, x, p_padded, s.search, static_cast<const float*>(s.ap),
                s.ctl, a, part_res(s));
@@ -927,6 +938,20 @@ static void pcg_iteration(Scene& s, int mode, float* x, int p_padded) {
     if (mode == APIC_SOLVER_REFERENCE)
         launch(pdl, k_gamma_exact, 1, kGammaThreads, kGammaSmem, st, B, s.ctl, 0, s.pcg_h, s.pcg_cap, s.pcg_dyn_cap,
                s.pcg_set_cond ? 1 : 0);
+}
+
+// Iterations in the body of the PCG loop.  Going round a graph's WHILE node
+// costs 5 us; within the body the next iteration's first kernel is a
+// programmatic dependent like the others.  An iteration that the body holds
+// beyond the solve's last one costs its kernels' launches (they return at
+// once).  Two iterations pay up to 768^2 cells, per iteration: 64^2 29.7 -> 28.3
+// us, 216^2 36.6 -> 34.1, 512^2 46.6 -> 46.0, 768^2 55.6 -> 55.0; not at 1024^2
+// (57.8, 58.0) and 1000 x 600 (70.5, 71.1).  Four are 2% faster where a solve
+// takes 16 iterations or more and 1-2% slower where it takes 6 to 8.  The
+// reference mode's solves take 3 to 9 and six kernels each: 128^2 67.1 us, with
+// two 68.3.
+static int loop_body(const Scene& s, int mode) {
+    return mode != APIC_SOLVER_REFERENCE && s.cells <= 768u * 768u ? 2 : 1;
 }
 
 // PCG setup (src/apic.rs:1885-1892) followed by a device-controlled WHILE
@@ -965,7 +990,8 @@ static cudaError_t build_pcg(Scene& s, GraphCursor& c, int mode, float* x, int p
     s.pcg_dyn_cap = dyn_cap;
     s.pcg_set_cond = true;
     e = capture_into(s, body, [&]() {
-        pcg_iteration(s, mode, x, p_padded);
+        const int n = loop_body(s, mode);
+        for (int k = 0; k < n; ++k) pcg_iteration(s, mode, x, p_padded, k == 0, n % 2 == 0 ? (k + 1) & 1 : -1);
         return cudaGetLastError();
     });
     s.pcg_set_cond = false;
@@ -1072,7 +1098,7 @@ static cudaError_t eager_pcg(Scene& s, int mode, float* x, int p_padded, uint32_
         cudaError_t e = read_ctl(s);
         if (e != cudaSuccess) return e;
         if (s.ctl_host->pcg_done || s.ctl_host->pcg_iters >= cap) break;
-        pcg_iteration(s, mode, x, p_padded);
+        pcg_iteration(s, mode, x, p_padded, true, -1);
     }
     return cudaGetLastError();
 }

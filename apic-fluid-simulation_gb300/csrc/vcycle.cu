@@ -115,8 +115,9 @@ __device__ __forceinline__ F2 kb_up(Blk bk, const Level& c, const Level& f, tile
     return acc;
 }
 template <bool kRz>
+// sel: the base residual's buffer, or -1: as Ctl::res_sel says.
 __global__ void __launch_bounds__(kTileBlock, 4) k_up(Level c, Level f, int lf, const Ctl* ctl, int base,
-                                                        float2* part) {
+                                                        float2* part, int sel) {
     __shared__ tile::Shared sh;
     const uint32_t count = ctl->tile_count[lf];
     const uint32_t id = blockIdx.x < count ? f.tiles[blockIdx.x] : 0u;
@@ -125,7 +126,8 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_up(Level c, Level f, int lf, 
     if (blockIdx.x < count) tile::up_load_const(f, id, g);
     pdl_wait();
     if (ctl->pcg_done) return;
-    const F2 acc = kb_up<kRz>(hw_blk(), c, f, sh, g, id, count, base ? pcg::cur_res(f, ctl) : f.res, last, extra);
+    const float* res = !base ? f.res : sel < 0 ? pcg::cur_res(f, ctl) : sel ? f.res2 : f.res;
+    const F2 acc = kb_up<kRz>(hw_blk(), c, f, sh, g, id, count, res, last, extra);
     if (kRz) block_store<kTileBlock>(hw_blk(), acc, part);
 }
 
@@ -310,7 +312,7 @@ void plan_vcycle(Scene& s) {
 // One V-cycle on s.stream: z = M^-1 r in lv[0].err.  Two kernels per level
 // (k_down, k_up) above the levels that the distributed-shared-memory cluster
 // or the shared-memory tail holds, or above the coarsest level's CG.
-void enqueue_vcycle(Scene& s, bool base_done, const ExitArgs& exit_in) {
+void enqueue_vcycle(Scene& s, bool base_done, const ExitArgs& exit_in, int sel) {
     cudaStream_t st = s.stream;
     Level* L = s.lv;
     const int last = s.nlevels - 1;
@@ -353,9 +355,9 @@ void enqueue_vcycle(Scene& s, bool base_done, const ExitArgs& exit_in) {
     }
     for (int k = l - 1; k >= 1; --k)
         launch(pdl, k_up<false>, tile_grid(L[k]), kTileBlock, 0, st, L[k + 1], L[k], k,
-               static_cast<const Ctl*>(s.ctl), 0, static_cast<float2*>(nullptr));
+               static_cast<const Ctl*>(s.ctl), 0, static_cast<float2*>(nullptr), -1);
     launch(pdl, base_done ? k_up<true> : k_up<false>, tile_grid(L[0]), kTileBlock, 0, st, L[1], L[0], 0,
-           static_cast<const Ctl*>(s.ctl), 1, part_rz(s));
+           static_cast<const Ctl*>(s.ctl), 1, part_rz(s), sel);
 }
 
 }  // namespace apic

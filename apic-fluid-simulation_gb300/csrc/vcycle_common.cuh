@@ -89,10 +89,17 @@ __device__ __forceinline__ float cg_reduce(F2 v, bool& any, CgSlot& sh, uint32_t
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) sh.w[warp] = make_float4(v.hi, v.lo, kAny && any ? 1.0f : 0.0f, 0.0f);
     cg_bar(nwarps);
-    const float4 q = lane < nwarps ? sh.w[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    v = warp_sum(F2{q.x, q.y});
+    // (up to 8 warps: four copies of their results, three levels of the tree)
+    const uint32_t from = nwarps <= 8u ? lane & 7u : lane;
+    const float4 q = from < nwarps ? sh.w[from] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    v = F2{q.x, q.y};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (o > 4 && nwarps <= 8u) continue;
+        v = f2_add(v, F2{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
+    }
     if (kAny) any = __any_sync(0xffffffffu, q.z != 0.0f);
-    return float(f2_value(v));
+    return v.hi;  // (the rounded value of a normalised double-float)
 }
 
 // The reference solver mode's sums (solve_coarse_exact, :627-629, :660,
