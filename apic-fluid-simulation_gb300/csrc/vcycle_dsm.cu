@@ -136,8 +136,8 @@ __device__ __forceinline__ void dsm_restrict(const Band& f, Put put) {
             x = q - row * cw;
         }
         const int i = (2 * row + dy) * w + 2 * x;
-        const float d0 = left_over(f.r, f.d, f.px, f.py, f.e, i, i, w);
-        const float d1 = left_over(f.r, f.d, f.px, f.py, f.e, i + 1, i + 1, w);
+        const float2 two = left_over(f.r, f.d, f.px, f.py, f.e, i, w);
+        const float d0 = two.x, d1 = two.y;
         const float d2 = __shfl_down_sync(0xffffffffu, d0, 1), d3 = __shfl_down_sync(0xffffffffu, d1, 1);
         if (dy == 0) put(row, x, (((0.0f + d0) + d1) + d2) + d3);
     }
