@@ -14,7 +14,7 @@
 //   k_coarsen        one multigrid level from its finer level (:1499-1602).
 //   k_gradient       pressure projection per face (:1958-2055), fused with the
 //                    post-force add (:2453-2458).
-//   k_extrapolate2   two Jacobi sweeps of velocity extrapolation for u and v
+//   k_extrapolate    two Jacobi sweeps of velocity extrapolation for u and v
 //                    in shared-memory tiles (:2266-2350).
 //
 // Cell stages run one warp per non-zero 32-bit mask word ("segment"): lane k
@@ -542,17 +542,22 @@ __global__ void __launch_bounds__(256) k_gradient(uint32_t uf, uint32_t vf, int 
     }
 }
 
-// Velocity extrapolation, two Jacobi sweeps per launch (src/apic.rs:2266-2350
-// runs four, swapping buffers after each).  A CTA owns a kExTX x kExTY tile
-// of one face field (u: (W+1) x H, v: W x (H+1)) and stages the tile plus a
-// two-face halo in shared memory; sweep 1 runs on the halo-shrunk region,
-// sweep 2 on the tile, which is written out.  A neighbour outside the field
-// reads as invalid, which is exactly the reference's x > 0 / x < width /
+// Velocity extrapolation: the four Jacobi sweeps of src/apic.rs:2266-2350 (it
+// swaps buffers after each) on tiles of one face field (u: (W+1) x H, v: W x
+// (H+1)) with a halo as wide as the sweeps of a launch, in shared memory; each
+// sweep runs on a region one face smaller on each side than the one before,
+// the last one on the tile, which is written out.  A neighbour outside the
+// field reads as invalid, which is exactly the reference's x > 0 / x < width /
 // y > 0 / y < height guards, and every face adds its valid neighbours in the
 // reference's order (x-1, x+1, y-1, y+1) before the one division, so each
 // sweep's values and flags are bit-identical to a sweep over the whole grid.
-constexpr int kExTX = 128, kExTY = 24, kExHalo = 2;
-constexpr int kExRX = kExTX + 2 * kExHalo, kExRY = kExTY + 2 * kExHalo;
+// A tile whose staged faces are all valid, or all invalid, is what the sweeps
+// would leave it as: most of a large grid.
+template <int kTX, int kTY, int kSweeps>
+struct ExTile {
+    static constexpr int TX = kTX, TY = kTY, N = kSweeps;
+    static constexpr int RX = kTX + 2 * kSweeps, RY = kTY + 2 * kSweeps;
+};
 
 struct ExField {
     const float* in;
@@ -563,60 +568,71 @@ struct ExField {
     int tiles_x;       // tiles per row of tiles
 };
 
+template <int kRX>
 __device__ __forceinline__ void ex_face(const float* val, const uint8_t* ok, int i, float* nv, uint8_t* nok) {
     if (ok[i]) { *nv = val[i]; *nok = 1; return; }
     float sum = 0.0f;
     uint32_t cnt = 0;
     if (ok[i - 1]) { sum += val[i - 1]; cnt++; }
     if (ok[i + 1]) { sum += val[i + 1]; cnt++; }
-    if (ok[i - kExRX]) { sum += val[i - kExRX]; cnt++; }
-    if (ok[i + kExRX]) { sum += val[i + kExRX]; cnt++; }
+    if (ok[i - kRX]) { sum += val[i - kRX]; cnt++; }
+    if (ok[i + kRX]) { sum += val[i + kRX]; cnt++; }
     if (cnt > 0) { *nv = sum / float(cnt); *nok = 1; }
     else { *nv = val[i]; *nok = 0; }
 }
 
-__global__ void __launch_bounds__(256) k_extrapolate2(ExField fu, ExField fv, int tiles_u) {
-    __shared__ float s_val[2][kExRX * kExRY];
-    __shared__ uint8_t s_ok[2][kExRX * kExRY];
+template <class T>
+__global__ void __launch_bounds__(256) k_extrapolate(ExField fu, ExField fv, int tiles_u) {
+    __shared__ float s_val[2][T::RX * T::RY];
+    __shared__ uint8_t s_ok[2][T::RX * T::RY];
     const bool is_u = int(blockIdx.x) < tiles_u;
     const ExField& F = is_u ? fu : fv;
     const int t = is_u ? int(blockIdx.x) : int(blockIdx.x) - tiles_u;
-    const int x0 = (t % F.tiles_x) * kExTX - kExHalo, y0 = (t / F.tiles_x) * kExTY - kExHalo;
+    const int x0 = (t % F.tiles_x) * T::TX - T::N, y0 = (t / F.tiles_x) * T::TY - T::N;
     pdl_wait();
-    for (int i = threadIdx.x; i < kExRX * kExRY; i += blockDim.x) {
-        const int gx = x0 + i % kExRX, gy = y0 + i / kExRX;
+    bool some = false, all = true;  // of the staged faces inside the field: valid
+#pragma unroll 4
+    for (int i = threadIdx.x; i < T::RX * T::RY; i += 256) {
+        const int gx = x0 + i % T::RX, gy = y0 + i / T::RX;
         float v = 0.0f;
         uint8_t k = 0;
         if (gx >= 0 && gx < F.w && gy >= 0 && gy < F.h) {
             const size_t g = size_t(gy) * F.w + gx;
             v = F.in[g];
             k = F.in_ok[g];
+            some = some || k;
+            all = all && k;
         }
         s_val[0][i] = v;
         s_ok[0][i] = k;
     }
-    __syncthreads();
-    // sweep 1 on the region one face inside the staged one (faces outside
-    // the field stay invalid)
-    for (int j = threadIdx.x; j < (kExRX - 2) * (kExRY - 2); j += blockDim.x) {
-        const int rx = 1 + j % (kExRX - 2), ry = 1 + j / (kExRX - 2);
-        const int i = ry * kExRX + rx;
-        const int gx = x0 + rx, gy = y0 + ry;
-        float v = 0.0f;
-        uint8_t k = 0;
-        if (gx >= 0 && gx < F.w && gy >= 0 && gy < F.h) ex_face(s_val[0], s_ok[0], i, &v, &k);
-        s_val[1][i] = v;
-        s_ok[1][i] = k;
+    const bool mixed = __syncthreads_or(some) && !__syncthreads_and(all);
+    int cur = 0;
+    if (mixed) {
+#pragma unroll
+        for (int n = 1; n < T::N; ++n) {
+            // faces outside the field stay invalid
+            const int rx_n = T::RX - 2 * n, cells = rx_n * (T::RY - 2 * n);
+            for (int j = threadIdx.x; j < cells; j += 256) {
+                const int rx = n + j % rx_n, ry = n + j / rx_n, i = ry * T::RX + rx;
+                const int gx = x0 + rx, gy = y0 + ry;
+                float v = 0.0f;
+                uint8_t k = 0;
+                if (gx >= 0 && gx < F.w && gy >= 0 && gy < F.h) ex_face<T::RX>(s_val[cur], s_ok[cur], i, &v, &k);
+                s_val[cur ^ 1][i] = v;
+                s_ok[cur ^ 1][i] = k;
+            }
+            __syncthreads();
+            cur ^= 1;
+        }
     }
-    __syncthreads();
-    // sweep 2 on the tile, written out
-    for (int j = threadIdx.x; j < kExTX * kExTY; j += blockDim.x) {
-        const int rx = kExHalo + j % kExTX, ry = kExHalo + j / kExTX;
+    for (int j = threadIdx.x; j < T::TX * T::TY; j += 256) {
+        const int rx = T::N + j % T::TX, ry = T::N + j / T::TX, i = ry * T::RX + rx;
         const int gx = x0 + rx, gy = y0 + ry;
         if (gx >= F.w || gy >= F.h) continue;
-        float v;
-        uint8_t k;
-        ex_face(s_val[1], s_ok[1], ry * kExRX + rx, &v, &k);
+        float v = s_val[cur][i];
+        uint8_t k = s_ok[cur][i];
+        if (mixed) ex_face<T::RX>(s_val[cur], s_ok[cur], i, &v, &k);
         const size_t g = size_t(gy) * F.w + gx;
         F.out[g] = v;
         F.out_ok[g] = k;
@@ -747,24 +763,35 @@ cudaError_t launch_post_forces(Scene& s) {
     return cudaGetLastError();
 }
 
+template <class T> static void extrapolate(Scene& s, bool from_alt) {
+    const int W = int(s.W), H = int(s.H);
+    auto field = [](const float* in, const uint8_t* in_ok, float* out, uint8_t* out_ok, int w, int h) {
+        return ExField{in, in_ok, out, out_ok, w, h, int(div_up(uint32_t(w), T::TX))};
+    };
+    const ExField fu = from_alt ? field(s.u_alt, s.valid_u_alt, s.u, s.valid_u, W + 1, H)
+                                : field(s.u, s.valid_u, s.u_alt, s.valid_u_alt, W + 1, H);
+    const ExField fv = from_alt ? field(s.v_alt, s.valid_v_alt, s.v, s.valid_v, W, H + 1)
+                                : field(s.v, s.valid_v, s.v_alt, s.valid_v_alt, W, H + 1);
+    const uint32_t tiles_u = uint32_t(fu.tiles_x) * div_up(uint32_t(fu.h), T::TY);
+    const uint32_t tiles_v = uint32_t(fv.tiles_x) * div_up(uint32_t(fv.h), T::TY);
+    launch(s.use_pdl, k_extrapolate<T>, tiles_u + tiles_v, 256, 0, s.stream, fu, fv, int(tiles_u));
+}
+
 // The reference's four sweeps as two launches of two sweeps each:
 // u, v -> u_alt, v_alt -> u, v (the result ends where the next stages read it).
+// Up to 512^2 cells the grid's tiles are few and a tile's rounds set the time:
+// 32 x 8 tiles, three rounds a sweep; above, the halo's share of the traffic
+// does: 64 x 16.  The four sweeps, 32 x 8 / 64 x 16 / 128 x 24 (every size before):
+// 64^2 9.5 / 13.6 / 22.3 us, 256^2 10.5 / 15.7 / 26.8, 512^2 15.4 / 16.3 / 27.9,
+// 1024^2 34.8 / 27.7 / 37.4, 4096^2 (noise) 510 / 348 / 350.
 cudaError_t launch_extrapolate(Scene& s) {
-    auto field = [](const float* in, const uint8_t* in_ok, float* out, uint8_t* out_ok, int w, int h) {
-        ExField f;
-        f.in = in; f.in_ok = in_ok; f.out = out; f.out_ok = out_ok; f.w = w; f.h = h;
-        f.tiles_x = int(div_up(uint32_t(w), kExTX));
-        return f;
-    };
-    const int W = int(s.W), H = int(s.H);
-    const uint32_t tiles_u = div_up(uint32_t(W + 1), kExTX) * div_up(uint32_t(H), kExTY);
-    const uint32_t tiles_v = div_up(uint32_t(W), kExTX) * div_up(uint32_t(H + 1), kExTY);
-    launch(s.use_pdl, k_extrapolate2, tiles_u + tiles_v, 256, 0, s.stream,
-           field(s.u, s.valid_u, s.u_alt, s.valid_u_alt, W + 1, H), field(s.v, s.valid_v, s.v_alt, s.valid_v_alt, W, H + 1),
-           int(tiles_u));
-    launch(s.use_pdl, k_extrapolate2, tiles_u + tiles_v, 256, 0, s.stream,
-           field(s.u_alt, s.valid_u_alt, s.u, s.valid_u, W + 1, H), field(s.v_alt, s.valid_v_alt, s.v, s.valid_v, W, H + 1),
-           int(tiles_u));
+    if (s.cells <= 512u * 512u) {
+        extrapolate<ExTile<32, 8, 2>>(s, false);
+        extrapolate<ExTile<32, 8, 2>>(s, true);
+    } else {
+        extrapolate<ExTile<64, 16, 2>>(s, false);
+        extrapolate<ExTile<64, 16, 2>>(s, true);
+    }
     return cudaGetLastError();
 }
 
