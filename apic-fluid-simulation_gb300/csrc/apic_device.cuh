@@ -282,6 +282,43 @@ __device__ __forceinline__ bool block_sum_last(Blk bk, double v, double* partial
     return true;
 }
 
+// The same for two sums at once (the second one's partials behind the first's).
+template <int kThreads>
+__device__ __forceinline__ bool block_sum_last(Blk bk, double2 v, double* partials, double* partials2,
+                                               uint32_t* counter, double2* total) {
+    __shared__ double2 s_w2[kThreads / 32];
+    __shared__ bool s_last2;
+    v = make_double2(warp_sum(v.x), warp_sum(v.y));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) s_w2[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double2 b = make_double2(0.0, 0.0);
+        for (int w = 0; w < kThreads / 32; ++w) b = make_double2(b.x + s_w2[w].x, b.y + s_w2[w].y);
+        partials[bk.id] = b.x;
+        partials2[bk.id] = b.y;
+        __threadfence();
+        s_last2 = atomicAdd(counter, 1u) == bk.n - 1;
+    }
+    __syncthreads();
+    if (!s_last2) return false;
+    __threadfence();
+    const volatile double *p = partials, *p2 = partials2;
+    double2 t = make_double2(0.0, 0.0);
+    for (uint32_t b = threadIdx.x; b < bk.n; b += kThreads) t = make_double2(t.x + p[b], t.y + p2[b]);
+    t = make_double2(warp_sum(t.x), warp_sum(t.y));
+    __syncthreads();
+    if (lane == 0) s_w2[warp] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double2 a = make_double2(0.0, 0.0);
+        for (int w = 0; w < kThreads / 32; ++w) a = make_double2(a.x + s_w2[w].x, a.y + s_w2[w].y);
+        *total = a;
+        *counter = 0;
+    }
+    return true;
+}
+
 // ---- double-float sums ---------------------------------------------------
 // An unevaluated sum hi + lo of two floats (about 48 significant bits).  Sums
 // of FP32 products accumulate in this form with FP32 instructions only:

@@ -95,9 +95,16 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_u32(uint32_t v, uint32_
 // npad, a multiple of 8, lanes; keys of lanes n .. npad-1 are never read).
 __global__ void __launch_bounds__(256) k_p2g_bin_keys(const PartPtrs* __restrict__ pp, uint32_t n, int W, int H,
                                                       CellSize cs, uint32_t* __restrict__ keys,
-                                                      uint32_t* __restrict__ fluid, uint32_t* __restrict__ head) {
+                                                      uint32_t* __restrict__ fluid, uint32_t* __restrict__ head,
+                                                      uint32_t* __restrict__ lo, uint32_t* __restrict__ hi) {
     pdl_wait();
     clear_sort_head(head);
+    // the cells' runs, empty until k_p2g_bounds (a grid with particles has even
+    // sides, so whole vectors)
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < uint32_t(W) * uint32_t(H) / 4u; c += gridDim.x * blockDim.x) {
+        reinterpret_cast<uint4*>(lo)[c] = make_uint4(0u, 0u, 0u, 0u);
+        reinterpret_cast<uint4*>(hi)[c] = make_uint4(0u, 0u, 0u, 0u);
+    }
     const uint32_t i0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
     const bool any = i0 < n;
     float4 px = make_float4(0.0f, 0.0f, 0.0f, 0.0f), py = px;
@@ -1064,8 +1071,8 @@ __global__ void k_swap_tables(PartPtrs* pp) {
 
 static CellSize cell_size(const Scene& s) { return CellSize{s.dx, exact_reciprocal(s.dx)}; }
 
-// P2G stage; bin_lo / bin_hi and the base fluid mask must be zero (the
-// caller clears them), every accumulator entry is written.
+// P2G stage; the base fluid mask, and without particles bin_lo / bin_hi, must be
+// zero (the caller clears them), every accumulator entry is written.
 cudaError_t launch_p2g(Scene& s) {
     const bool ref = p2g_reference_order(s);
     cudaError_t e = cudaFuncSetAttribute(k_p2g_gather, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1074,7 +1081,7 @@ cudaError_t launch_p2g(Scene& s) {
     const uint32_t* svals = s.bin_vals;
     if (s.n > 0) {
         launch(s.use_pdl, k_p2g_bin_keys, div_up(s.n, 1024), 256, 0, s.stream, static_cast<const PartPtrs*>(s.pp), s.n,
-               int(s.W), int(s.H), cell_size(s), s.bin_keys, s.lv[0].fluid, s.sort_scratch);
+               int(s.W), int(s.H), cell_size(s), s.bin_keys, s.lv[0].fluid, s.sort_scratch, s.bin_lo, s.bin_hi);
         uint32_t *kres, *vres;
         e = radix_sort_pairs(s.bin_keys, s.bin_vals, s.bin_keys_alt, s.bin_vals_alt, s.sort_scratch, s.n,
                              bin_key_bits(s), 0, s.stream, s.use_pdl, &kres, &vres, &s.ctl->status);

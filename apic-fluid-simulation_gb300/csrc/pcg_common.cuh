@@ -314,6 +314,51 @@ __device__ __forceinline__ double ph_true_residual(const Level& B, uint32_t nseg
     return rr;
 }
 
+// A relative solve's start in one pass: b64 = res, pressure = 0 and ||b||^2
+// (x), and for refinement (mixed) the true residual of the starting p64
+// (ph_true_residual's terms: kept where warm, else zero, whose residual is b),
+// x = 0 and its ||r||^2 (y).
+__device__ __forceinline__ double2 ph_solve_start(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps,
+                                                  double* b64, double* p64, float* x, float* pressure, int warm,
+                                                  int mixed) {
+    double bb = 0.0, rr = 0.0;
+    const uint32_t W = B.w;
+    APIC_BASE_ALL(B, nseg, warp, nwarps) {
+        const uint32_t c = raw_ + W;
+        const long long raw = raw_;
+        const float res = B.res[c];
+        const double b = double(res);
+        double r = b;
+        if (warm) {
+            const float dg = B.diag[c], pxc = B.px[c], pxl = B.px[c - 1], pyc = B.py[c], pyd = B.py[c - W];
+            const double pc = p64[c], pr = p64[c + 1], pl = p64[c - 1], pu = p64[c + W], pd = p64[c - W];
+            const bool fr = fluid_raw(B.fluid, raw + 1, B.cells), fl = fluid_raw(B.fluid, raw - 1, B.cells);
+            const bool fu = fluid_raw(B.fluid, raw + W, B.cells);
+            const bool fd = fluid_raw(B.fluid, raw - (long long)W, B.cells);
+            double v = double(dg) * pc;
+            double t = v + double(pxc) * pr;
+            v = fr ? t : v;
+            t = v + double(pxl) * pl;
+            v = fl ? t : v;
+            t = v + double(pyc) * pu;
+            v = fu ? t : v;
+            t = v + double(pyd) * pd;
+            v = fd ? t : v;
+            r = b - v;
+        }
+        if (!fluid_) continue;
+        b64[c] = b;
+        pressure[raw_] = 0.0f;
+        bb += b * b;
+        if (!warm) p64[c] = 0.0;
+        if (!mixed) continue;
+        rr += r * r;
+        if (warm) B.res[c] = float(r);
+        x[c] = 0.0f;
+    }
+    return make_double2(bb, rr);
+}
+
 // p64 += x, or (finalize) pressure = float(p64).
 __device__ __forceinline__ void ph_accumulate(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps,
                                               double* p64, const float* x, float* pressure, int finalize) {

@@ -465,12 +465,14 @@ struct StageTimer {
     }
 };
 
-// P2G writes every accumulator entry; it needs empty cell runs and a clear
-// fluid mask.
+// P2G writes every accumulator entry; it needs a clear fluid mask, and empties
+// the cells' runs itself where there are particles.
 cudaError_t clear_p2g_targets(Scene& s) {
     cudaStream_t st = s.stream;
-    cudaMemsetAsync(s.bin_lo, 0, sizeof(uint32_t) * s.cells, st);
-    cudaMemsetAsync(s.bin_hi, 0, sizeof(uint32_t) * s.cells, st);
+    if (s.n == 0) {
+        cudaMemsetAsync(s.bin_lo, 0, sizeof(uint32_t) * s.cells, st);
+        cudaMemsetAsync(s.bin_hi, 0, sizeof(uint32_t) * s.cells, st);
+    }
     cudaMemsetAsync(s.lv[0].fluid, 0, sizeof(uint32_t) * s.lv[0].words, st);
     return cudaGetLastError();
 }

@@ -55,8 +55,8 @@ __device__ __forceinline__ void pcg_reset(Ctl* ctl) {
     ctl->res_sel = 0;  // a solve's right-hand side is in the first buffer
 }
 
-__global__ void k_pcg_begin(Ctl* ctl, int stamp) {
-    if (stamp) ctl->solve_t0 = global_ns();
+__global__ void k_pcg_begin(Ctl* ctl) {
+    pdl_wait();
     pcg_reset(ctl);
 }
 
@@ -66,26 +66,55 @@ __global__ void k_pcg_begin(Ctl* ctl, int stamp) {
 // grid (bk), run by the single-scene kernel with the hardware's and by the
 // batch kernel (one launch over many scenes, batch.h) with the scene's.
 
-__global__ void __launch_bounds__(kSegBlock) k_clear_pressure(Level B, float* p, const Ctl* ctl) {
+// The reference mode's solve starts here: its PCG state and a zero pressure.
+__global__ void __launch_bounds__(kSegBlock) k_reference_start(Level B, float* p, Ctl* ctl) {
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl->solve_t0 = global_ns();
+        pcg_reset(ctl);
+    }
     pcg::ph_clear_pressure(B, ctl->seg_count[0], gwarp(), gnwarps(), p);
 }
 
+// Entry of the PCG loop: go on while not converged and under the iteration
+// cap (src/apic.rs:1894-1899); dyn_cap reads the remaining budget of a
+// refinement.  Inside the loop the same decision is taken by the kernel that
+// runs the residual's exit test (pcg::loop_decision) or, in the reference
+// mode, by k_gamma_exact.
+__device__ __forceinline__ bool pcg_entry(const Ctl* ctl, uint32_t cap, int dyn_cap) {
+    const uint32_t c = dyn_cap ? ctl->inner_cap : cap;
+    return !ctl->pcg_done && ctl->pcg_iters < c;
+}
+
+// The loop that a kernel which ends a solve's setup opens (set 0: none).
+struct LoopEntry {
+    cudaGraphConditionalHandle h = 0;
+    uint32_t cap = 0;
+    int dyn_cap = 0;
+    int set = 0;
+};
+
 // s = z and gamma = r.z (src/apic.rs:1887-1892).
 // In the reference mode k_gamma_exact forms gamma and the exit instead.
-__device__ __forceinline__ void kb_pcg_start(Blk bk, const Level& B, float* s, Ctl* ctl, double* partials, int mode) {
+// True in the one thread that formed gamma.
+__device__ __forceinline__ bool kb_pcg_start(Blk bk, const Level& B, float* s, Ctl* ctl, double* partials, int mode) {
     F2 acc = pcg::ph_start(B, ctl->seg_count[0], blk_warp(bk), blk_nwarps(bk), s);
-    if (mode == APIC_SOLVER_REFERENCE) return;
+    if (mode == APIC_SOLVER_REFERENCE) return false;
     double tot;
     if (block_sum_last<kSegBlock>(bk, acc, partials, &ctl->red_counter, &tot) && threadIdx.x == 0) {
         float gamma = float(tot);
         ctl->gamma = gamma;
         ctl->dgamma = tot;
-        if (mode == APIC_SOLVER_REFERENCE ? (gamma < kSafety) : !(gamma != 0.0f)) ctl->pcg_done = 1;
+        if (!(gamma != 0.0f)) ctl->pcg_done = 1;
+        return true;
     }
+    return false;
 }
-__global__ void __launch_bounds__(kSegBlock) k_pcg_start(Level B, float* s, Ctl* ctl, double* partials, int mode) {
+__global__ void __launch_bounds__(kSegBlock) k_pcg_start(Level B, float* s, Ctl* ctl, double* partials, int mode,
+                                                         LoopEntry loop) {
     pdl_wait();
-    kb_pcg_start(hw_blk(), B, s, ctl, partials, mode);
+    if (kb_pcg_start(hw_blk(), B, s, ctl, partials, mode) && loop.set)
+        cudaGraphSetConditional(loop.h, pcg_entry(ctl, loop.cap, loop.dyn_cap) ? 1u : 0u);
 }
 
 // s' = z + beta s, Ap = A s' and this block's part of delta = s'.Ap
@@ -370,6 +399,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
         ctl->gamma = g;
         ctl->dgamma = double(g);
         if (g < kSafety) ctl->pcg_done = 1;
+        if (set_cond) cudaGraphSetConditional(h, pcg_entry(ctl, cap, dyn_cap) ? 1u : 0u);
     } else {
         pcg::finish_rz_reference(ctl, g);
         if (set_cond) {
@@ -385,6 +415,7 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
 // = all fluid cells): the position of a segment's cells in the reference's
 // ascending fluid list.  One block, once per solve.
 __global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, uint32_t* seg_pre) {
+    pdl_wait();
     const uint32_t nseg = ctl->seg_count[0];
     __shared__ uint32_t sw[32];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -509,25 +540,17 @@ __device__ __forceinline__ void kb_mixed_init(Blk bk, const Level& B, double* b6
     double tot;
     if (block_sum_last<kSegBlock>(bk, bb, partials, &ctl->red_counter, &tot) && threadIdx.x == 0) ctl->bnorm2 = tot;
 }
-__global__ void __launch_bounds__(kSegBlock) k_mixed_init(Level B, double* b64, double* p64, Ctl* ctl,
-                                                          double* partials, int warm) {
-    kb_mixed_init(hw_blk(), B, b64, p64, ctl, partials, warm);
-}
-
 // True relative residual of p64 (flags: see pcg::ph_true_residual).
-__device__ __forceinline__ void kb_true_residual(Blk bk, const Level& B, const double* b64, const double* p64,
+// True in the one thread that formed it.
+__device__ __forceinline__ bool kb_true_residual(Blk bk, const Level& B, const double* b64, const double* p64,
                                                  float* x, Ctl* ctl, double* partials, int flags) {
     if ((flags & 1) && bk.id == 0 && threadIdx.x == 0) ctl->res_sel = 0;
     double rr = pcg::ph_true_residual(B, ctl->seg_count[0], blk_warp(bk), blk_nwarps(bk), b64, p64, x, flags);
     double tot;
-    if (block_sum_last<kSegBlock>(bk, rr, partials, &ctl->red_counter, &tot) && threadIdx.x == 0)
-        ctl->true_rel = ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0;
+    if (!block_sum_last<kSegBlock>(bk, rr, partials, &ctl->red_counter, &tot) || threadIdx.x != 0) return false;
+    ctl->true_rel = ctl->bnorm2 > 0.0 ? sqrt(tot / ctl->bnorm2) : 0.0;
+    return true;
 }
-__global__ void __launch_bounds__(kSegBlock) k_true_residual(Level B, const double* b64, const double* p64, float* x,
-                                                             Ctl* ctl, double* partials, int flags) {
-    kb_true_residual(hw_blk(), B, b64, p64, x, ctl, partials, flags);
-}
-
 // p64 += x (finalize 0; the refinement also counts the inner solve's
 // iterations), or pressure = float(p64) (finalize 1).
 __device__ __forceinline__ void kb_mixed_accumulate(Blk bk, const Level& B, double* p64, const float* x,
@@ -535,31 +558,7 @@ __device__ __forceinline__ void kb_mixed_accumulate(Blk bk, const Level& B, doub
     pcg::ph_accumulate(B, ctl->seg_count[0], blk_warp(bk), blk_nwarps(bk), p64, x, pressure, finalize);
     if (!finalize && bk.id == 0 && threadIdx.x == 0) ctl->used_iters += ctl->pcg_iters;
 }
-__global__ void __launch_bounds__(kSegBlock) k_mixed_accumulate(Level B, double* p64, const float* x, float* pressure,
-                                                                Ctl* ctl, int finalize) {
-    kb_mixed_accumulate(hw_blk(), B, p64, x, pressure, ctl, finalize);
-}
-
-__global__ void __launch_bounds__(kSegBlock) k_pressure_to64(Level B, const float* pressure, double* p64,
-                                                             const Ctl* ctl) {
-    pcg::ph_pressure_to64(B, ctl->seg_count[0], gwarp(), gnwarps(), pressure, p64);
-}
-
 // ---- loop control (device side; each sets a graph conditional) ------------
-
-// Entry of the PCG loop: go on while not converged and under the iteration
-// cap (src/apic.rs:1894-1899); dyn_cap reads the remaining budget of a
-// refinement.  Inside the loop the same decision is taken by the kernel that
-// runs the residual's exit test (pcg::loop_decision) or, in the reference
-// mode, by k_gamma_exact.
-__device__ __forceinline__ bool pcg_entry(const Ctl* ctl, uint32_t cap, int dyn_cap) {
-    const uint32_t c = dyn_cap ? ctl->inner_cap : cap;
-    return !ctl->pcg_done && ctl->pcg_iters < c;
-}
-__global__ void k_pcg_cond(const Ctl* __restrict__ ctl, cudaGraphConditionalHandle h, uint32_t cap, int dyn_cap) {
-    pdl_wait();
-    cudaGraphSetConditional(h, pcg_entry(ctl, cap, dyn_cap) ? 1u : 0u);
-}
 
 __device__ __forceinline__ void finish_solve(Ctl* ctl, uint32_t cap) {
     ctl->solve_ns += global_ns() - ctl->solve_t0;
@@ -568,13 +567,20 @@ __device__ __forceinline__ void finish_solve(Ctl* ctl, uint32_t cap) {
 }
 __global__ void k_finish_solve(Ctl* ctl, uint32_t cap) { finish_solve(ctl, cap); }
 
+// The FP32 mode's end: p64 = pressure, for its true residual.
+__global__ void __launch_bounds__(kSegBlock) k_pressure_to64(Level B, const float* pressure, double* p64, Ctl* ctl,
+                                                             uint32_t cap) {
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) finish_solve(ctl, cap);
+    pcg::ph_pressure_to64(B, ctl->seg_count[0], gwarp(), gnwarps(), pressure, p64);
+}
+
 __device__ __forceinline__ void rel_begin(Ctl* ctl, double tol, uint32_t cap) {
     pcg::set_target(ctl, tol);
     ctl->inner_cap = cap;
     ctl->refinements = 0;
     ctl->used_iters = 0;
 }
-__global__ void k_rel_begin(Ctl* ctl, double tol, uint32_t cap) { rel_begin(ctl, tol, cap); }
 
 // Refinement loop: go on while the FP64 true residual is above tol and
 // iterations remain.  Each inner FP32 solve reduces its own right-hand side
@@ -596,9 +602,39 @@ __device__ __forceinline__ bool refine_cond(Ctl* ctl, double tol, uint32_t cap) 
     ctl->cond = cont ? 1u : 0u;
     return cont;
 }
-__global__ void k_refine_cond(Ctl* ctl, cudaGraphConditionalHandle h, double tol, uint32_t cap, int graph) {
-    const bool cont = refine_cond(ctl, tol, cap);
-    if (graph) cudaGraphSetConditional(h, cont ? 1u : 0u);
+// The true residual, and the refinement loop's decision on it (decide).
+__global__ void __launch_bounds__(kSegBlock) k_true_residual(Level B, const double* b64, const double* p64, float* x,
+                                                             Ctl* ctl, double* partials, int flags, int decide,
+                                                             double tol, LoopEntry loop) {
+    pdl_wait();
+    if (!kb_true_residual(hw_blk(), B, b64, p64, x, ctl, partials, flags) || !decide) return;
+    const bool cont = refine_cond(ctl, tol, loop.cap);
+    if (loop.set) cudaGraphSetConditional(loop.h, cont ? 1u : 0u);
+}
+
+// A relative solve's start (pcg::ph_solve_start) with its targets and, mixed,
+// the refinement loop's first decision.  One kernel: the five that stood here
+// (||b||, zero pressure, targets, true residual, decision) took 25 us of a
+// small scene's substep.
+__global__ void __launch_bounds__(kSegBlock) k_solve_start(Level B, double* b64, double* p64, float* x,
+                                                           float* pressure, Ctl* ctl, double* partials, int warm,
+                                                           int mixed, double tol, LoopEntry loop) {
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl->solve_t0 = global_ns();
+        ctl->res_sel = 0;
+    }
+    const double2 sums = pcg::ph_solve_start(B, ctl->seg_count[0], gwarp(), gnwarps(), b64, p64, x, pressure, warm, mixed);
+    double2 tot;
+    if (!block_sum_last<kSegBlock>(hw_blk(), sums, partials, partials + kMaxRedBlocks, &ctl->red_counter, &tot) ||
+        threadIdx.x != 0)
+        return;
+    ctl->bnorm2 = tot.x;
+    rel_begin(ctl, tol, loop.cap);
+    if (!mixed) return;
+    ctl->true_rel = tot.x > 0.0 ? sqrt(tot.y / tot.x) : 0.0;
+    const bool cont = refine_cond(ctl, tol, loop.cap);
+    if (loop.set) cudaGraphSetConditional(loop.h, cont ? 1u : 0u);
 }
 
 __device__ __forceinline__ void refine_end(Ctl* ctl, double tol) {
@@ -608,7 +644,13 @@ __device__ __forceinline__ void refine_end(Ctl* ctl, double tol) {
     ctl->pcg_iters_total += ctl->used_iters;
     if (ctl->true_rel > tol) ctl->not_converged++;
 }
-__global__ void k_refine_end(Ctl* ctl, double tol) { refine_end(ctl, tol); }
+
+__global__ void __launch_bounds__(kSegBlock) k_mixed_accumulate(Level B, double* p64, const float* x, float* pressure,
+                                                                Ctl* ctl, int finalize, double tol) {
+    pdl_wait();
+    kb_mixed_accumulate(hw_blk(), B, p64, x, pressure, ctl, finalize);
+    if (finalize && blockIdx.x == 0 && threadIdx.x == 0) refine_end(ctl, tol);
+}
 
 // ---- the same phases over a batch of scenes (batch.h) ----------------------
 // Segment phases: persistent CTAs walk the listed items of their gate (each a
@@ -954,29 +996,36 @@ static int loop_body(const Scene& s, int mode) {
     return mode != APIC_SOLVER_REFERENCE && s.cells <= 768u * 768u ? 2 : 1;
 }
 
-// PCG setup (src/apic.rs:1885-1892) followed by a device-controlled WHILE
-// loop over iterations.
-// begin: reset the PCG state first (the refinement loop's k_refine_cond has
-// already done so for its inner solves).
-static cudaError_t build_pcg(Scene& s, GraphCursor& c, int mode, float* x, int p_padded, uint32_t cap, int dyn_cap,
-                             bool clear_pressure, bool begin = true) {
+// PCG setup (src/apic.rs:1885-1892): z = M^-1 r, s = z, gamma, the loop's entry.
+// begin: reset the PCG state first (the refinement loop's decision has already
+// done so for its inner solves).
+static void enqueue_pcg_start(Scene& s, int mode, bool begin, const LoopEntry& loop) {
     const Level& B = s.lv[0];
-    uint32_t g = seg_grid(B.words);
+    const uint32_t g = seg_grid(B.words);
+    cudaStream_t st = s.stream;
+    const bool pdl = s.use_pdl;
+    if (mode == APIC_SOLVER_REFERENCE) {
+        launch(pdl, k_reference_start, g, kSegBlock, 0, st, B, s.pressure, s.ctl);
+        launch(pdl, k_seg_prefix, 1, 1024, 0, st, B, static_cast<const Ctl*>(s.ctl), s.seg_pre);
+    } else if (begin) {
+        launch(pdl, k_pcg_begin, 1, 1, 0, st, s.ctl);
+    }
+    enqueue_vcycle(s);
+    launch(pdl, k_pcg_start, g, kSegBlock, 0, st, B, s.search, s.ctl, s.partials, mode, loop);
+    if (mode == APIC_SOLVER_REFERENCE)
+        launch(pdl, k_gamma_exact, 1, kGammaThreads, kGammaSmem, st, B, s.ctl, 1, loop.h, loop.cap, loop.dyn_cap,
+               loop.set);
+}
+
+// The setup followed by a device-controlled WHILE loop over iterations.
+static cudaError_t build_pcg(Scene& s, GraphCursor& c, int mode, float* x, int p_padded, uint32_t cap, int dyn_cap,
+                             bool begin = true) {
     cudaGraphConditionalHandle h;
     cudaError_t e = cudaGraphConditionalHandleCreate(&h, c.g, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return e;
+    const LoopEntry loop{h, cap, dyn_cap, 1};
     e = capture_into(s, c, [&]() {
-        cudaStream_t st = s.stream;
-        // only the reference-mode solve clears the pressure, and it starts here
-        if (begin) k_pcg_begin<<<1, 1, 0, st>>>(s.ctl, clear_pressure ? 1 : 0);
-        if (clear_pressure) k_clear_pressure<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.ctl);
-        if (mode == APIC_SOLVER_REFERENCE) k_seg_prefix<<<1, 1024, 0, st>>>(B, s.ctl, s.seg_pre);
-        enqueue_vcycle(s);
-        launch(s.use_pdl, k_pcg_start, g, kSegBlock, 0, st, B, s.search, s.ctl, s.partials, mode);
-        if (mode == APIC_SOLVER_REFERENCE)
-            launch(s.use_pdl, k_gamma_exact, 1, kGammaThreads, kGammaSmem, st, B, s.ctl, 1,
-                   cudaGraphConditionalHandle(0), 0u, 0, 0);
-        launch(s.use_pdl, k_pcg_cond, 1, 1, 0, st, static_cast<const Ctl*>(s.ctl), h, cap, dyn_cap);
+        enqueue_pcg_start(s, mode, begin, loop);
         return cudaGetLastError();
     });
     if (e != cudaSuccess) return e;
@@ -1008,7 +1057,7 @@ cudaError_t build_solve(Scene& s, GraphCursor& c) {
     s.p64_valid = false;
     cudaError_t e;
     if (mode == APIC_SOLVER_REFERENCE) {
-        e = build_pcg(s, c, mode, s.pressure, 0, 100, 0, true);
+        e = build_pcg(s, c, mode, s.pressure, 0, 100, 0);
         if (e != cudaSuccess) return e;
         return capture_into(s, c, [&]() {
             k_finish_solve<<<1, 1, 0, s.stream>>>(s.ctl, 100);
@@ -1016,47 +1065,42 @@ cudaError_t build_solve(Scene& s, GraphCursor& c) {
         });
     }
     const double tol = double(s.rel_tol);
+    const bool mixed = mode == APIC_SOLVER_REL_MIXED;
+    cudaGraphConditionalHandle hr = 0;
+    if (mixed) {
+        e = cudaGraphConditionalHandleCreate(&hr, c.g, 0, cudaGraphCondAssignDefault);
+        if (e != cudaSuccess) return e;
+    }
+    const LoopEntry refine{hr, s.max_iter, 0, mixed ? 1 : 0}, none{};
     e = capture_into(s, c, [&]() {
-        cudaStream_t st = s.stream;
-        k_mixed_init<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.ctl, s.partials, warm_start(s));
-        k_clear_pressure<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.ctl);
-        k_rel_begin<<<1, 1, 0, st>>>(s.ctl, tol, s.max_iter);
+        launch(s.use_pdl, k_solve_start, g, kSegBlock, 0, s.stream, B, s.b64, s.p64, s.corr, s.pressure, s.ctl,
+               s.partials, int(warm_start(s)), mixed ? 1 : 0, tol, refine);
         return cudaGetLastError();
     });
     if (e != cudaSuccess) return e;
-    if (mode == APIC_SOLVER_REL_FP32) {
-        e = build_pcg(s, c, APIC_SOLVER_REL_FP32, s.pressure, 0, s.max_iter, 1, false);
+    auto true_residual = [&](int flags, int decide, const LoopEntry& loop) {
+        launch(s.use_pdl, k_true_residual, g, kSegBlock, 0, s.stream, B, static_cast<const double*>(s.b64),
+               static_cast<const double*>(s.p64), s.corr, s.ctl, s.partials, flags, decide, tol, loop);
+    };
+    if (!mixed) {
+        e = build_pcg(s, c, APIC_SOLVER_REL_FP32, s.pressure, 0, s.max_iter, 1);
         if (e != cudaSuccess) return e;
         // true residual of the FP32 pressure that the projection will use
         return capture_into(s, c, [&]() {
-            cudaStream_t st = s.stream;
-            k_finish_solve<<<1, 1, 0, st>>>(s.ctl, s.max_iter);
-            k_pressure_to64<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.p64, s.ctl);
-            k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 1);
+            k_pressure_to64<<<g, kSegBlock, 0, s.stream>>>(B, s.pressure, s.p64, s.ctl, s.max_iter);
+            true_residual(1, 0, none);
             return cudaGetLastError();
         });
     }
     // APIC_SOLVER_REL_MIXED: r = b - A p in FP64, FP32 PCG on A d = r, p += d.
-    cudaGraphConditionalHandle hr;
-    e = cudaGraphConditionalHandleCreate(&hr, c.g, 0, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) return e;
-    e = capture_into(s, c, [&]() {
-        cudaStream_t st = s.stream;
-        k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 3);
-        k_refine_cond<<<1, 1, 0, st>>>(s.ctl, hr, tol, s.max_iter, 1);
-        return cudaGetLastError();
-    });
-    if (e != cudaSuccess) return e;
     GraphCursor body;
     e = add_conditional_with(c, cudaGraphCondTypeWhile, hr, &body);
     if (e != cudaSuccess) return e;
-    e = build_pcg(s, body, APIC_SOLVER_REL_FP32, s.corr, 1, s.max_iter, 1, false, false);
+    e = build_pcg(s, body, APIC_SOLVER_REL_FP32, s.corr, 1, s.max_iter, 1, false);
     if (e != cudaSuccess) return e;
     e = capture_into(s, body, [&]() {
-        cudaStream_t st = s.stream;
-        k_mixed_accumulate<<<g, kSegBlock, 0, st>>>(B, s.p64, s.corr, s.pressure, s.ctl, 0);
-        k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 3);
-        k_refine_cond<<<1, 1, 0, st>>>(s.ctl, hr, tol, s.max_iter, 1);
+        k_mixed_accumulate<<<g, kSegBlock, 0, s.stream>>>(B, s.p64, s.corr, s.pressure, s.ctl, 0, tol);
+        true_residual(3, 1, refine);
         return cudaGetLastError();
     });
     if (e != cudaSuccess) return e;
@@ -1064,9 +1108,7 @@ cudaError_t build_solve(Scene& s, GraphCursor& c) {
     // the projection uses the FP64 pressure; its true residual is the one reported
     s.p64_valid = true;
     return capture_into(s, c, [&]() {
-        cudaStream_t st = s.stream;
-        k_mixed_accumulate<<<g, kSegBlock, 0, st>>>(B, s.p64, s.corr, s.pressure, s.ctl, 1);
-        k_refine_end<<<1, 1, 0, st>>>(s.ctl, tol);
+        k_mixed_accumulate<<<g, kSegBlock, 0, s.stream>>>(B, s.p64, s.corr, s.pressure, s.ctl, 1, tol);
         return cudaGetLastError();
     });
 }
@@ -1080,17 +1122,8 @@ static cudaError_t read_ctl(Scene& s) {
 }
 
 // PCG setup and iterations until the device flags convergence or the cap.
-static cudaError_t eager_pcg(Scene& s, int mode, float* x, int p_padded, uint32_t cap, bool clear_pressure) {
-    const Level& B = s.lv[0];
-    uint32_t g = seg_grid(B.words);
-    cudaStream_t st = s.stream;
-    k_pcg_begin<<<1, 1, 0, st>>>(s.ctl, clear_pressure ? 1 : 0);
-    if (clear_pressure) k_clear_pressure<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.ctl);
-    if (mode == APIC_SOLVER_REFERENCE) k_seg_prefix<<<1, 1024, 0, st>>>(B, s.ctl, s.seg_pre);
-    enqueue_vcycle(s);
-    k_pcg_start<<<g, kSegBlock, 0, st>>>(B, s.search, s.ctl, s.partials, mode);
-    if (mode == APIC_SOLVER_REFERENCE)
-        k_gamma_exact<<<1, kGammaThreads, kGammaSmem, st>>>(B, s.ctl, 1, cudaGraphConditionalHandle(0), 0u, 0, 0);
+static cudaError_t eager_pcg(Scene& s, int mode, float* x, int p_padded, uint32_t cap) {
+    enqueue_pcg_start(s, mode, true, LoopEntry{});
     s.pcg_set_cond = false;
     s.pcg_cap = cap;
     s.pcg_dyn_cap = 0;
@@ -1112,34 +1145,30 @@ cudaError_t run_solve_eager(Scene& s) {
     s.p64_valid = false;
     cudaError_t e;
     if (mode == APIC_SOLVER_REFERENCE) {
-        if ((e = eager_pcg(s, mode, s.pressure, 0, 100, true)) != cudaSuccess) return e;
+        if ((e = eager_pcg(s, mode, s.pressure, 0, 100)) != cudaSuccess) return e;
         k_finish_solve<<<1, 1, 0, st>>>(s.ctl, 100);
         return cudaGetLastError();
     }
     const double tol = double(s.rel_tol);
-    k_mixed_init<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.ctl, s.partials, warm_start(s));
-    k_clear_pressure<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.ctl);
-    k_rel_begin<<<1, 1, 0, st>>>(s.ctl, tol, s.max_iter);
-    if (mode == APIC_SOLVER_REL_FP32) {
-        if ((e = eager_pcg(s, mode, s.pressure, 0, s.max_iter, false)) != cudaSuccess) return e;
-        k_finish_solve<<<1, 1, 0, st>>>(s.ctl, s.max_iter);
-        k_pressure_to64<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.p64, s.ctl);
-        k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 1);
+    const bool mixed = mode == APIC_SOLVER_REL_MIXED;
+    const LoopEntry refine{0, s.max_iter, 0, 0};
+    k_solve_start<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.pressure, s.ctl, s.partials, int(warm_start(s)),
+                                            mixed ? 1 : 0, tol, refine);
+    if (!mixed) {
+        if ((e = eager_pcg(s, mode, s.pressure, 0, s.max_iter)) != cudaSuccess) return e;
+        k_pressure_to64<<<g, kSegBlock, 0, st>>>(B, s.pressure, s.p64, s.ctl, s.max_iter);
+        k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 1, 0, tol, refine);
         return cudaGetLastError();
     }
-    k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 3);
-    k_refine_cond<<<1, 1, 0, st>>>(s.ctl, 0, tol, s.max_iter, 0);
     for (;;) {
         if ((e = read_ctl(s)) != cudaSuccess) return e;
         if (!s.ctl_host->cond) break;
-        if ((e = eager_pcg(s, APIC_SOLVER_REL_FP32, s.corr, 1, s.ctl_host->inner_cap, false)) != cudaSuccess) return e;
-        k_mixed_accumulate<<<g, kSegBlock, 0, st>>>(B, s.p64, s.corr, s.pressure, s.ctl, 0);
-        k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 3);
-        k_refine_cond<<<1, 1, 0, st>>>(s.ctl, 0, tol, s.max_iter, 0);
+        if ((e = eager_pcg(s, APIC_SOLVER_REL_FP32, s.corr, 1, s.ctl_host->inner_cap)) != cudaSuccess) return e;
+        k_mixed_accumulate<<<g, kSegBlock, 0, st>>>(B, s.p64, s.corr, s.pressure, s.ctl, 0, tol);
+        k_true_residual<<<g, kSegBlock, 0, st>>>(B, s.b64, s.p64, s.corr, s.ctl, s.partials, 3, 1, tol, refine);
     }
     s.p64_valid = true;
-    k_mixed_accumulate<<<g, kSegBlock, 0, st>>>(B, s.p64, s.corr, s.pressure, s.ctl, 1);
-    k_refine_end<<<1, 1, 0, st>>>(s.ctl, tol);
+    k_mixed_accumulate<<<g, kSegBlock, 0, st>>>(B, s.p64, s.corr, s.pressure, s.ctl, 1, tol);
     return cudaGetLastError();
 }
 
