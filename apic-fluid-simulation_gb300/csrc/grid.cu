@@ -315,14 +315,23 @@ __global__ void __launch_bounds__(kSegBlock) k_laplacian(const uint32_t* __restr
 __device__ __forceinline__ void coarsen_word(const Level& f, const Level& c, uint32_t word, uint32_t lane) {
     const uint32_t raw = word * 32u + lane;
     bool on = false;
-    uint32_t cx = 0, cy = 0;
+    // every load at once (a level with a coarser one has even sides, so a row of
+    // children is a pair, inside the padded arrays and 8-byte aligned), then
+    // the mask decides
+    uint32_t bits[2] = {0u, 0u};
+    float2 d[2], x[2], y[2];
     if (raw < c.cells) {
+        uint32_t cx, cy;
         raw_xy(raw, c.w, c.wshift, cx, cy);
-        for (uint32_t dy = 0; dy < 2; ++dy)
-            for (uint32_t dx = 0; dx < 2; ++dx) {
-                uint32_t fx = cx * 2 + dx, fy = cy * 2 + dy;
-                if (fx < f.w && fy < f.h && bit_at(f.fluid, fy * f.w + fx)) on = true;
-            }
+#pragma unroll
+        for (uint32_t dy = 0; dy < 2; ++dy) {
+            const uint32_t fr = (2u * cy + dy) * f.w + 2u * cx, fp = fr + f.w;
+            bits[dy] = (f.fluid[fr >> 5] >> (fr & 31u)) & 3u;
+            d[dy] = *reinterpret_cast<const float2*>(f.diag + fp);
+            x[dy] = *reinterpret_cast<const float2*>(f.px + fp);
+            y[dy] = *reinterpret_cast<const float2*>(f.py + fp);
+        }
+        on = (bits[0] | bits[1]) != 0u;
     }
     const uint32_t ballot = __ballot_sync(0xffffffffu, on);
     if (lane == 0) c.fluid[word] = ballot;
@@ -338,19 +347,21 @@ __device__ __forceinline__ void coarsen_word(const Level& f, const Level& c, uin
         return;
     }
     float diag = 0.0f, px = 0.0f, py = 0.0f;
-    for (uint32_t dy = 0; dy < 2; ++dy)
-        for (uint32_t dx = 0; dx < 2; ++dx) {
-            uint32_t fx = cx * 2 + dx, fy = cy * 2 + dy;
-            if (fx >= f.w || fy >= f.h) continue;
-            uint32_t fr = fy * f.w + fx, fp = fr + f.w;
-            if (bit_at(f.fluid, fr)) {
-                diag += f.diag[fp];
-                if (dx == 0) diag += 2.0f * f.px[fp];
-                if (dy == 0) diag += 2.0f * f.py[fp];
-                if (dx == 1) px += f.px[fp];
-                if (dy == 1) py += f.py[fp];
-            }
+#pragma unroll
+    for (uint32_t dy = 0; dy < 2; ++dy) {
+        if (bits[dy] & 1u) {
+            diag += d[dy].x;
+            diag += 2.0f * x[dy].x;
+            if (dy == 0) diag += 2.0f * y[dy].x;
+            if (dy == 1) py += y[dy].x;
         }
+        if (bits[dy] & 2u) {
+            diag += d[dy].y;
+            if (dy == 0) diag += 2.0f * y[dy].y;
+            px += x[dy].y;
+            if (dy == 1) py += y[dy].y;
+        }
+    }
     uint32_t cp = raw + c.w;
     float fd = diag * 0.5f;
     c.diag[cp] = fd;
@@ -404,8 +415,12 @@ __global__ void __launch_bounds__(kOneThreads) k_compact_one(const uint32_t* __r
     compact_one(fluid, words, seg, level, ctl);
 }
 
-// The smallest levels, [first, n), by one CTA: each level's coarsening (a
-// warp per mask word), then its segment list, with CTA barriers between.
+// The smallest levels, [first, n), by one CTA: a level's coarsening by a warp
+// per mask word, with a CTA barrier between levels, then every level's
+// segment list by a warp of its own.  What it takes is the latency of each
+// level's loads and stores, one after another (128^2 scene, four levels: 18.0
+// -> 9.3 us against lists between the levels and loads behind their masks).
+constexpr uint32_t kTailWords = 128;  // mask words of a level here at most
 struct TailLevels {
     int first, n;
     Level lv[kMaxLevels];
@@ -418,9 +433,21 @@ __global__ void __launch_bounds__(kOneThreads) k_coarsen_tail(TailLevels t, Ctl*
         const Level& c = t.lv[l];
         for (uint32_t w = warp; w < c.words; w += kOneThreads / 32u) coarsen_word(f, c, w, lane);
         __syncthreads();
-        compact_one(c.fluid, c.words, c.seg, l, ctl);
-        __syncthreads();
     }
+    const int l = t.first + int(warp);
+    if (l >= t.n) return;
+    const Level& c = t.lv[l];
+    uint32_t m[kTailWords / 32u];
+#pragma unroll
+    for (uint32_t k = 0; k < kTailWords / 32u; ++k) m[k] = 32u * k + lane < c.words ? c.fluid[32u * k + lane] : 0u;
+    uint32_t count = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kTailWords / 32u; ++k) {
+        const uint32_t some = __ballot_sync(0xffffffffu, m[k] != 0u);
+        if (m[k]) c.seg[count + uint32_t(__popc(some & ((1u << lane) - 1u)))] = 32u * k + lane;
+        count += uint32_t(__popc(some));
+    }
+    if (lane == 0) ctl->seg_count[l] = count;
 }
 
 // The ascending list of a level's tiles that hold fluid, one CTA per level
@@ -726,7 +753,6 @@ cudaError_t launch_build_pressure(Scene& s) {
 // Levels of at most kTailWords mask words (4096 cells: 64^2 and below) are
 // built together by one CTA; each larger level by a coarsening launch and
 // its segment list.
-constexpr uint32_t kTailWords = 128;
 cudaError_t launch_multilevel(Scene& s) {
     int l = 1;
     for (; l < s.nlevels && s.lv[l].words > kTailWords; ++l) {
