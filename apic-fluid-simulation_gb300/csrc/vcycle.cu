@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kTailThreads) k_coarse_solve(Level L, float* _
                                                                float* __restrict__ cr, Ctl* __restrict__ ctl,
                                                                int exact, int nsm, ExitArgs exit) {
     extern __shared__ uint32_t sm[];
-    CgArrays A{L.fluid, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, cs, cap, cr, nsm > 3};
+    CgArrays A{L.fluid, L.w, L.cells, L.diag, L.px, L.py, L.res, L.err, cs, cap, cr};
     float* f = reinterpret_cast<float*>(sm + L.words);
     auto copy = [&](float* dst, const float* src) {
         for (uint32_t i = threadIdx.x; i < L.padded; i += kTailThreads) cp_async4(dst + i, src + i);

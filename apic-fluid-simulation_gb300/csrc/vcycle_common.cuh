@@ -124,15 +124,13 @@ __device__ __forceinline__ float serial_sum8(const float* prod, uint32_t n) {
     return s;
 }
 
-// The level a CG runs on.  own: diag, px, py and cs lie in this CTA's shared
-// memory and may be overwritten.
+// The level a CG runs on.
 struct CgArrays {
     const uint32_t* bits;
     uint32_t w, cells;
     float *diag, *px, *py;
     const float* res;
     float *err, *cs, *cap, *cr;
-    bool own;
 };
 constexpr uint32_t kCgMaxK = 10;  // cells per thread held in registers
 
@@ -140,13 +138,13 @@ constexpr uint32_t kCgMaxK = 10;  // cells per thread held in registers
 // `nwarps` warps of a CTA.  Cell k of a thread is threadIdx.x + k * threads.
 // exact: the dot products are the reference's serial FP32 sums (reference
 // solver mode).
-//   K == 1: a cell's coefficients, vectors and the neighbours that count in
-//     registers, the directions in cs.
-//   K > 1:  the vectors of K cells in registers; diag, px and py (own) are
-//     first zeroed wherever the reference skips a term, so the loops run over
-//     all cells without a test (a term of zero leaves a sum as it was).
+//   K == 1: a cell's coefficients and vectors in registers, the directions in
+//     cs.
+//   K > 1:  the vectors of K cells in registers.
 //   K == 0: everything in memory (levels of more than kCgMaxK cells per
 //     thread).
+// The coefficients are zero outside the fluid and so are the directions, so a
+// term that the reference skips adds zero.
 struct CgShared {
     CgSlot slot[2];
     float dot;
@@ -160,35 +158,25 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
     const uint32_t W = A.w, cells = A.cells;
     const uint32_t nwords = (cells + 31u) >> 5;
     uint32_t nfl = 0;  // fluid cells of the level
-    for (uint32_t k = lane; k < nwords; k += 32) nfl += uint32_t(__popc(A.bits[k]));
-    nfl = __reduce_add_sync(0xffffffffu, nfl);
-    if (K > 0 && exact) {
-        for (uint32_t word = threadIdx.x; word < nwords; word += threads) {
-            uint32_t c = 0;
-            for (uint32_t k = 0; k < word; ++k) c += uint32_t(__popc(A.bits[k]));
-            sh.pre[word] = c;
-        }
-    }
-    // neighbours that count (right, left, up, down), bit 4: the cell is fluid
-    auto links = [&](uint32_t r) -> uint32_t {
-        if (r >= cells || !bit_at(A.bits, r)) return 0u;
-        const long long q = r;
-        return 16u | (fluid_raw(A.bits, q + 1, cells) ? 1u : 0u) | (fluid_raw(A.bits, q - 1, cells) ? 2u : 0u) |
-               (fluid_raw(A.bits, q + W, cells) ? 4u : 0u) | (fluid_raw(A.bits, q - (long long)W, cells) ? 8u : 0u);
+    auto count = [&] {
+        for (uint32_t k = lane; k < nwords; k += 32) nfl += uint32_t(__popc(A.bits[k]));
+        nfl = __reduce_add_sync(0xffffffffu, nfl);
     };
-    auto apply = [&](uint32_t c, uint32_t nb, float d, float sc, float pxc, float pxl, float pyc, float pyd) {
-        // (all four loads first: they lie inside the padded array)
-        const float sr = A.cs[c + 1], sl = A.cs[c - 1], su = A.cs[c + W], sd = A.cs[c - W];
+    if (exact) {
+        count();
+        if (K > 0)
+            for (uint32_t word = threadIdx.x; word < nwords; word += threads) {
+                uint32_t c = 0;
+                for (uint32_t k = 0; k < word; ++k) c += uint32_t(__popc(A.bits[k]));
+                sh.pre[word] = c;
+            }
+    }
+    auto apply = [&](uint32_t c, float d, float sc, float pxc, float pxl, float pyc, float pyd) {
         float v = d * sc;
-        float t = __fmaf_rn(pxc, sr, v);
-        v = (nb & 1u) ? t : v;
-        t = __fmaf_rn(pxl, sl, v);
-        v = (nb & 2u) ? t : v;
-        t = __fmaf_rn(pyc, su, v);
-        v = (nb & 4u) ? t : v;
-        t = __fmaf_rn(pyd, sd, v);
-        v = (nb & 8u) ? t : v;
-        return v;
+        v = __fmaf_rn(pxc, A.cs[c + 1], v);
+        v = __fmaf_rn(pxl, A.cs[c - 1], v);
+        v = __fmaf_rn(pyc, A.cs[c + W], v);
+        return __fmaf_rn(pyd, A.cs[c - W], v);
     };
     // exact sums: the fluid cells' products are staged at cap in fluid order
     auto stage = [&](uint32_t r, float q) {
@@ -215,53 +203,32 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
         return sh.dot;
     };
     constexpr int KR = K > 0 ? K : 1;
-    uint32_t nb = 0;
     float d = 0.0f, pxc = 0.0f, pxl = 0.0f, pyc = 0.0f, pyd = 0.0f;  // K == 1
     float rv[KR], x[KR], av[KR];
 #pragma unroll
     for (int k = 0; k < KR; ++k) rv[k] = x[k] = av[k] = 0.0f;
+    // r.r first: where it is below the exit, as in many V-cycles of a relative
+    // solve, nothing else is needed.  The directions are zero outside the
+    // fluid and in the padding.
     F2 g{0.0f, 0.0f};
     bool more = false;
-    if constexpr (K == 1) {
-        if (exact) cg_bar(nwarps);  // sh.pre
-        nb = links(threadIdx.x);
-        if (nb) {
-            const uint32_t c = threadIdx.x + W;
-            d = A.diag[c];
-            pxc = A.px[c];
-            pxl = A.px[c - 1];
-            pyc = A.py[c];
-            pyd = A.py[c - W];
-            rv[0] = A.res[c];
-            A.cs[c] = rv[0];
-        }
-        const float q = rv[0] * rv[0];
-        if (exact && nb) stage(threadIdx.x, q);
-        g = F2{q, 0.0f};
-    } else if constexpr (K > 1) {
-        for (uint32_t c = threadIdx.x; c < cells + 2u * W; c += threads) {
-            const long long r = (long long)c - W;
-            const bool f = fluid_raw(A.bits, r, cells) != 0;
-            if (!f || !fluid_raw(A.bits, r + 1, cells)) A.px[c] = 0.0f;
-            if (!f || !fluid_raw(A.bits, r + W, cells)) A.py[c] = 0.0f;
-            if (!f) A.diag[c] = 0.0f;
-            A.cs[c] = f ? A.res[c] : 0.0f;
-        }
-        cg_bar(nwarps);
+    if (exact && K > 0) cg_bar(nwarps);  // sh.pre
+    for (uint32_t c = threadIdx.x; c < 2u * W; c += threads) A.cs[c < W ? c : cells + c] = 0.0f;
+    if constexpr (K > 0) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const uint32_t r = threadIdx.x + uint32_t(k) * threads;
             if (r >= cells) continue;
-            rv[k] = A.cs[r + W];
+            rv[k] = bit_at(A.bits, r) ? A.res[r + W] : 0.0f;
+            A.cs[r + W] = rv[k];
             const float q = rv[k] * rv[k];
             if (exact) stage(r, q);
-            g = f2_add(g, q);
+            g = K == 1 ? F2{q, 0.0f} : f2_add(g, q);
         }
     } else {
         for (uint32_t r = threadIdx.x; r < cells; r += threads) {
-            if (!bit_at(A.bits, r)) continue;
             const uint32_t c = r + W;
-            const float q = A.res[c];
+            const float q = bit_at(A.bits, r) ? A.res[c] : 0.0f;
             A.err[c] = 0.0f;
             A.cr[c] = q;
             A.cs[c] = q;
@@ -273,16 +240,28 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
         gamma = K > 0 ? serial() : serial_cells(A.cr, A.cr);
     else
         gamma = cg_reduce<false>(g, more, sh.slot[0], nwarps);
-    const uint32_t max_it = gamma < 1e-12f ? 0u : min(nfl, 100u);
+    uint32_t max_it = 0;
+    if (!(gamma < 1e-12f)) {
+        if (!exact) count();
+        max_it = min(nfl, 100u);
+        if (K == 1 && threadIdx.x < cells) {
+            const uint32_t c = threadIdx.x + W;
+            d = A.diag[c];
+            pxc = A.px[c];
+            pxl = A.px[c - 1];
+            pyc = A.py[c];
+            pyd = A.py[c - W];
+        }
+    }
     for (uint32_t it = 0; it < max_it; ++it) {
         // (the directions are visible: a barrier follows their update)
         F2 dsum{0.0f, 0.0f};
         if constexpr (K == 1) {
             float q = 0.0f;
-            if (nb) {
+            if (threadIdx.x < cells) {
                 const uint32_t c = threadIdx.x + W;
                 const float sc = A.cs[c];
-                av[0] = apply(c, nb, d, sc, pxc, pxl, pyc, pyd);
+                av[0] = apply(c, d, sc, pxc, pxl, pyc, pyd);
                 q = sc * av[0];
                 if (exact) stage(threadIdx.x, q);
             }
@@ -294,11 +273,7 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
                 if (r >= cells) continue;
                 const uint32_t c = r + W;
                 const float sc = A.cs[c];
-                float v = A.diag[c] * sc;
-                v = __fmaf_rn(A.px[c], A.cs[c + 1], v);
-                v = __fmaf_rn(A.px[c - 1], A.cs[c - 1], v);
-                v = __fmaf_rn(A.py[c], A.cs[c + W], v);
-                v = __fmaf_rn(A.py[c - W], A.cs[c - W], v);
+                const float v = apply(c, A.diag[c], sc, A.px[c], A.px[c - 1], A.py[c], A.py[c - W]);
                 av[k] = v;
                 const float q = sc * v;
                 if (exact) stage(r, q);
@@ -306,11 +281,10 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
             }
         } else {
             for (uint32_t r = threadIdx.x; r < cells; r += threads) {
-                const uint32_t n = links(r);
-                if (!n) continue;
+                if (!bit_at(A.bits, r)) continue;
                 const uint32_t c = r + W;
                 const float sc = A.cs[c];
-                const float v = apply(c, n, A.diag[c], sc, A.px[c], A.px[c - 1], A.py[c], A.py[c - W]);
+                const float v = apply(c, A.diag[c], sc, A.px[c], A.px[c - 1], A.py[c], A.py[c - W]);
                 A.cap[c] = v;
                 dsum = f2_add(dsum, sc * v);
             }
@@ -358,7 +332,7 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 const uint32_t r = threadIdx.x + uint32_t(k) * threads;
-                if (r >= cells || (K == 1 && !nb)) continue;
+                if (r >= cells) continue;
                 A.cs[r + W] = rv[k] + (beta * A.cs[r + W]);
             }
         } else {
@@ -439,9 +413,9 @@ static __device__ __noinline__ void cg_one_warp(const CgArrays& A, bool exact) {
     if (on) A.err[c] = x;
 }
 
-// A level of up to 32 cells takes one warp, up to 1024 one cell per thread of as many warps as that needs; above, all threads hold 4,
-// 6 or 10 cells each; beyond 10240 cells (or without shared-memory copies to
-// overwrite) the cells stay in memory.
+// A level of up to 32 cells takes one warp, up to 1024 one cell per thread of
+// as many warps as that needs; above, all threads hold 4, 6 or 10 cells each;
+// beyond 10240 cells they stay in memory.
 static __device__ __forceinline__ void cta_coarse_cg(const CgArrays& A, bool exact) {
     __shared__ CgShared sh;
     const uint32_t need = (A.cells + 31u) >> 5, all = blockDim.x >> 5;
@@ -451,11 +425,11 @@ static __device__ __forceinline__ void cta_coarse_cg(const CgArrays& A, bool exa
             cg_one_warp(A, exact);
         else if (need <= all)
             cg_warps<1>(A, sh, nwarps, exact);
-        else if (A.own && need <= 4u * all)
+        else if (need <= 4u * all)
             cg_warps<4>(A, sh, nwarps, exact);
-        else if (A.own && need <= 6u * all)
+        else if (need <= 6u * all)
             cg_warps<6>(A, sh, nwarps, exact);
-        else if (A.own && need <= kCgMaxK * all)
+        else if (need <= kCgMaxK * all)
             cg_warps<int(kCgMaxK)>(A, sh, nwarps, exact);
         else
             cg_warps<0>(A, sh, nwarps, exact);
@@ -723,7 +697,7 @@ __device__ __forceinline__ void cta_tail_levels(const TailParams& tp, uint32_t* 
     }
     float* cg = reinterpret_cast<float*>(f.bits + f.words + 6u * f.padded);  // three vectors behind the last level
     cta_coarse_cg(CgArrays{f.bits, f.w, f.cells, f.diag, f.px, f.py, f.res, f.err, cg, cg + f.padded,
-                           cg + 2u * f.padded, true},
+                           cg + 2u * f.padded},
                   tp.exact != 0);
     for (int l = n - 2; l >= 0; --l) {
         const SmemLevel c = f;
