@@ -437,6 +437,17 @@ inline cudaError_t launch(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 bloc
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 uint32_t seg_grid(uint32_t words);     // blocks for a segment kernel over `words` words
+// segments of a warp's step in the SpMV, and its blocks on the base level
+// (five resident CTAs per SM): four where the rows are whole vectors and the
+// level is larger than 256^2; on smaller ones only the latency of a step counts
+// (an iteration of 120^2 32.0 us with one segment, 33.1 with four; 488^2 50.2 and
+// 48.8, 1024^2 58.6 and 58.2, 4096^2 646 and 626, 634 with four CTAs per SM)
+inline __host__ __device__ uint32_t spmv_segs(const Level& B) { return B.w % 4u == 0u && B.words > 2048u ? 4u : 1u; }
+inline uint32_t spmv_grid(const Level& B) {
+    if (spmv_segs(B) == 1u) return seg_grid(B.words);
+    const uint32_t b = div_up(B.words, 4u * uint32_t(kSegWarps)), cap = 152u * 5u;
+    return b < cap ? b : cap;
+}
 // blocks for a tile kernel on a level, and for its base level's block partials
 inline uint32_t tile_grid(const Level& L) {
     return L.ntiles < kMaxTileBlocks ? (L.ntiles ? L.ntiles : 1u) : kMaxTileBlocks;

@@ -232,6 +232,7 @@ BScene make_bscene(Scene& s) {
         t.grid[l] = seg_grid(s.lv[l].words);
     }
     t.tgrid = tile_grid(s.lv[0]);
+    t.sgrid = spmv_grid(s.lv[0]);
     t.ctl = s.ctl;
     t.search = s.search;
     t.ap = s.ap;

@@ -38,6 +38,7 @@ struct BScene {
     Level lv[kMaxLevels];
     uint32_t grid[kMaxLevels];  // seg_grid of each level: the scene's own launch size
     uint32_t tgrid;             // tile_grid of the base level
+    uint32_t sgrid;             // spmv_grid of the base level
     Ctl* ctl;
     float *search, *ap, *corr, *pressure;
     double *b64, *p64, *partials;
@@ -93,10 +94,10 @@ inline __host__ __device__ uint32_t kinds_for(int max_tail) { return uint32_t(ma
 // a tile holds as many cells as 16 segments
 inline __host__ __device__ uint32_t tile_chunk(Shape sh) { return sh.chunk_segs > 16u ? sh.chunk_segs / 16u : 1u; }
 #ifdef __CUDACC__
-// Blocks of the scene's base-level launch that hold a segment (at least one).
+// Blocks of the scene's SpMV launch that hold a segment (at least one).
 __device__ __forceinline__ uint32_t busy_blocks(const BScene& s) {
-    const uint32_t b = (s.ctl->seg_count[0] + kSegWarps - 1) / kSegWarps;
-    return b < 1u ? 1u : (b < s.grid[0] ? b : s.grid[0]);
+    const uint32_t per = kSegWarps * spmv_segs(s.lv[0]), b = (s.ctl->seg_count[0] + per - 1) / per;
+    return b < 1u ? 1u : (b < s.sgrid ? b : s.sgrid);
 }
 // ... of its base level's tile launch that hold a tile (at least one).
 __device__ __forceinline__ uint32_t busy_tile_blocks(const BScene& s) {

@@ -143,7 +143,8 @@ __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nse
     // the buffer this iteration's update writes the residual to (read by the
     // kernels after this one)
     if (bk.id == 0 && threadIdx.x == 0) ctl->res_sel = (ctl->pcg_iters + 1u) & 1u;
-    F2 acc = pcg::ph_spmv_search(B, nseg, blk_warp(bk), blk_nwarps(bk), s, beta, bv, ap, w0);
+    const F2 acc = spmv_segs(B) == 4u ? pcg::ph_spmv_search4(B, nseg, blk_warp(bk), blk_nwarps(bk), s, beta, bv, ap, w0)
+                                      : pcg::ph_spmv_search(B, nseg, blk_warp(bk), blk_nwarps(bk), s, beta, bv, ap, w0);
     block_store<kSegBlock>(bk, acc, part);
 }
 // first: of its loop body (counted).
@@ -152,7 +153,8 @@ __global__ void __launch_bounds__(kSegBlock) k_spmv_dot(Level B, const float* s,
     // the base segment list is written by the substep's setup: load this
     // warp's first word before waiting on the previous kernel
     const uint32_t nseg = ctl->seg_count[0];
-    const uint32_t w0 = gwarp() < nseg ? B.seg[gwarp()] : 0xFFFFFFFFu;
+    const uint32_t s0 = spmv_segs(B) == 4u ? 4u * gwarp() + ((threadIdx.x & 31u) >> 3) : gwarp();
+    const uint32_t w0 = s0 < nseg ? B.seg[s0] : 0xFFFFFFFFu;
     pdl_wait();
     if (first && blockIdx.x == 0 && threadIdx.x == 0) ctl->pcg_bodies++;
     kb_spmv_dot(hw_blk(), B, nseg, w0, s, ap, ctl, part, mode, rz, nrz);
@@ -810,8 +812,8 @@ __global__ void __launch_bounds__(kSegBlock, 8) k_bat_spmv_dot(const BScene* __r
         if (!bat_gate(ctl, kGatePcg)) return;
         const uint32_t nseg = ctl->seg_count[0], end = group_end(S, item, sh);
         for (uint32_t b = item * sh.block_group; b < end; ++b) {
-            kb_spmv_dot(Blk{b, S.grid[0]}, S.lv[0], nseg, 0xFFFFFFFFu, S.search, S.ap, ctl, bs_part_sap(S), kRel,
-                        bs_part_rz(S), S.grid[0], &ctl->b_rz);
+            kb_spmv_dot(Blk{b, S.sgrid}, S.lv[0], nseg, 0xFFFFFFFFu, S.search, S.ap, ctl, bs_part_sap(S), kRel,
+                        bs_part_rz(S), S.tgrid, &ctl->b_rz);
             __syncthreads();  // block_store's shared slots are reused by the next block
         }
     });
@@ -825,7 +827,7 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_update_down(const BScene*
         Ctl* ctl = S.ctl;
         if (!bat_gate(ctl, kGatePcg)) return;
         const uint32_t count = ctl->tile_count[0], end = tile_group_end(S, item, shp);
-        const StepArgs a{bs_part_sap(S), S.grid[0], kRel, nullptr, nullptr, bs_part_rz(S), S.tgrid};
+        const StepArgs a{bs_part_sap(S), S.sgrid, kRel, nullptr, nullptr, bs_part_rz(S), S.tgrid};
         for (uint32_t b = item * shp.block_group; b < end; ++b) {
             tile::DownRegs g;
             const uint32_t id = b < count ? S.lv[0].tiles[b] : 0u;
@@ -953,17 +955,17 @@ ExitArgs exit_args(const Scene& s, int mode) {
 // the next one (inside k_spmv_dot / k_update_down).
 static void pcg_iteration(Scene& s, int mode, float* x, int p_padded, bool first, int sel) {
     const Level& B = s.lv[0];
-    const uint32_t g = seg_grid(B.words), tg = tile_grid(B);
+    const uint32_t g = seg_grid(B.words), tg = tile_grid(B), sg = spmv_grid(B);
     cudaStream_t st = s.stream;
     const bool pdl = s.use_pdl, tiled = s.nlevels >= 2;
     const uint32_t nrz = tiled ? tg : g;
-    launch(pdl && !first, k_spmv_dot, g, kSegBlock, 0, st, B, static_cast<const float*>(s.search), s.ap, s.ctl,
+    launch(pdl && !first, k_spmv_dot, sg, kSegBlock, 0, st, B, static_cast<const float*>(s.search), s.ap, s.ctl,
            part_sap(s), mode, static_cast<const float2*>(part_rz(s)), nrz, first ? 1 : 0);
     if (mode == APIC_SOLVER_REFERENCE)
         launch(pdl, k_delta_exact, div_up(B.cells, kDeltaChunk), kDeltaThreads, 0, st, B,
                static_cast<const float*>(s.search), static_cast<const float*>(s.ap),
                static_cast<const uint32_t*>(s.seg_pre), s.ctl, s.exact_parts);
-    const StepArgs a{part_sap(s), g, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
+    const StepArgs a{part_sap(s), sg, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
     if (tiled) {
         launch(pdl, k_update_down, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
                static_cast<const float*>(s.ap), s.ctl, a, part_res(s), sel);
