@@ -225,6 +225,7 @@ __device__ __forceinline__ tile::Update update_args(const Level& B, const Ctl* c
     return tile::Update{second ? B.res : B.res2, ap, B.err, s, p, p_padded, second ? B.res2 : B.res};
 }
 // (after the dependency wait; g: the first tile's constants, if the block has one)
+template <bool kAll>
 __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Level& C, tile::Shared& sh,
                                                tile::DownRegs& g, uint32_t count, uint32_t id, float* p, int p_padded,
                                                float* s, const float* ap, Ctl* ctl, const StepArgs& a, float4* part,
@@ -233,7 +234,7 @@ __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Lev
     const float beta = ctl->beta;
     const bool beta_valid = ctl->beta_valid != 0;
     const tile::Update u = update_args(B, ctl, p, p_padded, s, ap, sel);
-    if (bk.id < count) tile::down_load<true>(B, u.res, u, g);
+    if (bk.id < count) tile::down_load<true, kAll>(B, u.res, u, g);
     float alpha;
     if (!pcg_alpha(bk, ctl, a, &alpha, rz_sum, sap_sum)) return;
     float mx = 0.0f;
@@ -242,13 +243,14 @@ __device__ __forceinline__ void kb_update_down(Blk bk, const Level& B, const Lev
         if (i != bk.id) {
             id = B.tiles[i];
             __syncthreads();  // the tile before this one has been read
-            tile::down_load_const(B, id, g);
-            tile::down_load<true>(B, u.res, u, g);
+            tile::down_load_const<kAll>(B, id, g);
+            tile::down_load<true, kAll>(B, u.res, u, g);
         }
         tile::down_tile<true>(sh, B, C, id, g, u, alpha, beta, beta_valid, &acc, &mx);
     }
     block_store<kSegBlock>(bk, acc, mx, part);
 }
+template <bool kAll>
 __global__ void __launch_bounds__(kTileBlock, 4) k_update_down(Level B, Level C, float* p, int p_padded, float* s,
                                                                  const float* ap, Ctl* ctl, StepArgs a, float4* part,
                                                                  int sel) {
@@ -256,9 +258,9 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_update_down(Level B, Level C,
     const uint32_t count = ctl->tile_count[0];
     const uint32_t id = blockIdx.x < count ? B.tiles[blockIdx.x] : 0u;
     tile::DownRegs g;
-    if (blockIdx.x < count) tile::down_load_const(B, id, g);
+    if (blockIdx.x < count) tile::down_load_const<kAll>(B, id, g);
     pdl_wait();
-    kb_update_down(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part, sel);
+    kb_update_down<kAll>(hw_blk(), B, C, sh, g, count, id, p, p_padded, s, ap, ctl, a, part, sel);
 }
 
 // The update alone, and the base level's first red sweep (grids without a
@@ -831,8 +833,8 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_update_down(const BScene*
         for (uint32_t b = item * shp.block_group; b < end; ++b) {
             tile::DownRegs g;
             const uint32_t id = b < count ? S.lv[0].tiles[b] : 0u;
-            if (b < count) tile::down_load_const(S.lv[0], id, g);
-            kb_update_down(Blk{b, S.tgrid}, S.lv[0], S.lv[1], sh, g, count, id, into_corr ? S.corr : S.pressure,
+            if (b < count) tile::down_load_const<true>(S.lv[0], id, g);
+            kb_update_down<true>(Blk{b, S.tgrid}, S.lv[0], S.lv[1], sh, g, count, id, into_corr ? S.corr : S.pressure,
                            into_corr, S.search, S.ap, ctl, a, bs_part_res(S), -1, &ctl->b_rz, &ctl->b_sap);
             __syncthreads();
         }
@@ -967,7 +969,7 @@ static void pcg_iteration(Scene& s, int mode, float* x, int p_padded, bool first
                static_cast<const uint32_t*>(s.seg_pre), s.ctl, s.exact_parts);
     const StepArgs a{part_sap(s), sg, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
     if (tiled) {
-        launch(pdl, k_update_down, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
+        launch(pdl, tile::reads_all(B) ? k_update_down<true> : k_update_down<false>, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
                static_cast<const float*>(s.ap), s.ctl, a, part_res(s), sel);
         // the V-cycle's next kernel runs the residual's exit test, its last
         // one stores the parts of r.z

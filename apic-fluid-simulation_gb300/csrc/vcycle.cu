@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(kSegBlock) k_smooth(Level L, int li, const Ctl
 // an iteration the first of these kernels after the update also runs the
 // update's exit test and the loop's decision, in an extra block beside the
 // sweeps; later kernels see its verdict.
+template <bool kAll>
 __device__ __forceinline__ void kb_down(Blk bk, const Level& f, const Level& c, tile::Shared& sh, tile::DownRegs& g,
                                         uint32_t id, uint32_t end, const float* res) {
     const tile::Update none{};
@@ -70,12 +71,13 @@ __device__ __forceinline__ void kb_down(Blk bk, const Level& f, const Level& c, 
         if (i != bk.id) {
             id = f.tiles[i];
             __syncthreads();  // the tile before this one has been read
-            tile::down_load_const(f, id, g);
+            tile::down_load_const<kAll>(f, id, g);
         }
-        tile::down_load<false>(f, res, none, g);
+        tile::down_load<false, kAll>(f, res, none, g);
         tile::down_tile<false>(sh, f, c, id, g, none, 0.0f, 0.0f, false, nullptr, nullptr);
     }
 }
+template <bool kAll>
 __global__ void __launch_bounds__(kTileBlock, 4) k_down(Level f, Level c, int lf, Ctl* ctl, ExitArgs exit) {
     __shared__ tile::Shared sh;
     const uint32_t extra = exit.on ? 1u : 0u;
@@ -90,16 +92,16 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_down(Level f, Level c, int lf
     const uint32_t count = ctl->tile_count[lf];
     const uint32_t id = bk.id < count ? f.tiles[bk.id] : 0u;
     tile::DownRegs g;
-    if (bk.id < count) tile::down_load_const(f, id, g);
+    if (bk.id < count) tile::down_load_const<kAll>(f, id, g);
     pdl_wait();
     if (ctl->pcg_done) return;
-    kb_down(bk, f, c, sh, g, id, count, lf == 0 ? pcg::cur_res(f, ctl) : f.res);
+    kb_down<kAll>(bk, f, c, sh, g, id, count, lf == 0 ? pcg::cur_res(f, ctl) : f.res);
 }
 
 // The prolongation from c and level f's black and red sweeps; kRz: the base
 // level in an iteration, whose part of r.z is stored too (the next iteration
 // sums the parts).
-template <bool kRz>
+template <bool kRz, bool kAll>
 __device__ __forceinline__ F2 kb_up(Blk bk, const Level& c, const Level& f, tile::Shared& sh, tile::UpRegs& g,
                                     uint32_t id, uint32_t end, const float* res, uint32_t last, uint32_t extra) {
     F2 acc{0.0f, 0.0f};
@@ -107,15 +109,15 @@ __device__ __forceinline__ F2 kb_up(Blk bk, const Level& c, const Level& f, tile
         if (i != bk.id) {
             id = f.tiles[i];
             __syncthreads();  // the tile before this one has been read
-            tile::up_load_const(f, id, g);
+            tile::up_load_const<kAll>(f, id, g);
         }
-        tile::up_load(c, f, res, last, extra, g);
+        tile::up_load<kAll>(c, f, res, last, extra, g);
         tile::up_tile<kRz>(sh, f, g, &acc);
     }
     return acc;
 }
-template <bool kRz>
 // sel: the base residual's buffer, or -1: as Ctl::res_sel says.
+template <bool kRz, bool kAll>
 __global__ void __launch_bounds__(kTileBlock, 4) k_up(Level c, Level f, int lf, const Ctl* ctl, int base,
                                                         float2* part, int sel) {
     __shared__ tile::Shared sh;
@@ -123,11 +125,11 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_up(Level c, Level f, int lf, 
     const uint32_t id = blockIdx.x < count ? f.tiles[blockIdx.x] : 0u;
     const uint32_t last = base ? ctl->last_fluid : 0xFFFFFFFFu, extra = base ? ctl->pad_count : 0u;
     tile::UpRegs g;
-    if (blockIdx.x < count) tile::up_load_const(f, id, g);
+    if (blockIdx.x < count) tile::up_load_const<kAll>(f, id, g);
     pdl_wait();
     if (ctl->pcg_done) return;
     const float* res = !base ? f.res : sel < 0 ? pcg::cur_res(f, ctl) : sel ? f.res2 : f.res;
-    const F2 acc = kb_up<kRz>(hw_blk(), c, f, sh, g, id, count, res, last, extra);
+    const F2 acc = kb_up<kRz, kAll>(hw_blk(), c, f, sh, g, id, count, res, last, extra);
     if (kRz) block_store<kTileBlock>(hw_blk(), acc, part);
 }
 
@@ -199,8 +201,8 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_down(const BScene* __rest
         if (i0 >= end) return;
         const uint32_t id = S.lv[lf].tiles[i0];
         tile::DownRegs g;
-        tile::down_load_const(S.lv[lf], id, g);
-        kb_down(Blk{i0, 1u}, S.lv[lf], S.lv[lf + 1], sh, g, id, end,
+        tile::down_load_const<true>(S.lv[lf], id, g);
+        kb_down<true>(Blk{i0, 1u}, S.lv[lf], S.lv[lf + 1], sh, g, id, end,
                 lf == 0 ? pcg::cur_res(S.lv[0], ctl) : S.lv[lf].res);
     });
 }
@@ -217,8 +219,8 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_up(const BScene* __restri
         const uint32_t id = S.lv[lf].tiles[i0];
         const uint32_t last = base ? ctl->last_fluid : 0xFFFFFFFFu, extra = base ? ctl->pad_count : 0u;
         tile::UpRegs g;
-        tile::up_load_const(S.lv[lf], id, g);
-        kb_up<false>(Blk{i0, 1u}, S.lv[lf + 1], S.lv[lf], sh, g, id, end,
+        tile::up_load_const<true>(S.lv[lf], id, g);
+        kb_up<false, true>(Blk{i0, 1u}, S.lv[lf + 1], S.lv[lf], sh, g, id, end,
                      base ? pcg::cur_res(S.lv[0], ctl) : S.lv[lf].res, last, extra);
     });
 }
@@ -235,8 +237,8 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_bat_up_rz(const BScene* __res
             const Blk bk{b, S.tgrid};
             tile::UpRegs g;
             const uint32_t id = b < count ? S.lv[0].tiles[b] : 0u;
-            if (b < count) tile::up_load_const(S.lv[0], id, g);
-            const F2 acc = kb_up<true>(bk, S.lv[1], S.lv[0], sh, g, id, count, pcg::cur_res(S.lv[0], ctl),
+            if (b < count) tile::up_load_const<true>(S.lv[0], id, g);
+            const F2 acc = kb_up<true, true>(bk, S.lv[1], S.lv[0], sh, g, id, count, pcg::cur_res(S.lv[0], ctl),
                                        ctl->last_fluid, ctl->pad_count);
             block_store<kTileBlock>(bk, acc, bs_part_rz(S));
             __syncthreads();  // shared slots and the tile are reused by the next block
@@ -328,7 +330,7 @@ void enqueue_vcycle(Scene& s, bool base_done, const ExitArgs& exit_in, int sel) 
     const bool dsm = s.use_dsm && s.dsm_first < s.dsm_tail && s.dsm_tail < s.nlevels;
     ExitArgs exit = exit_in;
     auto down = [&](int l) {
-        launch(pdl, k_down, tile_grid(L[l]) + (exit.on ? 1u : 0u), kTileBlock, 0, st, L[l], L[l + 1], l, s.ctl, exit);
+        launch(pdl, tile::reads_all(L[l]) ? k_down<true> : k_down<false>, tile_grid(L[l]) + (exit.on ? 1u : 0u), kTileBlock, 0, st, L[l], L[l + 1], l, s.ctl, exit);
         exit.on = 0;
     };
     if (!base_done) down(0);
@@ -354,9 +356,11 @@ void enqueue_vcycle(Scene& s, bool base_done, const ExitArgs& exit_in, int sel) 
         down(l);
     }
     for (int k = l - 1; k >= 1; --k)
-        launch(pdl, k_up<false>, tile_grid(L[k]), kTileBlock, 0, st, L[k + 1], L[k], k,
+        launch(pdl, tile::reads_all(L[k]) ? k_up<false, true> : k_up<false, false>, tile_grid(L[k]), kTileBlock, 0, st, L[k + 1], L[k], k,
                static_cast<const Ctl*>(s.ctl), 0, static_cast<float2*>(nullptr), -1);
-    launch(pdl, base_done ? k_up<true> : k_up<false>, tile_grid(L[0]), kTileBlock, 0, st, L[1], L[0], 0,
+    const bool all = tile::reads_all(L[0]);
+    auto up = base_done ? (all ? k_up<true, true> : k_up<true, false>) : all ? k_up<false, true> : k_up<false, false>;
+    launch(pdl, up, tile_grid(L[0]), kTileBlock, 0, st, L[1], L[0], 0,
            static_cast<const Ctl*>(s.ctl), 1, part_rz(s), sel);
 }
 
