@@ -69,34 +69,43 @@ __device__ __forceinline__ float search_at(const float* z, const float* s, float
     return beta_valid ? z[q] + (beta * s[q]) : s[q];
 }
 
-// Ap' = A s' (the FMA chain of :1833-1846); returns s'.Ap'.
+// Ap' = A s' at raw cell `raw` of the grid (the FMA chain of :1833-1846); *sc:
+// s' there.
+__device__ __forceinline__ float apply_search(const Level& B, uint32_t raw, const float* s, float beta,
+                                              bool beta_valid, float* s_here) {
+    const long long W = B.w, q = raw;
+    const float* z = B.err;
+    const uint32_t c = raw + B.w;
+    const bool fr = fluid_raw(B.fluid, q + 1, B.cells), fl = fluid_raw(B.fluid, q - 1, B.cells);
+    const bool fu = fluid_raw(B.fluid, q + W, B.cells), fd = fluid_raw(B.fluid, q - W, B.cells);
+    const float sc = search_at(z, s, beta, beta_valid, c);
+    const float sr = search_at(z, s, beta, beta_valid, c + 1), sl = search_at(z, s, beta, beta_valid, c - 1);
+    const float su = search_at(z, s, beta, beta_valid, c + uint32_t(W));
+    const float sd = search_at(z, s, beta, beta_valid, c - uint32_t(W));
+    const float pxc = B.px[c], pxl = B.px[c - 1], pyc = B.py[c], pyd = B.py[c - W];
+    float v = B.diag[c] * sc;
+    float t = __fmaf_rn(pxc, sr, v);
+    v = fr ? t : v;
+    t = __fmaf_rn(pxl, sl, v);
+    v = fl ? t : v;
+    t = __fmaf_rn(pyc, su, v);
+    v = fu ? t : v;
+    t = __fmaf_rn(pyd, sd, v);
+    v = fd ? t : v;
+    *s_here = sc;
+    return v;
+}
+
+// Ap' over the segments; returns s'.Ap'.
 __device__ __forceinline__ F2 ph_spmv_search(const Level& B, uint32_t nseg, uint32_t warp, uint32_t nwarps,
                                              const float* s, float beta, bool beta_valid, float* ap,
                                              uint32_t w0 = 0xFFFFFFFFu) {
     F2 acc{0.0f, 0.0f};
-    const long long W = B.w;
-    const float* z = B.err;
     APIC_BASE_ALL_W0(B, nseg, warp, nwarps, w0) {
-        const long long raw = raw_;
-        const uint32_t c = raw_ + B.w;
-        const bool fr = fluid_raw(B.fluid, raw + 1, B.cells), fl = fluid_raw(B.fluid, raw - 1, B.cells);
-        const bool fu = fluid_raw(B.fluid, raw + W, B.cells), fd = fluid_raw(B.fluid, raw - W, B.cells);
-        const float sc = search_at(z, s, beta, beta_valid, c);
-        const float sr = search_at(z, s, beta, beta_valid, c + 1), sl = search_at(z, s, beta, beta_valid, c - 1);
-        const float su = search_at(z, s, beta, beta_valid, c + uint32_t(W));
-        const float sd = search_at(z, s, beta, beta_valid, c - uint32_t(W));
-        const float pxc = B.px[c], pxl = B.px[c - 1], pyc = B.py[c], pyd = B.py[c - W];
-        float v = B.diag[c] * sc;
-        float t = __fmaf_rn(pxc, sr, v);
-        v = fr ? t : v;
-        t = __fmaf_rn(pxl, sl, v);
-        v = fl ? t : v;
-        t = __fmaf_rn(pyc, su, v);
-        v = fu ? t : v;
-        t = __fmaf_rn(pyd, sd, v);
-        v = fd ? t : v;
+        float sc;
+        const float v = apply_search(B, raw_, s, beta, beta_valid, &sc);
         if (!fluid_) continue;
-        ap[c] = v;
+        ap[raw_ + B.w] = v;
         acc = f2_add(acc, v * sc);
     }
     return acc;

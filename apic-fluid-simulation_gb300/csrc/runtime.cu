@@ -735,7 +735,7 @@ int apic::create_scene(uint32_t width, uint32_t height, float cell_size, const a
     AL(s.ctl, 1);
     AL(s.partials, kPartialDoubles);
     AL(s.exact_parts, s.cells / 8192 + 1);
-    AL(s.seg_pre, s.lv[0].words + 1);
+    AL(s.seg_pre, s.lv[0].words + 1 + s.cells / 8192u + 2u);  // and the segments that k_delta_exact's chunks start in
     s.scan_tmp_len = 3 * (div_up(max_words, 1024) + 1);
     AL(s.scan_tmp, s.scan_tmp_len);
 #undef AL

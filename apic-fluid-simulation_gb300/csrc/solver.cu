@@ -117,25 +117,24 @@ __global__ void __launch_bounds__(kSegBlock) k_pcg_start(Level B, float* s, Ctl*
         cudaGraphSetConditional(loop.h, pcg_entry(ctl, loop.cap, loop.dyn_cap) ? 1u : 0u);
 }
 
-// s' = z + beta s, Ap = A s' and this block's part of delta = s'.Ap
-// (apply_matrix_and_dot, src/apic.rs:1823-1863; the search update
-// :1945-1954 is folded in).  k_pcg_update sums the parts.
-// In the relative modes the previous iteration's r.z arrives as the parts
-// its V-cycle stored (rz): every block sums them into gamma' and forms
-// beta = gamma' / gamma (:1934-1943); a zero r.z ends the solve (k_pcg_update
-// records it).  Block 0 keeps beta for k_pcg_update.
+// The relative modes' s' = z + beta s, Ap = A s' and this block's part of delta =
+// s'.Ap (apply_matrix_and_dot, src/apic.rs:1823-1863; the search update
+// :1945-1954 is folded in).  The update sums the parts.  The previous
+// iteration's r.z arrives as the parts its V-cycle stored (rz): every block
+// sums them into gamma' and forms beta = gamma' / gamma (:1934-1943); a zero
+// r.z ends the solve (the update records it).  Block 0 keeps beta for the
+// update.
 // (after the dependency wait; w0: this warp's first segment word)
 // rz_sum: the parts' sum formed once beforehand (batched solves), else null.
 __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nseg, uint32_t w0, const float* s,
-                                            float* ap, Ctl* ctl, float2* part, int mode, const float2* rz,
+                                            float* ap, Ctl* ctl, float2* part, const float2* rz,
                                             uint32_t nrz, const float* rz_sum = nullptr) {
     const bool done = ctl->pcg_done != 0, bv = ctl->beta_valid != 0;
     float beta = ctl->beta;
     const float gamma = ctl->gamma;
-    float ng = 0.0f;
-    if (mode != APIC_SOLVER_REFERENCE) ng = rz_sum ? *rz_sum : sum_partials<kSegBlock>(rz, nrz);
+    const float ng = rz_sum ? *rz_sum : sum_partials<kSegBlock>(rz, nrz);
     if (done) return;
-    if (mode != APIC_SOLVER_REFERENCE && bv) {
+    if (bv) {
         if (!(ng != 0.0f)) return;
         beta = ng / gamma;
         if (bk.id == 0 && threadIdx.x == 0) ctl->beta = beta;
@@ -148,8 +147,8 @@ __device__ __forceinline__ void kb_spmv_dot(Blk bk, const Level& B, uint32_t nse
     block_store<kSegBlock>(bk, acc, part);
 }
 // first: of its loop body (counted).
-__global__ void __launch_bounds__(kSegBlock) k_spmv_dot(Level B, const float* s, float* ap, Ctl* ctl, float2* part,
-                                                        int mode, const float2* rz, uint32_t nrz, int first) {
+__global__ void __launch_bounds__(kSegBlock, 5) k_spmv_dot(Level B, const float* s, float* ap, Ctl* ctl, float2* part,
+                                                        const float2* rz, uint32_t nrz, int first) {
     // the base segment list is written by the substep's setup: load this
     // warp's first word before waiting on the previous kernel
     const uint32_t nseg = ctl->seg_count[0];
@@ -157,7 +156,7 @@ __global__ void __launch_bounds__(kSegBlock) k_spmv_dot(Level B, const float* s,
     const uint32_t w0 = s0 < nseg ? B.seg[s0] : 0xFFFFFFFFu;
     pdl_wait();
     if (first && blockIdx.x == 0 && threadIdx.x == 0) ctl->pcg_bodies++;
-    kb_spmv_dot(hw_blk(), B, nseg, w0, s, ap, ctl, part, mode, rz, nrz);
+    kb_spmv_dot(hw_blk(), B, nseg, w0, s, ap, ctl, part, rz, nrz);
 }
 
 // delta (the sum of k_spmv_dot's parts, formed by every block) gives alpha or
@@ -417,17 +416,26 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
 
 // Fluid cells before each base segment (seg_pre[k], k <= nseg; seg_pre[nseg]
 // = all fluid cells): the position of a segment's cells in the reference's
-// ascending fluid list.  One block, once per solve.
-__global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, uint32_t* seg_pre) {
+// ascending fluid list; and the segment that holds the first cell of each of
+// the chunks of k_delta_exact (chunk_seg).  One block, once per solve, four
+// segments a thread and round.
+__global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, uint32_t* seg_pre, uint32_t* chunk_seg) {
     pdl_wait();
     const uint32_t nseg = ctl->seg_count[0];
     __shared__ uint32_t sw[32];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     uint32_t carry = 0;
-    for (uint32_t k0 = 0; k0 < nseg; k0 += 1024) {
-        const uint32_t k = k0 + t;
-        const uint32_t v = k < nseg ? uint32_t(__popc(B.fluid[B.seg[k]])) : 0u;
-        uint32_t x = v;
+    for (uint32_t k0 = 0; k0 < nseg; k0 += 4096) {
+        const uint32_t k = k0 + 4u * t;
+        uint32_t v[4], x = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) v[j] = k + j < nseg ? B.seg[k + j] : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            v[j] = k + j < nseg ? uint32_t(__popc(B.fluid[v[j]])) : 0u;
+            x += v[j];
+        }
+        const uint32_t own = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -445,7 +453,15 @@ __global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, ui
             sw[lane] = u;
         }
         __syncthreads();
-        if (k < nseg) seg_pre[k] = carry + (warp > 0 ? sw[warp - 1] : 0u) + x - v;
+        uint32_t at = carry + (warp > 0 ? sw[warp - 1] : 0u) + x - own;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            if (k + j >= nseg) break;
+            seg_pre[k + j] = at;
+            const uint32_t c = (at + kDeltaChunk - 1u) / kDeltaChunk;  // the first chunk that starts here or later
+            if (c * kDeltaChunk < at + v[j]) chunk_seg[c] = k + j;
+            at += v[j];
+        }
         const uint32_t tot = sw[31];
         __syncthreads();
         carry += tot;
@@ -453,62 +469,63 @@ __global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, ui
     if (t == 0) seg_pre[nseg] = carry;
 }
 
-// delta = apply_matrix_and_dot's sum (:1823-1863): s'.Ap over the fluid cells
-// in ascending order, in chunks of 8192 cells each summed serially from zero
-// (rayon's par_chunks(8192)); k_pcg_update then adds the chunk sums in chunk
-// order.  s' is the iteration's search direction, z + beta s (k_spmv_dot
-// evaluates the same expression).  One block per chunk: warps 1..15 stage the
-// products in fluid order in shared memory (positions from seg_pre), a
-// stretch of segments at a time, while thread 0 adds those staged before, in
-// order, the loads ahead of its add chain: a chunk costs its 8192 dependent
-// adds.  (Staged as a whole first, and added with each product's load in the
-// chain, a PCG iteration of a 256^2 grid with 30657 fluid cells took 117 us;
-// with this and the r.z sum's rows it takes 82.)
+// Ap = A s' and delta, apply_matrix_and_dot's sum (:1823-1863): s'.Ap over the
+// fluid cells in ascending order, in chunks of 8192 cells each summed serially
+// from zero (rayon's par_chunks(8192)); the update then adds the chunk sums in
+// chunk order.  s' is the iteration's search direction, z + beta s (the search
+// update :1945-1954 is folded in).  One block per chunk: warps 1..15 form Ap and
+// stage the products in fluid order in shared memory (positions from
+// seg_pre), a stretch of segments at a time, while thread 0 adds those staged
+// before, in order, the loads ahead of its add chain: a chunk costs its 8192
+// dependent adds, and Ap is formed behind them.  An iteration of a 256^2 grid
+// with 30657 fluid cells: 117 us staged as a whole first, 82 with this chain and
+// the r.z sum's rows; Ap formed here instead of by a kernel before, and the
+// chunk's segments from a table instead of a binary search, took 3 us more off
+// it (64^2 44.2 -> 41.4, 256^2 88.1 -> 85.4, 1024^2 355 -> 349, moving scenes).
 constexpr int kDeltaThreads = 512;
 constexpr uint32_t kDeltaStretch = 60;  // segments staged at a time (15 warps, four each)
+// first: of its loop body (counted).
 __global__ void __launch_bounds__(kDeltaThreads) k_delta_exact(Level B, const float* __restrict__ s,
-                                                               const float* __restrict__ ap,
-                                                               const uint32_t* __restrict__ seg_pre, Ctl* ctl,
-                                                               float* __restrict__ parts) {
+                                                               float* __restrict__ ap,
+                                                               const uint32_t* __restrict__ seg_pre,
+                                                               const uint32_t* __restrict__ chunk_seg, Ctl* ctl,
+                                                               float* __restrict__ parts, int first) {
     __shared__ __align__(16) float prod[kDeltaChunk];
-    __shared__ uint32_t s_k0, s_k1;
     pdl_wait();
-    if (ctl->pcg_done) return;
-    const uint32_t nseg = ctl->seg_count[0];
-    const uint32_t nfluid = seg_pre[nseg];
-    const uint32_t c = blockIdx.x;
-    const uint32_t f0 = c * kDeltaChunk;
-    if (f0 >= nfluid) return;
-    const uint32_t f1 = min(f0 + kDeltaChunk, nfluid);
-    if (threadIdx.x < 2) {
-        // segments [k0, k1) hold fluid cells f0 .. f1-1 (every segment holds
-        // at least one): the last k with seg_pre[k] <= f0, the first with
-        // seg_pre[k] >= f1
-        const uint32_t want = threadIdx.x == 0 ? f0 + 1u : f1;
-        uint32_t lo = 0, hi = nseg;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) / 2;
-            if (seg_pre[mid] < want) lo = mid + 1; else hi = mid;
-        }
-        if (threadIdx.x == 0) s_k0 = lo - 1u;
-        else s_k1 = lo;
-    }
-    __syncthreads();
     const float beta = ctl->beta;
     const bool beta_valid = ctl->beta_valid != 0;
+    const uint32_t nseg = ctl->seg_count[0], nfluid = ctl->fluid_cells;
+    const uint32_t c = blockIdx.x;
+    const uint32_t f0 = c * kDeltaChunk;
+    if (c == 0 && threadIdx.x == 0 && first) ctl->pcg_bodies++;
+    if (ctl->pcg_done) return;
+    // the buffer this iteration's update writes the residual to
+    if (c == 0 && threadIdx.x == 0) ctl->res_sel = (ctl->pcg_iters + 1u) & 1u;
+    if (f0 >= nfluid) return;
+    const uint32_t f1 = min(f0 + kDeltaChunk, nfluid);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t k0 = s_k0, k1 = s_k1;
+    // segments [k0, k1) hold fluid cells f0 .. f1-1 (the last one may hold cells
+    // of the next chunk too)
+    const uint32_t k0 = chunk_seg[c];
+    uint32_t k1 = nseg;
+    if (f1 < nfluid) {
+        k1 = chunk_seg[c + 1];
+        if (seg_pre[k1] < f1) ++k1;
+    }
     auto stage = [&](uint32_t from) {
         const uint32_t end = min(from + kDeltaStretch, k1);
 #pragma unroll 4
         for (uint32_t k = from + warp - 1u; k < end; k += kDeltaThreads / 32 - 1) {
-            const uint32_t w = B.seg[k];
-            const uint32_t m = B.fluid[w];
+            const uint32_t w = B.seg[k], raw = w * 32u + lane;
+            const uint32_t m = B.fluid[w], pre = seg_pre[k];
+            if (raw >= B.cells) continue;
+            float sc;
+            const float v = pcg::apply_search(B, raw, s, beta, beta_valid, &sc);
             if (!((m >> lane) & 1u)) continue;
-            const uint32_t pos = seg_pre[k] + uint32_t(__popc(m & ((1u << lane) - 1u)));
+            const uint32_t pos = pre + uint32_t(__popc(m & ((1u << lane) - 1u)));
             if (pos < f0 || pos >= f1) continue;
-            const uint32_t cidx = w * 32u + lane + B.w;
-            prod[pos - f0] = ap[cidx] * pcg::search_at(B.err, s, beta, beta_valid, cidx);
+            ap[raw + B.w] = v;
+            prod[pos - f0] = v * sc;
         }
     };
     if (warp != 0) stage(k0);
@@ -814,7 +831,7 @@ __global__ void __launch_bounds__(kSegBlock, 8) k_bat_spmv_dot(const BScene* __r
         if (!bat_gate(ctl, kGatePcg)) return;
         const uint32_t nseg = ctl->seg_count[0], end = group_end(S, item, sh);
         for (uint32_t b = item * sh.block_group; b < end; ++b) {
-            kb_spmv_dot(Blk{b, S.sgrid}, S.lv[0], nseg, 0xFFFFFFFFu, S.search, S.ap, ctl, bs_part_sap(S), kRel,
+            kb_spmv_dot(Blk{b, S.sgrid}, S.lv[0], nseg, 0xFFFFFFFFu, S.search, S.ap, ctl, bs_part_sap(S),
                         bs_part_rz(S), S.tgrid, &ctl->b_rz);
             __syncthreads();  // block_store's shared slots are reused by the next block
         }
@@ -952,6 +969,9 @@ ExitArgs exit_args(const Scene& s, int mode) {
     return a;
 }
 
+// (behind the prefix counts of the base level's segments)
+static uint32_t* chunk_seg(const Scene& s) { return s.seg_pre + s.lv[0].words + 1; }
+
 // One PCG iteration (src/apic.rs:1899-1955); x receives alpha * s.  The
 // search update that ends the reference's iteration happens at the start of
 // the next one (inside k_spmv_dot / k_update_down).
@@ -961,12 +981,13 @@ static void pcg_iteration(Scene& s, int mode, float* x, int p_padded, bool first
     cudaStream_t st = s.stream;
     const bool pdl = s.use_pdl, tiled = s.nlevels >= 2;
     const uint32_t nrz = tiled ? tg : g;
-    launch(pdl && !first, k_spmv_dot, sg, kSegBlock, 0, st, B, static_cast<const float*>(s.search), s.ap, s.ctl,
-           part_sap(s), mode, static_cast<const float2*>(part_rz(s)), nrz, first ? 1 : 0);
     if (mode == APIC_SOLVER_REFERENCE)
-        launch(pdl, k_delta_exact, div_up(B.cells, kDeltaChunk), kDeltaThreads, 0, st, B,
-               static_cast<const float*>(s.search), static_cast<const float*>(s.ap),
-               static_cast<const uint32_t*>(s.seg_pre), s.ctl, s.exact_parts);
+        launch(pdl && !first, k_delta_exact, div_up(B.cells, kDeltaChunk), kDeltaThreads, 0, st, B,
+               static_cast<const float*>(s.search), s.ap, static_cast<const uint32_t*>(s.seg_pre),
+               static_cast<const uint32_t*>(chunk_seg(s)), s.ctl, s.exact_parts, first ? 1 : 0);
+    else
+        launch(pdl && !first, k_spmv_dot, sg, kSegBlock, 0, st, B, static_cast<const float*>(s.search), s.ap, s.ctl,
+               part_sap(s), static_cast<const float2*>(part_rz(s)), nrz, first ? 1 : 0);
     const StepArgs a{part_sap(s), sg, mode, s.exact_parts, s.seg_pre, part_rz(s), nrz};
     if (tiled) {
         launch(pdl, tile::reads_all(B) ? k_update_down<true> : k_update_down<false>, tg, kTileBlock, 0, st, B, s.lv[1], x, p_padded, s.search,
@@ -1010,7 +1031,7 @@ static void enqueue_pcg_start(Scene& s, int mode, bool begin, const LoopEntry& l
     const bool pdl = s.use_pdl;
     if (mode == APIC_SOLVER_REFERENCE) {
         launch(pdl, k_reference_start, g, kSegBlock, 0, st, B, s.pressure, s.ctl);
-        launch(pdl, k_seg_prefix, 1, 1024, 0, st, B, static_cast<const Ctl*>(s.ctl), s.seg_pre);
+        launch(pdl, k_seg_prefix, 1, 1024, 0, st, B, static_cast<const Ctl*>(s.ctl), s.seg_pre, chunk_seg(s));
     } else if (begin) {
         launch(pdl, k_pcg_begin, 1, 1, 0, st, s.ctl);
     }
