@@ -219,29 +219,67 @@ __device__ __forceinline__ float smoothed_guarded(const float* sm, const float* 
     return c < cells ? smoothed_at(sm, dens, fluid, c) : 0.0f;
 }
 
-__global__ void __launch_bounds__(kSegBlock) k_smooth_density(const uint32_t* __restrict__ fluid,
-                                                               const uint32_t* __restrict__ seg,
-                                                               const Ctl* __restrict__ ctl, uint32_t W, uint32_t cells,
-                                                               const float* __restrict__ src, float* __restrict__ dst) {
+// A tile of a grid with a halo as wide as the sweeps that one launch runs on it.
+template <int kTX, int kTY, int kSweeps>
+struct SweepTile {
+    static constexpr int TX = kTX, TY = kTY, N = kSweeps;
+    static constexpr int RX = kTX + 2 * kSweeps, RY = kTY + 2 * kSweeps;
+};
+
+// The three smoothing passes of the density over the fluid cells (src/apic.rs:
+// 1649-1685) in one launch, on tiles with a halo of three in shared memory.
+// A cell's neighbours are those of its flat index (the cell after a row's last
+// one is the next row's first), which a staged position's are too.  Three
+// launches before, each reading what the one before wrote: 128^2 11.4 -> 4.6 us,
+// the build stage 308 -> 259 us at 4096^2.
+template <class T>
+__global__ void __launch_bounds__(256) k_smooth_density(const uint32_t* __restrict__ fluid, uint32_t W, uint32_t H,
+                                                        const float* __restrict__ src, float* __restrict__ dst,
+                                                        uint32_t tiles_x) {
+    __shared__ float s_val[2][T::RX * T::RY];
+    __shared__ uint8_t s_on[T::RX * T::RY];
+    const int x0 = int(blockIdx.x % tiles_x) * T::TX - T::N, y0 = int(blockIdx.x / tiles_x) * T::TY - T::N;
+    const long long cells = (long long)W * H;
     pdl_wait();
-    const uint32_t nseg = ctl->seg_count[0];
-    const int lane = threadIdx.x & 31;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nseg; s += nw) {
-        uint32_t word = seg[s];
-        uint32_t bits = fluid[word];
-        if (!((bits >> lane) & 1u)) continue;
-        long long raw = (long long)word * 32 + lane;
-        float fl = float(fluid_raw(fluid, raw - 1, cells)), fr = float(fluid_raw(fluid, raw + 1, cells));
-        float fb = float(fluid_raw(fluid, raw - (long long)W, cells)), ft = float(fluid_raw(fluid, raw + (long long)W, cells));
-        float sum = src[raw] * 4.0f;
-        float weight = 4.0f;
-        if (fl != 0.0f) sum += src[raw - 1];
-        if (fr != 0.0f) sum += src[raw + 1];
-        if (fb != 0.0f) sum += src[raw - W];
-        if (ft != 0.0f) sum += src[raw + W];
-        weight += fl + fr + fb + ft;
-        dst[raw] = sum / weight;
+    bool some = false;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < T::RX * T::RY; i += 256) {
+        const int x = x0 + i % T::RX, y = y0 + i / T::RX;
+        const long long raw = (long long)y * W + x;
+        const bool in = raw >= 0 && raw < cells;
+        const bool on = in && bit_at(fluid, uint32_t(raw));
+        s_val[0][i] = in ? src[raw] : 0.0f;
+        s_on[i] = on;
+        some = some || on;
+    }
+    if (!__syncthreads_or(some)) return;
+    int cur = 0;
+#pragma unroll
+    for (int n = 1; n <= T::N; ++n) {
+        const int rx_n = T::RX - 2 * n, count = rx_n * (T::RY - 2 * n);
+        for (int j = threadIdx.x; j < count; j += 256) {
+            const int rx = n + j % rx_n, ry = n + j / rx_n, i = ry * T::RX + rx;
+            if (!s_on[i]) continue;
+            const float* v = s_val[cur];
+            const float fl = float(s_on[i - 1]), fr = float(s_on[i + 1]);
+            const float fb = float(s_on[i - T::RX]), ft = float(s_on[i + T::RX]);
+            float sum = v[i] * 4.0f;
+            float weight = 4.0f;
+            if (fl != 0.0f) sum += v[i - 1];
+            if (fr != 0.0f) sum += v[i + 1];
+            if (fb != 0.0f) sum += v[i - T::RX];
+            if (ft != 0.0f) sum += v[i + T::RX];
+            weight += fl + fr + fb + ft;
+            const float out = sum / weight;
+            if (n < T::N) {
+                s_val[cur ^ 1][i] = out;
+            } else {
+                const int x = x0 + rx, y = y0 + ry;
+                if (x < int(W) && y < int(H)) dst[size_t(y) * W + x] = out;
+            }
+        }
+        if (n < T::N) __syncthreads();
+        cur ^= 1;
     }
 }
 
@@ -415,16 +453,77 @@ __global__ void __launch_bounds__(kOneThreads) k_compact_one(const uint32_t* __r
     compact_one(fluid, words, seg, level, ctl);
 }
 
+// The base level's list by one CTA (up to kOneWords mask words: 512^2 cells),
+// with what k_compact_count and k_compact_write do besides: the mask cleaned of
+// obstacles, the totals, the last fluid cell.
+__global__ void __launch_bounds__(kOneThreads) k_compact_base(uint32_t* __restrict__ fluid,
+                                                               const uint32_t* __restrict__ obstacle, uint32_t words,
+                                                               uint32_t* __restrict__ seg, uint32_t W,
+                                                               Ctl* __restrict__ ctl) {
+    constexpr uint32_t kPer = kOneWords / kOneThreads;
+    __shared__ uint32_t s_cells[kOneThreads / 32], s_last[kOneThreads / 32];
+    pdl_wait();
+    const uint32_t per = (words + kOneThreads - 1) / kOneThreads, w0 = threadIdx.x * per;
+    uint32_t m[kPer], nz = 0, cells = 0, last = 0;  // last: the last fluid cell, one up
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k)
+        m[k] = k < per ? load_clean_word(fluid, obstacle, w0 + k, words, true) : 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+        if (!m[k]) continue;
+        ++nz;
+        cells += uint32_t(__popc(m[k]));
+        last = (w0 + k) * 32u + 32u - uint32_t(__clz(m[k]));
+    }
+    uint32_t tot;
+    uint32_t off = scan_1024(nz, &tot);
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k)
+        if (m[k]) seg[off++] = w0 + k;
+    cells = __reduce_add_sync(0xffffffffu, cells);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if ((threadIdx.x & 31u) == 0) {
+        s_cells[threadIdx.x >> 5] = cells;
+        s_last[threadIdx.x >> 5] = last;
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    cells = __reduce_add_sync(0xffffffffu, s_cells[threadIdx.x]);
+    last = __reduce_max_sync(0xffffffffu, s_last[threadIdx.x]);
+    if (threadIdx.x != 0) return;
+    ctl->seg_count[0] = tot;
+    ctl->fluid_cells = cells;
+    ctl->last_fluid = last > 0 ? last - 1u + W : 0u;
+    ctl->pad_count = (8u - cells % 8u) % 8u;
+}
+
 // The smallest levels, [first, n), by one CTA: a level's coarsening by a warp
 // per mask word, with a CTA barrier between levels, then every level's
 // segment list by a warp of its own.  What it takes is the latency of each
 // level's loads and stores, one after another (128^2 scene, four levels: 18.0
 // -> 9.3 us against lists between the levels and loads behind their masks).
 constexpr uint32_t kTailWords = 128;  // mask words of a level here at most
+constexpr uint32_t kTailTileGroups = 64;
 struct TailLevels {
     int first, n;
+    int tiles;  // the tile lists too
     Level lv[kMaxLevels];
 };
+// Whether one of the tile's cells is fluid.
+__device__ __forceinline__ bool tile_holds_fluid(const Level& L, uint32_t i) {
+    const uint32_t x0 = (i % L.tiles_x) * kTileX, y0 = (i / L.tiles_x) * kTileY;
+    const uint32_t rows = min(kTileY, L.h - y0), n = min(kTileX, L.w - x0);
+    const uint32_t mask = n >= 32u ? 0xffffffffu : (1u << n) - 1u;
+    uint32_t any = 0;
+#pragma unroll 8
+    for (uint32_t y = 0; y < rows; ++y) {
+        const uint32_t raw = (y0 + y) * L.w + x0, sh = raw & 31u;
+        uint32_t bits = L.fluid[raw >> 5] >> sh;
+        if (sh && (raw >> 5) + 1u < L.words) bits |= L.fluid[(raw >> 5) + 1u] << (32u - sh);
+        any |= bits & mask;
+    }
+    return any != 0;
+}
 __global__ void __launch_bounds__(kOneThreads) k_coarsen_tail(TailLevels t, Ctl* __restrict__ ctl) {
     pdl_wait();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -433,6 +532,36 @@ __global__ void __launch_bounds__(kOneThreads) k_coarsen_tail(TailLevels t, Ctl*
         const Level& c = t.lv[l];
         for (uint32_t w = warp; w < c.words; w += kOneThreads / 32u) coarsen_word(f, c, w, lane);
         __syncthreads();
+    }
+    if (t.tiles) {
+        // groups of 32 tiles over the levels with a coarser one, a warp each:
+        // which hold fluid, then each group's place behind those before it
+        __shared__ uint32_t s_votes[kTailTileGroups];
+        uint32_t g0 = 0;
+        for (int l = 0; l + 1 < t.n; ++l) {
+            const uint32_t ntiles = t.lv[l].ntiles, groups = (ntiles + 31u) / 32u;
+            for (uint32_t g = (warp - g0) & 31u; g < groups; g += 32u) {
+                const uint32_t i = 32u * g + lane;
+                const uint32_t votes = __ballot_sync(0xffffffffu, i < ntiles && tile_holds_fluid(t.lv[l], i));
+                if (lane == 0) s_votes[g0 + g] = votes;
+            }
+            g0 += groups;
+        }
+        __syncthreads();
+        g0 = 0;
+        for (int l = 0; l + 1 < t.n; ++l) {
+            const uint32_t groups = (t.lv[l].ntiles + 31u) / 32u;
+            for (uint32_t g = (warp - g0) & 31u; g < groups; g += 32u) {
+                const uint32_t votes = s_votes[g0 + g];
+                uint32_t before = 0;
+                for (uint32_t k = lane; k < g; k += 32u) before += uint32_t(__popc(s_votes[g0 + k]));
+                before = __reduce_add_sync(0xffffffffu, before);
+                if ((votes >> lane) & 1u)
+                    t.lv[l].tiles[before + uint32_t(__popc(votes & ((1u << lane) - 1u)))] = 32u * g + lane;
+                if (g + 1u == groups && lane == 0) ctl->tile_count[l] = before + uint32_t(__popc(votes));
+            }
+            g0 += groups;
+        }
     }
     const int l = t.first + int(warp);
     if (l >= t.n) return;
@@ -458,20 +587,6 @@ struct TileLists {
     int n;
     Level lv[kMaxLevels];
 };
-__device__ __forceinline__ bool tile_holds_fluid(const Level& L, uint32_t i) {
-    const uint32_t x0 = (i % L.tiles_x) * kTileX, y0 = (i / L.tiles_x) * kTileY;
-    const uint32_t rows = min(kTileY, L.h - y0), n = min(kTileX, L.w - x0);
-    const uint32_t mask = n >= 32u ? 0xffffffffu : (1u << n) - 1u;
-    uint32_t any = 0;
-#pragma unroll 8
-    for (uint32_t y = 0; y < rows; ++y) {
-        const uint32_t raw = (y0 + y) * L.w + x0, sh = raw & 31u;
-        uint32_t bits = L.fluid[raw >> 5] >> sh;
-        if (sh && (raw >> 5) + 1u < L.words) bits |= L.fluid[(raw >> 5) + 1u] << (32u - sh);
-        any |= bits & mask;
-    }
-    return any != 0;
-}
 __global__ void __launch_bounds__(256) k_tile_flags(Level L) {
     pdl_wait();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
@@ -580,12 +695,6 @@ __global__ void __launch_bounds__(256) k_gradient(uint32_t uf, uint32_t vf, int 
 // sweep's values and flags are bit-identical to a sweep over the whole grid.
 // A tile whose staged faces are all valid, or all invalid, is what the sweeps
 // would leave it as: most of a large grid.
-template <int kTX, int kTY, int kSweeps>
-struct ExTile {
-    static constexpr int TX = kTX, TY = kTY, N = kSweeps;
-    static constexpr int RX = kTX + 2 * kSweeps, RY = kTY + 2 * kSweeps;
-};
-
 struct ExField {
     const float* in;
     const uint8_t* in_ok;
@@ -710,6 +819,10 @@ static cudaError_t compact_level(Scene& s, int level, const uint32_t* obstacle) 
                L.seg, level, s.ctl);
         return cudaGetLastError();
     }
+    if (L.words <= kOneWords) {
+        launch(s.use_pdl, k_compact_base, 1, kOneThreads, 0, s.stream, L.fluid, obstacle, L.words, L.seg, L.w, s.ctl);
+        return cudaGetLastError();
+    }
     uint32_t nb = div_up(L.words, kCompactWords);
     if (nb == 0) nb = 1;  // the last block records the (empty) level's totals
     launch(s.use_pdl, k_compact_count, nb, 256, 0, s.stream, L.fluid, obstacle, L.words, s.scan_tmp);
@@ -739,12 +852,17 @@ cudaError_t launch_tile_lists(Scene& s) {
 cudaError_t launch_base_lists(Scene& s) { return compact_level(s, 0, s.obstacle); }
 cudaError_t launch_level_lists(Scene& s, int level) { return compact_level(s, level, nullptr); }
 
+template <class T> static void smooth_density(Scene& s) {
+    const uint32_t tiles_x = div_up(s.W, T::TX);
+    launch(s.use_pdl, k_smooth_density<T>, tiles_x * div_up(s.H, T::TY), 256, 0, s.stream,
+           static_cast<const uint32_t*>(s.lv[0].fluid), s.W, s.H, static_cast<const float*>(s.density), s.sm_a, tiles_x);
+}
+
 cudaError_t launch_build_pressure(Scene& s) {
     const Level& B = s.lv[0];
     uint32_t g = seg_grid(B.words);
-    launch(s.use_pdl, k_smooth_density, g, kSegBlock, 0, s.stream, B.fluid, B.seg, s.ctl, s.W, s.cells, s.density, s.sm_a);
-    launch(s.use_pdl, k_smooth_density, g, kSegBlock, 0, s.stream, B.fluid, B.seg, s.ctl, s.W, s.cells, s.sm_a, s.sm_b);
-    launch(s.use_pdl, k_smooth_density, g, kSegBlock, 0, s.stream, B.fluid, B.seg, s.ctl, s.W, s.cells, s.sm_b, s.sm_a);
+    if (s.cells <= 512u * 512u) smooth_density<SweepTile<32, 8, 3>>(s);
+    else smooth_density<SweepTile<64, 16, 3>>(s);
     launch(s.use_pdl, k_laplacian, g, kSegBlock, 0, s.stream, B.fluid, s.obstacle, B.seg, s.ctl, s.W, s.cells, s.dx, s.u, s.v,
                                                s.sm_a, s.density, B.res, B.diag, B.inv_diag, B.px, B.py);
     return cudaGetLastError();
@@ -765,8 +883,15 @@ cudaError_t launch_multilevel(Scene& s) {
         TailLevels t;
         t.first = l;
         t.n = s.nlevels;
-        for (int k = 0; k < s.nlevels; ++k) t.lv[k] = s.lv[k];
+        uint32_t groups = 0;
+        for (int k = 0; k < s.nlevels; ++k) {
+            t.lv[k] = s.lv[k];
+            if (k + 1 < s.nlevels) groups += div_up(s.lv[k].ntiles, 32);
+        }
+        // up to 512^2 cells: a launch less
+        t.tiles = groups <= kTailTileGroups ? 1 : 0;
         launch(s.use_pdl, k_coarsen_tail, 1, kOneThreads, 0, s.stream, t, s.ctl);
+        if (t.tiles) return cudaGetLastError();
     }
     return launch_tile_lists(s);
 }
@@ -812,11 +937,11 @@ template <class T> static void extrapolate(Scene& s, bool from_alt) {
 // 1024^2 34.8 / 27.7 / 37.4, 4096^2 (noise) 510 / 348 / 350.
 cudaError_t launch_extrapolate(Scene& s) {
     if (s.cells <= 512u * 512u) {
-        extrapolate<ExTile<32, 8, 2>>(s, false);
-        extrapolate<ExTile<32, 8, 2>>(s, true);
+        extrapolate<SweepTile<32, 8, 2>>(s, false);
+        extrapolate<SweepTile<32, 8, 2>>(s, true);
     } else {
-        extrapolate<ExTile<64, 16, 2>>(s, false);
-        extrapolate<ExTile<64, 16, 2>>(s, true);
+        extrapolate<SweepTile<64, 16, 2>>(s, false);
+        extrapolate<SweepTile<64, 16, 2>>(s, true);
     }
     return cudaGetLastError();
 }

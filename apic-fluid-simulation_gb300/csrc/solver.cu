@@ -66,16 +66,6 @@ __global__ void k_pcg_begin(Ctl* ctl) {
 // grid (bk), run by the single-scene kernel with the hardware's and by the
 // batch kernel (one launch over many scenes, batch.h) with the scene's.
 
-// The reference mode's solve starts here: its PCG state and a zero pressure.
-__global__ void __launch_bounds__(kSegBlock) k_reference_start(Level B, float* p, Ctl* ctl) {
-    pdl_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctl->solve_t0 = global_ns();
-        pcg_reset(ctl);
-    }
-    pcg::ph_clear_pressure(B, ctl->seg_count[0], gwarp(), gnwarps(), p);
-}
-
 // Entry of the PCG loop: go on while not converged and under the iteration
 // cap (src/apic.rs:1894-1899); dyn_cap reads the remaining budget of a
 // refinement.  Inside the loop the same decision is taken by the kernel that
@@ -417,11 +407,21 @@ __global__ void __launch_bounds__(kGammaThreads) k_gamma_exact(Level B, Ctl* ctl
 // Fluid cells before each base segment (seg_pre[k], k <= nseg; seg_pre[nseg]
 // = all fluid cells): the position of a segment's cells in the reference's
 // ascending fluid list; and the segment that holds the first cell of each of
-// the chunks of k_delta_exact (chunk_seg).  One block, once per solve, four
-// segments a thread and round.
-__global__ void __launch_bounds__(1024) k_seg_prefix(Level B, const Ctl* ctl, uint32_t* seg_pre, uint32_t* chunk_seg) {
+// the chunks of k_delta_exact (chunk_seg).  The reference mode's solve starts
+// here: block 0 resets the PCG state and counts, four segments a thread and
+// round; the others clear the pressure.
+__global__ void __launch_bounds__(1024) k_reference_start(Level B, float* p, Ctl* ctl, uint32_t* seg_pre,
+                                                          uint32_t* chunk_seg) {
     pdl_wait();
     const uint32_t nseg = ctl->seg_count[0];
+    if (blockIdx.x != 0) {
+        pcg::ph_clear_pressure(B, nseg, (blockIdx.x - 1u) * 32u + (threadIdx.x >> 5), (gridDim.x - 1u) * 32u, p);
+        return;
+    }
+    if (threadIdx.x == 0) {
+        ctl->solve_t0 = global_ns();
+        pcg_reset(ctl);
+    }
     __shared__ uint32_t sw[32];
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     uint32_t carry = 0;
@@ -1030,8 +1030,8 @@ static void enqueue_pcg_start(Scene& s, int mode, bool begin, const LoopEntry& l
     cudaStream_t st = s.stream;
     const bool pdl = s.use_pdl;
     if (mode == APIC_SOLVER_REFERENCE) {
-        launch(pdl, k_reference_start, g, kSegBlock, 0, st, B, s.pressure, s.ctl);
-        launch(pdl, k_seg_prefix, 1, 1024, 0, st, B, static_cast<const Ctl*>(s.ctl), s.seg_pre, chunk_seg(s));
+        launch(pdl, k_reference_start, 1u + std::min(div_up(B.words, 32), 304u), 1024, 0, st, B, s.pressure, s.ctl,
+               s.seg_pre, chunk_seg(s));
     } else if (begin) {
         launch(pdl, k_pcg_begin, 1, 1, 0, st, s.ctl);
     }
