@@ -68,6 +68,7 @@ cudaError_t scratch_for_current_context(uint32_t** out) {
 __global__ void k_keys_from_positions(const float* __restrict__ px, const float* __restrict__ py, uint32_t n,
                                       CellSize cs, float max_x, float max_y, uint32_t* __restrict__ keys,
                                       uint32_t* __restrict__ vals, uint32_t* __restrict__ head) {
+    pdl_wait();
     clear_sort_head(head);
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
