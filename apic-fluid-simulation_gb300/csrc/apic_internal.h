@@ -67,7 +67,7 @@ struct Ctl {
     float alpha;
     float beta;
     uint32_t beta_valid;    // beta belongs to this solve (the search direction is z + beta s)
-    uint32_t delta_stop;    // k_pcg_update found s.Ap unusable; the next kernel turns it into pcg_done
+    uint32_t delta_stop;    // the update found s.Ap unusable; the next kernel turns it into pcg_done
     unsigned long long solve_t0;  // %globaltimer at the start of the running solve (ns)
     unsigned long long solve_ns;  // summed solve time of this update (ns)
     uint32_t max_r_bits;    // max |r| (float bits)

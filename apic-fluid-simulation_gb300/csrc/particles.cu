@@ -1,6 +1,6 @@
 // particles.cu — particle <-> grid transfers on the GPU.
 //
-//   k_p2g       transfer_particles_to_grid's scatter (src/apic.rs:1237-1426):
+//   k_p2g_*     transfer_particles_to_grid's scatter (src/apic.rs:1237-1426):
 //               APIC momentum and weight to the 4 u and 4 v faces, temporal
 //               weight w_t (:1246-1248), cell-centred density (:1260-1284) and
 //               the fluid bit of the particle's cell (:1358-1360).
@@ -12,11 +12,9 @@
 //   k_permute   gather of the nine fields by the sorted `val` (:1068-1110).
 //
 // The reference sums P2G contributions with float CAS loops, so its sums come
-// in thread-schedule order.  Here a CTA first sums its particles'
-// contributions in shared memory (hardware float atomics) over the window of
-// faces and cells they touch, then adds each touched entry to global memory
-// once; both levels are likewise order-dependent at the last bit.  Every other result of these kernels is computed lane by lane with the
-// reference's operation order.
+// in thread-schedule order.  Here every face is summed by one thread in a fixed
+// order (below).  Every other result of these kernels is computed lane by lane
+// with the reference's operation order.
 #include <cuda_runtime.h>
 
 #include <climits>

@@ -245,7 +245,7 @@ __device__ __forceinline__ void loop_decision(Ctl* ctl, int mode, cudaGraphCondi
     if (set_cond) cudaGraphSetConditional(h, cont ? 1u : 0u);
 }
 
-// The exits that k_pcg_update leaves to the next kernel: its delta stop, or
+// The exits that the update leaves to the next kernel: its delta stop, or
 // the residual test on its block parts, max|r| < solve_error (reference
 // mode, src/apic.rs:1929-1932) or ||r|| <= target * ||b||.  Run by one
 // block, after the caller's dependency wait.

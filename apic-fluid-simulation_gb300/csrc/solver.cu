@@ -9,13 +9,14 @@
 // multiple of 8, :1487-1494) and plain CG on the coarsest level
 // (solve_coarse_exact :618-704, one CTA here).
 //
-// Every kernel is a grid-stride loop over the level's segment list whose
-// length lives in device memory, and returns at once when the device-side
+// The kernels walk the level's segment list or its list of fluid tiles, whose
+// lengths live in device memory, and return at once when the device-side
 // `pcg_done` flag is set, so an iteration costs no host round trip.  Dot
-// products accumulate FP32 products in FP64 and are reduced deterministically
-// (per-block partials summed in block order by the last block).  The
-// reference's alpha/beta/gamma are FP32 and so are they here: the FP64 sums
-// are rounded to float before the reference's FP32 divisions.
+// products sum FP32 products in double-float (FP64 in the refinement) and are
+// reduced deterministically: per-block partials, summed in block order by the
+// kernel that needs the total.  The reference's alpha/beta/gamma are FP32 and
+// so are they here: the sums are rounded to float before the reference's FP32
+// divisions.
 //
 // Solver modes: APIC_SOLVER_REFERENCE keeps the reference's exits (max|r| <
 // solve_error, gamma/delta < 1e-5, 100 iterations).  APIC_SOLVER_REL_FP32
@@ -760,7 +761,7 @@ __global__ void __launch_bounds__(kBatCtlThreads) k_bat_pcg_cond(const BScene* _
 // scene's decision.  CTA 0 lists the scenes that go on and sets the loop
 // condition; CTA 1 + i sums scene i's r.z parts (stored by the V-cycle's
 // last kernel) for the next iteration, once instead of in every block of
-// k_spmv_dot and k_pcg_update (the same function of the same parts).
+// k_spmv_dot and k_update_down (the same function of the same parts).
 __global__ void __launch_bounds__(kSegBlock) k_bat_round_end(const BScene* __restrict__ tab, uint32_t n, BCtl* bc,
                                                             cudaGraphConditionalHandle h, BListRef l3) {
     pdl_wait();

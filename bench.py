@@ -397,7 +397,7 @@ def run_gpu_arm(args, world, rank, local):
                        "true_residual_rel_max": max(true_res) if true_res else None,
                        "l2": "flushed (256 MB write) between timed steps", "parallelism": f"replicas x{world}",
                        "solve_form": "graph of per-phase kernels",
-                       "vcycle": "one kernel per sweep and transfer" + (
+                       "vcycle": "two tile kernels per level (down, up)" + (
                            "; coarse levels in one cluster's distributed shared memory" if dsm else ""),
                        "launch": ("stage by stage" if args.eager else "one CUDA graph per update")
                        + ("" if args.no_pdl else "; programmatic dependent launch in the PCG loop")},
@@ -557,8 +557,8 @@ def roofline(iters, solve_ms, steps, counts, peak, peak_kind):
     achieved = per_iter * iters / sec / 1e9
     traffic = solve_traffic()
     return {"bound": "hbm", "kernel": "pressure solve: MG-preconditioned CG (per iteration k_spmv_dot, "
-                                      "k_pcg_update, k_smooth_exit, the V-cycle's sweep and transfer kernels, "
-                                      "k_vcycle_dsm, k_prolong_red_rz)",
+                                      "k_update_down, the V-cycle's tile kernels k_down and k_up, "
+                                      "k_vcycle_dsm)",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
             "traffic": traffic, "traffic_unit": "DRAM bytes per PCG iteration" if traffic else None,
             "algorithmic_bytes_per_iteration": per_iter, "iterations": iters,
@@ -705,7 +705,8 @@ def run_batched(args, world=1, rank=0, local=0):
                              "block_group": chosen["block_group"],
                              "how": "the library's batch tuner: the first calls for this makeup of scenes try the "
                                     "stream-per-scene form and the joint form with 12 shapes, each twice, cost = "
-                                    "wall time per PCG iteration over all scenes; the lowest mean cost is kept"},
+                                    "wall time per PCG iteration over all scenes; the lowest mean cost is kept "
+                                    "(three shapes only where each costs more than 1.5 times the streams)"},
                    "cuda_device_max_connections": os.environ.get("CUDA_DEVICE_MAX_CONNECTIONS", "8 (default)"),
                    "dsm_vcycle": not args.no_dsm},
         "batched_vs_plain": {"updates_compared": cmp_steps, "batched": sub_cmp / cmp_s, "plain": sub_plain / plain_s,
