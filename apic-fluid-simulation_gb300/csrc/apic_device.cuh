@@ -552,39 +552,4 @@ __device__ __forceinline__ void sum_max_partials(const float4* part, uint32_t n,
     }
 }
 
-// Same pattern for a maximum of non-negative values (exact in any order).
-template <int kThreads>
-__device__ __forceinline__ bool block_max_last(float v, double* partials, uint32_t* counter, float* total) {
-    __shared__ float s_m[kThreads / 32];
-    __shared__ bool s_last;
-    v = warp_maxf(v);
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) s_m[warp] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float b = 0.0f;
-        for (int w = 0; w < kThreads / 32; ++w) b = fmaxf(b, s_m[w]);
-        partials[blockIdx.x] = double(b);
-        __threadfence();
-        s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_last) return false;
-    __threadfence();
-    const volatile double* vp = partials;
-    float t = 0.0f;
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += kThreads) t = fmaxf(t, float(vp[b]));
-    t = warp_maxf(t);
-    __syncthreads();
-    if (lane == 0) s_m[warp] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float a = 0.0f;
-        for (int w = 0; w < kThreads / 32; ++w) a = fmaxf(a, s_m[w]);
-        *total = a;
-        *counter = 0;
-    }
-    return true;
-}
-
 }  // namespace apic

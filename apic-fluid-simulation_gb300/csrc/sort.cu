@@ -37,7 +37,6 @@ namespace {
 constexpr uint32_t kMaxBuckets = 1u << kMaxDigitBits;
 constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr uint32_t kMaxPasses = 4;
 // Scratch words in front of the tiles' published counts: every digit's
 // histogram (passes * buckets <= 3072) and a tile counter per pass.
 constexpr uint32_t kSortHead = kSortHeadWords;
