@@ -257,6 +257,7 @@ struct Scene {
     uint32_t max_iter = 500;
     bool vmax_valid = false;
     bool world_ready = false;
+    bool masks_written = false;  // a caller wrote u_open / v_open since they were formed from the obstacles
     bool has_ext = false, has_post = false;
 
     // measurement

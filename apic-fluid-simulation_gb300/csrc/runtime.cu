@@ -363,6 +363,7 @@ int upload_world(apic_handle* h) {
     CK(cudaMemcpyAsync(s.u_open, uo.data(), sizeof(uint32_t) * uo.size(), cudaMemcpyHostToDevice, s.stream));
     CK(cudaMemcpyAsync(s.v_open, vo.data(), sizeof(uint32_t) * vo.size(), cudaMemcpyHostToDevice, s.stream));
     s.world_ready = true;
+    s.masks_written = false;
     return APIC_OK;
 }
 
@@ -1177,6 +1178,7 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
     CK(cudaMemcpy(d.dev, src, bytes, cudaMemcpyHostToDevice));
     if (field == APIC_F_VEL_X || field == APIC_F_VEL_Y) s.vmax_valid = false;
     if (field == APIC_F_PRESSURE) s.p64_valid = false;
+    if (field == APIC_F_U_OPEN_BITS || field == APIC_F_V_OPEN_BITS) s.masks_written = true;
     if (field == APIC_F_OBSTACLE_BITS) {
         std::memcpy(h->obstacle_host.data(), src, bytes);
         int rc = upload_world(h);
@@ -1435,8 +1437,10 @@ int apic_restore(apic_handle* h, const void* src, uint64_t bytes) {
         if ((rc = reset_tables(s))) return rc;
     }
     uint64_t off = uint64_t(NPF) * hd.lanes * 4;
+    // the obstacles and the open-face masks that follow from them, where the
+    // snapshot's differ from the scene's or a caller wrote masks of its own
     const uint64_t obst = uint64_t(hd.obstacle_words) * 8;
-    if (std::memcmp(h->obstacle_host.data(), in + off, obst) != 0) {
+    if (s.masks_written || std::memcmp(h->obstacle_host.data(), in + off, obst) != 0) {
         std::memcpy(h->obstacle_host.data(), in + off, obst);
         if ((rc = upload_world(h))) return rc;
     }
