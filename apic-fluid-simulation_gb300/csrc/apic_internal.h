@@ -326,7 +326,7 @@ cudaError_t radix_sort_pairs_digits(uint32_t* keys, uint32_t* vals, uint32_t* ke
 bool radix_sort_in_alt(int bits);     // radix_sort_pairs over `bits` bits ends in the alt buffers
 int sort_digit_bits(int bits);        // ... its digit width
 uint32_t sort_scratch_words(uint32_t n, int bits, int dbits);
-uint32_t sort_scratch_words(const Scene& s, uint32_t n);  // enough for the scene's two sorts
+uint32_t sort_scratch_words(const Scene& s, uint32_t n);  // enough for the scene's two sorts of up to n pairs
 int bin_key_bits(const Scene& s);
 bool sort_result_in_alt(const Scene& s);  // where launch_sort leaves the Morton-sorted pairs
 int morton_key_bits(uint32_t width, uint32_t height);

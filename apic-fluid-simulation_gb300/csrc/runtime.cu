@@ -367,9 +367,12 @@ int upload_world(apic_handle* h) {
     return APIC_OK;
 }
 
-int alloc_particles(Scene& s, uint32_t npad, uint32_t n) {
+// Particle buffers for npad lanes.  Every buffer, the sort's scratch too, is
+// sized by the capacity, so a set that fits allocates nothing.
+int alloc_particles(Scene& s, uint32_t npad) {
     if (npad <= s.part_cap && s.part_cap > 0) return APIC_OK;
     free_particles(s);
+    s.n = s.nchunks = s.npad = 0;  // what the scene holds should an allocation fail
     const cudaStream_t st = s.stream;
     for (int f = 0; f < NPF; ++f) {
         CK(dalloc(&s.part[f], npad, st));
@@ -379,7 +382,7 @@ int alloc_particles(Scene& s, uint32_t npad, uint32_t n) {
     CK(dalloc(&s.keys_alt, npad, st)); CK(dalloc(&s.vals_alt, npad, st));
     CK(dalloc(&s.bin_keys, npad, st)); CK(dalloc(&s.bin_vals, npad, st));
     CK(dalloc(&s.bin_keys_alt, npad, st)); CK(dalloc(&s.bin_vals_alt, npad, st));
-    CK(dalloc(&s.sort_scratch, sort_scratch_words(s, n), st));
+    CK(dalloc(&s.sort_scratch, sort_scratch_words(s, npad), st));
     s.part_cap = npad;
     return APIC_OK;
 }
@@ -396,13 +399,8 @@ int reset_tables(Scene& s) {
 int load_particles(apic_handle* h, uint32_t n, const float* px, const float* py, const float* vx, const float* vy) {
     Scene& s = h->s;
     uint32_t nchunks = (n + 7) / 8, npad = nchunks * 8;
-    int rc = alloc_particles(s, npad, n);
+    int rc = alloc_particles(s, npad);
     if (rc != APIC_OK) return rc;
-    // sort scratch may need to grow when n grows within the same capacity
-    if (n != s.n) {
-        dfree(s.sort_scratch, s.stream);
-        CK(dalloc(&s.sort_scratch, sort_scratch_words(s, n), s.stream));
-    }
     // a new particle set: the next mixed solve starts from zero pressure
     if (s.p64) CK(cudaMemsetAsync(s.p64, 0, sizeof(double) * (uint64_t(s.cells) + 2ull * s.W), s.stream));
     // the given numbers straight from the caller's arrays (pageable memory is

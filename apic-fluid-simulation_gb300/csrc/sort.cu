@@ -383,7 +383,8 @@ static int digit_bits(int bits) {
 
 // Tile size of a sort: small sorts take small tiles, for which the look-back
 // is short and more SMs work; from 256 K pairs on 4096 pairs a tile.
-static int tile_items(uint32_t n) { return n <= 65536u ? 2 : n <= 262144u ? 4 : 8; }
+constexpr uint32_t kTile2Pairs = 65536u, kTile4Pairs = 262144u;
+static int tile_items(uint32_t n) { return n <= kTile2Pairs ? 2 : n <= kTile4Pairs ? 4 : 8; }
 static uint32_t sort_tiles(uint32_t n) { return div_up(n, uint32_t(tile_items(n)) * kSortThreads); }
 static int sort_passes(int bits, int dbits) { return dbits > 0 ? (bits + dbits - 1) / dbits : 0; }
 static size_t pass_smem(int items, int dbits) {
@@ -434,7 +435,11 @@ uint32_t sort_scratch_words(uint32_t n, int bits, int dbits) {
 }
 uint32_t sort_scratch_words(const Scene& s, uint32_t n) {
     const int m = key_bits(s), b = bin_key_bits(s);
-    return std::max(sort_scratch_words(n, m, digit_bits(m)), sort_scratch_words(n, b, digit_bits(b)));
+    uint32_t words = 0;
+    // (the largest counts of each tile size: fewer pairs may make more tiles)
+    for (uint32_t k : {n, std::min(n, kTile2Pairs), std::min(n, kTile4Pairs)})
+        words = std::max({words, sort_scratch_words(k, m, digit_bits(m)), sort_scratch_words(k, b, digit_bits(b))});
+    return words;
 }
 
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* scratch,
