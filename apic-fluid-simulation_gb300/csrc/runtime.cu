@@ -1163,16 +1163,17 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
     Scene& s = h->s;
     CK(cudaStreamSynchronize(s.stream));
     PartPtrs pp = read_ptrs(s);
-    if (field == APIC_F_RESIDUAL) {  // a solve starts from the first buffer
-        CK(cudaMemset(&s.ctl->res_sel, 0, sizeof(uint32_t)));
-        s.ctl_host->res_sel = 0;
-    }
     FieldDesc d = describe(h, field, &pp);
     if (!d.ok || field == APIC_F_FLUID_LIST || field == APIC_F_SORT_KEYS || field == APIC_F_SORT_VALS)
         return fail(APIC_ERR_INVALID_ARG, "field not writable: " + std::to_string(field));
     if (bytes != d.count * d.elem) return fail(APIC_ERR_INVALID_ARG, "size mismatch");
     if (bytes == 0) return APIC_OK;
     if (!src) return fail(APIC_ERR_INVALID_ARG, "null source");
+    if (field == APIC_F_RESIDUAL) {  // a solve starts from the first buffer
+        CK(cudaMemset(&s.ctl->res_sel, 0, sizeof(uint32_t)));
+        s.ctl_host->res_sel = 0;
+        d = describe(h, field, &pp);
+    }
     CK(cudaMemcpy(d.dev, src, bytes, cudaMemcpyHostToDevice));
     if (field == APIC_F_VEL_X || field == APIC_F_VEL_Y) s.vmax_valid = false;
     if (field == APIC_F_PRESSURE) s.p64_valid = false;
