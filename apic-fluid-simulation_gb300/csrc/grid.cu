@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(256) k_extrapolate(ExField fu, ExField fv, int
         if (gx >= 0 && gx < F.w && gy >= 0 && gy < F.h) {
             const size_t g = size_t(gy) * F.w + gx;
             v = F.in[g];
-            k = F.in_ok[g];
+            k = F.in_ok[g] != 0;  // (a caller may have written any byte; a sweep writes 1)
             some = some || k;
             all = all && k;
         }
