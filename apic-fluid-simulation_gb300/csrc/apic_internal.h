@@ -258,6 +258,7 @@ struct Scene {
     bool vmax_valid = false;
     bool world_ready = false;
     bool masks_written = false;  // a caller wrote u_open / v_open since they were formed from the obstacles
+    bool mg_written = false;     // a caller wrote a coarse level's mask or coefficients
     bool has_ext = false, has_post = false;
 
     // measurement
@@ -354,7 +355,7 @@ cudaError_t launch_post_forces(Scene& s);
 cudaError_t launch_extrapolate(Scene& s);
 cudaError_t launch_smoothed_view(Scene& s, float* out);
 cudaError_t launch_level_lists(Scene& s, int level);
-cudaError_t launch_mask_level(Scene& s, int level);  // zero a coarse level's coefficients outside its fluid
+cudaError_t launch_mask_level(Scene& s, int level);  // zero a coarse level's coefficients that touch no fluid pair
 cudaError_t launch_tile_lists(Scene& s);  // every level's fluid tiles
 // solver.cu: the solve is recorded into graphs (apic_graph.h: build_solve)
 // solver.cu: the same solve launched kernel by kernel with host loop control

@@ -409,14 +409,18 @@ __device__ __forceinline__ void coarsen_word(const Level& f, const Level& c, uin
 }
 
 // The same zeros on a coarse level whose mask or coefficients a caller wrote
-// (padding included).
+// (padding included), and no coupling from a fluid cell to one that is not.
 __global__ void __launch_bounds__(256) k_mask_level(Level c) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.padded || fluid_raw(c.fluid, (long long)i - c.w, c.cells)) return;
-    c.diag[i] = 0.0f;
-    c.inv_diag[i] = 0.0f;
-    c.px[i] = 0.0f;
-    c.py[i] = 0.0f;
+    if (i >= c.padded) return;
+    const long long raw = (long long)i - c.w;
+    const bool on = fluid_raw(c.fluid, raw, c.cells) != 0;
+    if (!on) {
+        c.diag[i] = 0.0f;
+        c.inv_diag[i] = 0.0f;
+    }
+    if (!on || !fluid_raw(c.fluid, raw + 1, c.cells)) c.px[i] = 0.0f;
+    if (!on || !fluid_raw(c.fluid, raw + c.w, c.cells)) c.py[i] = 0.0f;
 }
 
 // One coarse level from its finer level: one warp per coarse mask word.

@@ -554,6 +554,25 @@ float bits_to_float(uint32_t b) {
     return f;
 }
 
+// A V-cycle's stage on levels that a caller wrote.  The kernels that hold levels
+// in shared memory take every cell of them, which is right for the levels that
+// the setup builds (zero coefficients outside the fluid, no coupling out of it, no
+// coarse cell left out whose finer cells are fluid).  Here the tile kernels, which
+// ask the mask, take every level but the coarsest, and the levels' errors start at
+// zero, as the reference's do.
+template <class F> int on_written_levels(Scene& s, F run) {
+    if (!s.mg_written) return run();
+    for (int l = 1; l < s.nlevels; ++l) CK(cudaMemsetAsync(s.lv[l].err, 0, sizeof(float) * s.lv[l].padded, s.stream));
+    const int tail = s.tail_first;
+    const bool dsm = s.use_dsm;
+    s.tail_first = s.nlevels;
+    s.use_dsm = false;
+    const int rc = run();
+    s.tail_first = tail;
+    s.use_dsm = dsm;
+    return rc;
+}
+
 int valid_handle(apic_handle* h) {
     if (!h) return fail(APIC_ERR_INVALID_ARG, "null handle");
     return APIC_OK;
@@ -1189,6 +1208,7 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
         CK(cudaStreamSynchronize(s.stream));
     }
     if (field >= APIC_F_MG_FLUID_BITS) {
+        s.mg_written = true;
         const int level = field / APIC_F_MG_LEVEL_STRIDE + 1;
         CK(launch_mask_level(s, level));
         if (field % APIC_F_MG_LEVEL_STRIDE == APIC_F_MG_FLUID_BITS) {
@@ -1641,12 +1661,18 @@ int apic_debug_run_stage(apic_handle* h, int stage, float dt) {
             break;
         case APIC_STAGE_FORCES: CK(launch_external_forces(s)); break;
         case APIC_STAGE_BUILD: CK(launch_base_lists(s)); CK(launch_build_pressure(s)); break;
-        case APIC_STAGE_MG: CK(launch_base_lists(s)); CK(launch_multilevel(s)); break;
+        case APIC_STAGE_MG:
+            CK(launch_base_lists(s));
+            CK(launch_multilevel(s));
+            s.mg_written = false;
+            break;
         case APIC_STAGE_PCG: {
             k_begin_update<<<1, 1, 0, st>>>(s.ctl, 0.0f, 0u, s.has_ext ? 1u : 0u, s.has_post ? 1u : 0u);
             k_set_dt<<<1, 1, 0, st>>>(s.ctl, dt, s.has_ext ? 1u : 0u, s.has_post ? 1u : 0u);
-            CK(run_solve_eager(s));
-            int rc = sync_ctl(s);
+            int rc = on_written_levels(s, [&]() -> int {
+                CK(run_solve_eager(s));
+                return sync_ctl(s);
+            });
             if (rc) return rc;
             const Ctl& c = *s.ctl_host;
             s.stats.pcg_iterations = c.pcg_iters;
@@ -1667,8 +1693,12 @@ int apic_debug_run_stage(apic_handle* h, int stage, float dt) {
         case APIC_STAGE_VMAX: CK(launch_vmax(s)); s.vmax_valid = true; break;
         case APIC_STAGE_VCYCLE:
             k_begin_update<<<1, 1, 0, st>>>(s.ctl, 0.0f, 0u, 0u, 0u);  // clears the solve's done flag
-            enqueue_vcycle(s);
-            CK(cudaGetLastError());
+            if (int rc = on_written_levels(s, [&]() -> int {
+                    enqueue_vcycle(s);
+                    CK(cudaGetLastError());
+                    return APIC_OK;
+                }))
+                return rc;
             break;
         default: return fail(APIC_ERR_INVALID_ARG, "unknown stage");
     }

@@ -305,9 +305,9 @@ void plan_vcycle(Scene& s) {
     if (s.tail_first < s.nlevels) {
         s.tail_smem = bytes;
         cudaFuncSetAttribute(k_vcycle_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTailSmemBudget));
-    } else {
-        cudaFuncSetAttribute(k_coarse_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoarseSmemBudget));
     }
+    // (also where the tail holds every level: levels that a caller wrote take this kernel)
+    cudaFuncSetAttribute(k_coarse_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoarseSmemBudget));
     plan_vcycle_dsm(s);
 }
 
