@@ -355,7 +355,7 @@ cudaError_t launch_post_forces(Scene& s);
 cudaError_t launch_extrapolate(Scene& s);
 cudaError_t launch_smoothed_view(Scene& s, float* out);
 cudaError_t launch_level_lists(Scene& s, int level);
-cudaError_t launch_mask_level(Scene& s, int level);  // zero a coarse level's coefficients that touch no fluid pair
+cudaError_t launch_mask_level(Scene& s, int level);  // zero a level's coefficients outside its fluid and out of it
 cudaError_t launch_tile_lists(Scene& s);  // every level's fluid tiles
 // solver.cu: the solve is recorded into graphs (apic_graph.h: build_solve)
 // solver.cu: the same solve launched kernel by kernel with host loop control

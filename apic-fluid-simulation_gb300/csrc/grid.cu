@@ -408,8 +408,9 @@ __device__ __forceinline__ void coarsen_word(const Level& f, const Level& c, uin
     c.py[cp] = py * 0.5f;
 }
 
-// The same zeros on a coarse level whose mask or coefficients a caller wrote
-// (padding included), and no coupling from a fluid cell to one that is not.
+// The same zeros on a coarsest level whose mask or coefficients a caller wrote
+// (padding included), and no coupling from a fluid cell to one that is not: its
+// CG runs over all cells too.
 __global__ void __launch_bounds__(256) k_mask_level(Level c) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.padded) return;

@@ -558,18 +558,39 @@ float bits_to_float(uint32_t b) {
 // in shared memory take every cell of them, which is right for the levels that
 // the setup builds (zero coefficients outside the fluid, no coupling out of it, no
 // coarse cell left out whose finer cells are fluid).  Here the tile kernels, which
-// ask the mask, take every level but the coarsest, and the levels' errors start at
-// zero, as the reference's do.
+// ask the mask, take every level but the coarsest, whose coefficients are masked
+// for the stage and given back as they were written; and the levels' errors start
+// at zero, as the reference's do.
 template <class F> int on_written_levels(Scene& s, F run) {
     if (!s.mg_written) return run();
     for (int l = 1; l < s.nlevels; ++l) CK(cudaMemsetAsync(s.lv[l].err, 0, sizeof(float) * s.lv[l].padded, s.stream));
+    const Level& C = s.lv[s.nlevels - 1];
+    float* const coeff[] = {C.diag, C.inv_diag, C.px, C.py};
+    float* kept = nullptr;
+    if (dalloc(&kept, 4 * size_t(C.padded), s.stream) != cudaSuccess)
+        return fail(APIC_ERR_OOM, "out of device memory (coarse coefficients)");
+    auto copy = [&](bool back) -> int {
+        for (int k = 0; k < 4; ++k) {
+            float* at = kept + size_t(k) * C.padded;
+            CK(cudaMemcpyAsync(back ? coeff[k] : at, back ? at : coeff[k], sizeof(float) * C.padded,
+                               cudaMemcpyDeviceToDevice, s.stream));
+        }
+        return APIC_OK;
+    };
     const int tail = s.tail_first;
     const bool dsm = s.use_dsm;
-    s.tail_first = s.nlevels;
-    s.use_dsm = false;
-    const int rc = run();
-    s.tail_first = tail;
-    s.use_dsm = dsm;
+    int rc = copy(false);
+    if (rc == APIC_OK && launch_mask_level(s, s.nlevels - 1) != cudaSuccess) rc = fail(APIC_ERR_CUDA, "coarse mask");
+    if (rc == APIC_OK) {
+        s.tail_first = s.nlevels;
+        s.use_dsm = false;
+        rc = run();
+        s.tail_first = tail;
+        s.use_dsm = dsm;
+        const int back = copy(true);
+        if (rc == APIC_OK) rc = back;
+    }
+    dfree(kept, s.stream);
     return rc;
 }
 
@@ -1209,13 +1230,11 @@ int apic_write_field(apic_handle* h, int field, const void* src, uint64_t bytes)
     }
     if (field >= APIC_F_MG_FLUID_BITS) {
         s.mg_written = true;
-        const int level = field / APIC_F_MG_LEVEL_STRIDE + 1;
-        CK(launch_mask_level(s, level));
         if (field % APIC_F_MG_LEVEL_STRIDE == APIC_F_MG_FLUID_BITS) {
-            CK(launch_level_lists(s, level));
+            CK(launch_level_lists(s, field / APIC_F_MG_LEVEL_STRIDE + 1));
             CK(launch_tile_lists(s));
+            CK(cudaStreamSynchronize(s.stream));
         }
-        CK(cudaStreamSynchronize(s.stream));
     }
     if (field == APIC_F_EXT_FORCE_U || field == APIC_F_EXT_FORCE_V) s.has_ext = true;
     if (field == APIC_F_POST_FORCE_U || field == APIC_F_POST_FORCE_V) s.has_post = true;

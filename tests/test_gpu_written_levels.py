@@ -71,3 +71,30 @@ def test_written_masks(gpu_lib, w, h):
     g.run_stage("vcycle", 1 / 1000)
     fl = fluid_padded(g)
     eq(g.read_field("error")[fl], want[fl], "z")
+
+
+@pytest.mark.parametrize("w,h", GRIDS)
+def test_coefficients_before_masks(gpu_lib, w, h):
+    """The order of the writes does not matter, and what was written stays, also
+    outside the mask and after a V-cycle."""
+    if A.device_count() == 0:
+        pytest.skip("no CUDA device")
+    g, rng = make(w, h), np.random.default_rng(2)
+    built = read_levels(g, w, h)
+    for l, (bits, _) in enumerate(built):  # a first mask without any cell
+        g.write_field(A.mg_field("fluid_bits", l), np.zeros_like(bits))
+    for l, (bits, co) in enumerate(built):
+        lw, lh = sides(w, h, l)
+        out = ~V.Level(lw, lh, bits, *(co[n] for n in NAMES)).on
+        for n in NAMES:  # values outside the mask that nothing may read
+            co[n] = np.where(out, rng.uniform(1, 2, co[n].size), co[n]).astype(np.float32)
+            g.write_field(A.mg_field(n, l), co[n])
+        g.write_field(A.mg_field("fluid_bits", l), bits)
+    want = expected(g, w, h, built)
+    g.run_stage("vcycle", 1 / 1000)
+    fl = fluid_padded(g)
+    eq(g.read_field("error")[fl], want[fl], "z")
+    for l, (bits, co) in enumerate(built):
+        eq(g.read_field(A.mg_field("fluid_bits", l)), bits, f"level {l} mask")
+        for n in NAMES:
+            eq(g.read_field(A.mg_field(n, l)), co[n], f"level {l} {n}")
