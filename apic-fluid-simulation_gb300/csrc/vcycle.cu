@@ -94,7 +94,9 @@ __global__ void __launch_bounds__(kTileBlock, 4) k_down(Level f, Level c, int lf
     tile::DownRegs g;
     if (bk.id < count) tile::down_load_const<kAll>(f, id, g);
     pdl_wait();
-    if (ctl->pcg_done) return;
+    // (block 0 may be writing the flag: the block's threads must agree on it, or
+    // some would sweep a tile that others have left)
+    if (exit.on ? __syncthreads_or(ctl->pcg_done != 0) != 0 : ctl->pcg_done != 0) return;
     kb_down<kAll>(bk, f, c, sh, g, id, count, lf == 0 ? pcg::cur_res(f, ctl) : f.res);
 }
 
