@@ -64,7 +64,7 @@ __device__ __forceinline__ float prolonged(float e, float ec, uint32_t reps) {
 
 // ---- the coarsest level's CG -------------------------------------------------
 
-// Sum (double-float) and a vote over the first `nwarps` warps of the CTA,
+// Sum, rounded to FP32, and a vote over the first `nwarps` warps of the CTA,
 // returned to each of their threads: a shuffle tree per warp, one barrier of
 // those warps, and the same tree over the warps' results in every warp, so
 // no second barrier broadcasts it.  sh: one slot per warp; two calls in a row
@@ -72,34 +72,77 @@ __device__ __forceinline__ float prolonged(float e, float ec, uint32_t reps) {
 // readers of the first from its next writers).  A CG iteration is bound by the latency of
 // its two sums.  In FP64, with every warp adding all warps' doubles, GB300's
 // FP64 rate bound them: a PCG iteration of a 216^2 scene (27^2 coarsest
-// cells) took 70.7 us, of a 488^2 one (61^2) 76.7, and now 48 and 59.  A
-// double-float holds 48 bits of a sum that is rounded to 24: over 2700 random
-// sums of 9 to 9375 products its rounded value was the FP64 sum's every time.
+// cells) took 70.7 us, of a 488^2 one (61^2) 76.7, and 48 and 59 with
+// double-float sums.  A double-float holds 48 bits where FP64 holds 53, so the
+// result is checked: where the sum could round to another float within its
+// error bound, or is not finite (a double-float overflows to NaN), the terms are
+// summed again in FP64: one in some 5000 sums of random squares, one in 100 of
+// random terms of both signs, and no rounded sum of 83000 was wrong.  The check
+// takes 0.2 us of an iteration with 27^2 coarsest cells (33.5 -> 33.7), 0.8 with
+// 61^2 (41.5 -> 42.3) and 2.6 with 125 x 75 (62.0 -> 64.5).
 struct CgSlot {
     float4 w[32];
 };
 __device__ __forceinline__ void cg_bar(uint32_t nwarps) {
     asm volatile("bar.sync 1, %0;" ::"r"(nwarps * 32u) : "memory");
 }
-// any: whether it holds in any thread (kAny).
-template <bool kAny>
-__device__ __forceinline__ float cg_reduce(F2 v, bool& any, CgSlot& sh, uint32_t nwarps) {
+// The sum in FP64 of a, or a b, over the cells of each thread (r, r + threads,
+// ...: those it wrote itself) that bits holds; every thread of the warps takes part.
+static __device__ __noinline__ float cg_sum64(const float* a, const float* b, const uint32_t* bits, uint32_t cells,
+                                              double* wide, uint32_t nwarps) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double t = 0.0;
+    for (uint32_t r = threadIdx.x; r < cells; r += nwarps * 32u)
+        if (bit_at(bits, r)) t += double(b ? a[r] * b[r] : a[r]);
+    t = warp_sum(t);
+    if (lane == 0) wide[warp] = t;
+    cg_bar(nwarps);
+    return float(warp_sum(lane < nwarps ? wide[lane] : 0.0));
+}
+// A thread's terms of a sum: their double-float sum and, where they may have both
+// signs, the sum of their magnitudes.
+struct CgTerms {
+    F2 v{0.0f, 0.0f};
+    float mag = 0.0f;
+    template <bool kSigned> __device__ __forceinline__ void add(float q) {
+        v = f2_add(v, q);
+        if (kSigned) mag += fabsf(q);
+    }
+    template <bool kSigned> __device__ __forceinline__ void set(float q) {
+        v = F2{q, 0.0f};
+        if (kSigned) mag = fabsf(q);
+    }
+};
+// any: whether it holds in any thread (kAny).  eps: the error bound of a sum, in
+// units of its terms' magnitudes (bounded by the largest of a thread's times
+// the threads: two votes instead of ten shuffles); sum64(): the sum in FP64.
+// exact: only the vote counts.
+template <bool kAny, bool kSigned, class Sum64>
+__device__ __forceinline__ float cg_reduce(const CgTerms& t, bool& any, CgSlot& sh, uint32_t nwarps, float eps,
+                                           bool exact, Sum64 sum64) {
+    F2 v = t.v;
+    float mag = t.mag;
+    if (kSigned) mag = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mag)));
     v = warp_sum(v);
     if (kAny) any = __any_sync(0xffffffffu, any);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) sh.w[warp] = make_float4(v.hi, v.lo, kAny && any ? 1.0f : 0.0f, 0.0f);
+    if (lane == 0) sh.w[warp] = make_float4(v.hi, v.lo, kAny && any ? 1.0f : 0.0f, mag);
     cg_bar(nwarps);
     // (up to 8 warps: four copies of their results, three levels of the tree)
     const uint32_t from = nwarps <= 8u ? lane & 7u : lane;
     const float4 q = from < nwarps ? sh.w[from] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     v = F2{q.x, q.y};
+    if (kSigned) mag = float(nwarps * 32u) * __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(q.w)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         if (o > 4 && nwarps <= 8u) continue;
         v = f2_add(v, F2{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
     }
     if (kAny) any = __any_sync(0xffffffffu, q.z != 0.0f);
-    return v.hi;  // (the rounded value of a normalised double-float)
+    // (the same in every warp: the same values through the same tree)
+    const float e = eps * (kSigned ? mag : v.hi), up = v.hi + (v.lo + e), down = v.hi + (v.lo - e);
+    if (up == down || exact) return up;
+    return sum64();
 }
 
 // The reference solver mode's sums (solve_coarse_exact, :627-629, :660,
@@ -147,6 +190,7 @@ constexpr uint32_t kCgMaxK = 10;  // cells per thread held in registers
 // term that the reference skips adds zero.
 struct CgShared {
     CgSlot slot[2];
+    double wide[32];
     float dot;
     uint32_t pre[32 * kCgMaxK];  // exact: fluid cells before each mask word
 };
@@ -210,8 +254,21 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
     // r.r first: where it is below the exit, as in many V-cycles of a relative
     // solve, nothing else is needed.  The directions are zero outside the
     // fluid and in the padding.
-    F2 g{0.0f, 0.0f};
+    CgTerms g;
     bool more = false;
+    // a double-float add errs by at most 5 * 2^-48 of its operands' magnitudes;
+    // a thread adds its cells, the two trees add ten times
+    const float eps = float((K > 0 ? uint32_t(K) : cells / threads) + 16u) * 0x1p-45f;
+    // (cells in registers put their terms into cap, which only the exact sums use)
+    auto rr64 = [&]() {
+        if constexpr (K == 0) return cg_sum64(A.cr + W, A.cr + W, A.bits, cells, sh.wide, nwarps);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+            if (r < cells) A.cap[r] = rv[k] * rv[k];
+        }
+        return cg_sum64(A.cap, nullptr, A.bits, cells, sh.wide, nwarps);
+    };
     if (exact && K > 0) cg_bar(nwarps);  // sh.pre
     for (uint32_t c = threadIdx.x; c < 2u * W; c += threads) A.cs[c < W ? c : cells + c] = 0.0f;
     if constexpr (K > 0) {
@@ -223,7 +280,8 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
             A.cs[r + W] = rv[k];
             const float q = rv[k] * rv[k];
             if (exact) stage(r, q);
-            g = K == 1 ? F2{q, 0.0f} : f2_add(g, q);
+            if constexpr (K == 1) g.template set<false>(q);
+            else g.template add<false>(q);
         }
     } else {
         for (uint32_t r = threadIdx.x; r < cells; r += threads) {
@@ -232,14 +290,14 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
             A.err[c] = 0.0f;
             A.cr[c] = q;
             A.cs[c] = q;
-            g = f2_add(g, q * q);
+            g.template add<false>(q * q);
         }
     }
     float gamma;
     if (exact)
         gamma = K > 0 ? serial() : serial_cells(A.cr, A.cr);
     else
-        gamma = cg_reduce<false>(g, more, sh.slot[0], nwarps);
+        gamma = cg_reduce<false, false>(g, more, sh.slot[0], nwarps, eps, exact, rr64);
     uint32_t max_it = 0;
     if (!(gamma < 1e-12f)) {
         if (!exact) count();
@@ -255,7 +313,7 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
     }
     for (uint32_t it = 0; it < max_it; ++it) {
         // (the directions are visible: a barrier follows their update)
-        F2 dsum{0.0f, 0.0f};
+        CgTerms dsum;
         if constexpr (K == 1) {
             float q = 0.0f;
             if (threadIdx.x < cells) {
@@ -265,7 +323,7 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
                 q = sc * av[0];
                 if (exact) stage(threadIdx.x, q);
             }
-            dsum = F2{q, 0.0f};
+            dsum.template set<true>(q);
         } else if constexpr (K > 1) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
@@ -277,7 +335,7 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
                 av[k] = v;
                 const float q = sc * v;
                 if (exact) stage(r, q);
-                dsum = f2_add(dsum, q);
+                dsum.template add<true>(q);
             }
         } else {
             for (uint32_t r = threadIdx.x; r < cells; r += threads) {
@@ -286,18 +344,26 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
                 const float sc = A.cs[c];
                 const float v = apply(c, A.diag[c], sc, A.px[c], A.px[c - 1], A.py[c], A.py[c - W]);
                 A.cap[c] = v;
-                dsum = f2_add(dsum, sc * v);
+                dsum.template add<true>(sc * v);
             }
         }
         float delta;
         if (exact)
             delta = K > 0 ? serial() : serial_cells(A.cs, A.cap);
         else
-            delta = cg_reduce<false>(dsum, more, sh.slot[1], nwarps);
+            delta = cg_reduce<false, true>(dsum, more, sh.slot[1], nwarps, eps, false, [&]() {
+                if constexpr (K == 0) return cg_sum64(A.cs + W, A.cap + W, A.bits, cells, sh.wide, nwarps);
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const uint32_t r = threadIdx.x + uint32_t(k) * threads;
+                    if (r < cells) A.cap[r] = A.cs[r + W] * av[k];
+                }
+                return cg_sum64(A.cap, nullptr, A.bits, cells, sh.wide, nwarps);
+            });
         if (fabsf(delta) < 1e-5f) break;
         const float alpha = gamma / delta;
         more = false;  // some |r| is not below the exit (max|r| < 1e-6)
-        F2 ng{0.0f, 0.0f};
+        CgTerms ng;
         if constexpr (K > 0) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
@@ -308,7 +374,8 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
                 more = more || fabsf(rv[k]) >= 1e-6f;
                 const float q = rv[k] * rv[k];
                 if (exact) stage(r, q);
-                ng = K == 1 ? F2{q, 0.0f} : f2_add(ng, q);
+                if constexpr (K == 1) ng.template set<false>(q);
+                else ng.template add<false>(q);
             }
         } else {
             for (uint32_t r = threadIdx.x; r < cells; r += threads) {
@@ -318,12 +385,12 @@ static __device__ __noinline__ void cg_warps(const CgArrays& arrays, CgShared& s
                 const float nr = A.cr[c] - alpha * A.cap[c];
                 A.cr[c] = nr;
                 more = more || fabsf(nr) >= 1e-6f;
-                ng = f2_add(ng, nr * nr);
+                ng.template add<false>(nr * nr);
             }
         }
         // the exit's test and the next r.r in one reduction (the latter is
         // dropped when the former ends the loop)
-        float new_gamma = cg_reduce<true>(ng, more, sh.slot[0], nwarps);
+        float new_gamma = cg_reduce<true, false>(ng, more, sh.slot[0], nwarps, eps, exact, rr64);
         if (!more) break;
         if (exact) new_gamma = K > 0 ? serial() : serial_cells(A.cr, A.cr);
         const float beta = new_gamma / gamma;
