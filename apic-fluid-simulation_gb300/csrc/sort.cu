@@ -175,6 +175,10 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const uint32_t* __re
     if (threadIdx.x == 0) s_tile = atomicAdd(head + 3072 + pass, 1u);
     __syncthreads();
     const uint32_t tile = s_tile, ntiles = gridDim.x;
+    // calls that overlap on one scratch (apic_morton_sort_noalloc on two streams)
+    // share its counters: a number past this launch's tiles has neither keys nor
+    // published counts in the scratch
+    if (tile >= ntiles) return;
     const uint32_t tile0 = tile * kTileKeys, base = tile0 + warp * (32u * kItems);
     uint32_t k[kItems], v[kItems], rk[kItems];
 #pragma unroll
