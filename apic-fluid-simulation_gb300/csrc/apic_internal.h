@@ -107,7 +107,6 @@ enum : uint32_t {
     kStatusBadStep = 2u,
     kStatusP2gLayout = 8u,  // a particle's staggered stencil left the bins P2G searches (never expected)
     kStatusBounds = 16u,    // checked build (APIC_BOUNDS_CHECK): an index left its buffer
-    kStatusSortWait = 32u,  // a bounded wait of the radix sort gave up (never expected)
 };
 
 struct Level {
@@ -317,8 +316,8 @@ void free_render(Scene& s);
 // sorted pairs stay where the last pass wrote them (*keys_out / *vals_out:
 // keys/vals or keys_alt/vals_alt).  iota >= 0: the values are the pair's index
 // >> iota (vals is only a buffer then).  scratch: sort_scratch_words, its head
-// zeroed (clear_sort_head).  status: where a bounded wait that gave up or an
-// index outside the buffers is recorded (may be null).
+// zeroed (clear_sort_head).  status: where an index outside the buffers is
+// recorded (may be null).
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t* scratch,
                              uint32_t n, int bits, int iota, cudaStream_t st, bool pdl, uint32_t** keys_out,
                              uint32_t** vals_out, uint32_t* status = nullptr);

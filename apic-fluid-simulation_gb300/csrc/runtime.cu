@@ -928,7 +928,6 @@ int update_finish(apic_handle* h) {
                                   uint64_t(c.pcg_bodies) * s.kn_pcg + uint64_t(c.refinements_total) * s.kn_refine;
     if (c.status & kStatusBounds)
         return fail(APIC_ERR_CUDA, "bounds check: an index left its buffer (build with APIC_BOUNDS_CHECK)");
-    if (c.status & kStatusSortWait) return fail(APIC_ERR_TIMEOUT, "radix sort: a bounded device wait gave up");
     if (c.status & kStatusP2gLayout)
         return fail(APIC_ERR_CUDA, "P2G: a particle's stencil left the cells its faces gather from (internal error)");
     if (c.status & kStatusBadStep) return fail(APIC_ERR_NONFINITE, "substep size is not positive (non-finite velocities)");

@@ -18,7 +18,8 @@
 // Adinets and Merrill, "Onesweep", 2022): a tile that knows its own place
 // publishes the running total, so later tiles stop there.  Tiles take their
 // numbers from a counter as they start, so a tile only waits for tiles that
-// are running or done; the wait is bounded all the same.  Only the bits below
+// are running or done; the wait is bounded all the same, and a tile whose wait
+// runs out counts the keys before it.  Only the bits below
 // the bit length of the largest possible key are sorted: higher bits are zero
 // for every key, so their passes would be identities.  The digit width is
 // chosen per sort for the fewest passes (20-bit keys of a 1024^2 grid: two
@@ -43,7 +44,12 @@ constexpr uint32_t kSortHead = kSortHeadWords;
 // A published count: the tile's own, with bit 31 the total up to and with it.
 constexpr uint32_t kNotReady = 0xFFFFFFFFu, kInclusive = 0x80000000u;
 constexpr int kLookback = 8;             // earlier tiles read at once
-constexpr uint32_t kSpinLimit = 1u << 22;  // rounds of reads before a wait gives up (seconds)
+// Rounds of reads before a tile stops waiting and counts the keys before it
+// itself (some 50 ms; a macro so that a test can let every wait run out).
+#ifndef APIC_SORT_SPIN_LIMIT
+#define APIC_SORT_SPIN_LIMIT (1u << 16)
+#endif
+constexpr uint32_t kSpinLimit = APIC_SORT_SPIN_LIMIT;
 
 // Four particles per thread with 16-byte loads and stores: the particle
 // arrays and the key buffers hold npad (a multiple of 8) lanes, so lanes
@@ -154,7 +160,7 @@ __device__ __forceinline__ void publish(uint32_t* p, uint32_t v) {
 // memory (dynamic): per-warp counts of each digit (16 bits), their tile-wide
 // start and global offset, the tile's pairs in sorted order.
 template <int kItems, int kPer>
-__global__ void __launch_bounds__(kSortThreads) k_sort_pass(const uint32_t* __restrict__ keys,
+__global__ void __launch_bounds__(kSortThreads, 2) k_sort_pass(const uint32_t* __restrict__ keys,
                                                             const uint32_t* __restrict__ vals, uint32_t n, int shift,
                                                             int dbits, int pass, int iota, uint32_t* __restrict__ head,
                                                             uint32_t* __restrict__ okeys, uint32_t* __restrict__ ovals,
@@ -333,11 +339,22 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const uint32_t* __re
 #pragma unroll
         for (int j = 0; j < kPer; ++j) goff[d0 + j] = global[j] - local[j];
     }
-    if (__syncthreads_or(lost)) {  // (never expected) leave the output alone
-        if (threadIdx.x == 0 && status) atomicOr(status, kStatusSortWait);
-        return;
-    }
     const uint32_t here = min(kTileKeys, n - tile0);
+    if (__syncthreads_or(lost)) {  // (never expected)
+        for (uint32_t i = threadIdx.x; i < nbk; i += kSortThreads) sm[i] = 0u;  // (the warps' counts are used up)
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < tile0; i += kSortThreads) atomicAdd(&sm[(keys[i] >> shift) & mask], 1u);
+        __syncthreads();
+        if (lost) {
+#pragma unroll
+            for (uint32_t j = 0; j < kPer; ++j) {
+                const uint32_t d = d0 + j, own = (d + 1u < nbk ? lstart[d + 1u] : here) - lstart[d];
+                publish(state + d, (sm[d] + own) | kInclusive);
+                goff[d] += sm[d];
+            }
+        }
+        __syncthreads();
+    }
     for (uint32_t q = threadIdx.x; q < here; q += kSortThreads) {
         const uint32_t key = sk[q], pos = goff[(key >> shift) & mask] + q;
         if (pos >= n) {  // (scratch overwritten by an overlapping call)
