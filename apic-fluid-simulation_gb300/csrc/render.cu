@@ -173,12 +173,6 @@ __global__ void __launch_bounds__(kTileThreads) k_splat_raster(const uint32_t* _
     __shared__ uint32_t list[kWarps][kWindow];            // quads that touch the warp's pixels
     __shared__ uint16_t cover[kWarps][kWindow];           // bit k: column k of the 8; bit 8 + k: row k of the 4
     __shared__ uint32_t masks[kWarps][kWindow / 32][32];  // per lane: which of them cover its pixel
-    for (int t = threadIdx.x; t < (kTex + 2) * (kTex + 2); t += kTileThreads) {
-        const int x = min(max(t % (kTex + 2) - 1, 0), kTex - 1), y = min(max(t / (kTex + 2) - 1, 0), kTex - 1);
-        tex[t] = float(circle_alpha(x, y)) / 255.0f;
-    }
-    d8[threadIdx.x] = float(threadIdx.x) / 255.0f;
-    __syncthreads();
     const uint32_t tile = blockIdx.x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t px0 = (tile % p.ntx) * kTile + (warp & 1u) * 8u, py0 = (tile / p.ntx) * kTile + (warp >> 1) * 4u;
@@ -187,6 +181,18 @@ __global__ void __launch_bounds__(kTileThreads) k_splat_raster(const uint32_t* _
     const float cx = float(px) + 0.5f, cy = float(py) + 0.5f;
     uint32_t dr = p.bg & 0xFFu, dg = (p.bg >> 8) & 0xFFu, db = (p.bg >> 16) & 0xFFu;
     const uint32_t b0 = start[tile], b1 = end[tile];
+    // most tiles of a large frame with few particles: no tables for them
+    // (3840 x 2160 without any 163 -> 47 us, with 20000 240 -> 165)
+    if (b0 == b1) {
+        if (px < p.width && py < p.height) frame[size_t(py) * p.width + px] = p.bg | (0xFFu << 24);
+        return;
+    }
+    for (int t = threadIdx.x; t < (kTex + 2) * (kTex + 2); t += kTileThreads) {
+        const int x = min(max(t % (kTex + 2) - 1, 0), kTex - 1), y = min(max(t / (kTex + 2) - 1, 0), kTex - 1);
+        tex[t] = float(circle_alpha(x, y)) / 255.0f;
+    }
+    d8[threadIdx.x] = float(threadIdx.x) / 255.0f;
+    __syncthreads();
     uint32_t n = 0;
     for (uint32_t base = b0; base < b1; base += 32u * kRasterGroups) {
         uint32_t id[kRasterGroups];
