@@ -1482,6 +1482,15 @@ int apic_restore(apic_handle* h, const void* src, uint64_t bytes) {
         if ((rc = upload_world(h))) return rc;
     }
     off += obst;
+    // pending forces are the snapshot's: what this handle has gathered goes
+    // (apic_add_radial_force adds to the fields)
+    auto drop = [&](bool pending, float* u, float* v) -> int {
+        if (!pending) return APIC_OK;
+        CK(cudaMemsetAsync(u, 0, uint64_t(s.uf) * 4, s.stream));
+        CK(cudaMemsetAsync(v, 0, uint64_t(s.vf) * 4, s.stream));
+        return APIC_OK;
+    };
+    if ((rc = drop(s.has_ext, s.ext_u, s.ext_v)) || (rc = drop(s.has_post, s.post_u, s.post_v))) return rc;
     s.has_ext = s.has_post = false;
     auto forces = [&](float* u, float* v) -> int {
         CK(cudaMemcpyAsync(u, in + off, uint64_t(s.uf) * 4, cudaMemcpyHostToDevice, s.stream));
