@@ -357,6 +357,7 @@ int upload_world(apic_handle* h) {
     Scene& s = h->s;
     std::vector<uint32_t> uo, vo;
     open_masks(s, h->obstacle_host, uo, vo);
+    s.masks_written = true;  // until the three copies are on their way
     // in order on the scene's stream (pageable sources are staged before each call returns)
     CK(cudaMemcpyAsync(s.obstacle, h->obstacle_host.data(), sizeof(uint32_t) * h->obstacle_host.size(),
                        cudaMemcpyHostToDevice, s.stream));
@@ -827,8 +828,10 @@ int apic_set_particles(apic_handle* h, uint32_t n, const float* px, const float*
     // recorded graphs hold the particle count and its buffers, which an equal
     // count leaves as they are
     if (n != h->s.n || h->s.part_cap == 0) invalidate_graphs(h->s);
-    int rc = load_particles(h, n, px, py, vx, vy);
-    if (rc == APIC_OK) CK(cudaStreamSynchronize(h->s.stream));
+    const int rc = load_particles(h, n, px, py, vx, vy);
+    // (after a failure too: copies in flight read the caller's arrays)
+    const cudaError_t e = cudaStreamSynchronize(h->s.stream);
+    if (rc == APIC_OK) CK(e);
     return rc;
 }
 
@@ -1468,52 +1471,58 @@ int apic_restore(apic_handle* h, const void* src, uint64_t bytes) {
     }
     if (s.npad != hd.lanes) return fail(APIC_ERR_INVALID_ARG, "snapshot lane count differs");
     CK(cudaStreamSynchronize(s.stream));
-    if (hd.lanes) {
-        for (int k = 0; k < NPF; ++k)
-            CK(cudaMemcpyAsync(s.part[k], f[k], uint64_t(hd.lanes) * 4, cudaMemcpyHostToDevice, s.stream));
-        if ((rc = reset_tables(s))) return rc;
-    }
-    uint64_t off = uint64_t(NPF) * hd.lanes * 4;
-    // the obstacles and the open-face masks that follow from them, where the
-    // snapshot's differ from the scene's or a caller wrote masks of its own
-    const uint64_t obst = uint64_t(hd.obstacle_words) * 8;
-    if (s.masks_written || std::memcmp(h->obstacle_host.data(), in + off, obst) != 0) {
-        std::memcpy(h->obstacle_host.data(), in + off, obst);
-        if ((rc = upload_world(h))) return rc;
-    }
-    off += obst;
-    // pending forces are the snapshot's: what this handle has gathered goes
-    // (apic_add_radial_force adds to the fields)
-    auto drop = [&](bool pending, float* u, float* v) -> int {
-        if (!pending) return APIC_OK;
-        CK(cudaMemsetAsync(u, 0, uint64_t(s.uf) * 4, s.stream));
-        CK(cudaMemsetAsync(v, 0, uint64_t(s.vf) * 4, s.stream));
-        return APIC_OK;
-    };
-    if ((rc = drop(s.has_ext, s.ext_u, s.ext_v)) || (rc = drop(s.has_post, s.post_u, s.post_v))) return rc;
-    s.has_ext = s.has_post = false;
-    auto forces = [&](float* u, float* v) -> int {
-        CK(cudaMemcpyAsync(u, in + off, uint64_t(s.uf) * 4, cudaMemcpyHostToDevice, s.stream));
-        CK(cudaMemcpyAsync(v, in + off + uint64_t(s.uf) * 4, uint64_t(s.vf) * 4, cudaMemcpyHostToDevice, s.stream));
-        off += uint64_t(s.uf + s.vf) * 4;
-        return APIC_OK;
-    };
-    if (hd.has_ext) {
-        if ((rc = forces(s.ext_u, s.ext_v))) return rc;
-        s.has_ext = true;
-    }
-    if (hd.has_post) {
-        if ((rc = forces(s.post_u, s.post_v))) return rc;
-        s.has_post = true;
-    }
-    // the pressure the next mixed solve starts from (zero where none was saved)
-    const uint64_t p64_bytes = sizeof(double) * (uint64_t(s.cells) + 2ull * s.W);
-    if (hd.p64_words) CK(cudaMemcpyAsync(s.p64, in + off, p64_bytes, cudaMemcpyHostToDevice, s.stream));
-    else CK(cudaMemsetAsync(s.p64, 0, p64_bytes, s.stream));
-    k_restore_clock<<<1, 1, 0, s.stream>>>(s.ctl, hd.timestamp, hd.prev_deltatime);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(s.stream));  // src is the caller's again
     s.vmax_valid = false;
+    auto load = [&]() -> int {
+        if (hd.lanes) {
+            for (int k = 0; k < NPF; ++k)
+                CK(cudaMemcpyAsync(s.part[k], f[k], uint64_t(hd.lanes) * 4, cudaMemcpyHostToDevice, s.stream));
+            if ((rc = reset_tables(s))) return rc;
+        }
+        uint64_t off = uint64_t(NPF) * hd.lanes * 4;
+        // the obstacles and the open-face masks that follow from them, where the
+        // snapshot's differ from the scene's or a caller wrote masks of its own
+        const uint64_t obst = uint64_t(hd.obstacle_words) * 8;
+        if (s.masks_written || std::memcmp(h->obstacle_host.data(), in + off, obst) != 0) {
+            std::memcpy(h->obstacle_host.data(), in + off, obst);
+            if ((rc = upload_world(h))) return rc;
+        }
+        off += obst;
+        // pending forces are the snapshot's: what this handle has gathered goes
+        // (apic_add_radial_force adds to the fields)
+        auto drop = [&](bool pending, float* u, float* v) -> int {
+            if (!pending) return APIC_OK;
+            CK(cudaMemsetAsync(u, 0, uint64_t(s.uf) * 4, s.stream));
+            CK(cudaMemsetAsync(v, 0, uint64_t(s.vf) * 4, s.stream));
+            return APIC_OK;
+        };
+        if ((rc = drop(s.has_ext, s.ext_u, s.ext_v)) || (rc = drop(s.has_post, s.post_u, s.post_v))) return rc;
+        s.has_ext = s.has_post = false;
+        auto forces = [&](float* u, float* v) -> int {
+            CK(cudaMemcpyAsync(u, in + off, uint64_t(s.uf) * 4, cudaMemcpyHostToDevice, s.stream));
+            CK(cudaMemcpyAsync(v, in + off + uint64_t(s.uf) * 4, uint64_t(s.vf) * 4, cudaMemcpyHostToDevice, s.stream));
+            off += uint64_t(s.uf + s.vf) * 4;
+            return APIC_OK;
+        };
+        if (hd.has_ext) {
+            if ((rc = forces(s.ext_u, s.ext_v))) return rc;
+            s.has_ext = true;
+        }
+        if (hd.has_post) {
+            if ((rc = forces(s.post_u, s.post_v))) return rc;
+            s.has_post = true;
+        }
+        // the pressure the next mixed solve starts from (zero where none was saved)
+        const uint64_t p64_bytes = sizeof(double) * (uint64_t(s.cells) + 2ull * s.W);
+        if (hd.p64_words) CK(cudaMemcpyAsync(s.p64, in + off, p64_bytes, cudaMemcpyHostToDevice, s.stream));
+        else CK(cudaMemsetAsync(s.p64, 0, p64_bytes, s.stream));
+        k_restore_clock<<<1, 1, 0, s.stream>>>(s.ctl, hd.timestamp, hd.prev_deltatime);
+        CK(cudaGetLastError());
+        return APIC_OK;
+    };
+    rc = load();
+    const cudaError_t e = cudaStreamSynchronize(s.stream);  // src is the caller's again, after a failure too
+    if (rc) return rc;
+    CK(e);
     return apic_set_solver(h, hd.solver_mode, hd.rel_tol, hd.max_iterations);
 }
 
